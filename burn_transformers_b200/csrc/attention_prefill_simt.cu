@@ -1,8 +1,15 @@
 // Causal attention for steps that bring several tokens per sequence, with plain 32-bit
 // arithmetic: scores, online softmax, and the value mix are all fused multiply-adds in 32-bit,
 // so this kernel serves the true 32-bit path (and any head size the tensor-core kernel refuses).
-// One warp owns a query; lanes own keys for the scores and channels for the value mix.
 // The S x S score plane is never stored.
+//
+// A block is 32 queries of one (sequence, head) and walks their keys in tiles of 64; a thread holds 4 queries x 4 keys of the
+// scores and 4 queries x 4 channels (of every 64) of the output, so that a 16-byte read of shared memory, which takes a warp
+// four cycles of the multiprocessor, feeds eight multiply-adds: these reads are what bounds it.  Keys, values and queries
+// lie in shared memory as rows (+ 4 numbers: eight consecutive rows meet all 32 banks once).  A tile's keys are asked for by
+// cp.async when the scores of the tile before it are done, its values when that tile's value mix is.  The version with a warp
+// a query and a lane a key (two reads for each multiply-add of the scores, a shuffle and two reads for each of the mix) took
+// 204 us for GPT-2 small's 12 heads at prompts of 37, 268 and 499 tokens; this one 75.
 //
 // Query t of sequence s sits at position past[s] + (t - seq_start[s]); key j is visible when
 // j <= position (causal) and j > position - window (window > 0).  A query that sees no key
@@ -11,17 +18,21 @@
 
 namespace bt {
 
-constexpr int PF_BQ = 16;      // queries per block
-constexpr int PF_BK = 32;      // keys per tile
-constexpr int PF_WARPS = 8;
-constexpr int PF_MAXI = 8;     // head_dim <= 256
+constexpr int PF_BQ = 32;      // queries per block
+constexpr int PF_BK = 64;      // keys per tile
+constexpr int PF_THREADS = 128;
+constexpr int PF_MAXG = 4;     // groups of 64 channels: head_dim <= 256
 
-template <typename T>
-__global__ void __launch_bounds__(PF_WARPS * 32)
+// numbers between rows of queries, keys and values in shared memory
+__host__ __device__ __forceinline__ int pf_stride(int head_dim) { return (head_dim + 3) / 4 * 4 + 4; }
+
+// G: groups of 64 channels that hold a head.  VEC: 32-bit rows whose heads start on 16-byte boundaries.
+template <typename T, int G, bool VEC>
+__global__ void __launch_bounds__(PF_THREADS)
 attention_prefill_simt_kernel(const T* __restrict__ q, long long q_row_stride, KvView kv, T* __restrict__ out,
                               const int* __restrict__ seq_start, const int* __restrict__ past_len, int n_heads,
                               int n_kv_heads, int head_dim, float scale, int causal, int window) {
-  extern __shared__ float smem[];
+  extern __shared__ __align__(16) float smem[];
   const int seq = blockIdx.y, head = blockIdx.z;
   const int t0 = seq_start[seq], n_new = seq_start[seq + 1] - t0;
   // longest tiles first: they see the most keys
@@ -32,14 +43,18 @@ attention_prefill_simt_kernel(const T* __restrict__ q, long long q_row_stride, K
   const int kv_len = past + n_new;
   const int kv_head = head / (n_heads / n_kv_heads);
   const int nq = min(PF_BQ, n_new - q0);
-  float* Qs = smem;                                // [PF_BQ][head_dim]
-  float* Ks = Qs + PF_BQ * head_dim;               // [PF_BK][head_dim + 1]
-  float* Vs = Ks + PF_BK * (head_dim + 1);         // [PF_BK][head_dim]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int S = pf_stride(head_dim), wide = S - 4;    // (channels past the head's are zeros)
+  float* Qs = smem;                        // [PF_BQ][S]
+  float* Ks = Qs + PF_BQ * S;              // [PF_BK][S]
+  float* Vs = Ks + PF_BK * S;              // [PF_BK][S]
+  float* Ps = Vs + PF_BK * S;              // [PF_BQ][PF_BK + 4]
+  constexpr int PS = PF_BK + 4;
+  const int tid = threadIdx.x;
+  const int tx = tid & 15, ty = tid >> 4;  // keys tx, tx + 16, ... and channels 4 tx .. (of every 64); queries 4 ty ..
 
-  for (int i = tid; i < PF_BQ * head_dim; i += blockDim.x) {
-    const int r = i / head_dim, c = i - r * head_dim;
-    Qs[i] = r < nq ? to_float(q[(long long)(t0 + q0 + r) * q_row_stride + head * head_dim + c]) * scale : 0.f;
+  for (int i = tid; i < PF_BQ * wide; i += PF_THREADS) {
+    const int r = i / wide, c = i - r * wide;
+    Qs[r * S + c] = r < nq && c < head_dim ? to_float(q[(long long)(t0 + q0 + r) * q_row_stride + head * head_dim + c]) * scale : 0.f;
   }
   // key range this block can see
   const int pos_first = past + q0, pos_last = past + q0 + nq - 1;
@@ -47,80 +62,170 @@ attention_prefill_simt_kernel(const T* __restrict__ q, long long q_row_stride, K
   int k_lo = window > 0 ? max(0, pos_first - window + 1) : 0;
   const int tile_lo = k_lo / PF_BK, tile_hi = (k_hi + PF_BK - 1) / PF_BK;
 
-  float m[2], l[2], acc[2][PF_MAXI];
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    m[u] = -INFINITY;
-    l[u] = 0.f;
-#pragma unroll
-    for (int i = 0; i < PF_MAXI; ++i) acc[u][i] = 0.f;
-  }
-
-  for (int tile = tile_lo; tile < tile_hi; ++tile) {
-    __syncthreads();
-    {  // stage the tile: 8 threads per key row
-      const int r = tid >> 3, part = tid & 7;
-      const int kp = tile * PF_BK + r;
-      if (kp < kv_len) {
-        const T* kr = kv_row<T>(kv.k, kv, seq, kv_head, n_kv_heads, head_dim, kp);
-        const T* vr = kv_row<T>(kv.v, kv, seq, kv_head, n_kv_heads, head_dim, kp);
-        for (int c = part; c < head_dim; c += 8) {
-          Ks[r * (head_dim + 1) + c] = to_float(kr[c]);
-          Vs[r * head_dim + c] = to_float(vr[c]);
+  // a tile's rows of keys or values; rows past the sequence's end are zeros
+  auto stage = [&](int tile, const void* base, float* dst) {
+    if (tile < tile_hi) {
+      if constexpr (VEC) {
+        const int pieces = head_dim / 4;
+        for (int i = tid; i < PF_BK * pieces; i += PF_THREADS) {
+          const int r = i / pieces, c = (i - r * pieces) * 4, kp = tile * PF_BK + r;
+          const bool in = kp < kv_len;
+          const T* src = kv_row<T>(base, kv, seq, kv_head, n_kv_heads, head_dim, in ? kp : kv_len - 1) + c;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst + r * S + c)),
+                       "l"(src), "r"(in ? 16 : 0) : "memory");
         }
       } else {
-        for (int c = part; c < head_dim; c += 8) {
-          Ks[r * (head_dim + 1) + c] = 0.f;
-          Vs[r * head_dim + c] = 0.f;
+        for (int i = tid; i < PF_BK * wide; i += PF_THREADS) {
+          const int r = i / wide, c = i - r * wide, kp = tile * PF_BK + r;
+          dst[r * S + c] = kp < kv_len && c < head_dim
+                               ? to_float(kv_row<T>(base, kv, seq, kv_head, n_kv_heads, head_dim, kp)[c]) : 0.f;
         }
       }
     }
-    __syncthreads();
-    const int kp = tile * PF_BK + lane;
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+
+  float m[4], l[4], acc[4][4 * G];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int qi = warp + u * PF_WARPS;
-      if (qi >= nq) continue;  // uniform per warp
-      const int qpos = past + q0 + qi;
-      bool visible = kp < kv_len;
-      if (causal) visible = visible && kp <= qpos;
-      if (window > 0) visible = visible && kp > qpos - window;
-      float s = 0.f;
-      const float* qv = Qs + qi * head_dim;
-      const float* kvp = Ks + lane * (head_dim + 1);
-      for (int c = 0; c < head_dim; ++c) s = fmaf(qv[c], kvp[c], s);
-      s = visible ? s : -INFINITY;
-      const float m_new = fmaxf(m[u], warp_max(s));
-      if (m_new == -INFINITY) continue;  // nothing visible yet (uniform per warp)
-      const float p = visible ? expf(s - m_new) : 0.f;
-      const float corr = expf(m[u] - m_new);  // m = -inf gives 0
-      l[u] = l[u] * corr + warp_sum(p);
-      m[u] = m_new;
+  for (int i = 0; i < 4; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.f;
 #pragma unroll
-      for (int i = 0; i < PF_MAXI; ++i) acc[u][i] *= corr;
-      for (int j = 0; j < PF_BK; ++j) {
-        const float pj = __shfl_sync(0xffffffffu, p, j);
-        const float* vrow = Vs + j * head_dim;
-#pragma unroll
-        for (int i = 0; i < PF_MAXI; ++i) {
-          const int c = lane + 32 * i;
-          if (c < head_dim) acc[u][i] = fmaf(pj, vrow[c], acc[u][i]);
-        }
-      }
-    }
+    for (int c = 0; c < 4 * G; ++c) acc[i][c] = 0.f;
   }
+
+  stage(tile_lo, kv.k, Ks);
+  stage(tile_lo, kv.v, Vs);
+  for (int tile = tile_lo; tile < tile_hi; ++tile) {
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");      // the keys (the values may still be on their way)
+    __syncthreads();
+    float s[4][4];
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int qi = warp + u * PF_WARPS;
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+#pragma unroll 4
+    for (int c = 0; c < wide; c += 4) {
+      float4 a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(Qs + (4 * ty + i) * S + c);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(Ks + (tx + 16 * j) * S + c);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s[i][j] = fmaf(a[i].x, b[j].x, s[i][j]);
+          s[i][j] = fmaf(a[i].y, b[j].y, s[i][j]);
+          s[i][j] = fmaf(a[i].z, b[j].z, s[i][j]);
+          s[i][j] = fmaf(a[i].w, b[j].w, s[i][j]);
+        }
+    }
+    __syncthreads();                        // everyone has read the keys
+    stage(tile + 1, kv.k, Ks);
+    // online softmax: a query's sixteen lanes agree on its maximum and sum
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int qpos = past + q0 + 4 * ty + i;
+      bool seen[4];
+      float top = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int kp = tile * PF_BK + tx + 16 * j;
+        seen[j] = kp < kv_len && (!causal || kp <= qpos) && (window <= 0 || kp > qpos - window);
+        if (seen[j]) top = fmaxf(top, s[i][j]);
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+      const float m_new = fmaxf(m[i], top);
+      const float m_use = m_new == -INFINITY ? 0.f : m_new;
+      const float corr = expf(m[i] - m_use);          // m = -inf gives 0
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float p = seen[j] ? expf(s[i][j] - m_use) : 0.f;
+        Ps[(4 * ty + i) * PS + tx + 16 * j] = p;
+        sum += p;
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      l[i] = l[i] * corr + sum;
+      m[i] = m_new;
+#pragma unroll
+      for (int c = 0; c < 4 * G; ++c) acc[i][c] *= corr;
+    }
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");      // the values (the next keys may still be on their way)
+    __syncthreads();                        // (and the weights, which a warp alone reads and writes)
+#pragma unroll 2
+    for (int k = 0; k < PF_BK; k += 4) {
+      float4 p[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(Ps + (4 * ty + i) * PS + k);
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        const int c = 64 * g + 4 * tx;
+        if (c >= wide) continue;
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const float4*>(Vs + (k + u) * S + c);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float w[4] = {p[i].x, p[i].y, p[i].z, p[i].w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            acc[i][4 * g] = fmaf(w[u], v[u].x, acc[i][4 * g]);
+            acc[i][4 * g + 1] = fmaf(w[u], v[u].y, acc[i][4 * g + 1]);
+            acc[i][4 * g + 2] = fmaf(w[u], v[u].z, acc[i][4 * g + 2]);
+            acc[i][4 * g + 3] = fmaf(w[u], v[u].w, acc[i][4 * g + 3]);
+          }
+        }
+      }
+    }
+    __syncthreads();                        // everyone has read the values
+    stage(tile + 1, kv.v, Vs);
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int qi = 4 * ty + i;
     if (qi >= nq) continue;
-    const float inv = l[u] > 0.f ? 1.f / l[u] : 0.f;
+    const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
     T* dst = out + (long long)(t0 + q0 + qi) * ((long long)n_heads * head_dim) + head * head_dim;
 #pragma unroll
-    for (int i = 0; i < PF_MAXI; ++i) {
-      const int c = lane + 32 * i;
-      if (c < head_dim) dst[c] = from_float<T>(acc[u][i] * inv);
-    }
+    for (int g = 0; g < G; ++g)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int c = 64 * g + 4 * tx + u;
+        if (c < head_dim) dst[c] = from_float<T>(acc[i][4 * g + u] * inv);
+      }
   }
+}
+
+template <typename T, int G, bool VEC>
+static int launch_pf(const void* q, long long q_row_stride, const KvView& view, void* out, const int* seq_start, const int* past_len,
+                     int n_seqs, int max_new, int n_heads, int n_kv_heads, int head_dim, float scale, int causal, int window,
+                     cudaStream_t stream) {
+  auto kern = attention_prefill_simt_kernel<T, G, VEC>;
+  constexpr size_t most = sizeof(float) * ((size_t)(PF_BQ + 2 * PF_BK) * (64 * G + 4) + (size_t)PF_BQ * (PF_BK + 4));
+  const size_t smem = sizeof(float) * ((size_t)(PF_BQ + 2 * PF_BK) * pf_stride(head_dim) + (size_t)PF_BQ * (PF_BK + 4));
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    BT_CHECK(e == cudaSuccess, "attention_prefill_simt: cannot reserve %zu bytes of shared memory", most);
+    configured = true;
+  }
+  const dim3 grid((max_new + PF_BQ - 1) / PF_BQ, n_seqs, n_heads);
+  kern<<<grid, PF_THREADS, smem, stream>>>((const T*)q, q_row_stride, view, (T*)out, seq_start, past_len, n_heads, n_kv_heads,
+                                           head_dim, scale, causal, window);
+  return 0;
+}
+
+template <typename T, bool VEC, typename... Args>
+static int launch_pf_sized(int head_dim, Args... args) {
+  if (head_dim <= 64) return launch_pf<T, 1, VEC>(args...);
+  if (head_dim <= 128) return launch_pf<T, 2, VEC>(args...);
+  if (head_dim <= 192) return launch_pf<T, 3, VEC>(args...);
+  return launch_pf<T, 4, VEC>(args...);
 }
 
 }  // namespace bt
@@ -134,32 +239,31 @@ extern "C" int bt_attention_prefill_simt(const void* q, long long q_row_stride, 
                                          int head_dim, float scale, int causal, int window, int dtype,
                                          cudaStream_t stream) {
   using namespace bt;
-  BT_CHECK(head_dim > 0 && head_dim <= 32 * PF_MAXI,
-           "attention_prefill_simt: head_dim %d must be at least 1 and at most %d", head_dim, 32 * PF_MAXI);
+  BT_CHECK(head_dim > 0 && head_dim <= 64 * PF_MAXG,
+           "attention_prefill_simt: head_dim %d must be at least 1 and at most %d", head_dim, 64 * PF_MAXG);
   BT_CHECK(n_heads > 0 && n_kv_heads > 0 && n_heads % n_kv_heads == 0,
            "attention_prefill_simt: %d query heads cannot share %d key heads", n_heads, n_kv_heads);
   BT_CHECK(n_seqs <= 65535 && n_heads <= 65535, "attention_prefill_simt: too many sequences or heads for one launch");
   if (n_seqs == 0 || max_new == 0) return 0;
   KvView view{k, v, kv_table, table_stride, table_len > 0 ? table_len : 1, page_size > 0 ? page_size : 1,
               kv_row_stride, seq_start};
-  dim3 grid((max_new + PF_BQ - 1) / PF_BQ, n_seqs, n_heads);
-  const size_t smem = sizeof(float) * ((size_t)PF_BQ * head_dim + (size_t)PF_BK * (head_dim + 1) + (size_t)PF_BK * head_dim);
-  cudaError_t e;
-  if (dtype == kF32) {
-    auto kern = attention_prefill_simt_kernel<float>;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    BT_CHECK(e == cudaSuccess, "attention_prefill_simt: cannot reserve %zu bytes of shared memory", smem);
-    kern<<<grid, PF_WARPS * 32, smem, stream>>>((const float*)q, q_row_stride, view, (float*)out, seq_start, past_len,
-                                                n_heads, n_kv_heads, head_dim, scale, causal, window);
+  // 16-byte copies need every head of every row on a 16-byte boundary
+  const bool vec = dtype == kF32 && head_dim % 4 == 0 && ((unsigned long long)k | (unsigned long long)v) % 16 == 0 &&
+                   (kv_table != nullptr || kv_row_stride % 4 == 0);
+  int rc;
+  if (dtype == kF32 && vec) {
+    rc = launch_pf_sized<float, true>(head_dim, q, q_row_stride, view, out, seq_start, past_len, n_seqs, max_new, n_heads, n_kv_heads,
+                                      head_dim, scale, causal, window, stream);
+  } else if (dtype == kF32) {
+    rc = launch_pf_sized<float, false>(head_dim, q, q_row_stride, view, out, seq_start, past_len, n_seqs, max_new, n_heads, n_kv_heads,
+                                       head_dim, scale, causal, window, stream);
   } else if (dtype == kBF16) {
-    auto kern = attention_prefill_simt_kernel<__nv_bfloat16>;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    BT_CHECK(e == cudaSuccess, "attention_prefill_simt: cannot reserve %zu bytes of shared memory", smem);
-    kern<<<grid, PF_WARPS * 32, smem, stream>>>((const __nv_bfloat16*)q, q_row_stride, view, (__nv_bfloat16*)out,
-                                                seq_start, past_len, n_heads, n_kv_heads, head_dim, scale, causal, window);
+    rc = launch_pf_sized<__nv_bfloat16, false>(head_dim, q, q_row_stride, view, out, seq_start, past_len, n_seqs, max_new, n_heads,
+                                               n_kv_heads, head_dim, scale, causal, window, stream);
   } else {
     return fail("attention_prefill_simt: unknown dtype %d", dtype);
   }
+  if (rc != 0) return rc;
   BT_LAUNCH_OK("attention_prefill_simt");
   return 0;
 }
