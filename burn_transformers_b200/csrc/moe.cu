@@ -18,8 +18,8 @@
 //                pair adds weight * input[t].
 //
 // The products exist as 32-bit multiply-adds (float32, and every shape), on tensor cores (bfloat16, mma.sync m16n8k16
-// with 32-bit accumulators, K a multiple of 8) and, for steps with few rows an expert, as a kernel that streams every
-// expert's weights once (bfloat16).  A row's result never depends on its neighbours in the tile.
+// with 32-bit accumulators, K a multiple of 8) and, for steps with few rows an expert, as a kernel that streams the weights
+// into registers (bfloat16).  A row's result never depends on its neighbours in the tile.
 #include "common.cuh"
 
 namespace bt {
@@ -469,79 +469,96 @@ moe_expert_mma_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* 
 }
 
 // ---- the products for few rows an expert (decode steps, bfloat16) ---------------------------------------------------
-// A block: one expert and 8 output columns (each of 4 warps two columns; for the first product the gate's and up's rows
-// of a column together).  The expert's rows, 8 at a time, lie in shared memory; a warp streams its columns' weight
-// rows once per 8 rows, a lane 16-byte pieces of K, sums in 32-bit, and the lanes' sums meet by shuffles.  Every weight
-// byte is read by one warp; a block whose expert got no row ends at once.
-constexpr int MF_ROWS = 8, MF_COLS = 8, MF_KC = 2048;
+// What bounds them is how many bytes of weights are asked for at once, so nothing is staged: a block takes a row tile (32
+// rows of one expert) and 32 rows of its weights (16 columns with both halves of the pair, or 32 columns), its eight warps
+// share K in pieces of 32, and a lane loads 16 bytes of a weight row (and of its tile rows) straight into the registers that
+// mma.sync m16n8k16 reads.  The fragments want a lane's numbers two by two, 8 apart; which k a place of the fragment
+// stands for is free as long as both operands agree, so the eight consecutive k of a lane's piece are its places of two
+// products.  The warps' sums meet in shared memory and are added in warp order.
+// The version before (an expert and 8 columns a block, 32-bit multiply-adds, every weight streamed once per 8 rows) took 135
+// us for the two products of 16 experts of 512 x 1,024 at 64 tokens of 4 choices (in a recorded layer, from the pairs'
+// sorting to the sum); this one 40.
+constexpr int MF_WARPS = 8, MF_ROWS = MS_BM, MF_W = 32, MF_KP = 32;
 
 template <int MODE>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(MF_WARPS * 32)
 moe_expert_few_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ w, void* __restrict__ out,
                       MoeArgs p) {
   constexpr bool IN = MODE != kMoeOut, PAIR = MODE == kMoeInPair;
-  __shared__ __align__(16) __nv_bfloat16 x_s[MF_ROWS][MF_KC];
+  constexpr int COLS = PAIR ? MF_W / 2 : MF_W;             // output columns of a block
+  __shared__ float sums[MF_WARPS][MF_ROWS][MF_W + 2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
   pdl_trigger();
   pdl_wait();
-  const int expert = blockIdx.y;
-  const int first = p.offsets[expert], count = p.offsets[expert + 1] - first;
-  if (count == 0) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * MF_COLS + warp * 2;
-  const __nv_bfloat16* w_e = w + (long long)expert * (PAIR ? 2 : 1) * p.N * p.K;
-  for (int r0 = 0; r0 < count; r0 += MF_ROWS) {
-    const int rows = min(MF_ROWS, count - r0);
-    float acc[PAIR ? 2 : 1][2][MF_ROWS] = {};
-    for (int k0 = 0; k0 < p.K; k0 += MF_KC) {
-      const int kc = min(MF_KC, p.K - k0);
-      __syncthreads();
-      for (int i = threadIdx.x; i < MF_ROWS * (kc / 8); i += 128) {
-        const int r = i / (kc / 8), c = (i - r * (kc / 8)) * 8;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (r < rows) {
-          const long long src = IN ? p.order[first + r0 + r] / p.top : first + r0 + r;
-          v = *reinterpret_cast<const uint4*>(a + src * p.a_row_stride + k0 + c);
-        }
-        *reinterpret_cast<uint4*>(&x_s[r][c]) = v;
-      }
-      __syncthreads();
+  int expert, row0, rows;
+  if (!moe_tile(p.offsets, p.tile_first, p.E, blockIdx.y, MF_ROWS, expert, row0, rows)) return;
+  const int n0 = blockIdx.x * COLS;
+  // this lane's weight rows (one of each group of eight) and tile rows (gid and gid + 8 of each sixteen); null: zeros
+  const __nv_bfloat16* w_row[MF_W / 8];
 #pragma unroll
-      for (int col = 0; col < 2; ++col) {
-        const int n = n0 + col;
-        if (n >= p.N) continue;
-        for (int k = lane * 8; k < kc; k += 256) {
-          float wv[PAIR ? 2 : 1][8];
-          load_piece(w_e + (long long)n * p.K + k0 + k, wv[0]);
-          if (PAIR) load_piece(w_e + (long long)(p.N + n) * p.K + k0 + k, wv[PAIR ? 1 : 0]);
+  for (int j = 0; j < MF_W / 8; ++j) {
+    const int c = j * 8 + gid, n = n0 + c % COLS;           // PAIR: the gate's 16 columns, then the up's
+    w_row[j] = n < p.N ? w + ((long long)expert * (PAIR ? 2 : 1) * p.N + (long long)(c / COLS) * p.N + n) * p.K : nullptr;
+  }
+  const __nv_bfloat16* a_row[4];
 #pragma unroll
-          for (int r = 0; r < MF_ROWS; ++r) {
-            float xv[8];
-            load_piece(&x_s[r][k], xv);
+  for (int i = 0; i < 4; ++i) {
+    const int r = i * 8 + gid;
+    a_row[i] = r < rows ? a + (long long)(IN ? p.order[row0 + r] / p.top : row0 + r) * p.a_row_stride : nullptr;
+  }
+  const bool two = rows > 16;                               // (uniform: the second sixteen rows hold something)
+  float acc[2][MF_W / 8][4] = {};
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  constexpr int AHEAD = 2;                                  // pieces a warp asks for at once
+  for (int k0 = warp * MF_KP; k0 < p.K; k0 += AHEAD * MF_WARPS * MF_KP) {
+    uint4 wv[AHEAD][MF_W / 8], av[AHEAD][4];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              acc[0][col][r] = fmaf(xv[u], wv[0][u], acc[0][col][r]);
-              if (PAIR) acc[PAIR ? 1 : 0][col][r] = fmaf(xv[u], wv[PAIR ? 1 : 0][u], acc[PAIR ? 1 : 0][col][r]);
-            }
-          }
-        }
-      }
+    for (int u = 0; u < AHEAD; ++u) {
+      const int k = k0 + u * MF_WARPS * MF_KP + tig * 8;
+      const bool in = k < p.K;                              // (K is a multiple of 8)
+#pragma unroll
+      for (int j = 0; j < MF_W / 8; ++j) wv[u][j] = in && w_row[j] ? __ldg(reinterpret_cast<const uint4*>(w_row[j] + k)) : zero;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) av[u][i] = in && a_row[i] ? *reinterpret_cast<const uint4*>(a_row[i] + k) : zero;
     }
 #pragma unroll
-    for (int col = 0; col < 2; ++col)
+    for (int u = 0; u < AHEAD; ++u)
 #pragma unroll
-      for (int r = 0; r < MF_ROWS; ++r) {
-        const float g = warp_sum(acc[0][col][r]);
-        const float u = PAIR ? warp_sum(acc[PAIR ? 1 : 0][col][r]) : 0.f;
-        const int n = n0 + col;
-        if (lane == 0 && r < rows && n < p.N) {
-          const long long row = first + r0 + r;
-          if (IN)
-            reinterpret_cast<__nv_bfloat16*>(out)[row * p.N + n] =
-                __float2bfloat16_rn(PAIR ? gated_pair(g, u, p.act, p.limit) : apply_activation(g, p.act));
-          else
-            reinterpret_cast<float*>(out)[row * p.N + n] = g * p.pair_weight[p.order[row]];
+      for (int m = 0; m < 2; ++m) {
+        if (m == 1 && !two) continue;
+        const uint4 lo = av[u][2 * m], hi = av[u][2 * m + 1];
+        const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
+#pragma unroll
+        for (int j = 0; j < MF_W / 8; ++j) {
+          const uint32_t b0[2] = {wv[u][j].x, wv[u][j].y}, b1[2] = {wv[u][j].z, wv[u][j].w};
+          mma_bf16_16816(acc[m][j], a0, b0);
+          mma_bf16_16816(acc[m][j], a1, b1);
         }
       }
+  }
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int j = 0; j < MF_W / 8; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<float2*>(&sums[warp][m * 16 + gid + 8 * h][j * 8 + tig * 2]) = make_float2(acc[m][j][2 * h], acc[m][j][2 * h + 1]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < rows * COLS; i += MF_WARPS * 32) {
+    const int r = i / COLS, c = i - r * COLS, n = n0 + c;
+    if (n >= p.N) continue;
+    float g = 0.f, u = 0.f;
+#pragma unroll
+    for (int v = 0; v < MF_WARPS; ++v) {
+      g += sums[v][r][c];
+      if (PAIR) u += sums[v][r][COLS + (PAIR ? c : 0)];
+    }
+    const long long row = row0 + r;
+    if (IN)
+      reinterpret_cast<__nv_bfloat16*>(out)[row * p.N + n] =
+          __float2bfloat16_rn(PAIR ? gated_pair(g, u, p.act, p.limit) : apply_activation(g, p.act));
+    else
+      reinterpret_cast<float*>(out)[row * p.N + n] = g * p.pair_weight[p.order[row]];
   }
 }
 
@@ -638,17 +655,21 @@ extern "C" int bt_moe_expert(int first, const void* a, long long a_row_stride, c
   const dim3 grid((N + MS_BN - 1) / MS_BN, tiles);
   const bool pieces = dtype == kBF16 && K % 8 == 0 && a_row_stride % 8 == 0 && (unsigned long long)a % 16 == 0 &&
                       (unsigned long long)w % 16 == 0;
-  if (pieces && tensor_cores && pairs <= 16 * E && E <= 65535) {
-    // few rows an expert (a decode step): every expert's weights streamed once per 8 of its rows
-    const dim3 few((N + MF_COLS - 1) / MF_COLS, E);
+  // few rows an expert (a decode step, a short prompt): up to 48 on average the kernel that streams its weights into
+  // registers is ahead of the one that stages both operands.  Measured for 16 experts of 512 x 1,024, the two products (us):
+  // 32 rows an expert 22 + 16 against 26 + 14, 50 rows 29 + 20 against 35 + 17, 75 rows 37 + 27 against 34 + 25; for 384 x
+  // 768 at 32 rows 15 + 13 against 18 + 13, 50 rows 22 + 15 against 21 + 13.
+  if (pieces && tensor_cores && pairs <= 48ll * E) {
+    const int cols = first == kMoeInPair ? MF_W / 2 : MF_W;
+    const dim3 few((N + cols - 1) / cols, tiles);
     if (first == kMoeInPair)
-      BT_PDL_OK("moe_expert", launch_pdl(moe_expert_few_kernel<kMoeInPair>, few, dim3(128), 0, stream, 1,
+      BT_PDL_OK("moe_expert", launch_pdl(moe_expert_few_kernel<kMoeInPair>, few, dim3(MF_WARPS * 32), 0, stream, 1,
                                          (const __nv_bfloat16*)a, (const __nv_bfloat16*)w, out, p));
     else if (first == kMoeInPlain)
-      BT_PDL_OK("moe_expert", launch_pdl(moe_expert_few_kernel<kMoeInPlain>, few, dim3(128), 0, stream, 1,
+      BT_PDL_OK("moe_expert", launch_pdl(moe_expert_few_kernel<kMoeInPlain>, few, dim3(MF_WARPS * 32), 0, stream, 1,
                                          (const __nv_bfloat16*)a, (const __nv_bfloat16*)w, out, p));
     else
-      BT_PDL_OK("moe_expert", launch_pdl(moe_expert_few_kernel<kMoeOut>, few, dim3(128), 0, stream, 1,
+      BT_PDL_OK("moe_expert", launch_pdl(moe_expert_few_kernel<kMoeOut>, few, dim3(MF_WARPS * 32), 0, stream, 1,
                                          (const __nv_bfloat16*)a, (const __nv_bfloat16*)w, out, p));
     return 0;
   }
