@@ -1,8 +1,11 @@
 // Attention over a latent cache on tensor cores (bfloat16): the same computation as latent_attention_kernel in
 // latent_attention.cu, with the scores and the value mix as mma.sync products.
 //
-// A block holds 64 rows, (token, head) pairs of one sequence, which all read the same key tiles of 32 cached rows.
-// Warps form 4 row groups of 16 rows; VW warps share a row group.  Per tile a warp computes the scores of its rows
+// A block holds 16 RG rows, (token, head) pairs of one sequence, which all read the same key tiles of 32 cached rows.
+// Warps form RG row groups of 16 rows; VW warps share a row group.  RG is 4, or 1 when a sequence brings no more than 16
+// rows (one token of up to 16 heads): with three of four row groups idle and 150 KB of shared memory a block (rank 512 + 64),
+// one such block a multiprocessor left most of the memory's latency uncovered; small blocks run two a multiprocessor.  64
+// sequences at context 250 to 510, 16 heads: 38 us before (five runs of keys a sequence), 25 now (four).  Per tile a warp computes the scores of its rows
 // against its 32 / VW keys over all rank + rot channels; the warps of a group exchange row maxima and sums through shared
 // memory and leave their weights there as bfloat16; then every warp multiplies the group's 16 x 32 weights with ITS
 // rank / VW channels of the tile's rows (values are the first `rank` channels of the key rows).  So no score is
@@ -13,7 +16,7 @@
 
 namespace bt {
 
-constexpr int LM_BM = 64;
+constexpr int LM_BM = 64;                 // rows of the larger block
 constexpr int LM_KT = 32;
 constexpr int LM_PAD = 8;                 // elements: rows of shared memory lie an odd number of 16-byte pieces apart
 constexpr int LM_PLD = LM_KT + LM_PAD;    // row length of the weights' tile
@@ -27,9 +30,9 @@ __device__ __forceinline__ void lm_cp_async16(unsigned dst, const void* src, int
 __device__ __forceinline__ void lm_cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void lm_cp_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// VW: warps per row group; VCT: the most value channels a warp owns (its accumulator's size)
-template <int VW, int VCT>
-__global__ void __launch_bounds__(128 * VW)
+// RG: row groups; VW: warps per row group; VCT: the most value channels a warp owns (its accumulator's size)
+template <int RG, int VW, int VCT>
+__global__ void __launch_bounds__(32 * RG * VW)
 latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long long q_row_stride,
                             const __nv_bfloat16* __restrict__ pool, const int* __restrict__ table, int table_stride,
                             int table_len, int page_size, const int* __restrict__ seq_start,
@@ -43,11 +46,11 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long long q_row
   constexpr float LOG2E = 1.4426950408889634f;
   const int dk = rank + rot, dkp = (dk + 15) & ~15, ld = dkp + LM_PAD;
   const int vc = rank / VW;                 // value channels per warp
-  __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(lm_smem);   // [64][ld]
-  __nv_bfloat16* k_s = q_s + LM_BM * ld;                            // [2][32][ld]
-  __nv_bfloat16* p_s = k_s + 2 * LM_KT * ld;                        // [4][16][LM_PLD]
-  float* red_max = reinterpret_cast<float*>(p_s + 4 * 16 * LM_PLD); // [4][VW][16]
-  float* red_sum = red_max + 4 * VW * 16;                           // [4][VW][16]
+  __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(lm_smem);   // [16 RG][ld]
+  __nv_bfloat16* k_s = q_s + 16 * RG * ld;                          // [2][32][ld]
+  __nv_bfloat16* p_s = k_s + 2 * LM_KT * ld;                        // [RG][16][LM_PLD]
+  float* red_max = reinterpret_cast<float*>(p_s + RG * 16 * LM_PLD);  // [RG][VW][16]
+  float* red_sum = red_max + RG * VW * 16;                          // [RG][VW][16]
   pdl_trigger();
   pdl_wait();
   const int seq = blockIdx.z, split = blockIdx.y;
@@ -64,7 +67,7 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long long q_row
   const bool active = rg * 16 < n_valid;
   const int chunks = dkp / 8;               // 16-byte pieces per row
   // the block's queries; rows past the valid ones and channels past rank + rot are zeros
-  for (int i = tid; i < LM_BM * chunks; i += blockDim.x) {
+  for (int i = tid; i < 16 * RG * chunks; i += blockDim.x) {
     const int r = i / chunks, c = i - r * chunks;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (r < n_valid && c * 8 < dk) {
@@ -103,21 +106,33 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long long q_row
   const int per = (n_tiles - tile_first + n_splits - 1) / n_splits;
   const int tile_lo = tile_first + split * per, tile_hi = min(n_tiles, tile_lo + per);
   const int row_chunks = dk / 8;
+  // a thread's pieces of a tile: from (row0, piece0) on, (step_row, step_piece) further each time (no division a piece)
+  constexpr int THREADS = 32 * RG * VW;
+  const int row0 = tid / row_chunks, piece0 = tid - row0 * row_chunks;
+  const int step_row = THREADS / row_chunks, step_piece = THREADS - step_row * row_chunks;
   auto load_tile = [&](int tile, int buf) {
+    // (the library's pages hold whole tiles: a tile's rows lie side by side)
     const int j0 = tile * LM_KT;
+    auto row_at = [&](int j) {
+      const int lp = j / page_size;
+      const int page = table[(long long)seq * table_stride + (lp % table_len)];
+      return pool + ((long long)page * page_size + (j - lp * page_size)) * dk;
+    };
+    const bool whole = page_size % LM_KT == 0;
+    const __nv_bfloat16* base = row_at(j0);
     __nv_bfloat16* dst = k_s + buf * LM_KT * ld;
-    for (int i = tid; i < LM_KT * row_chunks; i += blockDim.x) {
-      const int kk = i / row_chunks, c = i - kk * row_chunks;
-      const int j = j0 + kk;
+    int kk = row0, c = piece0;
+    while (kk < LM_KT) {
+      const bool in = j0 + kk <= last_pos;
       const __nv_bfloat16* src = pool;
-      int bytes = 0;
-      if (j <= last_pos) {
-        const int lp = j / page_size;
-        const int page = table[(long long)seq * table_stride + (lp % table_len)];
-        src = pool + ((long long)page * page_size + (j - lp * page_size)) * dk + c * 8;
-        bytes = 16;
+      if (in) src = (whole ? base + (long long)kk * dk : row_at(j0 + kk)) + c * 8;
+      lm_cp_async16(ds_smem(dst + kk * ld + c * 8), src, in ? 16 : 0);
+      kk += step_row;
+      c += step_piece;
+      if (c >= row_chunks) {
+        c -= row_chunks;
+        ++kk;
       }
-      lm_cp_async16(ds_smem(dst + kk * ld + c * 8), src, bytes);
     }
     lm_cp_commit();
   };
@@ -297,16 +312,21 @@ int launch_latent_attention_mma(const __nv_bfloat16* q, long long q_row_stride, 
            ((unsigned long long)out % 4) == 0, "latent_attention: queries and cache rows must lie on 16-byte boundaries");
   const int dk = rank + rot, dkp = (dk + 15) & ~15, ld = dkp + LM_PAD;
   const int vc = rank / vw;
-  const int hb = n_heads < LM_BM ? n_heads : LM_BM;
-  const int tq = LM_BM / hb;
+  // one token of few heads fills a quarter of the larger block at most; while every block has a multiprocessor to itself
+  // the larger one is ahead all the same, as all its warps copy (8 sequences of 13 runs: 9.8 against 12.6 us; 18: 17.9
+  // against 14.2; 64 of 4: 37.7 against 25.3)
+  const int rg = (long long)max_new * n_heads <= 16 && (long long)n_seqs * n_splits > sm_count() ? 1 : 4;
+  const int rows = 16 * rg;
+  const int hb = n_heads < rows ? n_heads : rows;
+  const int tq = rows / hb;
   const int head_tiles = (n_heads + hb - 1) / hb;
   const int token_tiles = (max_new + tq - 1) / tq;
-  const size_t smem = (size_t)(LM_BM + 2 * LM_KT) * ld * 2 + 4 * 16 * LM_PLD * 2 + 2 * 4 * vw * 16 * sizeof(float);
+  const size_t smem = (size_t)(rows + 2 * LM_KT) * ld * 2 + rg * 16 * LM_PLD * 2 + 2 * rg * vw * 16 * sizeof(float);
   BT_CHECK(smem <= 227 * 1024, "latent_attention: rank + rot = %d needs %zu bytes of shared memory", dk, smem);
-  const dim3 grid(token_tiles * head_tiles, n_splits, n_seqs), block(128 * vw);
-#define BT_LM(VW, VCT)                                                                                               \
+  const dim3 grid(token_tiles * head_tiles, n_splits, n_seqs), block(32 * rg * vw);
+#define BT_LM_SIZED(RG, VW, VCT)                                                                                               \
   do {                                                                                                               \
-    auto kernel = latent_attention_mma_kernel<VW, VCT>;                                                              \
+    auto kernel = latent_attention_mma_kernel<RG, VW, VCT>;                                                              \
     static size_t reserved = 0;   /* (the attribute is set again only when a call needs more than any before) */     \
     if (smem > 48 * 1024 && smem > reserved) {                                                                       \
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
@@ -318,12 +338,18 @@ int launch_latent_attention_mma(const __nv_bfloat16* q, long long q_row_stride, 
                          page_size, seq_start, past_len, sink, out, out_row_stride, part, n_heads, hb, tq, head_tiles, \
                          rank, rot, scale, n_splits, window));                                                       \
   } while (0)
+#define BT_LM(VW, VCT)                                  \
+  do {                                                  \
+    if (rg == 1) BT_LM_SIZED(1, VW, VCT);               \
+    else BT_LM_SIZED(4, VW, VCT);                       \
+  } while (0)
   if (vw == 1 && vc <= 32) BT_LM(1, 32);
   else if (vw == 1 && vc <= 64) BT_LM(1, 64);
   else if (vw == 1) BT_LM(1, 128);
   else if (vw == 2) BT_LM(2, 128);
   else BT_LM(4, 128);
 #undef BT_LM
+#undef BT_LM_SIZED
   return 0;
 }
 

@@ -114,11 +114,11 @@ class LatentAttention(Mixer):
         return CacheNeed(kv=KvSpec(1, self.latent_width, None, has_values=False))
 
     def _splits(self, ctx, rows_per_block: int) -> int:
-        """Runs the keys of a row tile are cut into: enough blocks to fill the GPU about twice, none when the step's
-        rows do that by themselves; at most one per 32 keys."""
+        """Runs the keys of a row tile are cut into: up to two blocks a multiprocessor, all of them at once, none when the
+        step's rows fill the GPU by themselves; at most one per 32 keys."""
         hb = min(self.n_heads, rows_per_block)
         tiles = -(-self.n_heads // hb) * -(-ctx.max_new // max(1, rows_per_block // hb)) * ctx.n_seqs
-        by_fill = -(-2 * _sm_count(ctx.ws.device) // max(1, tiles))
+        by_fill = 2 * _sm_count(ctx.ws.device) // max(1, tiles)
         span = ctx.ctx_bound if self.window is None else min(ctx.ctx_bound, self.window + 64)
         return int(max(1, min(by_fill, -(-span // 32), 64)))
 
