@@ -4,7 +4,7 @@
 // A block computes 128 x BN tiles of the output, one after another (one block per SM).  Its ten warps have fixed jobs:
 //   warp 0    asks the tensor memory accelerator (TMA) for the next 128 x 64 tile of A and BN x 64 tile of W
 //             (cp.async.bulk.tensor, 128-byte swizzle) into a ring of shared-memory stages;
-//   warp 1    one elected thread issues tcgen05.mma (M = 128, N = BN, K = 16, four per stage) whose accumulator
+//   warp 1    one elected thread issues tcgen05.mma (M = 128, or 256 for a pair, N = BN, K = 16, four per stage) whose accumulator
 //             lives in tensor memory (TMEM), and commits each stage back to the producer when it has been read;
 //   warps 2-9 wait for a tile's last commit and read the accumulator with tcgen05.ld (a warp reaches the 32 TMEM lanes
 //             of its quarter; the two warps of a quarter take half of the columns each).  A thread then holds 32
@@ -12,6 +12,11 @@
 //             stores (bfloat16 or 32-bit); with a 32-bit residual the warp first turns its patch through shared
 //             memory, so that four lanes read and write 64 contiguous bytes of a row.  There are two
 //             accumulators, so this runs while the next tile's products are already being issued.
+// What bounds the loop is the issuer at narrow tiles (0.25 us a k-block alone, 0.17 in a pair, up to 128 columns), the tensor
+// cores at wide ones, and for large calls what the whole GPU takes in from L2 and its power.  So two neighbouring blocks (a
+// cluster) may work on one tile of 256 x BN as a PAIR: each loads its own 128 rows of A and half of W's rows, and the tensor
+// cores of both read both halves of W (cta_group::2, issued by the pair's first block).  A block then takes in 16 KB + BN x
+// 64 bytes a k-block for the same products as 16 KB + BN x 128 alone.
 // Both operands are K-major (K contiguous): A as the activations are stored, W as [N, K].
 // The kernel is launched as a programmatic dependent: it sets itself up (barriers, tensor memory) and asks for its
 // first tiles of W while its predecessor still runs, and waits for it only before it touches activations.
@@ -42,20 +47,25 @@ struct TcParams {
 // tensor memory (2 x BN columns), so the epilogue of one tile runs while the products of the next are issued.
 // Shared memory: STAGES x (A tile 128 x 64, W tile BN x 64), each tile 1024-byte aligned, then a 32 x 20 float
 // patch per epilogue warp through which accumulator rows are turned into coalesced global rows.
-template <int BN, int STAGES>
+template <int BN, int STAGES, bool PAIR>
 __global__ void __launch_bounds__(TC_THREADS)
 linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, TcParams p) {
   extern __shared__ unsigned char tc_smem_raw[];
   __shared__ __align__(8) unsigned long long full[STAGES], empty[STAGES], acc_full[2], acc_empty[2];
   __shared__ unsigned tmem_base;
   __shared__ int failed;
-  constexpr unsigned A_BYTES = TC_BM * TC_BK * 2, W_BYTES = BN * TC_BK * 2;
+  constexpr int W_ROWS = PAIR ? BN / 2 : BN;           // of W that this block loads
+  constexpr unsigned A_BYTES = TC_BM * TC_BK * 2, W_BYTES = W_ROWS * TC_BK * 2;
+  constexpr unsigned STAGE_BYTES = (A_BYTES + W_BYTES) * (PAIR ? 2 : 1);      // what a stage's barrier counts
+  constexpr int BM = PAIR ? 2 * TC_BM : TC_BM;          // rows of a tile
   // columns of tensor memory from one accumulator to the other: a power of two, as the allocation has to be
   constexpr int ACC = BN <= 64 ? 64 : (BN <= 128 ? 128 : 256);
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<unsigned long long>(tc_smem_raw) + 1023ull) & ~1023ull);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (uniform for the compiler too)
   pdl_trigger();     // the next kernel may set itself up (and fetch its weights) while this one runs
-  const int tiles_m = (p.M + TC_BM - 1) / TC_BM, tiles_n = (p.N + BN - 1) / BN;
+  const int rank = PAIR ? (int)tc_rank() : 0;           // (the pair's first block is 0)
+  const int tile0 = (int)blockIdx.x / (PAIR ? 2 : 1), tile_step = (int)gridDim.x / (PAIR ? 2 : 1);
+  const int tiles_m = (p.M + BM - 1) / BM, tiles_n = (p.N + BN - 1) / BN;
   const int n_tiles = tiles_m * tiles_n;
   const int k_blocks = (p.K + TC_BK - 1) / TC_BK;
 
@@ -66,61 +76,81 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     }
     for (int b = 0; b < 2; ++b) {
       tc_bar_init(&acc_full[b], 1);
-      tc_bar_init(&acc_empty[b], TC_EPI_WARPS);       // one arrival per epilogue warp
+      tc_bar_init(&acc_empty[b], TC_EPI_WARPS * (PAIR ? 2 : 1));       // one arrival per epilogue warp (of both blocks)
     }
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == 1) {
     // two accumulators of BN 32-bit columns each (the count is a power of two of at least 32)
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc_smem(&tmem_base)), "r"(2 * ACC) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc_smem(&tmem_base)), "r"(2 * ACC) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc_smem(&tmem_base)), "r"(2 * ACC) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
+  if constexpr (PAIR) tc_cluster_sync();      // (the other block's barriers are set up as well)
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const unsigned tmem_acc = tmem_base;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc_elect()) {
       // The first stages' tiles of W are asked for before the kernel waits for its predecessor (programmatic dependent
       // launch): nothing of a step writes weights, so they travel while the previous kernel finishes.  Their tiles
       // of A follow after the wait.
-      const int pre = (int)blockIdx.x < n_tiles ? (k_blocks < STAGES ? k_blocks : STAGES) : 0;
+      const int pre = tile0 < n_tiles ? (k_blocks < STAGES ? k_blocks : STAGES) : 0;
+      auto expect = [&](int s) {
+        if (rank == 0) tc_bar_expect(&full[s], STAGE_BYTES);      // (a pair's copies all count on its first block's barrier)
+      };
+      auto load = [&](int s, bool weights, int kb, int row) {
+        unsigned char* dst = tiles + (size_t)s * (A_BYTES + W_BYTES) + (weights ? A_BYTES : 0);
+        if constexpr (PAIR) tc_tma_load_pair(dst, weights ? &map_w : &map_a, kb * TC_BK, row, tc_first_block(&full[s]));
+        else tc_tma_load(dst, weights ? &map_w : &map_a, kb * TC_BK, row, &full[s]);
+      };
       {
-        const int m0 = ((int)blockIdx.x % tiles_m) * TC_BM, n0 = ((int)blockIdx.x / tiles_m) * BN;
+        const int m0 = (tile0 % tiles_m) * BM + rank * TC_BM, n0 = (tile0 / tiles_m) * BN + rank * W_ROWS;
         for (int kb = 0; kb < pre; ++kb) {
-          tc_bar_expect(&full[kb], A_BYTES + W_BYTES);
-          tc_tma_load(tiles + (size_t)kb * (A_BYTES + W_BYTES) + A_BYTES, &map_w, kb * TC_BK, n0, &full[kb]);
+          expect(kb);
+          load(kb, true, kb, n0);
         }
         pdl_wait();
-        for (int kb = 0; kb < pre; ++kb) tc_tma_load(tiles + (size_t)kb * (A_BYTES + W_BYTES), &map_a, kb * TC_BK, m0, &full[kb]);
+        for (int kb = 0; kb < pre; ++kb) load(kb, false, kb, m0);
       }
-      int it = 0;                          // k-blocks loaded so far, over all tiles
-      for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * BN;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          if (it < pre) continue;          // asked for above
-          const int s = it % STAGES;
-          if (it >= STAGES && !tc_bar_wait(&empty[s], ((it / STAGES) - 1) & 1)) {
+      // the ring: stage `s`, waited for with the parity of its round (the first round's stages are free)
+      int kb = pre, s = pre == STAGES ? 0 : pre;
+      unsigned parity = pre == STAGES ? 0u : 1u;      // (of the round before: a fresh barrier's is complete)
+      for (int tile = tile0; tile < n_tiles; tile += tile_step, kb = 0) {
+        const int m0 = (tile % tiles_m) * BM + rank * TC_BM, n0 = (tile / tiles_m) * BN + rank * W_ROWS;
+        for (; kb < k_blocks; ++kb) {
+          if (!tc_bar_wait(&empty[s], parity)) {
             failed = 1;
             tile = n_tiles;
             break;
           }
-          tc_bar_expect(&full[s], A_BYTES + W_BYTES);
-          unsigned char* a_tile = tiles + (size_t)s * (A_BYTES + W_BYTES);
-          tc_tma_load(a_tile, &map_a, kb * TC_BK, m0, &full[s]);
-          tc_tma_load(a_tile + A_BYTES, &map_w, kb * TC_BK, n0, &full[s]);
+          expect(s);
+          load(s, false, kb, m0);
+          load(s, true, kb, n0);
+          if (++s == STAGES) {
+            s = 0;
+            parity ^= 1u;
+          }
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // instruction descriptor: 32-bit accumulator, bfloat16 operands, both K-major, N = BN, M = 128
-      const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(TC_BM >> 4) << 24);
-      int it = 0, local = 0;
+    // (the whole warp walks the ring and one elected lane issues, so that the operands stay in uniform registers: walked by
+    // the lane whose number is 0, a k-block cost the issuer 0.34 us whatever its width, and that bounded the loop)
+    if (rank == 0) {
+      // instruction descriptor: 32-bit accumulator, bfloat16 operands, both K-major, N = BN, M = 128 (256 for a pair)
+      const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(BM >> 4) << 24);
+      int s = 0, local = 0;
+      unsigned parity = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++local) {
+      for (int tile = tile0; tile < n_tiles && ok; tile += tile_step, ++local) {
         const int buf = local & 1;
         // the epilogue must have emptied this accumulator (it was last used two tiles ago)
         if (local >= 2 && !tc_bar_wait(&acc_empty[buf], ((local >> 1) - 1) & 1)) {
@@ -129,22 +159,37 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const unsigned d_tmem = tmem_acc + (unsigned)(buf * ACC);
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % STAGES;
-          if (!tc_bar_wait(&full[s], (it / STAGES) & 1)) {
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          if (!tc_bar_wait(&full[s], parity)) {
             failed = 1;
             ok = false;
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          unsigned char* a_tile = tiles + (size_t)s * (A_BYTES + W_BYTES);
-          const unsigned long long da = tc_desc(a_tile), dw = tc_desc(a_tile + A_BYTES);
+          if (tc_elect()) {
+            unsigned char* a_tile = tiles + (size_t)s * (A_BYTES + W_BYTES);
+            const unsigned long long da = tc_desc(a_tile), dw = tc_desc(a_tile + A_BYTES);
 #pragma unroll
-          for (int k = 0; k < TC_BK / 16; ++k)   // 16 bfloat16 = 32 bytes further along the row: +2 in 16-byte units
-            tc_mma(d_tmem, da + 2ull * k, dw + 2ull * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          tc_commit(&empty[s]);                  // arrives when these products have read the stage
+            for (int k = 0; k < TC_BK / 16; ++k) { // 16 bfloat16 = 32 bytes further along the row: +2 in 16-byte units
+              const unsigned more = (kb > 0 || k > 0) ? 1u : 0u;
+              if constexpr (PAIR) tc_mma_pair(d_tmem, da + 2ull * k, dw + 2ull * k, idesc, more);
+              else tc_mma(d_tmem, da + 2ull * k, dw + 2ull * k, idesc, more);
+            }
+            // arrives when these products have read the stage (in both blocks of a pair)
+            if constexpr (PAIR) tc_commit_pair(&empty[s]);
+            else tc_commit(&empty[s]);
+            // and, behind a tile's last ones, when every product issued so far has finished
+            if (kb + 1 == k_blocks) {
+              if constexpr (PAIR) tc_commit_pair(&acc_full[buf]);
+              else tc_commit(&acc_full[buf]);
+            }
+          }
+          __syncwarp();
+          if (++s == STAGES) {
+            s = 0;
+            parity ^= 1u;
+          }
         }
-        tc_commit(&acc_full[buf]);               // arrives when every product issued so far has finished
       }
     }
   } else {
@@ -156,9 +201,9 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     pdl_wait();      // the residual is read and the output written only when the previous kernel has finished
     const bool vec_ok = p.out_is_f32 ? (p.N % 4 == 0) : (p.N % 8 == 0);
     int local = 0;
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++local) {
+    for (int tile = tile0; tile < n_tiles; tile += tile_step, ++local) {
       const int buf = local & 1;
-      const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * BN;
+      const int m0 = (tile % tiles_m) * BM + rank * TC_BM, n0 = (tile / tiles_m) * BN;
       const bool ok = tc_bar_wait(&acc_full[buf], (local >> 1) & 1);
       if (!ok) {
         failed = 1;
@@ -278,33 +323,56 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       // this warp has read its part of the accumulator: hand the buffer back to the issuer
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       __syncwarp();
-      if (lane == 0) tc_bar_arrive(&acc_empty[buf]);
+      if (lane == 0) {
+        if constexpr (PAIR) tc_bar_arrive_at(tc_first_block(&acc_empty[buf]));
+        else tc_bar_arrive(&acc_empty[buf]);
+      }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
+  if (failed)          // (a wait ran out: copies may still be in flight, and must not land after the block has gone)
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+  if constexpr (PAIR) tc_cluster_sync();      // neither block's memory or barriers are touched by the other from here on
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_acc), "r"(2 * ACC) : "memory");
+    if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_acc), "r"(2 * ACC) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_acc), "r"(2 * ACC) : "memory");
   }
   if (threadIdx.x == 0 && failed && p.status) atomicExch(p.status, 2);
 }
 
-template <int BN, int STAGES>
+// A tile's shape, what a call costs beside its k-blocks (start, and the last tile's way out) and what a k-block costs, in ns,
+// measured at 1,024 and 2,048 rows with K from 768 to 4,096.  Against the version without pairs, whose issuer a single lane
+// walked (us a call, GPT-2's products with bias, GELU or residual): 2,048 rows: 768 x 3072 23.0 to 15.4, 768 x 768 10.2 to
+// 8.9, 2304 x 768 11.4 to 10.9, 3072 x 768 14.9 to 13.4; 1024 x 4096 30.3 to 19.0; 16,384 rows: 6400 x 1600 262 to 222,
+// 1600 x 6400 364 to 314, 4800 x 1600 201 to 177.
+struct TcTile {
+  int bn;
+  bool pair;
+  int once_ns, k_block_ns;
+};
+constexpr TcTile TC_TILES[] = {{256, false, 8900, 296}, {192, false, 7600, 265}, {128, false, 6400, 245}, {96, false, 5800, 250},
+                               {64, false, 5200, 233}, {256, true, 9400, 294}, {224, true, 8900, 260}, {192, true, 8400, 217},
+                               {160, true, 7900, 196}, {128, true, 7400, 170}, {96, true, 6900, 167}, {64, true, 6400, 163}};
+
+template <int BN, int STAGES, bool PAIR>
 static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mw, const TcParams& p, cudaStream_t stream) {
-  constexpr size_t smem = (size_t)STAGES * (TC_BM * TC_BK * 2 + BN * TC_BK * 2) + 1024 + (size_t)TC_EPI_WARPS * 32 * TC_PATCH_STRIDE * 4;
-  auto kern = linear_tcgen05_kernel<BN, STAGES>;
+  constexpr size_t smem = (size_t)STAGES * (TC_BM * TC_BK * 2 + (PAIR ? BN / 2 : BN) * TC_BK * 2) + 1024 + (size_t)TC_EPI_WARPS * 32 * TC_PATCH_STRIDE * 4;
+  static_assert(smem <= 227 * 1024, "a multiprocessor's shared memory");
+  auto kern = linear_tcgen05_kernel<BN, STAGES, PAIR>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     BT_CHECK(e == cudaSuccess, "linear_tcgen05: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     configured = true;
   }
-  const int n_tiles = ((p.N + BN - 1) / BN) * ((p.M + TC_BM - 1) / TC_BM);
-  const int sms = sm_count();
-  BT_CHECK(sms > 0, "linear_tcgen05: cannot read the number of multiprocessors of the current device");
-  const int blocks = n_tiles < sms ? n_tiles : sms;     // one persistent block per SM
-  BT_PDL_OK("linear_tcgen05", launch_pdl(kern, dim3(blocks), dim3(TC_THREADS), smem, stream, 1, ma, mw, p));
+  constexpr int GROUP = PAIR ? 2 : 1;
+  const int n_tiles = ((p.N + BN - 1) / BN) * ((p.M + GROUP * TC_BM - 1) / (GROUP * TC_BM));
+  const int groups = sm_count() / GROUP;
+  BT_CHECK(groups > 0, "linear_tcgen05: cannot read the number of multiprocessors of the current device");
+  const int blocks = (n_tiles < groups ? n_tiles : groups) * GROUP;     // one persistent block per SM
+  BT_PDL_OK("linear_tcgen05", launch_pdl(kern, dim3(blocks), dim3(TC_THREADS), smem, stream, GROUP, ma, mw, p));
   return 0;
 }
 
@@ -321,29 +389,44 @@ extern "C" int bt_linear_tcgen05(const void* a, const void* w, const float* bias
   BT_CHECK(bt_linear_tcgen05_supports(M, N, K), "linear_tcgen05: sizes M=%d N=%d K=%d are not supported", M, N, K);
   BT_CHECK(act >= 0 && act <= 2, "linear_tcgen05: unknown activation %d", act);
   BT_CHECK(!(residual && !out_is_f32), "linear_tcgen05: a residual needs a 32-bit output");
-  // The tile's width: wide tiles reuse every loaded row of A for more columns, narrow ones cover the GPU with fewer
-  // idle multiprocessors and fewer rounds.  Cost of a width = rounds of tiles over the multiprocessors x the time of
-  // a k-block at that width (measured: 0.31 us at 128 columns, 0.55 us at 256: about 37 + width); ties go to the wider.
-  const long long rows = (M + TC_BM - 1) / TC_BM;
+  // The tile: wide ones reuse every loaded row of A for more columns, narrow ones cover the GPU with fewer idle
+  // multiprocessors and fewer rounds; a pair takes in less and issues more products at once, a single block starts and ends
+  // sooner.  The least of (start and end + rounds of tiles x (k-blocks x their time + 0.4 us)) decides.
   const int sms = sm_count();
-  BT_CHECK(sms > 0, "linear_tcgen05: cannot read the number of multiprocessors of the current device");
+  BT_CHECK(sms > 1, "linear_tcgen05: cannot read the number of multiprocessors of the current device");
   int bn = 256;
+  bool pair = false;
   long long best = -1;
-  for (int width : {256, 192, 128, 96, 64}) {
-    const long long tiles = rows * ((N + width - 1) / width);
-    const long long cost = ((tiles + sms - 1) / sms) * (37 + width);
+  const int k_blocks = (K + TC_BK - 1) / TC_BK;
+  for (const TcTile& t : TC_TILES) {
+    const long long rows = t.pair ? 2 * TC_BM : TC_BM, groups = t.pair ? sms / 2 : sms;
+    const long long tiles = ((M + rows - 1) / rows) * ((N + t.bn - 1) / t.bn), rounds = (tiles + groups - 1) / groups;
+    // (more than three rounds: the whole GPU takes in no more than about 85 GB/s a multiprocessor)
+    const int taken_in = (TC_BM + (t.pair ? t.bn / 2 : t.bn)) * TC_BK * 2 / 85;
+    const long long per_block = rounds > 3 && taken_in > t.k_block_ns ? taken_in : t.k_block_ns;
+    const long long cost = t.once_ns + rounds * (k_blocks * per_block + 400);
     if (best < 0 || cost < best) {
       best = cost;
-      bn = width;
+      bn = t.bn;
+      pair = t.pair;
     }
   }
   CUtensorMap ma, mw;
   if (int rc = tensor_map_2d_bf16(&ma, a, (unsigned long long)M, (unsigned long long)K, (unsigned long long)K, TC_BM)) return rc;
-  if (int rc = tensor_map_2d_bf16(&mw, w, (unsigned long long)N, (unsigned long long)K, (unsigned long long)K, (unsigned)bn)) return rc;
+  if (int rc = tensor_map_2d_bf16(&mw, w, (unsigned long long)N, (unsigned long long)K, (unsigned long long)K, (unsigned)(pair ? bn / 2 : bn))) return rc;
   TcParams p{bias, residual, out, status, M, N, K, act, out_is_f32};
-  if (bn == 64) return launch_tc<64, 6>(ma, mw, p, stream);
-  if (bn == 96) return launch_tc<96, 6>(ma, mw, p, stream);
-  if (bn == 128) return launch_tc<128, 6>(ma, mw, p, stream);
-  if (bn == 192) return launch_tc<192, 5>(ma, mw, p, stream);
-  return launch_tc<256, 4>(ma, mw, p, stream);
+  if (pair) {
+    if (bn == 64) return launch_tc<64, 8, true>(ma, mw, p, stream);
+    if (bn == 96) return launch_tc<96, 8, true>(ma, mw, p, stream);
+    if (bn == 128) return launch_tc<128, 8, true>(ma, mw, p, stream);
+    if (bn == 160) return launch_tc<160, 7, true>(ma, mw, p, stream);
+    if (bn == 192) return launch_tc<192, 7, true>(ma, mw, p, stream);
+    if (bn == 224) return launch_tc<224, 6, true>(ma, mw, p, stream);
+    return launch_tc<256, 6, true>(ma, mw, p, stream);
+  }
+  if (bn == 64) return launch_tc<64, 8, false>(ma, mw, p, stream);
+  if (bn == 96) return launch_tc<96, 7, false>(ma, mw, p, stream);
+  if (bn == 128) return launch_tc<128, 6, false>(ma, mw, p, stream);
+  if (bn == 192) return launch_tc<192, 5, false>(ma, mw, p, stream);
+  return launch_tc<256, 4, false>(ma, mw, p, stream);
 }

@@ -53,6 +53,52 @@ __device__ __forceinline__ void tc_mma(unsigned tmem_d, unsigned long long a, un
 __device__ __forceinline__ void tc_commit(unsigned long long* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(tc_smem(bar)) : "memory");
 }
+// True for one lane of a converged warp, in a way that the compiler knows to be one lane.
+__device__ __forceinline__ bool tc_elect() {
+  unsigned one;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one != 0;
+}
+
+// ---- pairs of blocks (clusters of two, cta_group::2): the first block of the pair issues the products of both ----
+__device__ __forceinline__ unsigned tc_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+  return r;
+}
+// the address, in the pair, of what lies at `p` in this block's shared memory, but in the pair's first block
+__device__ __forceinline__ unsigned tc_first_block(const void* p) {
+  unsigned a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;\n" : "=r"(a) : "r"(tc_smem(p)));
+  return a;
+}
+__device__ __forceinline__ void tc_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+}
+// a copy into this block's shared memory that counts its bytes on a barrier of the pair's first block (`bar`: tc_first_block)
+__device__ __forceinline__ void tc_tma_load_pair(void* dst, const CUtensorMap* map, int col, int row, unsigned bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(
+          tc_smem(dst)),
+      "l"(map), "r"(col), "r"(row), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tc_mma_pair(unsigned tmem_d, unsigned long long a, unsigned long long b, unsigned idesc, unsigned accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrives at the barrier of both blocks when every product issued so far has finished
+__device__ __forceinline__ void tc_commit_pair(unsigned long long* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(tc_smem(bar)),
+               "h"((unsigned short)3)
+               : "memory");
+}
+__device__ __forceinline__ void tc_bar_arrive_at(unsigned bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+
 __device__ __forceinline__ void tc_ld16(unsigned taddr, float (&v)[16]) {
   unsigned r[16];
   asm volatile(
