@@ -599,6 +599,438 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
   if (threadIdx.x == 0 && *failed && p.status) atomicExch(p.status, 6);
 }
 
+// ---- the softmax form ------------------------------------------------------------------------------------------------
+// A block owns 128 queries of one (sequence, head); a thread of warps 0-3 owns one of them (TMEM lane = row):
+//   warps 0-3  read a tile's 128 scores into registers at once (and give the accumulator back: the next tile's S = Q K^T runs
+//              while this tile's weights are formed), keep the row's reference maximum and sum in 32-bit, and write the
+//              weights as bfloat16 into TENSOR MEMORY, from where P V takes them as its first operand;
+//   warp 4     one elected lane copies queries, keys and values by TMA (64 x 64 boxes, two stages);
+//   warp 5     walks the tiles; an elected lane issues S = Q K^T and O += P V, which accumulates over all tiles in TMEM.
+// The accumulated O is rescaled only when a row's maximum has grown by more than 2^8 over the reference its weights are
+// formed with (weights up to 2^8 lose nothing in bfloat16, whose rounding is relative, nor in the 32-bit sums); then the warps
+// wait for the products in flight, and read, multiply and write back their rows.
+// What bounds it is the special-function unit: 128 x 128 exponentials a tile are 1,024 cycles of a multiprocessor, and a
+// thread's other work between two tiles (load, maximum, pack, store) is hidden by a second block on the multiprocessor where
+// shared memory has room for it (heads of up to 64 channels; with values of 128, P takes the place of the scores it was made
+// of and the next scores wait for the product).  The version with eight softmax warps, P through shared memory and O taken
+// out of TMEM each tile had room for one block a multiprocessor: @@NUM@@
+constexpr int TS_SOFTMAX_WARPS = 4;
+constexpr int TS_THREADS = (TS_SOFTMAX_WARPS + 2) * 32;
+constexpr float TS_GROWTH = 8.f;                 // in powers of two
+
+__device__ __forceinline__ bool ta_elect() {
+  unsigned one;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one != 0;
+}
+// the first operand in tensor memory: lane = row, a column two consecutive k
+__device__ __forceinline__ void ta_mma_tmem(unsigned tmem_d, unsigned tmem_a, unsigned long long b, unsigned idesc, unsigned accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void ta_st32(unsigned taddr, const unsigned (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,"
+      "%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};\n" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
+      "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]),
+      "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void ta_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void ta_ld_wait1(unsigned (&a)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+               : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]), "+r"(a[8]),
+                 "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]), "+r"(a[14]), "+r"(a[15]), "+r"(a[16]),
+                 "+r"(a[17]), "+r"(a[18]), "+r"(a[19]), "+r"(a[20]), "+r"(a[21]), "+r"(a[22]), "+r"(a[23]), "+r"(a[24]),
+                 "+r"(a[25]), "+r"(a[26]), "+r"(a[27]), "+r"(a[28]), "+r"(a[29]), "+r"(a[30]), "+r"(a[31])
+               :
+               : "memory");
+}
+
+template <int HD, int HV>
+struct TsShape {
+  static constexpr int TILE_BYTES = HD / 64 * 2 * TA_BOX_BYTES, TILE_V = HV / 64 * 2 * TA_BOX_BYTES;
+  static constexpr size_t SMEM = (size_t)TILE_BYTES * (1 + TA_STAGES) + (size_t)TILE_V * TA_STAGES + 256;
+  static constexpr bool TWO = 2 * (SMEM + 1024) <= 228 * 1024;            // two blocks a multiprocessor
+  // tensor memory: S (128 columns), O (HV), P (64 columns of two keys each), 256 columns a block when two share the 512
+  static constexpr bool OVER = TWO && TA_BK + HV + 64 > 256;              // P over S
+  static constexpr int COLS = TWO ? 256 : 512;
+};
+
+template <int HD, int HV>
+__global__ void __launch_bounds__(TS_THREADS, TsShape<HD, HV>::TWO ? 2 : 1)
+attention_prefill_softmax_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
+                                 const __grid_constant__ CUtensorMap v_map, TaParams p) {
+  using Shape = TsShape<HD, HV>;
+  constexpr int CB = HD / 64, CBV = HV / 64;
+  constexpr int TILE_BYTES = Shape::TILE_BYTES, TILE_V = Shape::TILE_V;
+  constexpr bool OVER = Shape::OVER;
+  extern __shared__ __align__(1024) unsigned char ta_raw[];
+  unsigned char* Qs = ta_raw;
+  unsigned char* Ks = Qs + TILE_BYTES;                     // [stage]
+  unsigned char* Vs = Ks + TA_STAGES * TILE_BYTES;         // [stage]
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(Vs + TA_STAGES * TILE_V);
+  unsigned long long* q_full = bars;
+  unsigned long long* k_full = bars + 1;                   // [stage]
+  unsigned long long* k_empty = k_full + TA_STAGES;
+  unsigned long long* v_full = k_empty + TA_STAGES;
+  unsigned long long* v_empty = v_full + TA_STAGES;
+  unsigned long long* s_full = v_empty + TA_STAGES;        // one phase a tile, as all that follow
+  unsigned long long* s_free = s_full + 1;                 // the scores are in the softmax warps' registers
+  unsigned long long* p_ready = s_free + 1;
+  unsigned long long* o_done = p_ready + 1;                // P V of the tile has been added
+  unsigned* tmem_base = reinterpret_cast<unsigned*>(o_done + 1);
+  int* failed = reinterpret_cast<int*>(tmem_base + 1);
+
+  const int seq = (int)blockIdx.x / p.n_heads, head = (int)blockIdx.x % p.n_heads;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  // (sequence starts and lengths were written before the previous kernel started: safe to read before the wait)
+  const int t0 = p.seq_start[seq], n_new = p.seq_start[seq + 1] - t0;
+  const int q_tile = (int)gridDim.y - 1 - (int)blockIdx.y;      // (the longest blocks first)
+  const int q0 = q_tile * TA_BQ;
+  if (q0 >= n_new) return;
+  if ((ta_smem(ta_raw) & 1023u) != 0) {      // the swizzled layouts need the alignment: refuse rather than compute nonsense
+    if (threadIdx.x == 0 && p.status) atomicExch(p.status, 6);
+    return;
+  }
+  const int past = p.past_len[seq];
+  const int kv_len = past + n_new;
+  const int kv_head = head / (p.n_heads / p.n_kv_heads);
+  const int nq = min(TA_BQ, n_new - q0);
+  const int pos_first = past + q0, pos_last = past + q0 + nq - 1;
+  int key_lo = 0, key_hi = kv_len - 1;                                   // keys any query of the block can see
+  if (p.causal) key_hi = min(key_hi, pos_last);
+  if (p.window > 0) key_lo = max(0, pos_first - p.window + 1);
+  const int kt_lo = key_lo / TA_BK;
+  const int n_tiles = key_hi / TA_BK - kt_lo + 1;
+
+  if (threadIdx.x == 0) {
+    ta_bar_init(q_full, 1);
+    for (int s = 0; s < TA_STAGES; ++s) {
+      ta_bar_init(&k_full[s], 1);
+      ta_bar_init(&k_empty[s], 1);
+      ta_bar_init(&v_full[s], 1);
+      ta_bar_init(&v_empty[s], 1);
+    }
+    ta_bar_init(s_full, 1);
+    ta_bar_init(s_free, TS_SOFTMAX_WARPS);
+    ta_bar_init(p_ready, TS_SOFTMAX_WARPS);
+    ta_bar_init(o_done, 1);
+    *failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == TS_SOFTMAX_WARPS + 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(ta_smem(tmem_base)), "r"(Shape::COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  ta_fence_before();
+  __syncthreads();
+  ta_fence_after();
+  const unsigned tmem_s = *tmem_base, tmem_o = tmem_s + TA_BK, tmem_p = OVER ? tmem_s : tmem_o + (unsigned)HV;
+  // The next kernel's blocks come in once every block of this one has its tensor memory; on multiprocessors that have run
+  // out of query tiles they set themselves up while the longest tiles are still being worked on.
+  pdl_trigger();
+  pdl_wait();      // the projections (and the pages) of this step are complete from here on
+
+  if (warp == TS_SOFTMAX_WARPS) {
+    if (ta_elect()) {
+      // ---- producer ----
+      ta_bar_expect(q_full, TILE_BYTES);
+      for (int cb = 0; cb < CB; ++cb)
+        for (int h = 0; h < 2; ++h)
+          ta_tma(Qs + cb * 2 * TA_BOX_BYTES + h * TA_BOX_BYTES, &q_map, head * p.q_head_cols + cb * 64, t0 + q0 + h * 64, q_full);
+      // where the 64 keys of half h of tile `it` lie: their row in the tensor and the first columns of K and V
+      auto where = [&](int it, int h, int& row, int& col_k, int& col_v) {
+        const int kt = kt_lo + it;
+        if (p.table) {
+          // a page is one box; a half tile beyond the sequence's end repeats its last page (masked, but finite)
+          const int key = min(kt * TA_BK + h * 64, kv_len - 1);
+          const int page = p.table[(long long)seq * p.table_stride + (key / 64) % p.table_len];
+          row = (page * p.n_kv_heads + kv_head) * 64;
+          col_k = (head % p.maps) * p.k_map_cols;
+          col_v = 0;
+        } else if (p.kv_rows > 0) {
+          row = kv_head * p.kv_rows + t0 + kt * TA_BK + h * 64;
+          col_k = col_v = 0;
+        } else {
+          row = t0 + kt * TA_BK + h * 64;
+          col_k = p.k_col + kv_head * HD;
+          col_v = p.v_col + kv_head * HV;
+        }
+      };
+      auto load = [&](int it, bool values) {
+        const int s = it % TA_STAGES;
+        unsigned long long* bar = values ? &v_full[s] : &k_full[s];
+        unsigned char* dst = values ? Vs + s * TILE_V : Ks + s * TILE_BYTES;
+        ta_bar_expect(bar, values ? TILE_V : TILE_BYTES);
+        for (int h = 0; h < 2; ++h) {
+          int row, col_k, col_v;
+          where(it, h, row, col_k, col_v);
+          for (int cb = 0; cb < (values ? CBV : CB); ++cb)
+            ta_tma(dst + cb * 2 * TA_BOX_BYTES + h * TA_BOX_BYTES, values ? &v_map : &k_map, (values ? col_v : col_k) + cb * 64, row, bar);
+        }
+      };
+      for (int it = 0; it < min(n_tiles, TA_STAGES); ++it) {
+        load(it, false);
+        load(it, true);
+      }
+      // a stage of K is free when S of its tile is computed, a stage of V when its P V is
+      for (int it = 0; it + TA_STAGES < n_tiles; ++it) {
+        const int s = it % TA_STAGES;
+        const unsigned parity = (unsigned)(it / TA_STAGES) & 1u;
+        if (!ta_bar_wait(&k_empty[s], parity)) {
+          *failed = 1;
+          break;
+        }
+        load(it + TA_STAGES, false);
+        if (!ta_bar_wait(&v_empty[s], parity)) {
+          *failed = 1;
+          break;
+        }
+        load(it + TA_STAGES, true);
+      }
+    }
+  } else if (warp == TS_SOFTMAX_WARPS + 1) {
+    // ---- issuer.  Instruction descriptors: 32-bit accumulator, bfloat16 operands, M = 128; S: N = 128, both K-major;
+    // P V: N = HV, the first operand in tensor memory, the second MN-major ----
+    const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(TA_BK >> 3) << 17) | ((unsigned)(TA_BQ >> 4) << 24);
+    const unsigned idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(HV >> 3) << 17) | ((unsigned)(TA_BQ >> 4) << 24);
+    const unsigned long long desc_q = ta_desc(Qs, 16), desc_k = ta_desc(Ks, 16), desc_v = ta_desc(Vs, 2 * TA_BOX_BYTES);
+    // S of tile `it`, when its keys have landed and the softmax warps hold the tile before's scores
+    auto scores = [&](int it) -> bool {
+      const int s = it % TA_STAGES;
+      bool there = ta_bar_wait(&k_full[s], (it / TA_STAGES) & 1);
+      if (it > 0) there = there && ta_bar_wait(s_free, (it - 1) & 1);
+      if (OVER && it > 0) there = there && ta_bar_wait(o_done, (it - 1) & 1);      // (P lies where the scores go)
+      if (!__all_sync(0xffffffffu, there)) return false;      // (a wait that runs out must not part the lanes)
+      ta_fence_after();
+      if (ta_elect()) {
+        const unsigned long long dk = desc_k + (unsigned long long)(s * (TILE_BYTES >> 4));
+#pragma unroll
+        for (int k = 0; k < HD / 16; ++k) {      // 16 channels: 32 bytes further along the row, a box further every 64
+          const unsigned long long step = (k / 4) * (2 * TA_BOX_BYTES >> 4) + 2 * (k % 4);
+          ta_mma(tmem_s, desc_q + step, dk + step, idesc_s, k > 0 ? 1u : 0u);
+        }
+        ta_commit(s_full);
+        ta_commit(&k_empty[s]);
+      }
+      __syncwarp();
+      return true;
+    };
+    bool ok = __all_sync(0xffffffffu, ta_bar_wait(q_full, 0));
+    ok = ok && scores(0);
+    for (int it = 0; it < n_tiles && ok; ++it) {
+      const int s = it % TA_STAGES;
+      if (!OVER && it + 1 < n_tiles) ok = scores(it + 1);
+      ok = __all_sync(0xffffffffu, ok && ta_bar_wait(&v_full[s], (it / TA_STAGES) & 1) && ta_bar_wait(p_ready, it & 1));
+      if (!ok) break;
+      ta_fence_after();
+      if (ta_elect()) {
+        const unsigned long long dv = desc_v + (unsigned long long)(s * (TILE_V >> 4));
+#pragma unroll
+        for (int j = 0; j < TA_BK / 16; ++j)     // 16 keys further: 8 columns of P, 16 rows of V
+          ta_mma_tmem(tmem_o, tmem_p + 8u * j, dv + (unsigned long long)(j * (16 * 128 >> 4)), idesc_o, (it > 0 || j > 0) ? 1u : 0u);
+        ta_commit(o_done);
+        ta_commit(&v_empty[s]);
+      }
+      __syncwarp();
+      if (OVER && it + 1 < n_tiles) ok = scores(it + 1);
+    }
+    if (!ok && lane == 0) *failed = 1;
+  } else {
+    // ---- softmax: a thread a query row; warp w reaches TMEM lanes 32 w .. 32 w + 31 ----
+    const int r = warp * 32 + lane;
+    const int pos = past + q0 + r;
+    const unsigned lanes = (unsigned)(warp * 32) << 16;
+    float m = -INFINITY, l = 0.f;      // the reference maximum (base 2, scaled) and the sum of weights formed with it
+    bool ok = true;
+    for (int it = 0; it < n_tiles; ++it) {
+      const int key0 = (kt_lo + it) * TA_BK;
+      ok = __all_sync(0xffffffffu, ok && ta_bar_wait(s_full, it & 1));
+      if (!ok) break;                  // (uniform in the warp; the others run into their own bounds)
+      ta_fence_after();
+      unsigned a[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) ta_ld32_issue(tmem_s + lanes + 32u * c, a[c]);
+      ta_ld_wait(a[0], a[1]);
+      ta_ld_wait(a[2], a[3]);
+      ta_fence_before();
+      __syncwarp();
+      if (lane == 0) ta_bar_arrive(s_free);
+      // every key of the tile visible to every query of the block?  Then nothing is masked (the common tile).
+      const bool whole = key0 + TA_BK <= kv_len && (!p.causal || key0 + TA_BK - 1 <= pos_first) &&
+                         (p.window <= 0 || key0 > pos_last - p.window) && p.scale_log2 > 0.f;
+      float top = -INFINITY;
+      if (whole) {
+        float t4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; ++i) t4[c] = fmaxf(t4[c], __uint_as_float(a[c][i]));
+        top = fmaxf(fmaxf(t4[0], t4[1]), fmaxf(t4[2], t4[3])) * p.scale_log2;      // (the scale is positive on this path)
+      } else {
+        int lo = 0, hi = kv_len - 1;          // this row's visible keys, relative to the tile
+        if (p.causal) hi = min(hi, pos);
+        if (p.window > 0) lo = max(0, pos - p.window + 1);
+        lo -= key0;
+        hi -= key0;
+        // masked scores become what leaves a weight of 0 behind the scale, whatever its sign
+        const float never = p.scale_log2 > 0.f ? -INFINITY : INFINITY;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const bool seen = 32 * c + i >= lo && 32 * c + i <= hi;
+            top = fmaxf(top, seen ? __uint_as_float(a[c][i]) * p.scale_log2 : -INFINITY);
+            a[c][i] = seen ? a[c][i] : __float_as_uint(never);
+          }
+        if (p.scale_log2 == 0.f) {            // (0 times an infinity is no number: the weights are formed here instead)
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const bool seen = 32 * c + i >= lo && 32 * c + i <= hi;
+              a[c][i] = __float_as_uint(seen ? 0.f : -INFINITY);
+            }
+        }
+      }
+      bool taken = it == 0;            // whether the product of the tile before is known to have ended
+      const bool grown = top > m + TS_GROWTH || (m == -INFINITY && top > -INFINITY);
+      if (__any_sync(0xffffffffu, grown)) {
+        const float m_new = grown ? top : m;
+        const float alpha = grown ? ta_exp2(m - m_new) : 1.f;      // 0 for a row that had seen nothing yet
+        l *= alpha;
+        m = m_new;
+        if (it > 0) {
+          ok = __all_sync(0xffffffffu, ta_bar_wait(o_done, (it - 1) & 1));
+          if (!ok) break;
+          taken = true;
+          ta_fence_after();
+#pragma unroll 1
+          for (int c = 0; c < HV; c += 32) {
+            unsigned o[32];
+            ta_ld32_issue(tmem_o + lanes + (unsigned)c, o);
+            ta_ld_wait1(o);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            ta_st32(tmem_o + lanes + (unsigned)c, o);
+          }
+          ta_st_wait();
+        }
+      }
+      const float m_use = m == -INFINITY ? 0.f : m;
+      const float scale = p.scale_log2 == 0.f ? 1.f : p.scale_log2;
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      unsigned w[2][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          const float x = ta_exp2(fmaf(__uint_as_float(a[c][i]), scale, -m_use));
+          const float y = ta_exp2(fmaf(__uint_as_float(a[c][i + 1]), scale, -m_use));
+          sum[c] += x;
+          sum[c] += y;
+          w[c >> 1][(c & 1) * 16 + (i >> 1)] = ta_pack(x, y);
+        }
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      if (!taken) {                    // (the product of the tile before still reads P until then)
+        ok = __all_sync(0xffffffffu, ta_bar_wait(o_done, (it - 1) & 1));
+        if (!ok) break;
+        ta_fence_after();
+      }
+      ta_st32(tmem_p + lanes, w[0]);
+      ta_st32(tmem_p + lanes + 32u, w[1]);
+      ta_st_wait();
+      ta_fence_before();
+      __syncwarp();
+      if (lane == 0) ta_bar_arrive(p_ready);
+    }
+    if (ok) ok = __all_sync(0xffffffffu, ta_bar_wait(o_done, (n_tiles - 1) & 1));
+    if (!ok) *failed = 1;
+    ta_fence_after();
+    float inv = l > 0.f ? 1.f / l : 0.f;
+    if (p.sink != nullptr) {           // the denominator's other term, over the larger of the two exponents
+      const float sink2 = p.sink[head] * 1.4426950408889634f, top = fmaxf(m, sink2);
+      const float mine = ta_exp2(m - top);
+      inv = mine / fmaf(l, mine, ta_exp2(sink2 - top));
+    }
+    const long long token = t0 + q0 + r;
+    const bool mine = r < nq;
+    const __nv_bfloat16* gate = p.gate != nullptr && mine ? p.gate + token * p.gate_row + (long long)head * p.gate_head : nullptr;
+    if (gate != nullptr && p.gate_step == 0) inv *= __fdividef(1.f, 1.f + __expf(-to_float(gate[0])));
+    const long long at = token * ((long long)p.n_heads * p.v_dim) + head * p.v_dim;
+    if (ok) {
+#pragma unroll 1
+      for (int c0 = 0; c0 < HV; c0 += 32) {
+        unsigned raw[32];
+        ta_ld32_issue(tmem_o + lanes + (unsigned)c0, raw);
+        ta_ld_wait1(raw);
+        if (!mine) continue;
+#pragma unroll
+        for (int c = 0; c < 32; c += 8) {
+          if (c0 + c >= p.v_dim) continue;
+          float o[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(raw[c + i]) * inv;
+          if (gate != nullptr && p.gate_step != 0) {
+            const uint4 graw = *reinterpret_cast<const uint4*>(gate + c0 + c);
+            const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&graw);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float2 g = __bfloat1622float2(g2[i]);
+              o[2 * i] *= __fdividef(1.f, 1.f + __expf(-g.x));
+              o[2 * i + 1] *= __fdividef(1.f, 1.f + __expf(-g.y));
+            }
+          }
+          if (p.out32 != nullptr) {
+            float4* dst32 = reinterpret_cast<float4*>(p.out32 + at + c0 + c);
+            dst32[0] = make_float4(o[0], o[1], o[2], o[3]);
+            dst32[1] = make_float4(o[4], o[5], o[6], o[7]);
+          } else {
+            uint4 x;
+            x.x = ta_pack(o[0], o[1]);
+            x.y = ta_pack(o[2], o[3]);
+            x.z = ta_pack(o[4], o[5]);
+            x.w = ta_pack(o[6], o[7]);
+            *reinterpret_cast<uint4*>(p.out + at + c0 + c) = x;
+          }
+        }
+      }
+    }
+  }
+  ta_fence_before();
+  __syncthreads();
+  if (*failed)         // (a wait ran out: copies and products may still be in flight, and must not land after the block has gone)
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+  if (warp == TS_SOFTMAX_WARPS + 1) {
+    ta_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_s), "r"(Shape::COLS) : "memory");
+  }
+  if (threadIdx.x == 0 && *failed && p.status) atomicExch(p.status, 6);
+}
+
+template <int HD, int HV>
+static int launch_ts(const CUtensorMap& qm, const CUtensorMap& km, const CUtensorMap& vm, const TaParams& p, int n_seqs, int max_new,
+                     cudaStream_t stream) {
+  constexpr size_t smem = TsShape<HD, HV>::SMEM;
+  auto kern = attention_prefill_softmax_kernel<HD, HV>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    BT_CHECK(e == cudaSuccess, "attention_prefill_tcgen05: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+    configured = true;
+  }
+  const int q_tiles = (max_new + TA_BQ - 1) / TA_BQ;
+  BT_CHECK(q_tiles <= 65535, "attention_prefill_tcgen05: %d new tokens in one sequence are too many for one launch", max_new);
+  dim3 grid(n_seqs * p.n_heads, q_tiles);
+  BT_PDL_OK("attention_prefill_tcgen05", launch_pdl(kern, grid, dim3(TS_THREADS), smem, stream, 1, qm, km, vm, p));
+  return 0;
+}
+
 template <int HD, int HV, bool SIGMOID>
 static int launch_ta(const CUtensorMap& qm, const CUtensorMap& km, const CUtensorMap& vm, const TaParams& p, int n_seqs, int max_new,
                      cudaStream_t stream) {
@@ -676,8 +1108,8 @@ static int run_attention_prefill_tcgen05(const void* q, long long q_rows, long l
     if (v_dim == 64) return launch_ta<128, 64, true>(qm, km, vm, p, n_seqs, max_new, stream);
     return launch_ta<128, 128, true>(qm, km, vm, p, n_seqs, max_new, stream);
   }
-  if (head_dim == 64) return launch_ta<64, 64, false>(qm, km, vm, p, n_seqs, max_new, stream);
-  return launch_ta<128, 128, false>(qm, km, vm, p, n_seqs, max_new, stream);
+  if (head_dim == 64) return launch_ts<64, 64>(qm, km, vm, p, n_seqs, max_new, stream);
+  return launch_ts<128, 128>(qm, km, vm, p, n_seqs, max_new, stream);
 }
 
 extern "C" int bt_attention_prefill_tcgen05(const void* q, long long q_rows, long long q_row_stride, const void* k, const void* v,
@@ -738,10 +1170,10 @@ extern "C" int bt_sink_attention_tcgen05(const void* q, long long q_row, const v
   TaParams p{(__nv_bfloat16*)out, seq_start, past_len, nullptr, 0, 1, status, n_heads, n_heads, 0, 0,
              scale * 1.4426950408889634f, 1, window, 0, nullptr, dq, dv, (int)rows, sink, (const __nv_bfloat16*)gate,
              gate_row, gate_head, gate_step, nullptr, 1, 0};
-  if (dq <= 64 && dv <= 64) return launch_ta<64, 64, false>(qm, km, vm, p, n_seqs, max_new, stream);
-  if (dq <= 64) return launch_ta<64, 128, false>(qm, km, vm, p, n_seqs, max_new, stream);
-  if (dv <= 64) return launch_ta<128, 64, false>(qm, km, vm, p, n_seqs, max_new, stream);
-  return launch_ta<128, 128, false>(qm, km, vm, p, n_seqs, max_new, stream);
+  if (dq <= 64 && dv <= 64) return launch_ts<64, 64>(qm, km, vm, p, n_seqs, max_new, stream);
+  if (dq <= 64) return launch_ts<64, 128>(qm, km, vm, p, n_seqs, max_new, stream);
+  if (dv <= 64) return launch_ts<128, 64>(qm, km, vm, p, n_seqs, max_new, stream);
+  return launch_ts<128, 128>(qm, km, vm, p, n_seqs, max_new, stream);
 }
 
 // Causal attention in which every head is two maps over one value head, the maps' results left apart for a caller that
@@ -773,8 +1205,8 @@ extern "C" int bt_two_map_attention_tcgen05(const void* q, long long rows, int p
   if (int rc = tensor_map_2d_bf16(&vm, (const __nv_bfloat16*)pool + 2 * dim, pool_rows, v_dim, row, 64)) return rc;
   TaParams p{nullptr, seq_start, past_len, table, table_stride, table_len, status, 2 * n_heads, n_kv_heads, 0, 0,
              scale * 1.4426950408889634f, 1, 0, 0, nullptr, pad, v_dim, 0, nullptr, nullptr, 0, 0, 1, out, 2, dim};
-  if (pad == 64 && v_dim <= 64) return launch_ta<64, 64, false>(qm, km, vm, p, n_seqs, max_new, stream);
-  if (pad == 64) return launch_ta<64, 128, false>(qm, km, vm, p, n_seqs, max_new, stream);
-  if (v_dim <= 64) return launch_ta<128, 64, false>(qm, km, vm, p, n_seqs, max_new, stream);
-  return launch_ta<128, 128, false>(qm, km, vm, p, n_seqs, max_new, stream);
+  if (pad == 64 && v_dim <= 64) return launch_ts<64, 64>(qm, km, vm, p, n_seqs, max_new, stream);
+  if (pad == 64) return launch_ts<64, 128>(qm, km, vm, p, n_seqs, max_new, stream);
+  if (v_dim <= 64) return launch_ts<128, 64>(qm, km, vm, p, n_seqs, max_new, stream);
+  return launch_ts<128, 128>(qm, km, vm, p, n_seqs, max_new, stream);
 }

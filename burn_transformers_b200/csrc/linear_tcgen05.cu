@@ -153,14 +153,15 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       for (int tile = tile0; tile < n_tiles && ok; tile += tile_step, ++local) {
         const int buf = local & 1;
         // the epilogue must have emptied this accumulator (it was last used two tiles ago)
-        if (local >= 2 && !tc_bar_wait(&acc_empty[buf], ((local >> 1) - 1) & 1)) {
+        // (a wait that runs out must not part the warp's lanes)
+        if (!__all_sync(0xffffffffu, local < 2 || tc_bar_wait(&acc_empty[buf], ((local >> 1) - 1) & 1))) {
           failed = 1;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const unsigned d_tmem = tmem_acc + (unsigned)(buf * ACC);
         for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!tc_bar_wait(&full[s], parity)) {
+          if (!__all_sync(0xffffffffu, tc_bar_wait(&full[s], parity))) {
             failed = 1;
             ok = false;
             break;
