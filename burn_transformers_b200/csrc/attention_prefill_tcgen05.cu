@@ -618,6 +618,29 @@ constexpr int TS_SOFTMAX_WARPS = 4;
 constexpr int TS_THREADS = (TS_SOFTMAX_WARPS + 2) * 32;
 constexpr float TS_GROWTH = 8.f;                 // in powers of two
 
+// Two 32-bit numbers in one 64-bit register: a multiply-add or a sum of both is one instruction, each number rounded as by
+// itself.  A warp alone on its scheduler issues such an instruction every other cycle, so these halve what it waits for.
+__device__ __forceinline__ unsigned long long ta_two(unsigned lo, unsigned hi) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+  return v;
+}
+__device__ __forceinline__ void ta_halves(unsigned long long v, unsigned& lo, unsigned& hi) { asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v)); }
+__device__ __forceinline__ unsigned long long ta_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long ta_add2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ float ta_max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 __device__ __forceinline__ bool ta_elect() {
   unsigned one;
   asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
@@ -863,40 +886,45 @@ attention_prefill_softmax_kernel(const __grid_constant__ CUtensorMap q_map, cons
       if (lane == 0) ta_bar_arrive(s_free);
       // every key of the tile visible to every query of the block?  Then nothing is masked (the common tile).
       const bool whole = key0 + TA_BK <= kv_len && (!p.causal || key0 + TA_BK - 1 <= pos_first) &&
-                         (p.window <= 0 || key0 > pos_last - p.window) && p.scale_log2 > 0.f;
+                         (p.window <= 0 || key0 > pos_last - p.window);
+      const bool rising = p.scale_log2 > 0.f;      // the largest score has the largest weight
+      int lo = 0, hi = kv_len - 1;          // this row's visible keys, relative to the tile
+      if (p.causal) hi = min(hi, pos);
+      if (p.window > 0) lo = max(0, pos - p.window + 1);
+      lo -= key0;
+      hi -= key0;
+      if (!whole && rising) {
+        // a bit a key, 32 at a time: the bits become predicates several at once, so that a masked key costs one selection
+        // (two comparisons and a selection a key made the one masked tile of a causal block cost 2,700 cycles, not 500)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int first = lo - 32 * c, last = hi - 32 * c;
+          unsigned seen = last >= 31 ? 0xffffffffu : last < 0 ? 0u : (2u << last) - 1u;
+          seen &= first <= 0 ? 0xffffffffu : first > 31 ? 0u : 0xffffffffu << first;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) a[c][i] = (seen >> i) & 1u ? a[c][i] : __float_as_uint(-INFINITY);
+        }
+      }
       float top = -INFINITY;
-      if (whole) {
-        float t4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      if (rising) {
+        float t4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // (four chains side by side)
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+        for (int i = 0; i < 32; i += 2)
 #pragma unroll
-          for (int i = 0; i < 32; ++i) t4[c] = fmaxf(t4[c], __uint_as_float(a[c][i]));
-        top = fmaxf(fmaxf(t4[0], t4[1]), fmaxf(t4[2], t4[3])) * p.scale_log2;      // (the scale is positive on this path)
+          for (int c = 0; c < 4; ++c) t4[c] = ta_max3(t4[c], __uint_as_float(a[c][i]), __uint_as_float(a[c][i + 1]));
+        top = fmaxf(fmaxf(t4[0], t4[1]), fmaxf(t4[2], t4[3])) * p.scale_log2;
       } else {
-        int lo = 0, hi = kv_len - 1;          // this row's visible keys, relative to the tile
-        if (p.causal) hi = min(hi, pos);
-        if (p.window > 0) lo = max(0, pos - p.window + 1);
-        lo -= key0;
-        hi -= key0;
-        // masked scores become what leaves a weight of 0 behind the scale, whatever its sign
-        const float never = p.scale_log2 > 0.f ? -INFINITY : INFINITY;
+        // masked scores become what leaves a weight of 0 behind a negative scale; a scale of 0 is applied here (0 times an
+        // infinity is no number)
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
             const bool seen = 32 * c + i >= lo && 32 * c + i <= hi;
             top = fmaxf(top, seen ? __uint_as_float(a[c][i]) * p.scale_log2 : -INFINITY);
-            a[c][i] = seen ? a[c][i] : __float_as_uint(never);
+            if (p.scale_log2 == 0.f) a[c][i] = seen ? 0u : __float_as_uint(-INFINITY);
+            else a[c][i] = seen ? a[c][i] : __float_as_uint(INFINITY);
           }
-        if (p.scale_log2 == 0.f) {            // (0 times an infinity is no number: the weights are formed here instead)
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const bool seen = 32 * c + i >= lo && 32 * c + i <= hi;
-              a[c][i] = __float_as_uint(seen ? 0.f : -INFINITY);
-            }
-        }
       }
       bool taken = it == 0;            // whether the product of the tile before is known to have ended
       const bool grown = top > m + TS_GROWTH || (m == -INFINITY && top > -INFINITY);
@@ -924,19 +952,26 @@ attention_prefill_softmax_kernel(const __grid_constant__ CUtensorMap q_map, cons
       }
       const float m_use = m == -INFINITY ? 0.f : m;
       const float scale = p.scale_log2 == 0.f ? 1.f : p.scale_log2;
-      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      const unsigned long long scale2 = ta_two(__float_as_uint(scale), __float_as_uint(scale));
+      const unsigned long long shift2 = ta_two(__float_as_uint(-m_use), __float_as_uint(-m_use));
+      unsigned long long sum[4] = {0ull, 0ull, 0ull, 0ull};
       unsigned w[2][32];
 #pragma unroll
       for (int c = 0; c < 4; ++c)
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          const float x = ta_exp2(fmaf(__uint_as_float(a[c][i]), scale, -m_use));
-          const float y = ta_exp2(fmaf(__uint_as_float(a[c][i + 1]), scale, -m_use));
-          sum[c] += x;
-          sum[c] += y;
-          w[c >> 1][(c & 1) * 16 + (i >> 1)] = ta_pack(x, y);
+          unsigned x, y;
+          ta_halves(ta_fma2(ta_two(a[c][i], a[c][i + 1]), scale2, shift2), x, y);
+          x = __float_as_uint(ta_exp2(__uint_as_float(x)));
+          y = __float_as_uint(ta_exp2(__uint_as_float(y)));
+          sum[(i >> 1) & 3] = ta_add2(sum[(i >> 1) & 3], ta_two(x, y));
+          w[c >> 1][(c & 1) * 16 + (i >> 1)] = ta_pack(__uint_as_float(x), __uint_as_float(y));
         }
-      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      {
+        unsigned x, y;
+        ta_halves(ta_add2(ta_add2(sum[0], sum[1]), ta_add2(sum[2], sum[3])), x, y);
+        l += __uint_as_float(x) + __uint_as_float(y);
+      }
       if (!taken) {                    // (the product of the tile before still reads P until then)
         ok = __all_sync(0xffffffffu, ta_bar_wait(o_done, (it - 1) & 1));
         if (!ok) break;
