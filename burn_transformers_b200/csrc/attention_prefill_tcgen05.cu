@@ -1,22 +1,9 @@
 // Causal attention for steps that bring many tokens per sequence (prefill), bfloat16, on the fifth-generation
-// tensor cores: both products of a tile, S = Q K^T and O += P V, are tcgen05.mma with accumulators in tensor
+// tensor cores: both products of a tile, S = Q K^T and P V, are tcgen05.mma with accumulators in tensor
 // memory (TMEM); the S x S score plane is never stored.
 //
-// A block (one per multiprocessor) owns 128 queries of one (sequence, head) and walks over that sequence's keys in
-// tiles of 128.
-//   warps 0-7  softmax: query row r is TMEM lane r, and two threads share it (a warp reaches the lanes of quarter
-//              warp % 4; warps 0-3 take keys 0-63 of a tile and the lower half of the output channels, warps 4-7
-//              the rest).  A thread reads its part of S with tcgen05.ld, the pair agree on the row's maximum through
-//              shared memory, keep running maximum and sum in 32-bit (scores in base 2), write P = exp2(S - max) as
-//              bfloat16 into shared memory in the layout the tensor core reads (K-major, 128-byte swizzle), then
-//              add the tile's P V, read from TMEM, to their part of the row of the output, which lives in registers;
-//   warp 8     one lane asks the tensor memory accelerator (TMA) for the queries once and for each tile's keys and
-//              values (64 x 64 boxes, 128-byte swizzle) into two stages each;
-//   warp 9     one lane issues the products: S = Q K^T (both operands K-major) into one of two accumulators, so that
-//              the next tile's scores are computed while this tile's are weighed, and O_tile = P V (P K-major, V as
-//              it lies in memory: "MN-major", head channels contiguous) when P is written.  P and O_tile are
-//              double too: the softmax warps take a tile's P V only after they have written the next tile's P, so
-//              that the product runs while they compute.
+// A block owns 128 queries of one (sequence, head) and walks over that sequence's keys in tiles of 128.  There are two
+// kernels: the softmax (further below) and the sigmoid attention.
 // Blocks are numbered by falling length (every sequence and head of the last query tile first).
 // Keys and values come either from the rows of the step's own projections (sequences that start at position 0)
 // or from the pages of the cache (a page is one 64-row box).  Query t of sequence s sits at position
@@ -26,17 +13,29 @@
 // All hand-overs go through mbarriers; every wait is bounded, and a wait that runs out sets the status word:
 // the block still frees its tensor memory and returns.
 //
-// SIGMOID is the same walk for attention without a softmax: the weight of a visible key is sigmoid(score * scale +
-// bias[head]) and nothing is normalised, so the two threads of a row exchange no maximum, nothing is rescaled and
-// nothing divided at the end.  With a window, positions below `keep_first` stay visible to every later query: the tiles
-// that hold them and lie before the window's first tile are walked first (the products never ask where a tile lies).
+// The sigmoid attention has no softmax: the weight of a visible key is sigmoid(score * scale + bias[head]) and nothing is
+// normalised or rescaled.  With a window, positions below `keep_first` stay visible to every later query: the tiles that hold
+// them and lie before the window's first tile are walked first (the products never ask where a tile lies).  One block a
+// multiprocessor:
+//   warps 0-7  weights: query row r is TMEM lane r, and two threads share it (a warp reaches the lanes of quarter
+//              warp % 4; warps 0-3 take keys 0-63 of a tile and the lower half of the output channels, warps 4-7
+//              the rest).  A thread reads its part of S with tcgen05.ld, writes P as bfloat16 into shared memory in the
+//              layout the tensor core reads (K-major, 128-byte swizzle), then adds the tile's P V, read from TMEM, to their
+//              part of the row of the output, which lives in registers;
+//   warp 8     one lane asks the tensor memory accelerator (TMA) for the queries once and for each tile's keys and
+//              values (64 x 64 boxes, 128-byte swizzle) into two stages each;
+//   warp 9     one lane issues the products: S = Q K^T (both operands K-major) into one of two accumulators, so that
+//              the next tile's scores are computed while this tile's are weighed, and O_tile = P V (P K-major, V as
+//              it lies in memory: "MN-major", head channels contiguous) when P is written.  P and O_tile are
+//              double too: the warps take a tile's P V only after they have written the next tile's P, so
+//              that the product runs while they compute.
 //
 // The softmax form also takes heads whose channels are fewer than HD and HV (any multiples of 8): keys and values then
 // lie head by head, [head][token][channels], so that a box that reaches past a head's channels is filled with zeros by
 // the TMA; the queries' boxes may reach into the next head's channels, which meet those zeros.  Output channels past a
 // value head's are not stored.  Differential attention runs a head's two maps as two heads over one pool row [key 1 | key
-// 2 | value] (`maps`), with the queries padded by zeros to HD channels and the results left in 32-bit.  A sink, a number per head, adds exp(sink) to the softmax's denominator; a gate multiplies
-// the result by sigmoid(gate).
+// 2 | value] (`maps`), with the queries padded by zeros to HD channels and the results left in 32-bit.  A sink, a number per
+// head, adds exp(sink) to the softmax's denominator; a gate multiplies the result by sigmoid(gate).
 #include "api.h"
 #include "common.cuh"
 #include "tma.cuh"
@@ -44,7 +43,7 @@
 namespace bt {
 
 constexpr int TA_BQ = 128, TA_BK = 128;
-constexpr int TA_SOFTMAX_WARPS = 8;              // two threads per query row
+constexpr int TA_SOFTMAX_WARPS = 8;              // of the sigmoid form: two threads per query row
 constexpr int TA_THREADS = (TA_SOFTMAX_WARPS + 2) * 32;
 constexpr int TA_STAGES = 2;                     // (the issuer's code is written out for two)
 constexpr int TA_WAIT_LIMIT = 1 << 22;
@@ -61,8 +60,8 @@ struct TaParams {
   int k_col, v_col;            // packed: first column of the keys / values in a row of the projections
   float scale_log2;            // scale * log2(e)
   int causal, window;
-  int keep_first;              // SIGMOID, with a window: positions below this stay visible
-  const float* bias;           // SIGMOID: a number per head added to the scaled score (may be null)
+  int keep_first;              // sigmoid form, with a window: positions below this stay visible
+  const float* bias;           // sigmoid form: a number per head added to the scaled score (may be null)
   int q_head_cols;             // columns between query heads in a row of the projections
   int v_dim;                   // channels of a value head (at most HV), which lie side by side in `out`
   int kv_rows;                 // > 0: keys and values lie head by head, this many rows each (row: a token of the step)
@@ -169,17 +168,16 @@ constexpr int TA_TMEM_COLS = 512;
 //   K      [stage][HD / 64][128 keys][128 bytes], two stages;  V the same with HV, the values' head size (HD for the
 //          softmax attention; the sigmoid attention's keys and values may differ in size)
 //   P      [tile parity][2][128 rows][128 bytes]    (keys 0-63 | 64-127 of the tile)
-//   the row maxima the two threads of a row exchange [tile parity][2 halves][128] (at the end: their sums)
 //   barriers, the tensor-memory address, the failure flag
 template <int HD, int HV>
 constexpr size_t ta_smem_bytes() {
   return (size_t)(HD / 64) * 2 * TA_BOX_BYTES * (1 + TA_STAGES) + (size_t)(HV / 64) * 2 * TA_BOX_BYTES * TA_STAGES +
-         2 * 2 * 2 * TA_BOX_BYTES + 4 * 128 * 4 + 256;
+         2 * 2 * 2 * TA_BOX_BYTES + 256;
 }
 
-template <int HD, int HV, bool SIGMOID>
+template <int HD, int HV>
 __global__ void __launch_bounds__(TA_THREADS, 1)
-attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
+sigmoid_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                                  const __grid_constant__ CUtensorMap v_map, TaParams p) {
   constexpr int CB = HD / 64, CBV = HV / 64;               // 64-column boxes per row of a query or key head, of a value head
   constexpr int TILE_BYTES = CB * 2 * TA_BOX_BYTES;        // 128 rows of a query or key head
@@ -191,8 +189,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
   unsigned char* Ks = Qs + TILE_BYTES;                     // [stage]
   unsigned char* Vs = Ks + TA_STAGES * TILE_BYTES;         // [stage]
   unsigned char* Ps = Vs + TA_STAGES * TILE_V;                             // [tile parity][2 boxes]
-  float* x_max = reinterpret_cast<float*>(Ps + 2 * 2 * 2 * TA_BOX_BYTES);  // [tile parity][half][row]
-  unsigned long long* bars = reinterpret_cast<unsigned long long*>(x_max + 4 * 128);
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(Ps + 2 * 2 * 2 * TA_BOX_BYTES);
   unsigned long long* q_full = bars;                       // 1
   unsigned long long* k_full = bars + 1;                   // [stage]
   unsigned long long* k_empty = k_full + TA_STAGES;        // [stage]
@@ -230,8 +227,8 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
   if (p.causal) key_hi = min(key_hi, pos_last);
   if (p.window > 0) key_lo = max(0, pos_first - p.window + 1);
   const int kt_lo = key_lo / TA_BK, kt_hi = key_hi / TA_BK;
-  // tiles before the window's first that hold kept first positions (SIGMOID): walked first
-  const int kept_only = SIGMOID && p.window > 0 ? min((min(p.keep_first, key_hi + 1) + TA_BK - 1) / TA_BK, kt_lo) : 0;
+  // tiles before the window's first that hold kept first positions: walked first
+  const int kept_only = p.window > 0 ? min((min(p.keep_first, key_hi + 1) + TA_BK - 1) / TA_BK, kt_lo) : 0;
   const int n_tiles = kept_only + kt_hi - kt_lo + 1;
   auto tile_at = [&](int it) { return it < kept_only ? it : kt_lo + (it - kept_only); };
 
@@ -389,13 +386,12 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
       if (!ok) *failed = 1;
     }
   } else {
-    // ---- softmax: two threads per query row.  Warp w reaches the TMEM lanes of quarter w % 4 (rows 32 (w % 4) ..);
+    // ---- weights: two threads per query row.  Warp w reaches the TMEM lanes of quarter w % 4 (rows 32 (w % 4) ..);
     // warps 0-3 take keys 0-63 of a tile and the lower half of the output channels, warps 4-7 the rest ----
     const int half = warp >> 2;
     const int r = (warp & 3) * 32 + lane;
     const int pos = past + q0 + r;
     const unsigned lane_base = (unsigned)((warp & 3) * 32) << 16;
-    float m = -INFINITY, l = 0.f;
     float o[HH];
 #pragma unroll
     for (int i = 0; i < HH; ++i) o[i] = 0.f;
@@ -424,8 +420,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
       __syncwarp();
       if (lane == 0) ta_bar_arrive(&o_free[t & 1]);
     };
-    // (after a wait has run out the remaining waits are skipped, but every warp still runs every tile: the two
-    // warps of a row meet at a barrier in each)
+    // (after a wait has run out the remaining waits are skipped)
     for (int it = 0; it < n_tiles; ++it) {
       const int key0 = tile_at(it) * TA_BK;
       const unsigned s_addr = tmem_s + lane_base + (unsigned)((it & 1) * TA_BK + half * 64);
@@ -433,7 +428,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
       ta_fence_after();
       // every key of the tile visible to every query of the block?  Then nothing is masked (the common tile).
       const bool whole = key0 + TA_BK <= kv_len && (!p.causal || key0 + TA_BK - 1 <= pos_first) &&
-                         (p.window <= 0 || key0 > pos_last - p.window) && (SIGMOID || p.scale_log2 > 0.f);
+                         (p.window <= 0 || key0 > pos_last - p.window);
       int lo = 0, hi = kv_len - 1;          // this row's visible keys, then relative to this thread's 64 keys
       if (p.causal) hi = min(hi, pos);
       if (p.window > 0) lo = max(0, pos - p.window + 1);
@@ -443,64 +438,24 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
       ta_ld32_issue(s_addr, a);
       ta_ld32_issue(s_addr + 32u, b);
       ta_ld_wait(a, b);
-      float sum = 0.f, alpha = 1.f, m_new = m;
       float va[32], vb[32];
-      if constexpr (SIGMOID) {
-        // a weight is 1 / (1 + 2^-(score * scale + bias)) in base 2; kept first positions count beside the window's
-        const int kept = min(p.keep_first, pos + 1) - (key0 + half * 64);      // this thread's keys below it are seen
-        const float bias2 = p.bias != nullptr ? p.bias[head] * 1.4426950408889634f : 0.f;
-        if (whole) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            va[i] = __fdividef(1.f, 1.f + ta_exp2(-fmaf(__uint_as_float(a[i]), p.scale_log2, bias2)));
-            vb[i] = __fdividef(1.f, 1.f + ta_exp2(-fmaf(__uint_as_float(b[i]), p.scale_log2, bias2)));
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const bool sa = (i >= lo && i <= hi) || (p.window > 0 && i < kept && i <= hi);
-            const bool sb = (i + 32 >= lo && i + 32 <= hi) || (p.window > 0 && i + 32 < kept && i + 32 <= hi);
-            va[i] = sa ? __fdividef(1.f, 1.f + ta_exp2(-fmaf(__uint_as_float(a[i]), p.scale_log2, bias2))) : 0.f;
-            vb[i] = sb ? __fdividef(1.f, 1.f + ta_exp2(-fmaf(__uint_as_float(b[i]), p.scale_log2, bias2))) : 0.f;
-          }
-        }
-      } else {
-      // the row's maximum over this thread's keys, then over the row (the other thread's through shared memory)
-      float tile_max = -INFINITY;
-      if (whole) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) tile_max = fmaxf(tile_max, fmaxf(__uint_as_float(a[i]), __uint_as_float(b[i])));
-        tile_max *= p.scale_log2;       // (the scale is positive on this path)
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          tile_max = fmaxf(tile_max, (i >= lo && i <= hi) ? __uint_as_float(a[i]) * p.scale_log2 : -INFINITY);
-          tile_max = fmaxf(tile_max, (i + 32 >= lo && i + 32 <= hi) ? __uint_as_float(b[i]) * p.scale_log2 : -INFINITY);
-        }
-      }
-      x_max[((it & 1) * 2 + half) * 128 + r] = tile_max;
-      // the two warps of a quarter meet at a barrier of their own (64 threads); both run every tile, see below
-      asm volatile("bar.sync %0, 64;\n" ::"r"(1 + (warp & 3)) : "memory");
-      tile_max = fmaxf(tile_max, x_max[((it & 1) * 2 + (half ^ 1)) * 128 + r]);
-      m_new = fmaxf(m, tile_max);
-      const float m_use = m_new == -INFINITY ? 0.f : m_new;
-      alpha = ta_exp2(m - m_use);         // 0 for a row that had seen nothing yet
-      // weights, their sum, and P in shared memory: this thread's 64 keys are one box's row of 128 bytes
+      // a weight is 1 / (1 + 2^-(score * scale + bias)) in base 2; kept first positions count beside the window's
+      const int kept = min(p.keep_first, pos + 1) - (key0 + half * 64);      // this thread's keys below it are seen
+      const float bias2 = p.bias != nullptr ? p.bias[head] * 1.4426950408889634f : 0.f;
       if (whole) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          va[i] = ta_exp2(fmaf(__uint_as_float(a[i]), p.scale_log2, -m_use));
-          vb[i] = ta_exp2(fmaf(__uint_as_float(b[i]), p.scale_log2, -m_use));
-          sum += va[i] + vb[i];
+          va[i] = __fdividef(1.f, 1.f + ta_exp2(-fmaf(__uint_as_float(a[i]), p.scale_log2, bias2)));
+          vb[i] = __fdividef(1.f, 1.f + ta_exp2(-fmaf(__uint_as_float(b[i]), p.scale_log2, bias2)));
         }
       } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          va[i] = (i >= lo && i <= hi) ? ta_exp2(fmaf(__uint_as_float(a[i]), p.scale_log2, -m_use)) : 0.f;
-          vb[i] = (i + 32 >= lo && i + 32 <= hi) ? ta_exp2(fmaf(__uint_as_float(b[i]), p.scale_log2, -m_use)) : 0.f;
-          sum += va[i] + vb[i];
+          const bool sa = (i >= lo && i <= hi) || (p.window > 0 && i < kept && i <= hi);
+          const bool sb = (i + 32 >= lo && i + 32 <= hi) || (p.window > 0 && i + 32 < kept && i + 32 <= hi);
+          va[i] = sa ? __fdividef(1.f, 1.f + ta_exp2(-fmaf(__uint_as_float(a[i]), p.scale_log2, bias2))) : 0.f;
+          vb[i] = sb ? __fdividef(1.f, 1.f + ta_exp2(-fmaf(__uint_as_float(b[i]), p.scale_log2, bias2))) : 0.f;
         }
-      }
       }
       // (this P tile is free: its last products, of tile it - 2, were waited for before that tile's O was taken)
       unsigned char* box = Ps + (it & 1) * 2 * 2 * TA_BOX_BYTES + half * 2 * TA_BOX_BYTES + r * 128;
@@ -518,74 +473,33 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
         *reinterpret_cast<uint4*>(box + ((ch ^ (r & 7)) << 4)) = x;
         *reinterpret_cast<uint4*>(box + (((ch + 4) ^ (r & 7)) << 4)) = y;
       }
-      l = l * alpha + sum;
-      m = m_new;
       // P is written (generic proxy) and S is read: the issuer may go on
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       ta_fence_before();
       __syncwarp();
       if (lane == 0) ta_bar_arrive(&p_ready[it & 1]);
-      // the last tile's P V was computed while this tile's weights were: take it now, then age the sum by this
-      // tile's factor
+      // the last tile's P V was computed while this tile's weights were: take it now
       if (it > 0) {
         if (ok && !ta_bar_wait(&o_full[(it - 1) & 1], ((it - 1) >> 1) & 1)) ok = false;
         ta_fence_after();
         take_o(it - 1);
       }
-      if constexpr (!SIGMOID) {
-#pragma unroll
-        for (int i = 0; i < HH; ++i) o[i] *= alpha;
-      }
     }
     if (ok && !ta_bar_wait(&o_full[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1)) ok = false;
     ta_fence_after();
     take_o(n_tiles - 1);
-    // the row's sum is the two threads' (both hold the same maximum)
-    // (through the exchange buffer that the last tile did not use: nobody reads that one any more)
-    if constexpr (!SIGMOID) {
-      float* x_sum = x_max + (n_tiles & 1) * 2 * 128;
-      x_sum[half * 128 + r] = l;
-      asm volatile("bar.sync %0, 64;\n" ::"r"(1 + (warp & 3)) : "memory");
-      l += x_sum[(half ^ 1) * 128 + r];
-    }
     if (!ok) *failed = 1;
     if (ok && r < nq) {
-      float inv = SIGMOID ? 1.f : (l > 0.f ? 1.f / l : 0.f);
-      if constexpr (!SIGMOID) {
-        if (p.sink != nullptr) {       // the denominator's other term, over the larger of the two exponents
-          const float sink2 = p.sink[head] * 1.4426950408889634f, top = fmaxf(m, sink2);
-          const float mine = ta_exp2(m - top);
-          inv = mine / fmaf(l, mine, ta_exp2(sink2 - top));
-        }
-      }
       const long long token = t0 + q0 + r;
       __nv_bfloat16* dst = p.out + token * ((long long)p.n_heads * p.v_dim) + head * p.v_dim + half * HH;
-      const __nv_bfloat16* gate = p.gate != nullptr ? p.gate + token * p.gate_row + (long long)head * p.gate_head + half * HH * p.gate_step : nullptr;
-      if (gate != nullptr && p.gate_step == 0) inv *= __fdividef(1.f, 1.f + __expf(-to_float(gate[0])));
 #pragma unroll
       for (int c = 0; c < HH; c += 8) {
         if (half * HH + c >= p.v_dim) continue;
-        if (gate != nullptr && p.gate_step != 0) {
-          const uint4 raw = *reinterpret_cast<const uint4*>(gate + c);
-          const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float2 g = __bfloat1622float2(g2[i]);
-            o[c + 2 * i] *= __fdividef(1.f, 1.f + __expf(-g.x));
-            o[c + 2 * i + 1] *= __fdividef(1.f, 1.f + __expf(-g.y));
-          }
-        }
-        if (p.out32 != nullptr) {
-          float4* dst32 = reinterpret_cast<float4*>(p.out32 + token * ((long long)p.n_heads * p.v_dim) + head * p.v_dim + half * HH + c);
-          dst32[0] = make_float4(o[c] * inv, o[c + 1] * inv, o[c + 2] * inv, o[c + 3] * inv);
-          dst32[1] = make_float4(o[c + 4] * inv, o[c + 5] * inv, o[c + 6] * inv, o[c + 7] * inv);
-          continue;
-        }
         uint4 x;
-        x.x = ta_pack(o[c] * inv, o[c + 1] * inv);
-        x.y = ta_pack(o[c + 2] * inv, o[c + 3] * inv);
-        x.z = ta_pack(o[c + 4] * inv, o[c + 5] * inv);
-        x.w = ta_pack(o[c + 6] * inv, o[c + 7] * inv);
+        x.x = ta_pack(o[c], o[c + 1]);
+        x.y = ta_pack(o[c + 2], o[c + 3]);
+        x.z = ta_pack(o[c + 4], o[c + 5]);
+        x.w = ta_pack(o[c + 6], o[c + 7]);
         *reinterpret_cast<uint4*>(dst + c) = x;
       }
     }
@@ -613,7 +527,9 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
 // thread's other work between two tiles (load, maximum, pack, store) is hidden by a second block on the multiprocessor where
 // shared memory has room for it (heads of up to 64 channels; with values of 128, P takes the place of the scores it was made
 // of and the next scores wait for the product).  The version with eight softmax warps, P through shared memory and O taken
-// out of TMEM each tile had room for one block a multiprocessor: @@NUM@@
+// out of TMEM each tile had room for one block a multiprocessor.  16 sequences of 1,024 tokens, 25 heads of 64: 238 us
+// before, 125 now (0.75 us a tile and multiprocessor, 2.4 us a block); 8 x 512, 16 heads: 30.6 to 17.1 us; 2 x 1,024, 12
+// heads: 17.7 to 16.5 us (192 blocks: the time of one chain of eight tiles).
 constexpr int TS_SOFTMAX_WARPS = 4;
 constexpr int TS_THREADS = (TS_SOFTMAX_WARPS + 2) * 32;
 constexpr float TS_GROWTH = 8.f;                 // in powers of two
@@ -869,6 +785,7 @@ attention_prefill_softmax_kernel(const __grid_constant__ CUtensorMap q_map, cons
     const int r = warp * 32 + lane;
     const int pos = past + q0 + r;
     const unsigned lanes = (unsigned)(warp * 32) << 16;
+    const float scale = p.scale_log2 == 0.f ? 1.f : fabsf(p.scale_log2);
     float m = -INFINITY, l = 0.f;      // the reference maximum (base 2, scaled) and the sum of weights formed with it
     bool ok = true;
     for (int it = 0; it < n_tiles; ++it) {
@@ -887,13 +804,20 @@ attention_prefill_softmax_kernel(const __grid_constant__ CUtensorMap q_map, cons
       // every key of the tile visible to every query of the block?  Then nothing is masked (the common tile).
       const bool whole = key0 + TA_BK <= kv_len && (!p.causal || key0 + TA_BK - 1 <= pos_first) &&
                          (p.window <= 0 || key0 > pos_last - p.window);
-      const bool rising = p.scale_log2 > 0.f;      // the largest score has the largest weight
+      // from here on the largest score has the largest weight: a negative scale changes the scores' sign, a scale of 0 is
+      // applied to them at once
+      if (p.scale_log2 <= 0.f) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; ++i) a[c][i] = p.scale_log2 < 0.f ? a[c][i] ^ 0x80000000u : __float_as_uint(__uint_as_float(a[c][i]) * 0.f);
+      }
       int lo = 0, hi = kv_len - 1;          // this row's visible keys, relative to the tile
       if (p.causal) hi = min(hi, pos);
       if (p.window > 0) lo = max(0, pos - p.window + 1);
       lo -= key0;
       hi -= key0;
-      if (!whole && rising) {
+      if (!whole) {
         // a bit a key, 32 at a time: the bits become predicates several at once, so that a masked key costs one selection
         // (two comparisons and a selection a key made the one masked tile of a causal block cost 2,700 cycles, not 500)
 #pragma unroll
@@ -905,27 +829,12 @@ attention_prefill_softmax_kernel(const __grid_constant__ CUtensorMap q_map, cons
           for (int i = 0; i < 32; ++i) a[c][i] = (seen >> i) & 1u ? a[c][i] : __float_as_uint(-INFINITY);
         }
       }
-      float top = -INFINITY;
-      if (rising) {
-        float t4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // (four chains side by side)
+      float t4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // (four chains side by side)
 #pragma unroll
-        for (int i = 0; i < 32; i += 2)
+      for (int i = 0; i < 32; i += 2)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) t4[c] = ta_max3(t4[c], __uint_as_float(a[c][i]), __uint_as_float(a[c][i + 1]));
-        top = fmaxf(fmaxf(t4[0], t4[1]), fmaxf(t4[2], t4[3])) * p.scale_log2;
-      } else {
-        // masked scores become what leaves a weight of 0 behind a negative scale; a scale of 0 is applied here (0 times an
-        // infinity is no number)
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const bool seen = 32 * c + i >= lo && 32 * c + i <= hi;
-            top = fmaxf(top, seen ? __uint_as_float(a[c][i]) * p.scale_log2 : -INFINITY);
-            if (p.scale_log2 == 0.f) a[c][i] = seen ? 0u : __float_as_uint(-INFINITY);
-            else a[c][i] = seen ? a[c][i] : __float_as_uint(INFINITY);
-          }
-      }
+        for (int c = 0; c < 4; ++c) t4[c] = ta_max3(t4[c], __uint_as_float(a[c][i]), __uint_as_float(a[c][i + 1]));
+      const float top = fmaxf(fmaxf(t4[0], t4[1]), fmaxf(t4[2], t4[3])) * scale;
       bool taken = it == 0;            // whether the product of the tile before is known to have ended
       const bool grown = top > m + TS_GROWTH || (m == -INFINITY && top > -INFINITY);
       if (__any_sync(0xffffffffu, grown)) {
@@ -951,7 +860,6 @@ attention_prefill_softmax_kernel(const __grid_constant__ CUtensorMap q_map, cons
         }
       }
       const float m_use = m == -INFINITY ? 0.f : m;
-      const float scale = p.scale_log2 == 0.f ? 1.f : p.scale_log2;
       const unsigned long long scale2 = ta_two(__float_as_uint(scale), __float_as_uint(scale));
       const unsigned long long shift2 = ta_two(__float_as_uint(-m_use), __float_as_uint(-m_use));
       unsigned long long sum[4] = {0ull, 0ull, 0ull, 0ull};
@@ -1066,11 +974,11 @@ static int launch_ts(const CUtensorMap& qm, const CUtensorMap& km, const CUtenso
   return 0;
 }
 
-template <int HD, int HV, bool SIGMOID>
+template <int HD, int HV>
 static int launch_ta(const CUtensorMap& qm, const CUtensorMap& km, const CUtensorMap& vm, const TaParams& p, int n_seqs, int max_new,
                      cudaStream_t stream) {
   constexpr size_t smem = ta_smem_bytes<HD, HV>();
-  auto kern = attention_prefill_tcgen05_kernel<HD, HV, SIGMOID>;
+  auto kern = sigmoid_attention_tcgen05_kernel<HD, HV>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1138,10 +1046,10 @@ static int run_attention_prefill_tcgen05(const void* q, long long q_rows, long l
   BT_CHECK((v_dim == 64 || v_dim == 128) && (sigmoid || v_dim == head_dim),
            "attention_prefill_tcgen05: values of %d channels beside keys of %d are not supported", v_dim, head_dim);
   if (sigmoid) {
-    if (head_dim == 64 && v_dim == 64) return launch_ta<64, 64, true>(qm, km, vm, p, n_seqs, max_new, stream);
-    if (head_dim == 64) return launch_ta<64, 128, true>(qm, km, vm, p, n_seqs, max_new, stream);
-    if (v_dim == 64) return launch_ta<128, 64, true>(qm, km, vm, p, n_seqs, max_new, stream);
-    return launch_ta<128, 128, true>(qm, km, vm, p, n_seqs, max_new, stream);
+    if (head_dim == 64 && v_dim == 64) return launch_ta<64, 64>(qm, km, vm, p, n_seqs, max_new, stream);
+    if (head_dim == 64) return launch_ta<64, 128>(qm, km, vm, p, n_seqs, max_new, stream);
+    if (v_dim == 64) return launch_ta<128, 64>(qm, km, vm, p, n_seqs, max_new, stream);
+    return launch_ta<128, 128>(qm, km, vm, p, n_seqs, max_new, stream);
   }
   if (head_dim == 64) return launch_ts<64, 64>(qm, km, vm, p, n_seqs, max_new, stream);
   return launch_ts<128, 128>(qm, km, vm, p, n_seqs, max_new, stream);
