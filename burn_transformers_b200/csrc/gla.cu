@@ -165,7 +165,11 @@ static int launch_gla_scan(const T* proj, long long row_stride, int q_off, int k
 // e^{b_t - B_g(t)} (kept with q), e^{B_g(t) - B_(g(s)+1)} (formed per pair of groups and channel) and e^{B_(g(s)+1) - b_s}
 // (kept with k); inside a group the weights are products of one to three decays.  gla_chunk_kernel forms, per chunk, the
 // sums over s, the chunk's own contribution to the state, e^{b_end}, and q_t e^{b_t}; gla_prefix_kernel walks a sequence's
-// chunks; gla_carry_kernel adds the incoming state's part.  All 32-bit multiply-adds.
+// chunks; gla_carry_kernel adds the incoming state's part.  All 32-bit multiply-adds.  What bounds these kernels is the way
+// into and out of shared memory: rows are read and results written 16 bytes a lane where they lie on such boundaries (`vec`),
+// the state's product reads four tokens of a channel at once, B's rows have an odd length (with rows of 64, eight groups'
+// numbers of a channel lay in one bank).  2 x 1,024 tokens of 16 heads of 64 x 64 in a recorded layer: 63 + 8 + 20 us before,
+// 42 + 8 + 15 now.
 
 constexpr int GC = 64;     // tokens a chunk
 constexpr int GCP = 68;    // row length of the transposed tiles ([channel][token])
@@ -177,13 +181,14 @@ __global__ void __launch_bounds__(256)
 gla_chunk_kernel(const T* __restrict__ proj, long long row_stride, int q_off, int k_off, int v_off, float q_scale,
                  const float* __restrict__ dt, float log_scale, const int* __restrict__ seq_start, float* __restrict__ out,
                  long long out_row_stride, float* __restrict__ states, float* __restrict__ ends, float* __restrict__ aged_q,
-                 int max_chunks, int n_heads, int dim, int vdim, int col_blocks) {
+                 int max_chunks, int n_heads, int dim, int vdim, int col_blocks, int vec) {
   extern __shared__ __align__(16) float sm[];
   float* q_t = sm;                       // [dim][GCP]   q_t e^{b_t - B_g(t)}
   float* k_t = q_t + dim * GCP;          // [dim][GCP]   k_s e^{B_(g(s)+1) - b_s}; then k_s e^{b_end - b_s}
   float* v_s = k_t + dim * GCP;          // [GC][64]
   float* a_t = v_s + GC * 64;            // [GC][GCP]    a_t[s][t]: token t's weight on token s
-  float* bs = a_t + GC * GCP;            // [GG + 1][dim]  B_0 .. B_16
+  float* bs = a_t + GC * GCP;            // [GG + 1][bsp]  B_0 .. B_16
+  const int bsp = dim | 1;               // (an odd row length: a channel's numbers of several groups lie in several banks)
   pdl_trigger();
   pdl_wait();
   const int chunk = blockIdx.x, seq = blockIdx.z;
@@ -193,52 +198,84 @@ gla_chunk_kernel(const T* __restrict__ proj, long long row_stride, int q_off, in
   const int len = min(GC, n_new - chunk * GC);
   const long long row0 = first + (long long)chunk * GC;
   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15, warp = tid >> 5, lane = tid & 31;
-  for (int i = tid; i < GC * 64; i += 256) {
-    const int t = i >> 6, c = i & 63;
-    v_s[i] = (t < len && col0 + c < vdim)
-                 ? to_float(proj[(row0 + t) * row_stride + v_off + (long long)head * vdim + col0 + c]) : 0.f;
-  }
-  // a warp takes two groups, a lane a channel: the group's q, k and decays, and the weights inside the group
-  for (int g = warp * 2; g < warp * 2 + 2; ++g) {
-    float w00 = 0.f, w11 = 0.f, w22 = 0.f, w33 = 0.f, w10 = 0.f, w21 = 0.f, w32 = 0.f, w20 = 0.f, w31 = 0.f, w30 = 0.f;
-    for (int d = lane; d < dim; d += 32) {
-      float q[4], k[4], la[4], a[4];
+  constexpr int V = 16 / (int)sizeof(T);
+  if (vec) {
+#pragma unroll 2
+    for (int i = tid; i < GC * 64 / V; i += 256) {
+      const int t = i / (64 / V), c = i % (64 / V) * V;
+      float x[V];
+      unpack16(t < len && col0 + c < vdim
+                   ? __ldg(reinterpret_cast<const uint4*>(proj + (row0 + t) * row_stride + v_off + (long long)head * vdim + col0 + c))
+                   : make_uint4(0u, 0u, 0u, 0u), x);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = 4 * g + i;
-        q[i] = k[i] = la[i] = 0.f;
-        if (t < len) {
-          const T* src = proj + (row0 + t) * row_stride + (long long)head * dim + d;
-          q[i] = to_float(src[q_off]) * q_scale;
-          k[i] = to_float(src[k_off]);
-          la[i] = dt[((row0 + t) * n_heads + head) * dim + d] * log_scale;
-        }
-        a[i] = gla_exp<T>(la[i]);
-      }
-      bs[(g + 1) * dim + d] = (la[0] + la[1]) + (la[2] + la[3]);
-      const float a12 = a[1] * a[2], a23 = a[2] * a[3], a123 = a12 * a[3];
-      w00 = fmaf(q[0], k[0], w00);
-      w11 = fmaf(q[1], k[1], w11);
-      w22 = fmaf(q[2], k[2], w22);
-      w33 = fmaf(q[3], k[3], w33);
-      w10 = fmaf(q[1], k[0] * a[1], w10);
-      w21 = fmaf(q[2], k[1] * a[2], w21);
-      w32 = fmaf(q[3], k[2] * a[3], w32);
-      w20 = fmaf(q[2], k[0] * a12, w20);
-      w31 = fmaf(q[3], k[1] * a23, w31);
-      w30 = fmaf(q[3], k[0] * a123, w30);
-      const float p1 = a[0] * a[1], p2 = p1 * a[2], p3 = p2 * a[3];
-      *reinterpret_cast<float4*>(q_t + d * GCP + 4 * g) = make_float4(q[0] * a[0], q[1] * p1, q[2] * p2, q[3] * p3);
-      *reinterpret_cast<float4*>(k_t + d * GCP + 4 * g) = make_float4(k[0] * a123, k[1] * a23, k[2] * a[3], k[3]);
+      for (int u = 0; u < V; u += 4) *reinterpret_cast<float4*>(v_s + t * 64 + c + u) = make_float4(x[u], x[u + 1], x[u + 2], x[u + 3]);
     }
-    w00 = warp_sum(w00); w11 = warp_sum(w11); w22 = warp_sum(w22); w33 = warp_sum(w33); w10 = warp_sum(w10);
-    w21 = warp_sum(w21); w32 = warp_sum(w32); w20 = warp_sum(w20); w31 = warp_sum(w31); w30 = warp_sum(w30);
-    if (lane == 0) {
-      float* cell = a_t + 4 * g * GCP + 4 * g;      // [s][t]
-      *reinterpret_cast<float4*>(cell) = make_float4(w00, w10, w20, w30);
-      *reinterpret_cast<float4*>(cell + GCP) = make_float4(0.f, w11, w21, w31);
-      *reinterpret_cast<float4*>(cell + 2 * GCP) = make_float4(0.f, 0.f, w22, w32);
-      *reinterpret_cast<float4*>(cell + 3 * GCP) = make_float4(0.f, 0.f, 0.f, w33);
+  } else {
+    for (int i = tid; i < GC * 64; i += 256) {
+      const int t = i >> 6, c = i & 63;
+      v_s[i] = (t < len && col0 + c < vdim)
+                   ? to_float(proj[(row0 + t) * row_stride + v_off + (long long)head * vdim + col0 + c]) : 0.f;
+    }
+  }
+  // a warp takes two groups, a lane a channel: the groups' q, k and decays, and the weights inside a group (both groups'
+  // numbers are asked for before either's are used)
+  {
+    float w[2][10] = {};
+    for (int d = lane; d < dim; d += 32) {
+      float q[2][4], k[2][4], la[2][4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int t = 4 * (2 * warp + h) + i;
+          q[h][i] = k[h][i] = la[h][i] = 0.f;
+          if (t < len) {
+            const T* src = proj + (row0 + t) * row_stride + (long long)head * dim + d;
+            q[h][i] = to_float(src[q_off]);
+            k[h][i] = to_float(src[k_off]);
+            la[h][i] = dt[((row0 + t) * n_heads + head) * dim + d];
+          }
+        }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int g = 2 * warp + h;
+        float a[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          q[h][i] *= q_scale;
+          la[h][i] *= log_scale;
+          a[i] = gla_exp<T>(la[h][i]);
+        }
+        bs[(g + 1) * bsp + d] = (la[h][0] + la[h][1]) + (la[h][2] + la[h][3]);
+        const float a12 = a[1] * a[2], a23 = a[2] * a[3], a123 = a12 * a[3];
+        const float(&qh)[4] = q[h];
+        const float(&kh)[4] = k[h];
+        w[h][0] = fmaf(qh[0], kh[0], w[h][0]);
+        w[h][1] = fmaf(qh[1], kh[1], w[h][1]);
+        w[h][2] = fmaf(qh[2], kh[2], w[h][2]);
+        w[h][3] = fmaf(qh[3], kh[3], w[h][3]);
+        w[h][4] = fmaf(qh[1], kh[0] * a[1], w[h][4]);
+        w[h][5] = fmaf(qh[2], kh[1] * a[2], w[h][5]);
+        w[h][6] = fmaf(qh[3], kh[2] * a[3], w[h][6]);
+        w[h][7] = fmaf(qh[2], kh[0] * a12, w[h][7]);
+        w[h][8] = fmaf(qh[3], kh[1] * a23, w[h][8]);
+        w[h][9] = fmaf(qh[3], kh[0] * a123, w[h][9]);
+        const float p1 = a[0] * a[1], p2 = p1 * a[2], p3 = p2 * a[3];
+        *reinterpret_cast<float4*>(q_t + d * GCP + 4 * g) = make_float4(qh[0] * a[0], qh[1] * p1, qh[2] * p2, qh[3] * p3);
+        *reinterpret_cast<float4*>(k_t + d * GCP + 4 * g) = make_float4(kh[0] * a123, kh[1] * a23, kh[2] * a[3], kh[3]);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int i = 0; i < 10; ++i) w[h][i] = warp_sum(w[h][i]);
+      if (lane == 0) {
+        float* cell = a_t + 4 * (2 * warp + h) * GCP + 4 * (2 * warp + h);      // [s][t]
+        *reinterpret_cast<float4*>(cell) = make_float4(w[h][0], w[h][4], w[h][7], w[h][9]);
+        *reinterpret_cast<float4*>(cell + GCP) = make_float4(0.f, w[h][1], w[h][5], w[h][8]);
+        *reinterpret_cast<float4*>(cell + 2 * GCP) = make_float4(0.f, 0.f, w[h][2], w[h][6]);
+        *reinterpret_cast<float4*>(cell + 3 * GCP) = make_float4(0.f, 0.f, 0.f, w[h][3]);
+      }
     }
   }
   __syncthreads();
@@ -246,8 +283,8 @@ gla_chunk_kernel(const T* __restrict__ proj, long long row_stride, int q_off, in
     float sum = 0.f;
     bs[d] = 0.f;
     for (int g = 1; g <= GG; ++g) {
-      sum += bs[g * dim + d];
-      bs[g * dim + d] = sum;
+      sum += bs[g * bsp + d];
+      bs[g * bsp + d] = sum;
     }
     if (col_block == 0) ends[(((long long)seq * max_chunks + chunk) * n_heads + head) * dim + d] = gla_exp<T>(sum);
   }
@@ -255,7 +292,7 @@ gla_chunk_kernel(const T* __restrict__ proj, long long row_stride, int q_off, in
   if (col_block == 0)
     for (int i = tid; i < len * dim; i += 256) {
       const int t = i / dim, d = i - t * dim;
-      aged_q[((row0 + t) * n_heads + head) * dim + d] = q_t[d * GCP + t] * gla_exp<T>(bs[(t >> 2) * dim + d]);
+      aged_q[((row0 + t) * n_heads + head) * dim + d] = q_t[d * GCP + t] * gla_exp<T>(bs[(t >> 2) * bsp + d]);
     }
   // weights between groups: 120 pairs (later group gt, earlier group gs), each shared by two threads with half of the channels
   {
@@ -272,8 +309,8 @@ gla_chunk_kernel(const T* __restrict__ proj, long long row_stride, int q_off, in
     float* cell = a_t + 4 * gs * GCP + 4 * gt;
     if (live) {
       const int d_mid = (dim + 1) / 2, d_end = half ? dim : d_mid;
-      const float* bt_ = bs + gt * dim;
-      const float* bq = bs + (gs + 1) * dim;
+      const float* bt_ = bs + gt * bsp;
+      const float* bq = bs + (gs + 1) * bsp;
       for (int d = half ? d_mid : 0; d < d_end; ++d) {
         const float f = gla_exp<T>(bt_[d] - bq[d]);
         const float4 qv = *reinterpret_cast<const float4*>(q_t + d * GCP + gt * 4);
@@ -303,7 +340,7 @@ gla_chunk_kernel(const T* __restrict__ proj, long long row_stride, int q_off, in
   // k_s e^{b_end - b_s}
   for (int i = tid; i < GG * dim; i += 256) {
     const int g = i / dim, d = i - g * dim;
-    const float f = gla_exp<T>(bs[GG * dim + d] - bs[(g + 1) * dim + d]);
+    const float f = gla_exp<T>(bs[GG * bsp + d] - bs[(g + 1) * bsp + d]);
     float4* at = reinterpret_cast<float4*>(k_t + d * GCP + 4 * g);
     const float4 kv = *at;
     *at = make_float4(kv.x * f, kv.y * f, kv.z * f, kv.w * f);
@@ -329,11 +366,14 @@ gla_chunk_kernel(const T* __restrict__ proj, long long row_stride, int q_off, in
     for (int i = 0; i < 4; ++i) {
       const int t = ty * 4 + i;
       if (t >= len) break;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = col0 + tx * 4 + j;
-        if (c < vdim) out[(row0 + t) * out_row_stride + (long long)head * vdim + c] = acc[i][j];
+      float* o = out + (row0 + t) * out_row_stride + (long long)head * vdim + col0 + tx * 4;
+      if (vec) {
+        if (col0 + tx * 4 < vdim) *reinterpret_cast<float4*>(o) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        continue;
       }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (col0 + tx * 4 + j < vdim) o[j] = acc[i][j];
     }
   }
   __syncthreads();
@@ -345,23 +385,36 @@ gla_chunk_kernel(const T* __restrict__ proj, long long row_stride, int q_off, in
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    for (int sx = 0; sx < len; ++sx) {
-      const float4 vv = *reinterpret_cast<const float4*>(v_s + sx * 64 + tx * 4);
-      const float va[4] = {vv.x, vv.y, vv.z, vv.w};
+    for (int sx = 0; sx < len; sx += 4) {
+      // (tokens past the chunk's last one are zeros in both tiles)
+      float kw[4][4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float kv = i0 + i < dim ? k_t[(i0 + i) * GCP + sx] : 0.f;
+        const float4 kv = i0 + i < dim ? *reinterpret_cast<const float4*>(k_t + (i0 + i) * GCP + sx) : make_float4(0.f, 0.f, 0.f, 0.f);
+        kw[i][0] = kv.x; kw[i][1] = kv.y; kw[i][2] = kv.z; kw[i][3] = kv.w;
+      }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(kv, va[j], acc[i][j]);
+      for (int u = 0; u < 4; ++u) {
+        const float4 vv = *reinterpret_cast<const float4*>(v_s + (sx + u) * 64 + tx * 4);
+        const float va[4] = {vv.x, vv.y, vv.z, vv.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(kw[i][u], va[j], acc[i][j]);
       }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = col0 + tx * 4 + j;
-        if (i0 + i < dim && c < vdim) dst[(long long)(i0 + i) * vdim + c] = acc[i][j];
+    for (int i = 0; i < 4; ++i) {
+      if (i0 + i >= dim) break;
+      float* o = dst + (long long)(i0 + i) * vdim + col0 + tx * 4;
+      if (vec) {
+        if (col0 + tx * 4 < vdim) *reinterpret_cast<float4*>(o) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        continue;
       }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (col0 + tx * 4 + j < vdim) o[j] = acc[i][j];
+    }
   }
 }
 
@@ -404,7 +457,7 @@ gla_prefix_kernel(float* states, const float* __restrict__ ends, float* __restri
 __global__ void __launch_bounds__(256)
 gla_carry_kernel(const float* __restrict__ aged_q, const int* __restrict__ seq_start, float* __restrict__ out,
                  long long out_row_stride, const float* __restrict__ states, int max_chunks, int n_heads, int dim, int vdim,
-                 int col_blocks) {
+                 int col_blocks, int vec) {
   extern __shared__ __align__(16) float sm[];
   float* q_t = sm;                 // [dim][GCP]
   float* s_s = q_t + dim * GCP;    // [dim][64]
@@ -417,14 +470,32 @@ gla_carry_kernel(const float* __restrict__ aged_q, const int* __restrict__ seq_s
   const int len = min(GC, n_new - chunk * GC);
   const long long row0 = first + (long long)chunk * GC;
   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  for (int i = tid; i < GC * dim; i += 256) {
-    const int t = i / dim, d = i - t * dim;
-    q_t[d * GCP + t] = t < len ? aged_q[((row0 + t) * n_heads + head) * dim + d] : 0.f;
-  }
   const float* src = states + ((((long long)seq * max_chunks + chunk) * n_heads + head) * dim) * vdim + col0;
-  for (int i = tid; i < dim * 64; i += 256) {
-    const int d = i >> 6, c = i & 63;
-    s_s[i] = col0 + c < vdim ? src[(long long)d * vdim + c] : 0.f;
+  if (vec) {      // (a warp's lanes are 32 tokens, whose numbers meet all banks when they are written channel by channel)
+#pragma unroll 4
+    for (int i = tid; i < dim / 4 * GC; i += 256) {
+      const int t = i % GC, d = i / GC * 4;
+      const float4 x = t < len ? *reinterpret_cast<const float4*>(aged_q + ((row0 + t) * n_heads + head) * dim + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+      q_t[d * GCP + t] = x.x;
+      q_t[(d + 1) * GCP + t] = x.y;
+      q_t[(d + 2) * GCP + t] = x.z;
+      q_t[(d + 3) * GCP + t] = x.w;
+    }
+#pragma unroll 4
+    for (int i = tid; i < dim * 16; i += 256) {
+      const int d = i >> 4, c = (i & 15) * 4;
+      *reinterpret_cast<float4*>(s_s + d * 64 + c) =
+          col0 + c < vdim ? *reinterpret_cast<const float4*>(src + (long long)d * vdim + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  } else {
+    for (int i = tid; i < GC * dim; i += 256) {
+      const int t = i / dim, d = i - t * dim;
+      q_t[d * GCP + t] = t < len ? aged_q[((row0 + t) * n_heads + head) * dim + d] : 0.f;
+    }
+    for (int i = tid; i < dim * 64; i += 256) {
+      const int d = i >> 6, c = i & 63;
+      s_s[i] = col0 + c < vdim ? src[(long long)d * vdim + c] : 0.f;
+    }
   }
   __syncthreads();
   float acc[4][4];
@@ -445,11 +516,17 @@ gla_carry_kernel(const float* __restrict__ aged_q, const int* __restrict__ seq_s
   for (int i = 0; i < 4; ++i) {
     const int t = ty * 4 + i;
     if (t >= len) break;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = col0 + tx * 4 + j;
-      if (c < vdim) out[(row0 + t) * out_row_stride + (long long)head * vdim + c] += acc[i][j];
+    float* o = out + (row0 + t) * out_row_stride + (long long)head * vdim + col0 + tx * 4;
+    if (vec) {
+      if (col0 + tx * 4 < vdim) {
+        const float4 before = *reinterpret_cast<const float4*>(o);
+        *reinterpret_cast<float4*>(o) = make_float4(before.x + acc[i][0], before.y + acc[i][1], before.z + acc[i][2], before.w + acc[i][3]);
+      }
+      continue;
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (col0 + tx * 4 + j < vdim) o[j] += acc[i][j];
   }
 }
 
@@ -469,7 +546,7 @@ static int launch_gla_chunked(const T* proj, long long row_stride, int q_off, in
   const int col_blocks = (vdim + 63) / 64, max_chunks = (max_new + GC - 1) / GC;
   BT_CHECK((long long)n_heads * col_blocks <= 65535, "gla: %d heads x %d column blocks are too many", n_heads, col_blocks);
   const dim3 grid(max_chunks, n_heads * col_blocks, n_seqs), block(256);
-  const size_t smem_a = ((size_t)2 * dim * GCP + (size_t)GC * 64 + (size_t)GC * GCP + (size_t)(GG + 1) * dim) * sizeof(float);
+  const size_t smem_a = ((size_t)2 * dim * GCP + (size_t)GC * 64 + (size_t)GC * GCP + (size_t)(GG + 1) * (dim | 1)) * sizeof(float);
   const size_t smem_c = ((size_t)dim * GCP + (size_t)dim * 64) * sizeof(float);
   auto chunk_kernel = gla_chunk_kernel<T>;
   if (smem_a > 48 * 1024)
@@ -481,13 +558,17 @@ static int launch_gla_chunked(const T* proj, long long row_stride, int q_off, in
   float* states = scratch;
   float* ends = states + gla_state_floats(n_seqs, max_new, n_heads, dim, vdim);
   float* aged_q = ends + gla_end_floats(n_seqs, max_new, n_heads, dim);
+  // 16-byte accesses: every head of every row, of the results and of the scratch on such a boundary
+  constexpr int V = 16 / (int)sizeof(T);
+  const int vec = dim % 4 == 0 && vdim % V == 0 && v_off % V == 0 && row_stride % V == 0 && out_row_stride % 4 == 0 &&
+                  ((unsigned long long)proj | (unsigned long long)out | (unsigned long long)states | (unsigned long long)aged_q) % 16 == 0;
   BT_PDL_OK("gla_chunk", launch_pdl(chunk_kernel, grid, block, smem_a, stream, 1, proj, row_stride, q_off, k_off, v_off, q_scale,
                                     dt, log_scale, seq_start, out, out_row_stride, states, ends, aged_q, max_chunks, n_heads,
-                                    dim, vdim, col_blocks));
+                                    dim, vdim, col_blocks, vec));
   BT_PDL_OK("gla_prefix", launch_pdl(gla_prefix_kernel, dim3((dim * vdim + 255) / 256, n_heads, n_seqs), block, 0, stream, 1,
                                      states, (const float*)ends, state, slots, seq_start, max_chunks, n_heads, dim, vdim));
   BT_PDL_OK("gla_carry", launch_pdl(gla_carry_kernel, grid, block, smem_c, stream, 1, (const float*)aged_q, seq_start, out,
-                                    out_row_stride, (const float*)states, max_chunks, n_heads, dim, vdim, col_blocks));
+                                    out_row_stride, (const float*)states, max_chunks, n_heads, dim, vdim, col_blocks, vec));
   return 0;
 }
 

@@ -142,6 +142,11 @@ namespace bt {
 constexpr int LC = 64;    // tokens per chunk
 constexpr int LCP = 68;   // row length of the transposed tiles: 16-byte rows, four-way conflicts at most when they are written
 
+// What bounds the chunks' kernels is the way into and out of shared memory, not the multiply-adds: so rows are read 16 bytes a
+// lane where they lie on such boundaries (`vec`; a warp's lanes are 32 tokens, whose numbers meet all banks when they are
+// written channel by channel), the state's product reads four tokens of a channel at once, and results leave as 16 bytes.
+// 2 x 1,024 tokens of 16 heads of 64 x 64 (chunk / carry kernel in a recorded layer, us): 60 / 25 with a number a lane, 39 / 18 so.
+//
 // Tiles of shared memory hold their 64 tokens along the fast axis ([channel][token], rows of LCP floats), so that a
 // thread reads four tokens, or four value channels, with one 16-byte load and every product phase is 16 multiply-adds
 // per two such loads.  Threads form a 16 x 16 grid; thread (ty, tx) owns a 4 x 4 patch of every product.
@@ -152,7 +157,7 @@ __global__ void __launch_bounds__(256)
 lightning_chunk_kernel(const T* __restrict__ proj, long long row_stride, int q_off, int k_off, int v_off,
                        const int* __restrict__ seq_start, const float* __restrict__ decay, float* __restrict__ out,
                        long long out_row_stride, float* __restrict__ scratch, int max_chunks, int n_heads, int dim, int vdim,
-                       int cols, int col_blocks, int act) {
+                       int col_blocks, int act, int vec) {
   extern __shared__ __align__(16) float sm[];
   float* q_t = sm;                       // [dim][LCP]   q_t[d][t]
   float* k_t = q_t + dim * LCP;          // [dim][LCP]   k_t[d][s]
@@ -170,21 +175,48 @@ lightning_chunk_kernel(const T* __restrict__ proj, long long row_stride, int q_o
   const float lam = decay[head];
   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
   for (int i = tid; i <= LC; i += 256) pw[i] = powf(lam, (float)i);
-  for (int i = tid; i < LC * dim; i += 256) {
-    const int t = i / dim, d = i - t * dim;
-    float qv = 0.f, kv = 0.f;
-    if (t < len) {
-      const T* row = proj + (row0 + t) * row_stride + (long long)head * dim + d;
-      qv = feature(to_float(row[q_off]), act);
-      kv = feature(to_float(row[k_off]), act);
+  constexpr int V = 16 / (int)sizeof(T);
+  if (vec) {
+    const int groups = dim / V;
+#pragma unroll 4
+    for (int i = tid; i < 2 * groups * LC; i += 256) {
+      const int t = i % LC, g = i / LC;                    // (q's groups of channels, then k's)
+      const bool key = g >= groups;
+      const int d = (key ? g - groups : g) * V;
+      float x[V];
+      unpack16(t < len ? __ldg(reinterpret_cast<const uint4*>(proj + (row0 + t) * row_stride + (key ? k_off : q_off) + (long long)head * dim + d))
+                       : make_uint4(0u, 0u, 0u, 0u), x);
+      float* dst = (key ? k_t : q_t) + d * LCP + t;
+#pragma unroll
+      for (int u = 0; u < V; ++u) dst[u * LCP] = t < len ? feature(x[u], act) : 0.f;
     }
-    q_t[d * LCP + t] = qv;
-    k_t[d * LCP + t] = kv;
-  }
-  for (int i = tid; i < LC * 64; i += 256) {
-    const int t = i >> 6, c = i & 63;
-    v_s[i] = (t < len && col0 + c < vdim)
-                 ? feature(to_float(proj[(row0 + t) * row_stride + v_off + (long long)head * vdim + col0 + c]), act) : 0.f;
+#pragma unroll 2
+    for (int i = tid; i < LC * 64 / V; i += 256) {
+      const int t = i / (64 / V), c = i % (64 / V) * V;
+      const bool in = t < len && col0 + c < vdim;
+      float x[V];
+      unpack16(in ? __ldg(reinterpret_cast<const uint4*>(proj + (row0 + t) * row_stride + v_off + (long long)head * vdim + col0 + c))
+                  : make_uint4(0u, 0u, 0u, 0u), x);
+#pragma unroll
+      for (int u = 0; u < V; ++u) v_s[t * 64 + c + u] = in ? feature(x[u], act) : 0.f;
+    }
+  } else {
+    for (int i = tid; i < LC * dim; i += 256) {
+      const int t = i / dim, d = i - t * dim;
+      float qv = 0.f, kv = 0.f;
+      if (t < len) {
+        const T* row = proj + (row0 + t) * row_stride + (long long)head * dim + d;
+        qv = feature(to_float(row[q_off]), act);
+        kv = feature(to_float(row[k_off]), act);
+      }
+      q_t[d * LCP + t] = qv;
+      k_t[d * LCP + t] = kv;
+    }
+    for (int i = tid; i < LC * 64; i += 256) {
+      const int t = i >> 6, c = i & 63;
+      v_s[i] = (t < len && col0 + c < vdim)
+                   ? feature(to_float(proj[(row0 + t) * row_stride + v_off + (long long)head * vdim + col0 + c]), act) : 0.f;
+    }
   }
   __syncthreads();
   // scores of the chunk: tokens t = 4 ty .. and s = 4 tx ..
@@ -240,11 +272,14 @@ lightning_chunk_kernel(const T* __restrict__ proj, long long row_stride, int q_o
     for (int i = 0; i < 4; ++i) {
       const int t = ty * 4 + i;
       if (t >= len) break;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = col0 + tx * 4 + j;
-        if (c < vdim) out[(row0 + t) * out_row_stride + (long long)head * vdim + c] = acc[i][j];
+      float* o = out + (row0 + t) * out_row_stride + (long long)head * vdim + col0 + tx * 4;
+      if (vec) {
+        if (col0 + tx * 4 < vdim) *reinterpret_cast<float4*>(o) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        continue;
       }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (col0 + tx * 4 + j < vdim) o[j] = acc[i][j];
     }
   }
   // the chunk's contribution to the state: sum_s decay^(len-1-s) k_s[i] v_s[c], key channels 4 ty .. (+ 64, ...)
@@ -255,24 +290,39 @@ lightning_chunk_kernel(const T* __restrict__ proj, long long row_stride, int q_o
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    for (int sx = 0; sx < len; ++sx) {
-      const float w = pw[len - 1 - sx];
-      const float4 vv = *reinterpret_cast<const float4*>(v_s + sx * 64 + tx * 4);
-      const float va[4] = {vv.x * w, vv.y * w, vv.z * w, vv.w * w};
+    for (int sx = 0; sx < len; sx += 4) {
+      // (tokens past the chunk's last one are zeros in both tiles)
+      float w[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) w[u] = pw[max(len - 1 - sx - u, 0)];
+      float kw[4][4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float kv = i0 + i < dim ? k_t[(i0 + i) * LCP + sx] : 0.f;
+        const float4 kv = i0 + i < dim ? *reinterpret_cast<const float4*>(k_t + (i0 + i) * LCP + sx) : make_float4(0.f, 0.f, 0.f, 0.f);
+        kw[i][0] = kv.x * w[0]; kw[i][1] = kv.y * w[1]; kw[i][2] = kv.z * w[2]; kw[i][3] = kv.w * w[3];
+      }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(kv, va[j], acc[i][j]);
+      for (int u = 0; u < 4; ++u) {
+        const float4 vv = *reinterpret_cast<const float4*>(v_s + (sx + u) * 64 + tx * 4);
+        const float va[4] = {vv.x, vv.y, vv.z, vv.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(kw[i][u], va[j], acc[i][j]);
       }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = col0 + tx * 4 + j;
-        if (i0 + i < dim && c < vdim) dst[(long long)(i0 + i) * vdim + c] = acc[i][j];
+    for (int i = 0; i < 4; ++i) {
+      if (i0 + i >= dim) break;
+      float* o = dst + (long long)(i0 + i) * vdim + col0 + tx * 4;
+      if (vec) {
+        if (col0 + tx * 4 < vdim) *reinterpret_cast<float4*>(o) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        continue;
       }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (col0 + tx * 4 + j < vdim) o[j] = acc[i][j];
+    }
   }
 }
 
@@ -317,8 +367,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 lightning_carry_kernel(const T* __restrict__ proj, long long row_stride, int q_off, const int* __restrict__ seq_start,
                        const float* __restrict__ decay, float* __restrict__ out, long long out_row_stride,
-                       const float* __restrict__ scratch, int max_chunks, int n_heads, int dim, int vdim, int cols,
-                       int col_blocks, int act) {
+                       const float* __restrict__ scratch, int max_chunks, int n_heads, int dim, int vdim, int col_blocks,
+                       int act, int vec) {
   extern __shared__ __align__(16) float sm[];
   float* q_t = sm;                 // [dim][LCP], q_t[d][t] already scaled by decay^(t+1)
   float* s_s = q_t + dim * LCP;    // [dim][64]
@@ -332,15 +382,36 @@ lightning_carry_kernel(const T* __restrict__ proj, long long row_stride, int q_o
   const long long row0 = first + (long long)chunk * LC;
   const float lam = decay[head];
   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  for (int i = tid; i < LC * dim; i += 256) {
-    const int t = i / dim, d = i - t * dim;
-    q_t[d * LCP + t] = t < len ? feature(to_float(proj[(row0 + t) * row_stride + q_off + (long long)head * dim + d]), act) *
-                                     powf(lam, (float)(t + 1)) : 0.f;
-  }
+  float* pw = s_s + dim * 64;      // [LC + 1] powers of the decay
+  for (int i = tid; i <= LC; i += 256) pw[i] = powf(lam, (float)i);
+  __syncthreads();
+  constexpr int V = 16 / (int)sizeof(T);
   const float* src = scratch + ((((long long)seq * max_chunks + chunk) * n_heads + head) * dim) * vdim + col0;
-  for (int i = tid; i < dim * 64; i += 256) {
-    const int d = i >> 6, c = i & 63;
-    s_s[i] = col0 + c < vdim ? src[(long long)d * vdim + c] : 0.f;
+  if (vec) {
+#pragma unroll 2
+    for (int i = tid; i < dim / V * LC; i += 256) {
+      const int t = i % LC, d = i / LC * V;
+      float x[V];
+      unpack16(t < len ? __ldg(reinterpret_cast<const uint4*>(proj + (row0 + t) * row_stride + q_off + (long long)head * dim + d))
+                       : make_uint4(0u, 0u, 0u, 0u), x);
+#pragma unroll
+      for (int u = 0; u < V; ++u) q_t[(d + u) * LCP + t] = t < len ? feature(x[u], act) * pw[t + 1] : 0.f;
+    }
+#pragma unroll 4
+    for (int i = tid; i < dim * 16; i += 256) {
+      const int d = i >> 4, c = (i & 15) * 4;
+      *reinterpret_cast<float4*>(s_s + d * 64 + c) =
+          col0 + c < vdim ? *reinterpret_cast<const float4*>(src + (long long)d * vdim + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  } else {
+    for (int i = tid; i < LC * dim; i += 256) {
+      const int t = i / dim, d = i - t * dim;
+      q_t[d * LCP + t] = t < len ? feature(to_float(proj[(row0 + t) * row_stride + q_off + (long long)head * dim + d]), act) * pw[t + 1] : 0.f;
+    }
+    for (int i = tid; i < dim * 64; i += 256) {
+      const int d = i >> 6, c = i & 63;
+      s_s[i] = col0 + c < vdim ? src[(long long)d * vdim + c] : 0.f;
+    }
   }
   __syncthreads();
   float acc[4][4];
@@ -361,11 +432,17 @@ lightning_carry_kernel(const T* __restrict__ proj, long long row_stride, int q_o
   for (int i = 0; i < 4; ++i) {
     const int t = ty * 4 + i;
     if (t >= len) break;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = col0 + tx * 4 + j;
-      if (c < vdim) out[(row0 + t) * out_row_stride + (long long)head * vdim + c] += acc[i][j];
+    float* o = out + (row0 + t) * out_row_stride + (long long)head * vdim + col0 + tx * 4;
+    if (vec) {
+      if (col0 + tx * 4 < vdim) {
+        const float4 before = *reinterpret_cast<const float4*>(o);
+        *reinterpret_cast<float4*>(o) = make_float4(before.x + acc[i][0], before.y + acc[i][1], before.z + acc[i][2], before.w + acc[i][3]);
+      }
+      continue;
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (col0 + tx * 4 + j < vdim) o[j] += acc[i][j];
   }
 }
 
@@ -374,13 +451,16 @@ static int launch_lightning_chunked(const T* proj, long long row_stride, int q_o
                                     const int* slots, const int* seq_start, const float* decay, float* out,
                                     long long out_row_stride, float* scratch, int max_new, int n_seqs, int n_heads, int dim,
                                     int vdim, int act, cudaStream_t stream) {
-  const int cols = 64;
-  const int col_blocks = (vdim + cols - 1) / cols;
+  const int col_blocks = (vdim + 63) / 64;
   const int max_chunks = (max_new + LC - 1) / LC;
   BT_CHECK((long long)n_heads * col_blocks <= 65535, "lightning_scan: %d heads x %d column blocks are too many", n_heads, col_blocks);
   const dim3 grid(max_chunks, n_heads * col_blocks, n_seqs), block(256);
   const size_t smem_a = ((size_t)2 * dim * LCP + (size_t)LC * 64 + (size_t)LC * LCP + LC + 4) * sizeof(float);
-  const size_t smem_c = ((size_t)dim * LCP + (size_t)dim * 64) * sizeof(float);
+  const size_t smem_c = ((size_t)dim * LCP + (size_t)dim * 64 + LC + 4) * sizeof(float);
+  // 16-byte accesses: every head of every row, of the results and of the states on such a boundary
+  constexpr int V = 16 / (int)sizeof(T);
+  const int vec = dim % V == 0 && vdim % V == 0 && q_off % V == 0 && k_off % V == 0 && v_off % V == 0 && row_stride % V == 0 &&
+                  out_row_stride % 4 == 0 && ((unsigned long long)proj | (unsigned long long)out | (unsigned long long)scratch) % 16 == 0;
   auto chunk_kernel = lightning_chunk_kernel<T>;
   auto carry_kernel = lightning_carry_kernel<T>;
   if (smem_a > 48 * 1024)
@@ -391,13 +471,13 @@ static int launch_lightning_chunked(const T* proj, long long row_stride, int q_o
              "lightning_scan: cannot reserve %zu bytes of shared memory", smem_c);
   BT_PDL_OK("lightning_chunk", launch_pdl(chunk_kernel, grid, block, smem_a, stream, 1, proj, row_stride, q_off, k_off, v_off,
                                           seq_start, decay, out, out_row_stride, scratch, max_chunks, n_heads, dim, vdim,
-                                          cols, col_blocks, act));
+                                          col_blocks, act, vec));
   BT_PDL_OK("lightning_prefix", launch_pdl(lightning_prefix_kernel, dim3((dim * vdim + 255) / 256, n_heads, n_seqs), block, 0,
                                            stream, 1, scratch, state, slots, seq_start, decay, max_chunks, n_heads, dim,
                                            vdim));
   BT_PDL_OK("lightning_carry", launch_pdl(carry_kernel, grid, block, smem_c, stream, 1, proj, row_stride, q_off, seq_start,
                                           decay, out, out_row_stride, (const float*)scratch, max_chunks, n_heads, dim, vdim,
-                                          cols, col_blocks, act));
+                                          col_blocks, act, vec));
   return 0;
 }
 
