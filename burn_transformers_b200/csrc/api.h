@@ -214,6 +214,11 @@ int bt_moe_sort(const int* ids, int total, int E, int* offsets, int* tile_first,
 int bt_moe_expert(int first, const void* a, long long a_row_stride, const void* w, void* out, const int* offsets,
                   const int* tile_first, const int* order, const float* pair_weight, int pairs, int E, int top, int K,
                   int N, int act, float limit, int tensor_cores, int dtype, cudaStream_t stream);
+int bt_moe_expert_tcgen05_supports(int pairs, int E, int K, int N);
+int bt_moe_gather(const void* x, long long x_row_stride, const int* order, int top, void* out, int pairs, int K, cudaStream_t stream);
+int bt_moe_expert_tcgen05(int mode, const void* a, const void* w, void* out, const int* offsets, const int* order,
+                          const float* pair_weight, int* status, int pairs, int E, int K, int N, int act, float limit,
+                          cudaStream_t stream);
 int bt_moe_combine(const float* part, const int* place, float* stream_rows, long long n_tokens, int top, int width,
                    const int* ids, const float* weights, const float* input, int n_stored, int store,
                    cudaStream_t stream);

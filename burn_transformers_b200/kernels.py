@@ -549,7 +549,8 @@ _STATUS_TEXT = {1: "decode attention gave up waiting for a copy of cache pages",
                 5: "the matrix product for 17 to 64 rows gave up waiting for a stage of its pipeline",
                 6: "the tcgen05 prefill attention gave up waiting for a stage of its pipeline (or found its shared memory "
                    "misaligned)",
-                7: "the tcgen05 matrix product for few rows gave up waiting for a stage of its pipeline"}
+                7: "the tcgen05 matrix product for few rows gave up waiting for a stage of its pipeline",
+                8: "the experts' tcgen05 product gave up waiting for a stage of its pipeline"}
 
 
 def check_status(device) -> None:
@@ -1022,6 +1023,48 @@ def moe_expert(first: bool, a, w, out, offsets, tile_first, order, pair_weight, 
                                    _ptr(offsets), _ptr(tile_first), _ptr(order), _ptr(pair_weight), c_int(pairs), c_int(e),
                                    c_int(top), c_int(k), c_int(n), c_int(PAIR_RULES[activation]), c_float(limit),
                                    c_int(1 if tensor_cores else 0), c_int(_code(a.dtype)), _stream()))
+
+
+def moe_many_rows_supports(pairs, n_experts, k, n) -> bool:
+    """Whether `moe_expert_tcgen05` takes the product and is the one to take: bfloat16 steps with more rows an expert than
+    the kernel that streams the weights into registers is for (bt_moe_expert: 48 on average)."""
+    return pairs > 48 * n_experts and _supports("bt_moe_expert_tcgen05_supports", pairs, n_experts, k, n)
+
+
+def moe_gather(x, order, out, *, pairs, top):
+    """out[r] = x[order[r] // top] for the sorted rows r < pairs (bfloat16, rows of whole 16-byte pieces)."""
+    k = out.shape[1]
+    _need(x, "x", torch.bfloat16, (None, k))
+    _need(out, "out", torch.bfloat16, (None, k))
+    _need(order, "order", torch.int32)
+    if out.shape[0] < pairs or order.numel() < pairs:
+        raise ShapeError(f"moe_gather: {pairs} rows asked of shorter tensors")
+    _work(0.0, 4.0 * pairs * k)
+    _check(library().bt_moe_gather(_ptr(x), c_longlong(x.stride(0)), _ptr(order), c_int(top), _ptr(out), c_int(pairs), c_int(k),
+                                   _stream()))
+
+
+def moe_expert_tcgen05(first: bool, a, w, out, offsets, order, pair_weight, *, pairs, activation=None, limit: float = 0.0,
+                       gated: bool = True):
+    """One of the experts' two products on tcgen05 (csrc/moe_tcgen05.cu); as `moe_expert`, with `a` [pairs, K] sorted by
+    expert for both (`moe_gather`)."""
+    e, rows_w, k = w.shape
+    n = rows_w // 2 if first and gated else rows_w
+    _need(a, "a", torch.bfloat16, (None, k))
+    _need(w, "w", torch.bfloat16)
+    _need(out, "out", torch.bfloat16 if first else torch.float32, (None, n))
+    _need(offsets, "offsets", torch.int32)
+    _need(order, "order", torch.int32)
+    if min(out.shape[0], a.shape[0], order.numel()) < pairs or offsets.numel() < e + 1:
+        raise ShapeError(f"moe_expert_tcgen05: {pairs} rows asked of shorter tensors")
+    if a.stride(0) != k:
+        raise ShapeError("moe_expert_tcgen05: the sorted rows must lie side by side")
+    if activation not in (PAIR_RULES if gated else ACTIVATIONS):
+        raise ShapeError(f"moe_expert_tcgen05: unknown activation {activation!r}")
+    _work(2.0 * pairs * rows_w * k, w.numel() * w.element_size() + pairs * (k * a.element_size() + n * out.element_size()))
+    _check(library().bt_moe_expert_tcgen05(c_int((1 if gated else 2) if first else 0), _ptr(a), _ptr(w), _ptr(out), _ptr(offsets),
+                                           _ptr(order), _ptr(pair_weight), _ptr(kernel_status(a.device)), c_int(pairs), c_int(e),
+                                           c_int(k), c_int(n), c_int(PAIR_RULES[activation]), c_float(limit), _stream()))
 
 
 def moe_combine(part, place, stream_rows, *, n_tokens, top, ids=None, weights=None, identity_input=None, n_stored=0,

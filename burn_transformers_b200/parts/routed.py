@@ -154,8 +154,16 @@ class RoutedFeedForward(FeedForward):
         place = ctx.ws.take((pairs,), torch.int32)
         kernels.moe_sort(ids, offsets, tile_first, order, place, pairs=pairs, n_experts=routes)
         hidden = ctx.ws.take((pairs, self.inner), ctx.dtype)
+        part = ctx.ws.take((pairs, self.width), torch.float32)
+        if (ctx.dtype == torch.bfloat16 and kernels.moe_many_rows_supports(pairs, self.n_experts, self.width, self.inner)
+                and kernels.moe_many_rows_supports(pairs, self.n_experts, self.inner, self.width)):
+            rows = ctx.ws.take((pairs, self.width), ctx.dtype)
+            kernels.moe_gather(x, order, rows, pairs=pairs, top=top)
+            kernels.moe_expert_tcgen05(True, rows, self.w_in, hidden, offsets, order, None, pairs=pairs,
+                                       activation=self.activation, limit=self.limit, gated=self.gated)
+            kernels.moe_expert_tcgen05(False, hidden, self.w_out, part, offsets, order, weights, pairs=pairs)
+            return part, place, ids, weights
         kernels.moe_expert(True, x, self.w_in, hidden, offsets, tile_first, order, None, pairs=pairs, top=top,
                            activation=self.activation, limit=self.limit, gated=self.gated)
-        part = ctx.ws.take((pairs, self.width), torch.float32)
         kernels.moe_expert(False, hidden, self.w_out, part, offsets, tile_first, order, weights, pairs=pairs, top=top)
         return part, place, ids, weights
