@@ -73,6 +73,9 @@ int bt_sample(const float* logits, long long row_stride, int n_rows, int vocab, 
 int bt_advance(const int* ids, int* tokens, int* positions, int* past_len, int* ctx_len, int* counters, int n,
                cudaStream_t stream);
 int bt_linear_tcgen05_supports(int M, int N, int K);
+int bt_head_rows_tcgen05_supports(int M, int N, int K, long long a_row, long long out_row, long long head_stride);
+int bt_head_rows_tcgen05(const void* a, long long a_row, const void* w, void* out, long long out_row, long long head_stride, int* status,
+                         int M, int heads, int N, int K, cudaStream_t stream);
 int bt_linear_tcgen05(const void* a, const void* w, const float* bias, const float* residual, void* out, int* status,
                       int M, int N, int K, int act, int out_is_f32, cudaStream_t stream);
 // out[M, N] = act(x[M, K] @ w[N, K]^T + bias) (+ residual) for at most 128 bfloat16 rows over large weights, on the

@@ -40,6 +40,9 @@ struct TcParams {
   void* out;                // [M, N] 32-bit or bfloat16
   int* status;              // set to 1 when a bounded wait ran out
   int M, N, K, act, out_is_f32;
+  // head_cols > 0 (bfloat16 results only): column c of row r goes to out[(c / head_cols) * head_stride + r * out_row + c % head_cols]
+  int head_cols;
+  long long out_row, head_stride;
 };
 
 
@@ -299,11 +302,14 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             }
             __syncwarp();
             const int cq = lane & 3, rq = lane >> 2;
+            // (a chunk of 32 columns lies in one head)
+            const int head = p.head_cols > 0 ? col0 / p.head_cols : 0;
+            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out) + head * p.head_stride + (col0 - head * p.head_cols) + 8 * cq;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               const int r = rq + 8 * k, grow = m0 + quarter * 32 + r;
               const uint4 x = *reinterpret_cast<const uint4*>(patch8 + r * (TC_PATCH_STRIDE * 4) + 16 * cq);
-              if (grow < p.M) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (long long)grow * p.N + col0 + 8 * cq) = x;
+              if (grow < p.M) *reinterpret_cast<uint4*>(dst + (long long)grow * p.out_row) = x;
             }
             __syncwarp();      // the patch is free again
           }
@@ -383,13 +389,9 @@ extern "C" int bt_linear_tcgen05_supports(int M, int N, int K) {
   return M >= 1 && N >= 8 && K >= 8 && K % 8 == 0;   // rows of A and W are 16-byte multiples
 }
 
-// a: [M, K] bfloat16; w: [N, K] bfloat16; out: [M, N] 32-bit (out_is_f32) or bfloat16.
-extern "C" int bt_linear_tcgen05(const void* a, const void* w, const float* bias, const float* residual, void* out,
-                                 int* status, int M, int N, int K, int act, int out_is_f32, cudaStream_t stream) {
+static int run_linear_tcgen05(const void* a, long long a_row, const void* w, bt::TcParams p, cudaStream_t stream) {
   using namespace bt;
-  BT_CHECK(bt_linear_tcgen05_supports(M, N, K), "linear_tcgen05: sizes M=%d N=%d K=%d are not supported", M, N, K);
-  BT_CHECK(act >= 0 && act <= 2, "linear_tcgen05: unknown activation %d", act);
-  BT_CHECK(!(residual && !out_is_f32), "linear_tcgen05: a residual needs a 32-bit output");
+  const int M = p.M, N = p.N, K = p.K;
   // The tile: wide ones reuse every loaded row of A for more columns, narrow ones cover the GPU with fewer idle
   // multiprocessors and fewer rounds; a pair takes in less and issues more products at once, a single block starts and ends
   // sooner.  The least of (start and end + rounds of tiles x (k-blocks x their time + 0.4 us)) decides.
@@ -413,9 +415,8 @@ extern "C" int bt_linear_tcgen05(const void* a, const void* w, const float* bias
     }
   }
   CUtensorMap ma, mw;
-  if (int rc = tensor_map_2d_bf16(&ma, a, (unsigned long long)M, (unsigned long long)K, (unsigned long long)K, TC_BM)) return rc;
+  if (int rc = tensor_map_2d_bf16(&ma, a, (unsigned long long)M, (unsigned long long)K, (unsigned long long)a_row, TC_BM)) return rc;
   if (int rc = tensor_map_2d_bf16(&mw, w, (unsigned long long)N, (unsigned long long)K, (unsigned long long)K, (unsigned)(pair ? bn / 2 : bn))) return rc;
-  TcParams p{bias, residual, out, status, M, N, K, act, out_is_f32};
   if (pair) {
     if (bn == 64) return launch_tc<64, 8, true>(ma, mw, p, stream);
     if (bn == 96) return launch_tc<96, 8, true>(ma, mw, p, stream);
@@ -430,4 +431,28 @@ extern "C" int bt_linear_tcgen05(const void* a, const void* w, const float* bias
   if (bn == 128) return launch_tc<128, 6, false>(ma, mw, p, stream);
   if (bn == 192) return launch_tc<192, 5, false>(ma, mw, p, stream);
   return launch_tc<256, 4, false>(ma, mw, p, stream);
+}
+
+// a: [M, K] bfloat16; w: [N, K] bfloat16; out: [M, N] 32-bit (out_is_f32) or bfloat16.
+extern "C" int bt_linear_tcgen05(const void* a, const void* w, const float* bias, const float* residual, void* out,
+                                 int* status, int M, int N, int K, int act, int out_is_f32, cudaStream_t stream) {
+  using namespace bt;
+  BT_CHECK(bt_linear_tcgen05_supports(M, N, K), "linear_tcgen05: sizes M=%d N=%d K=%d are not supported", M, N, K);
+  BT_CHECK(act >= 0 && act <= 2, "linear_tcgen05: unknown activation %d", act);
+  BT_CHECK(!(residual && !out_is_f32), "linear_tcgen05: a residual needs a 32-bit output");
+  return run_linear_tcgen05(a, K, w, TcParams{bias, residual, out, status, M, N, K, act, out_is_f32, 0, N, 0}, stream);
+}
+
+// Per-head rows of one product: out[h][t][:] = a[t] @ w[h]^T for heads of N numbers (a multiple of 32), all bfloat16.
+// a: [M, K], rows a_row elements apart; w: [heads * N, K]; out: rows out_row apart, heads head_stride.
+extern "C" int bt_head_rows_tcgen05_supports(int M, int N, int K, long long a_row, long long out_row, long long head_stride) {
+  return M >= 1 && N >= 32 && N % 32 == 0 && K >= 8 && K % 8 == 0 && a_row >= K && a_row % 8 == 0 && out_row % 8 == 0 && head_stride % 8 == 0;
+}
+extern "C" int bt_head_rows_tcgen05(const void* a, long long a_row, const void* w, void* out, long long out_row, long long head_stride,
+                                    int* status, int M, int heads, int N, int K, cudaStream_t stream) {
+  using namespace bt;
+  BT_CHECK(heads > 0 && bt_head_rows_tcgen05_supports(M, N, K, a_row, out_row, head_stride) &&
+               ((unsigned long long)a | (unsigned long long)w | (unsigned long long)out) % 16 == 0,
+           "head_rows_tcgen05: sizes or strides that are not supported (M=%d heads=%d N=%d K=%d)", M, heads, N, K);
+  return run_linear_tcgen05(a, a_row, w, TcParams{nullptr, nullptr, out, status, M, heads * N, K, 0, 0, N, out_row, head_stride}, stream);
 }

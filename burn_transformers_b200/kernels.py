@@ -713,6 +713,29 @@ def head_linear(a, w, out, *, n_tokens, gate=None, tensor_cores=True):
                                     c_int(_code(w.dtype)), _stream()))
 
 
+def head_rows_supports(a, w, out, n_tokens) -> bool:
+    """Whether `head_rows` takes these views: bfloat16 rows of `a` that all heads share, weights [heads * N, K]."""
+    heads, n = out.shape[1], out.shape[2]
+    return (a.dtype == w.dtype == out.dtype == torch.bfloat16 and a.stride(1) == 1 and out.stride(2) == 1 and n_tokens > 64
+            and w.shape[0] == heads * n and w.is_contiguous()
+            and all(t.data_ptr() % 16 == 0 for t in (a, w, out))
+            and bool(library().bt_head_rows_tcgen05_supports(c_int(n_tokens), c_int(n), c_int(w.shape[1]), c_longlong(a.stride(0)),
+                                                             c_longlong(out.stride(0)), c_longlong(out.stride(1)))))
+
+
+def head_rows(a, w, out, *, n_tokens):
+    """out[t, h, :] = a[t] @ w[h * N .. (h + 1) * N]^T on the tcgen05 product: rows that all heads read (a [tokens, K], w
+    [heads * N, K], out a view [tokens, heads, N]; N a multiple of 32, see `head_rows_supports`)."""
+    heads, n = out.shape[1], out.shape[2]
+    k = w.shape[1]
+    if a.shape[1] != k or w.shape[0] != heads * n or min(a.shape[0], out.shape[0]) < n_tokens:
+        raise ShapeError(f"head_rows: {n_tokens} rows of a{list(a.shape)}, w{list(w.shape)} and out{list(out.shape)} do not fit")
+    _linear_work(n_tokens, heads * n, k, a, w, out)
+    _check(library().bt_head_rows_tcgen05(_ptr(a), c_longlong(a.stride(0)), _ptr(w), _ptr(out), c_longlong(out.stride(0)),
+                                          c_longlong(out.stride(1)), _ptr(kernel_status(a.device)), c_int(n_tokens), c_int(heads),
+                                          c_int(n), c_int(k), _stream()))
+
+
 def latent_attention_scratch_floats(n_tokens, n_heads, rank, n_splits) -> int:
     return int(library().bt_latent_attention_scratch_floats(c_int(n_tokens), c_int(n_heads), c_int(rank), c_int(n_splits)))
 

@@ -201,9 +201,15 @@ class LatentAttention(Mixer):
             mixed_heads = mixed.view(n, heads, self.vdim)
             if kernels.sink_attention_supports(q_heads, keys, values, gate, mixed_heads):
                 kernels.latent_gather(pool, ctx.positions, ctx.token_seq, table, group.table_len, rows, n_tokens=n)
-                latent = rows[:, :rank].unsqueeze(1).expand(n, heads, rank)
-                kernels.head_linear(latent, self.uk_heads_t, keys[:, :, :self.dim], n_tokens=n)
-                kernels.head_linear(latent, self.uv_heads, values, n_tokens=n)
+                # (all heads read the same latents: one product of all heads' weights, its columns filed head by head.  2,048
+                # tokens of rank 512 to 16 heads of 64: 20 and 18 us as a product a head on mma.sync, about 8 each so)
+                latent = rows[:, :rank]
+                for weight, by_head, made in ((self.t_uk_weight, self.uk_heads_t, keys[:, :, :self.dim]),
+                                              (self.t_uv_weight, self.uv_heads, values)):
+                    if kernels.head_rows_supports(latent, weight, made, n):
+                        kernels.head_rows(latent, weight, made, n_tokens=n)
+                    else:
+                        kernels.head_linear(latent.unsqueeze(1).expand(n, heads, rank), by_head, made, n_tokens=n)
                 if rot:
                     shared = rows[:, rank:].unsqueeze(1).expand(n, heads, rot)
                     kernels.rotary_interleaved(shared, keys[:, :, self.dim:], ctx.positions, freq, n_tokens=n, dims=0)
