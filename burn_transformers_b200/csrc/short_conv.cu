@@ -55,6 +55,61 @@ short_conv_kernel(const TIn* __restrict__ src, long long src_row_stride, const f
   }
 }
 
+// The same for steps of long runs: a thread a channel over SC_RUN tokens, its weights and the taps' inputs in registers, the
+// run's inputs all asked for before the first is used.  (A thread a number looked its sequence up, divided, and read every
+// tap's weight and input again: 2,440 tokens of 1,536 channels took 34 us in a recorded layer, 15 so.)
+constexpr int SC_RUN = 16;
+template <typename TIn, typename TOut, int TAPS>
+__global__ void __launch_bounds__(256)
+short_conv_run_kernel(const TIn* __restrict__ src, long long src_row_stride, const float* __restrict__ w,
+                      const float* __restrict__ bias, const float* __restrict__ state, const int* __restrict__ slots,
+                      const int* __restrict__ seq_start, const int* __restrict__ token_seq, TOut* __restrict__ out,
+                      long long out_row_stride, long long n_tokens, int channels, int act) {
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  const long long t0 = (long long)blockIdx.y * SC_RUN;
+  const bool owns = c < channels;
+  float wt[TAPS], before[TAPS > 1 ? TAPS - 1 : 1] = {};
+  pdl_trigger();
+#pragma unroll
+  for (int j = 0; j < TAPS; ++j) wt[j] = owns ? w[(long long)c * TAPS + j] : 0.f;
+  const float shift = owns && bias ? bias[c] : 0.f;
+  pdl_wait();
+  if (!owns) return;
+  const int n = (int)min((long long)SC_RUN, n_tokens - t0);
+  float u[SC_RUN];
+  int of[SC_RUN];
+#pragma unroll
+  for (int k = 0; k < SC_RUN; ++k) {
+    u[k] = k < n ? to_float(src[(t0 + k) * src_row_stride + c]) : 0.f;
+    of[k] = k < n ? token_seq[t0 + k] : 0;
+  }
+  int seq = -1;
+#pragma unroll
+  for (int k = 0; k < SC_RUN; ++k) {
+    if (k >= n) break;
+    const long long t = t0 + k;
+    if (of[k] != seq) {                    // (the run's first token, or a sequence's: the inputs before it)
+      seq = of[k];
+      const int r = (int)(t - seq_start[seq]);
+      const float* state_row = state + (long long)slots[seq] * (TAPS - 1) * channels + c;
+#pragma unroll
+      for (int j = 0; j < TAPS - 1; ++j) {
+        const int d = TAPS - 1 - j, idx = r - d;
+        before[j] = idx >= 0 ? to_float(src[(t - d) * src_row_stride + c]) : state_row[(long long)(TAPS - 1 + idx) * channels];
+      }
+    }
+    float y = shift;
+#pragma unroll
+    for (int j = 0; j < TAPS - 1; ++j) y = fmaf(wt[j], before[j], y);
+    y = fmaf(wt[TAPS - 1], u[k], y);
+#pragma unroll
+    for (int j = 0; j + 1 < TAPS - 1; ++j) before[j] = before[j + 1];
+    if (TAPS > 1) before[TAPS > 1 ? TAPS - 2 : 0] = u[k];
+    if (act == 1) y = sc_silu(y);
+    out[t * out_row_stride + c] = from_float<TOut>(y);
+  }
+}
+
 template <typename TIn, typename TOut, int NV>
 __global__ void __launch_bounds__(128)
 short_conv_norm_kernel(const TIn* __restrict__ src, long long src_row_stride, const float* __restrict__ w,
@@ -147,6 +202,19 @@ static int launch_short_conv(const T* src, long long src_row_stride, const float
       if (group <= 64) BT_SCN(__nv_bfloat16, 2); else if (group <= 128) BT_SCN(__nv_bfloat16, 4); else BT_SCN(__nv_bfloat16, 8);
     }
 #undef BT_SCN
+  } else if (taps >= 2 && taps <= 4 && n_tokens > 4ll * n_seqs && (n_tokens + SC_RUN - 1) / SC_RUN <= 65535) {
+    // (runs of a few tokens would read the taps' inputs once a token all the same, one token after the other)
+    const dim3 grid((channels + 255) / 256, (unsigned)((n_tokens + SC_RUN - 1) / SC_RUN));
+#define BT_SCR(TOUT, TAPS)                                                                                             \
+  BT_PDL_OK("short_conv", launch_pdl(short_conv_run_kernel<T, TOUT, TAPS>, grid, dim3(256), 0, stream, 1, src, src_row_stride, w, \
+                                     bias, (const float*)state, slots, seq_start, token_seq, (TOUT*)out, out_row_stride, \
+                                     n_tokens, channels, act))
+    if (out_dtype == kF32) {
+      if (taps == 2) BT_SCR(float, 2); else if (taps == 3) BT_SCR(float, 3); else BT_SCR(float, 4);
+    } else {
+      if (taps == 2) BT_SCR(__nv_bfloat16, 2); else if (taps == 3) BT_SCR(__nv_bfloat16, 3); else BT_SCR(__nv_bfloat16, 4);
+    }
+#undef BT_SCR
   } else {
     const dim3 grid(sc_blocks(n_tokens * channels));
     if (out_dtype == kF32)
