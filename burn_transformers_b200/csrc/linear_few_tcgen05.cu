@@ -62,7 +62,7 @@ linear_few_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
   pdl_trigger();     // the next kernel may set itself up (and fetch its weights) while this one runs
   cg::cluster_group cluster = cg::this_cluster();
   const int split = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);      // (uniform for the compiler too)
   const int n0 = blockIdx.y * TF_BN;
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<unsigned long long>(tf_smem_raw) + 1023ull) & ~1023ull);
   const unsigned x_bytes = (unsigned)p.rows16 * TC_BK * 2, stage_bytes = TF_W_BYTES + x_bytes;     // [stage][W 16 KB | X]
@@ -101,7 +101,7 @@ linear_few_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
   for (int e = 0; e < 8; ++e) my_bias[e] = (p.bias && my_col + e < p.N) ? __ldg(p.bias + my_col + e) : 0.f;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc_elect()) {
       // ---- producer: the ring's boxes of W first, then the wait for the predecessor, then the rows ----
       const int early = min(k_blocks, stages);
       for (int kb = 0; kb < early; ++kb) {
@@ -123,26 +123,31 @@ linear_few_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---- issuer.  Instruction descriptor: 32-bit accumulator, bfloat16 operands, both K-major, N = rows16, M = 128
-      const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(p.rows16 >> 3) << 17) | ((unsigned)(TF_BN >> 4) << 24);
-      bool ok = true;
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        const int s = kb % stages;
-        if (!tc_bar_wait(&full[s], (kb / stages) & 1)) {
-          failed = 1;
-          ok = false;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    // ---- issuer: the warp walks the ring, an elected lane issues (see linear_tcgen05.cu).  Instruction descriptor: 32-bit
+    // accumulator, bfloat16 operands, both K-major, N = rows16, M = 128
+    const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(p.rows16 >> 3) << 17) | ((unsigned)(TF_BN >> 4) << 24);
+    int s = 0;
+    unsigned parity = 0;
+    for (int kb = 0; kb < k_blocks; ++kb) {
+      if (!__all_sync(0xffffffffu, tc_bar_wait(&full[s], parity))) {      // (a wait that runs out must not part the lanes)
+        failed = 1;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      if (tc_elect()) {
         unsigned char* w_tile = tiles + (size_t)s * stage_bytes;
         const unsigned long long dw = tc_desc(w_tile), dx = tc_desc(w_tile + TF_W_BYTES);
 #pragma unroll
         for (int k = 0; k < TC_BK / 16; ++k)     // 16 bfloat16 = 32 bytes further along the row: +2 in 16-byte units
           tc_mma(tmem_acc, dw + 2ull * k, dx + 2ull * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
         tc_commit(&empty[s]);                    // arrives when these products have read the stage
+        if (kb + 1 == k_blocks) tc_commit(&acc_full);          // and, behind the last ones, when every product has finished
       }
-      if (ok && k_blocks > 0) tc_commit(&acc_full);          // arrives when every product has finished
+      __syncwarp();
+      if (++s == stages) {
+        s = 0;
+        parity ^= 1u;
+      }
     }
   } else {
     // ---- the accumulator leaves tensor memory: warp w reaches lanes 32 (w % 4) .. + 31, the block's columns of that
