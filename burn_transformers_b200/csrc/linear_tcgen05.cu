@@ -43,6 +43,7 @@ struct TcParams {
   // head_cols > 0 (bfloat16 results only): column c of row r goes to out[(c / head_cols) * head_stride + r * out_row + c % head_cols]
   int head_cols;
   long long out_row, head_stride;
+  int band;                 // tiles of rows that go over all columns before the next rows are begun (at least 1)
 };
 
 
@@ -71,6 +72,13 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const int tiles_m = (p.M + BM - 1) / BM, tiles_n = (p.N + BN - 1) / BN;
   const int n_tiles = tiles_m * tiles_n;
   const int k_blocks = (p.K + TC_BK - 1) / TC_BK;
+  // Where a tile lies: bands of `band` tiles of rows, a band's rows first, then its columns (the band's A comes from L2 then)
+  auto place = [&](int tile, int& tm, int& tn) {
+    const int b = tile / (p.band * tiles_n), first = b * p.band, in_band = tile - first * tiles_n;
+    const int rows = min(p.band, tiles_m - first);
+    tn = in_band / rows;
+    tm = first + in_band - tn * rows;
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -115,7 +123,9 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         else tc_tma_load(dst, weights ? &map_w : &map_a, kb * TC_BK, row, &full[s]);
       };
       {
-        const int m0 = (tile0 % tiles_m) * BM + rank * TC_BM, n0 = (tile0 / tiles_m) * BN + rank * W_ROWS;
+        int tm = 0, tn = 0;
+        place(tile0, tm, tn);
+        const int m0 = tm * BM + rank * TC_BM, n0 = tn * BN + rank * W_ROWS;
         for (int kb = 0; kb < pre; ++kb) {
           expect(kb);
           load(kb, true, kb, n0);
@@ -127,7 +137,9 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       int kb = pre, s = pre == STAGES ? 0 : pre;
       unsigned parity = pre == STAGES ? 0u : 1u;      // (of the round before: a fresh barrier's is complete)
       for (int tile = tile0; tile < n_tiles; tile += tile_step, kb = 0) {
-        const int m0 = (tile % tiles_m) * BM + rank * TC_BM, n0 = (tile / tiles_m) * BN + rank * W_ROWS;
+        int tm, tn;
+        place(tile, tm, tn);
+        const int m0 = tm * BM + rank * TC_BM, n0 = tn * BN + rank * W_ROWS;
         for (; kb < k_blocks; ++kb) {
           if (!tc_bar_wait(&empty[s], parity)) {
             failed = 1;
@@ -207,7 +219,9 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     int local = 0;
     for (int tile = tile0; tile < n_tiles; tile += tile_step, ++local) {
       const int buf = local & 1;
-      const int m0 = (tile % tiles_m) * BM + rank * TC_BM, n0 = (tile / tiles_m) * BN;
+      int tm, tn;
+      place(tile, tm, tn);
+      const int m0 = tm * BM + rank * TC_BM, n0 = tn * BN;
       const bool ok = tc_bar_wait(&acc_full[buf], (local >> 1) & 1);
       if (!ok) {
         failed = 1;
@@ -359,6 +373,7 @@ struct TcTile {
   bool pair;
   int once_ns, k_block_ns;
 };
+constexpr long long TC_BAND = 16ll << 20;
 constexpr TcTile TC_TILES[] = {{256, false, 8900, 296}, {192, false, 7600, 265}, {128, false, 6400, 245}, {96, false, 5800, 250},
                                {64, false, 5200, 233}, {256, true, 9400, 294}, {224, true, 8900, 260}, {192, true, 8400, 217},
                                {160, true, 7900, 196}, {128, true, 7400, 170}, {96, true, 6900, 167}, {64, true, 6400, 163}};
@@ -414,6 +429,12 @@ static int run_linear_tcgen05(const void* a, long long a_row, const void* w, bt:
       pair = t.pair;
     }
   }
+  // Tiles of rows whose A is at most TC_BAND bytes go over all columns before the next rows are begun: with all rows first,
+  // an A beyond L2 (or in L2 beside a residual that streams through it) came from memory again for every tile of columns.
+  // GPT-2 XL's layer at 16 x 1,024 tokens 1,270 to 1,176 us with bands of 16 MB, about 1,200 with 40; no sum changes.
+  const long long tile_rows = pair ? 2 * TC_BM : TC_BM, tiles_m = (M + tile_rows - 1) / tile_rows;
+  const long long band = TC_BAND / (tile_rows * K * 2);
+  p.band = (int)(band < 1 ? 1 : (band < tiles_m ? band : tiles_m));
   CUtensorMap ma, mw;
   if (int rc = tensor_map_2d_bf16(&ma, a, (unsigned long long)M, (unsigned long long)K, (unsigned long long)a_row, TC_BM)) return rc;
   if (int rc = tensor_map_2d_bf16(&mw, w, (unsigned long long)N, (unsigned long long)K, (unsigned long long)K, (unsigned)(pair ? bn / 2 : bn))) return rc;
