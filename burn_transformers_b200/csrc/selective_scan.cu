@@ -13,9 +13,11 @@
 // sequence's last from a zero state and leaves, per channel, what it ends with, E[n], and the sum of its step sizes, d;
 // the state after the piece is then exp(A[n] d) * (state before it) + E[n], since the recurrence is linear in the state
 // and its decays multiply to exp(A[n] * sum dt).  The second launch gives every piece its own block, which first walks
-// the earlier pieces' (E, d) from the sequence's stored state to its own start and then runs its tokens as the single
+// the earlier pieces' (E, d) from the state before the run to its own start and then runs its tokens as the single
 // run would; the last piece writes the state back.  `ends`: [pieces of the step][channels][n_state + 1], where the
-// pieces of sequence s begin at first_row(s) / piece + s.
+// pieces of sequence s begin at first_row(s) / piece + s.  Nothing orders the second launch's blocks, so none of them may
+// read what another one writes: the first launch copies the stored state into the cell of the sequence's last piece (which
+// leaves no ends), and all pieces start from that copy.
 #include "common.cuh"
 
 namespace bt {
@@ -124,8 +126,15 @@ selective_scan_kernel(const T* __restrict__ x, long long x_row_stride, const T* 
   float* e_base = piece > 0 ? ends + ((long long)(first / piece + seq)) * es + (long long)(owns ? c : 0) * (n_state + 1) : nullptr;
   float* s_base = state + ((long long)slots[seq] * channels + (owns ? c : 0)) * n_state;
   float dt_sum = 0.f;
+  // the state before the run: where it is stored if this block alone reads and writes it, else its copy
+  float* before = n_pieces > 1 ? e_base + (long long)(n_pieces - 1) * es : s_base;
+  if (ENDS && owns && my_piece == 0) {
 #pragma unroll
-  for (int i = 0; i < NS; ++i) s[i] = !ENDS && owns && n0 + i < n_state ? s_base[n0 + i] : 0.f;
+    for (int i = 0; i < NS; ++i)
+      if (n0 + i < n_state) before[n0 + i] = s_base[n0 + i];
+  }
+#pragma unroll
+  for (int i = 0; i < NS; ++i) s[i] = !ENDS && owns && n0 + i < n_state ? before[n0 + i] : 0.f;
   if (!ENDS && owns) {
 #pragma unroll 4
     for (int j = 0; j < my_piece; ++j) {      // (several pieces' numbers are asked for at once)
