@@ -208,12 +208,8 @@ static int launch_pf(const void* q, long long q_row_stride, const KvView& view, 
   auto kern = attention_prefill_simt_kernel<T, G, VEC>;
   constexpr size_t most = sizeof(float) * ((size_t)(PF_BQ + 2 * PF_BK) * (64 * G + 4) + (size_t)PF_BQ * (PF_BK + 4));
   const size_t smem = sizeof(float) * ((size_t)(PF_BQ + 2 * PF_BK) * pf_stride(head_dim) + (size_t)PF_BQ * (PF_BK + 4));
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-    BT_CHECK(e == cudaSuccess, "attention_prefill_simt: cannot reserve %zu bytes of shared memory", most);
-    configured = true;
-  }
+  static SharedMemoryAllowance allowed;
+  BT_CHECK(allow_shared_memory(allowed, kern, most), "attention_prefill_simt: cannot reserve %zu bytes of shared memory", most);
   const dim3 grid((max_new + PF_BQ - 1) / PF_BQ, n_seqs, n_heads);
   kern<<<grid, PF_THREADS, smem, stream>>>((const T*)q, q_row_stride, view, (T*)out, seq_start, past_len, n_heads, n_kv_heads,
                                            head_dim, scale, causal, window);

@@ -961,12 +961,8 @@ static int launch_ts(const CUtensorMap& qm, const CUtensorMap& km, const CUtenso
                      cudaStream_t stream) {
   constexpr size_t smem = TsShape<HD, HV>::SMEM;
   auto kern = attention_prefill_softmax_kernel<HD, HV>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    BT_CHECK(e == cudaSuccess, "attention_prefill_tcgen05: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    configured = true;
-  }
+  static SharedMemoryAllowance allowed;
+  BT_CHECK(allow_shared_memory(allowed, kern, smem), "attention_prefill_tcgen05: cannot reserve %zu bytes of shared memory", smem);
   const int q_tiles = (max_new + TA_BQ - 1) / TA_BQ;
   BT_CHECK(q_tiles <= 65535, "attention_prefill_tcgen05: %d new tokens in one sequence are too many for one launch", max_new);
   dim3 grid(n_seqs * p.n_heads, q_tiles);
@@ -979,12 +975,8 @@ static int launch_ta(const CUtensorMap& qm, const CUtensorMap& km, const CUtenso
                      cudaStream_t stream) {
   constexpr size_t smem = ta_smem_bytes<HD, HV>();
   auto kern = sigmoid_attention_tcgen05_kernel<HD, HV>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    BT_CHECK(e == cudaSuccess, "attention_prefill_tcgen05: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    configured = true;
-  }
+  static SharedMemoryAllowance allowed;
+  BT_CHECK(allow_shared_memory(allowed, kern, smem), "attention_prefill_tcgen05: cannot reserve %zu bytes of shared memory", smem);
   const int q_tiles = (max_new + TA_BQ - 1) / TA_BQ;
   BT_CHECK(q_tiles <= 65535, "attention_prefill_tcgen05: %d new tokens in one sequence are too many for one launch", max_new);
   dim3 grid(n_seqs * p.n_heads, q_tiles);

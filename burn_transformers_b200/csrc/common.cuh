@@ -5,6 +5,8 @@
 #include <cstdint>
 #include <cstdio>
 
+#include "per_device.cuh"
+
 namespace bt {
 
 enum DType : int { kF32 = 0, kBF16 = 1 };
@@ -41,6 +43,16 @@ bool pdl_enabled();
 
 // Streaming multiprocessors of the current device (looked up once per device); 0 if it cannot be read.
 int sm_count();
+
+// Allows `kernel` that much dynamic shared memory on the current device; `kept`: the kernel's own (static) allowance.
+template <typename Kernel>
+inline bool allow_shared_memory(SharedMemoryAllowance& kept, Kernel* kernel, size_t bytes) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  return kept.allow(dev, bytes, [kernel](size_t n) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n) == cudaSuccess;
+  });
+}
 
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

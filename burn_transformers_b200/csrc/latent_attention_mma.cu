@@ -327,12 +327,9 @@ int launch_latent_attention_mma(const __nv_bfloat16* q, long long q_row_stride, 
 #define BT_LM_SIZED(RG, VW, VCT)                                                                                               \
   do {                                                                                                               \
     auto kernel = latent_attention_mma_kernel<RG, VW, VCT>;                                                              \
-    static size_t reserved = 0;   /* (the attribute is set again only when a call needs more than any before) */     \
-    if (smem > 48 * 1024 && smem > reserved) {                                                                       \
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
-      BT_CHECK(e == cudaSuccess, "latent_attention: cannot reserve %zu bytes of shared memory", smem);               \
-      reserved = smem;                                                                                               \
-    }                                                                                                                \
+    static SharedMemoryAllowance allowed;                                                                            \
+    if (smem > 48 * 1024)                                                                                            \
+      BT_CHECK(allow_shared_memory(allowed, kernel, smem), "latent_attention: cannot reserve %zu bytes of shared memory", smem); \
     BT_PDL_OK("latent_attention_mma",                                                                                \
               launch_pdl(kernel, grid, block, smem, stream, 1, q, q_row_stride, pool, table, table_stride, table_len, \
                          page_size, seq_start, past_len, sink, out, out_row_stride, part, n_heads, hb, tq, head_tiles, \

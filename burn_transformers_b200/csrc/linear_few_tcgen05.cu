@@ -322,13 +322,9 @@ extern "C" int bt_linear_few_tcgen05(const void* x, const void* w, const float* 
   if (int rc = tensor_map_2d_bf16(&mw, w, (unsigned long long)N, (unsigned long long)K, (unsigned long long)K, TF_BN)) return rc;
   const int tmem_cols = rows16 <= 32 ? 32 : (rows16 <= 64 ? 64 : 128);
   FewParams p{bias, residual, out, status, M, N, K, per * TC_BK, act, out_is_f32, rows16, stages, tmem_cols};
-  static bool configured = false;
-  if (!configured) {
-    const size_t most = TF_RING_BUDGET + 1024;
-    cudaError_t e = cudaFuncSetAttribute(linear_few_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-    BT_CHECK(e == cudaSuccess, "linear_few_tcgen05: cannot reserve %zu bytes of shared memory: %s", most, cudaGetErrorString(e));
-    configured = true;
-  }
+  constexpr size_t most = TF_RING_BUDGET + 1024;
+  static SharedMemoryAllowance allowed;
+  BT_CHECK(allow_shared_memory(allowed, linear_few_tcgen05_kernel, most), "linear_few_tcgen05: cannot reserve %zu bytes of shared memory", most);
   BT_PDL_OK("linear_few_tcgen05", launch_pdl(linear_few_tcgen05_kernel, dim3(split, n_tiles), dim3(TF_THREADS), smem, stream, split, mx, mw, p));
   return 0;
 }

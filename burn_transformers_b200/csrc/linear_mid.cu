@@ -273,14 +273,10 @@ extern "C" int bt_linear_mid(const void* a, const void* w, const float* bias, co
   BT_CHECK(n_tiles <= 65535, "linear_mid: N=%d needs too many column tiles", N);
   auto launch = [&](auto kernel, int bn_) -> int {
     const size_t smem = (size_t)lm_stages(bn_) * (LM_A_BYTES + bn_ * LM_BK * 2) + 1024 + (split > 1 ? (size_t)LM_BM * bn_ * 4 : 0);
-    static bool configured[3] = {false, false, false};
-    const int which = bn_ == 64 ? 2 : (bn_ == 32 ? 1 : 0);
-    if (!configured[which]) {
-      const size_t most = (size_t)lm_stages(bn_) * (LM_A_BYTES + bn_ * LM_BK * 2) + 1024 + (size_t)LM_BM * bn_ * 4;
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-      BT_CHECK(e == cudaSuccess, "linear_mid: cannot reserve %zu bytes of shared memory: %s", most, cudaGetErrorString(e));
-      configured[which] = true;
-    }
+    const size_t most = (size_t)lm_stages(bn_) * (LM_A_BYTES + bn_ * LM_BK * 2) + 1024 + (size_t)LM_BM * bn_ * 4;
+    static SharedMemoryAllowance allowed[3];      // (the three kernels are of one type: one by one)
+    BT_CHECK(allow_shared_memory(allowed[bn_ == 64 ? 2 : (bn_ == 32 ? 1 : 0)], kernel, most),
+             "linear_mid: cannot reserve %zu bytes of shared memory", most);
     BT_PDL_OK("linear_mid", launch_pdl(kernel, dim3(split, n_tiles), dim3(LM_THREADS), smem, stream, split, ma, mw, p));
     return 0;
   };

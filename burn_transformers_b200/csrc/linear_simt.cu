@@ -286,12 +286,8 @@ static int launch_fma(const float* A, const float* W, const float* bias, const f
                       int K, int act, int rows16, cudaStream_t stream) {
   using Tile = FmaTile<BM, BN, STAGES, W_IS_NK>;
   auto kern = linear_fma_kernel<BM, BN, TM, TN, STAGES, W_IS_NK>;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile::SMEM);
-    BT_CHECK(e == cudaSuccess, "linear: cannot reserve %zu bytes of shared memory: %s", Tile::SMEM, cudaGetErrorString(e));
-    configured = true;
-  }
+  static SharedMemoryAllowance allowed;
+  BT_CHECK(allow_shared_memory(allowed, kern, Tile::SMEM), "linear: cannot reserve %zu bytes of shared memory", Tile::SMEM);
   const int tiles_n = (N + BN - 1) / BN;
   const dim3 grid((unsigned)((long long)tiles_n * ((M + BM - 1) / BM)));
   kern<<<grid, FMA_THREADS, Tile::SMEM, stream>>>(A, W, bias, residual, out, M, N, K, act, tiles_n, rows16);

@@ -383,12 +383,8 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mw, const TcParam
   constexpr size_t smem = (size_t)STAGES * (TC_BM * TC_BK * 2 + (PAIR ? BN / 2 : BN) * TC_BK * 2) + 1024 + (size_t)TC_EPI_WARPS * 32 * TC_PATCH_STRIDE * 4;
   static_assert(smem <= 227 * 1024, "a multiprocessor's shared memory");
   auto kern = linear_tcgen05_kernel<BN, STAGES, PAIR>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    BT_CHECK(e == cudaSuccess, "linear_tcgen05: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    configured = true;
-  }
+  static SharedMemoryAllowance allowed;
+  BT_CHECK(allow_shared_memory(allowed, kern, smem), "linear_tcgen05: cannot reserve %zu bytes of shared memory", smem);
   constexpr int GROUP = PAIR ? 2 : 1;
   const int n_tiles = ((p.N + BN - 1) / BN) * ((p.M + GROUP * TC_BM - 1) / (GROUP * TC_BM));
   const int groups = sm_count() / GROUP;

@@ -292,12 +292,9 @@ extern "C" int bt_sink_attention(const void* q, long long q_row, int q_head, con
 #define BT_SA_KIND(VCT, SIGMOID)                                                                                  \
   do {                                                                                                            \
     auto kernel = sink_attention_mma_kernel<VCT, SIGMOID>;                                                        \
-    static size_t reserved = 0;                                                                                   \
-    if (smem > 48 * 1024 && smem > reserved) {                                                                    \
-      BT_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess, \
-               "sink_attention: cannot reserve %zu bytes of shared memory", smem);                                \
-      reserved = smem;                                                                                            \
-    }                                                                                                             \
+    static SharedMemoryAllowance allowed;                                                                         \
+    if (smem > 48 * 1024)                                                                                         \
+      BT_CHECK(allow_shared_memory(allowed, kernel, smem), "sink_attention: cannot reserve %zu bytes of shared memory", smem); \
     BT_PDL_OK("sink_attention", launch_pdl(kernel, grid, block, smem, stream, 1, p));                             \
   } while (0)
   if (dvp <= 32) BT_SA(32);
