@@ -154,7 +154,7 @@ linear_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     bool ok = true;
     for (int kb = 0; kb < my_blocks && ok; ++kb) {
       const int s = kb % LM_STAGES;
-      if (!lm_wait(&full[s], (kb / LM_STAGES) & 1)) {
+      if (!__all_sync(0xffffffffu, lm_wait(&full[s], (kb / LM_STAGES) & 1))) {      // (what follows is collective)
         ok = false;
         break;
       }

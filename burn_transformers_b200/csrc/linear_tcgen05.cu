@@ -222,8 +222,7 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       int tm, tn;
       place(tile, tm, tn);
       const int m0 = tm * BM + rank * TC_BM, n0 = tn * BN;
-      const bool ok = tc_bar_wait(&acc_full[buf], (local >> 1) & 1);
-      if (!ok) {
+      if (!__all_sync(0xffffffffu, tc_bar_wait(&acc_full[buf], (local >> 1) & 1))) {      // (what follows is collective)
         failed = 1;
         break;
       }
