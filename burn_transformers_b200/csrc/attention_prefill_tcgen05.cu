@@ -506,6 +506,7 @@ sigmoid_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
   }
   ta_fence_before();
   __syncthreads();
+  if (*failed) let_copies_land();
   if (warp == TA_SOFTMAX_WARPS + 1) {
     ta_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_s), "r"(TA_TMEM_COLS) : "memory");
@@ -947,8 +948,7 @@ attention_prefill_softmax_kernel(const __grid_constant__ CUtensorMap q_map, cons
   }
   ta_fence_before();
   __syncthreads();
-  if (*failed)         // (a wait ran out: copies and products may still be in flight, and must not land after the block has gone)
-    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+  if (*failed) let_copies_land();
   if (warp == TS_SOFTMAX_WARPS + 1) {
     ta_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_s), "r"(Shape::COLS) : "memory");

@@ -38,6 +38,12 @@ void count_launch();
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// For a block that gives up on a wait: its copies (and products) may still be in flight and must not land in memory that it
+// uses for something else, or has left.  About a millisecond, far longer than a copy takes.
+__device__ __forceinline__ void let_copies_land() {
+  for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+}
+
 // BT_NO_PDL=1 in the environment launches every kernel fully serialised (for measurements).
 bool pdl_enabled();
 

@@ -158,6 +158,7 @@ linear_few_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
       ok = __all_sync(0xffffffffu, tc_bar_wait(&acc_full, 0));      // (the reads below are collective)
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     }
+    if (!ok) let_copies_land();      // (the tile of sums goes over the ring)
 #pragma unroll 1
     for (int m0 = 32 * half; m0 < p.rows16; m0 += 64) {
       float v[32];
@@ -252,6 +253,7 @@ linear_few_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
   if (split > 1) cluster.sync();    // nobody leaves while a peer may still read its partial tile
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
+  if (failed) let_copies_land();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_acc), "r"(p.tmem_cols) : "memory");

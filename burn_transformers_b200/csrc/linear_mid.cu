@@ -227,6 +227,7 @@ linear_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     cluster.sync();    // nobody leaves while a peer may still read its partial tile
   }
   __syncthreads();
+  if (failed) let_copies_land();
   if (tid == 0 && failed && p.status) atomicExch(p.status, 5);
 }
 

@@ -351,8 +351,7 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
-  if (failed)          // (a wait ran out: copies may still be in flight, and must not land after the block has gone)
-    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+  if (failed) let_copies_land();
   if constexpr (PAIR) tc_cluster_sync();      // neither block's memory or barriers are touched by the other from here on
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");

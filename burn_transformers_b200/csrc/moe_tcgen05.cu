@@ -265,8 +265,7 @@ moe_expert_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
-  if (failed)          // (a wait ran out: copies may still be in flight, and must not land after the block has gone)
-    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+  if (failed) let_copies_land();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_acc), "r"(2 * ME_BN) : "memory");

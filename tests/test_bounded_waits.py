@@ -1,5 +1,5 @@
 """Waits that run out, read from the sources (no GPU is made to wait for something that never comes): lanes of a warp that works
-together give up together."""
+together give up together, and a block stays until the copies it asked for must have landed."""
 import re
 from pathlib import Path
 
@@ -34,3 +34,12 @@ def test_a_warp_gives_up_as_a_whole(name):
         jumps = any(word in " ".join(lines[at:at + 5]) for word in ("break;", "return false;"))
         if leaves and jumps and "__all_sync" not in line:
             assert any(one in header for header in branches(lines, at) for one in ONE_LANE), f"{name}:{at + 1}: {line.strip()}"
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_a_block_that_gives_up_stays_for_its_copies(name):
+    for kernel in (CSRC / name).read_text().split("__global__")[1:]:
+        kernel = kernel.split("\n}\n")[0]
+        if WAIT.search(kernel):
+            after = kernel[max(m.end() for m in WAIT.finditer(kernel)):]
+            assert re.search(r"__syncthreads\(\);\s+if \(\*?failed\) let_copies_land\(\);", after), name
