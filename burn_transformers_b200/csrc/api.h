@@ -132,6 +132,7 @@ int bt_latent_decode_prep(const void* proj, long long row_stride, int q_off, int
 int bt_latent_decode_finish(const float* part, const void* mixed_latent, int n_splits, const void* uv, const void* gate,
                             long long gate_row_stride, int gate_per_head, void* out, long long out_row_stride, int n_tokens, int n_heads,
                             int rank, int vdim, int dtype, cudaStream_t stream);
+int bt_latent_attention_ns(int rank, int rot, int n_heads, int n_seqs, int max_new, int n_tokens, int span, int n_splits);
 int bt_latent_attention_rows(int rank, int rot, int dtype, int tensor_cores);
 int bt_lightning_scan(const void* proj, long long row_stride, int q_off, int k_off, int v_off, float* state,
                       const int* slots, const int* seq_start, const float* decay, float* out, long long out_row_stride,

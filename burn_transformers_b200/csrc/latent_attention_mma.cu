@@ -299,6 +299,45 @@ static int lm_value_warps(int rank, int rot) {
 }
 
 int latent_attention_mma_rows() { return LM_BM; }
+
+static size_t lm_block_smem(int rank, int rot, int rg) {
+  const int ld = ((rank + rot + 15) & ~15) + LM_PAD;
+  return (size_t)(16 * rg + 2 * LM_KT) * ld * 2 + rg * 16 * LM_PLD * 2 + 2 * rg * lm_value_warps(rank, rot) * 16 * sizeof(float);
+}
+// One token of few heads fills a quarter of the larger block at most; while every block has a multiprocessor to itself the
+// larger one is ahead all the same, as all its warps copy (8 sequences of 13 runs: 9.8 against 12.6 us; 18: 17.9 against 14.2;
+// 64 of 4: 37.7 against 25.3)
+static int lm_row_groups(int n_seqs, int max_new, int n_heads, int n_splits) {
+  return (long long)max_new * n_heads <= 16 && (long long)n_seqs * n_splits > sm_count() ? 1 : 4;
+}
+
+// What a call is expected to take, in ns, for the caller that chooses how many runs the keys are cut into (0: no shape of
+// this kernel, or no device).  A tile of 32 keys costs `wave` a round of blocks and `load` a block of a multiprocessor, a round
+// costs `round`, and the join of runs `join` and `number` for a million partial results.  Fitted to 1,260 shapes (ranks 64 to 512, 1 to 290
+// sequences, contexts of 40 to 1,540): nine of ten estimates are within a third, and of two neighbouring numbers of runs the one
+// estimated lower was within 3 % of the faster in 94 of 100 shapes and slower by more than a tenth in 1.
+struct LmTime {
+  float once, wave, load, round, join, number;
+};
+constexpr LmTime LM_TIMES[2][4] = {      // blocks of 64 rows, of 16; ranks up to 64, 128, 256, 512
+    {{4240, 1060, 343, 0, 2810, 4780}, {5610, 1410, 616, 0, 2630, 4370}, {5880, 663, 1600, 0, 1630, 4200}, {3840, 3340, 0, 2650, 868, 4690}},
+    {{0, 1880, 35, 3770, 2820, 6960}, {0, 3790, 0, 4430, 2400, 6260}, {4760, 3010, 120, 0, 2340, 4420}, {6100, 2740, 721, 0, 0, 4850}}};
+
+extern "C" int bt_latent_attention_ns(int rank, int rot, int n_heads, int n_seqs, int max_new, int n_tokens, int span, int n_splits) {
+  const int vw = lm_value_warps(rank, rot), sms = sm_count();
+  if (vw == 0 || sms <= 0 || n_heads <= 0 || n_seqs <= 0 || max_new <= 0 || span <= 0 || n_splits <= 0) return 0;
+  const int rg = lm_row_groups(n_seqs, max_new, n_heads, n_splits), rows = 16 * rg;
+  const int hb = n_heads < rows ? n_heads : rows, tq = rows / hb;
+  const double blocks = (double)((n_heads + hb - 1) / hb) * ((max_new + tq - 1) / tq) * n_seqs * n_splits;
+  const int by_smem = (int)(228 * 1024 / (lm_block_smem(rank, rot, rg) + 1024)), by_threads = 16 / (rg * vw);      // (128 registers a thread)
+  const int places = sms * (by_smem < 1 || by_threads < 1 ? 1 : (by_smem < by_threads ? by_smem : by_threads));
+  const LmTime& t = LM_TIMES[rg == 1][rank <= 64 ? 0 : (rank <= 128 ? 1 : (rank <= 256 ? 2 : 3))];
+  const double tiles = (double)((((span + LM_KT - 1) / LM_KT) + n_splits - 1) / n_splits);
+  const double rounds = (double)((long long)((blocks + places - 1) / places)), load = blocks > sms ? blocks / sms : 1.0;
+  double ns = t.once + tiles * (t.wave * rounds + t.load * load) + t.round * rounds;
+  if (n_splits > 1) ns += t.join + t.number * 1e-6 * n_tokens * n_heads * rank * n_splits;
+  return ns < 2e9 ? (int)ns : 2000000000;
+}
 bool latent_attention_mma_supports(int rank, int rot) { return lm_value_warps(rank, rot) != 0; }
 
 int launch_latent_attention_mma(const __nv_bfloat16* q, long long q_row_stride, const __nv_bfloat16* pool, const int* table,
@@ -310,18 +349,14 @@ int launch_latent_attention_mma(const __nv_bfloat16* q, long long q_row_stride, 
   BT_CHECK(vw != 0, "latent_attention: rank %d, rot %d is no shape of the tensor-core kernel", rank, rot);
   BT_CHECK(((unsigned long long)q % 16) == 0 && ((unsigned long long)pool % 16) == 0 && (q_row_stride % 8) == 0 &&
            ((unsigned long long)out % 4) == 0, "latent_attention: queries and cache rows must lie on 16-byte boundaries");
-  const int dk = rank + rot, dkp = (dk + 15) & ~15, ld = dkp + LM_PAD;
-  const int vc = rank / vw;
-  // one token of few heads fills a quarter of the larger block at most; while every block has a multiprocessor to itself
-  // the larger one is ahead all the same, as all its warps copy (8 sequences of 13 runs: 9.8 against 12.6 us; 18: 17.9
-  // against 14.2; 64 of 4: 37.7 against 25.3)
-  const int rg = (long long)max_new * n_heads <= 16 && (long long)n_seqs * n_splits > sm_count() ? 1 : 4;
+  const int dk = rank + rot, vc = rank / vw;
+  const int rg = lm_row_groups(n_seqs, max_new, n_heads, n_splits);
   const int rows = 16 * rg;
   const int hb = n_heads < rows ? n_heads : rows;
   const int tq = rows / hb;
   const int head_tiles = (n_heads + hb - 1) / hb;
   const int token_tiles = (max_new + tq - 1) / tq;
-  const size_t smem = (size_t)(rows + 2 * LM_KT) * ld * 2 + rg * 16 * LM_PLD * 2 + 2 * rg * vw * 16 * sizeof(float);
+  const size_t smem = lm_block_smem(rank, rot, rg);
   BT_CHECK(smem <= 227 * 1024, "latent_attention: rank + rot = %d needs %zu bytes of shared memory", dk, smem);
   const dim3 grid(token_tiles * head_tiles, n_splits, n_seqs), block(32 * rg * vw);
 #define BT_LM_SIZED(RG, VW, VCT)                                                                                               \

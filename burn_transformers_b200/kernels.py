@@ -54,7 +54,7 @@ class KernelProfile:
 
     SKIP = ("bt_last_error", "bt_launch_count", "bt_abi_version", "bt_tensor_map", "bt_decode_flow_plan",
             "bt_decode_flow_phase_bytes", "bt_attention_decode_scratch_floats", "bt_latent_attention_scratch_floats",
-            "bt_latent_attention_rows", "bt_lightning_chunked_scratch_floats", "bt_sink_attention_supports",
+            "bt_latent_attention_rows", "bt_latent_attention_ns", "bt_lightning_chunked_scratch_floats", "bt_sink_attention_supports",
             "bt_mlstm_chunked_scratch_floats", "bt_moe_tile_rows", "bt_mlstm_scan_fuses", "bt_gla_scan_fuses")
 
     def __init__(self, context_hint: int | None = None):
@@ -744,6 +744,12 @@ def latent_attention_rows(rank, rot, dtype, tensor_cores=True) -> int:
     """Rows, (token, head) pairs, one block of the attention kernel holds for this shape."""
     return \
         int(library().bt_latent_attention_rows(c_int(rank), c_int(rot), c_int(_code(dtype)), c_int(1 if tensor_cores else 0)))
+
+
+def latent_attention_ns(rank, rot, n_heads, n_seqs, max_new, n_tokens, span, n_splits) -> int:
+    """What `latent_attention` on tensor cores is expected to take for these sizes (0: it does not take them); `span`: the keys
+    a row sees at most."""
+    return int(library().bt_latent_attention_ns(*map(c_int, (rank, rot, n_heads, n_seqs, max_new, n_tokens, span, n_splits))))
 
 
 def latent_attention(q, out, pool, table, table_len, seq_start, past_len, *, n_tokens, n_seqs, max_new, n_heads, rank,

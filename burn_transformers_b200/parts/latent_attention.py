@@ -114,13 +114,19 @@ class LatentAttention(Mixer):
         return CacheNeed(kv=KvSpec(1, self.latent_width, None, has_values=False))
 
     def _splits(self, ctx, rows_per_block: int) -> int:
-        """Runs the keys of a row tile are cut into: up to two blocks a multiprocessor, all of them at once, none when the
-        step's rows fill the GPU by themselves; at most one per 32 keys."""
+        """Runs the keys of a row tile are cut into: about two blocks a multiprocessor, none when the step's rows fill the GPU by
+        themselves; at most one per 32 keys.  Of the two numbers around two blocks the tensor-core kernel takes the one that
+        its sizes make the faster: cut once, 160 row tiles of rank 512 behind 100 keys take 87 us instead of 41, for the join of the
+        runs, and 160 of rank 128 behind 900 take 66 instead of 113."""
         hb = min(self.n_heads, rows_per_block)
         tiles = -(-self.n_heads // hb) * -(-ctx.max_new // max(1, rows_per_block // hb)) * ctx.n_seqs
-        by_fill = 2 * _sm_count(ctx.ws.device) // max(1, tiles)
+        blocks, tiles = 2 * _sm_count(ctx.ws.device), max(1, tiles)
         span = ctx.ctx_bound if self.window is None else min(ctx.ctx_bound, self.window + 64)
-        return int(max(1, min(by_fill, -(-span // 32), 64)))
+        more, fewer = (int(max(1, min(runs, -(-span // 32), 64))) for runs in (-(-blocks // tiles), blocks // tiles))
+        if more == fewer or ctx.dtype != torch.bfloat16:
+            return more
+        return min((more, fewer), key=lambda runs: kernels.latent_attention_ns(
+            self.kv_rank, self.rot_dim, self.n_heads, ctx.n_seqs, ctx.max_new, ctx.n_tokens, span, runs))
 
     # `forward(..., store=True)` writes the result into `residual` instead of adding it (rows that hold nothing yet)
     can_store = True
