@@ -219,6 +219,7 @@ int bt_moe_expert(int first, const void* a, long long a_row_stride, const void* 
                   const int* tile_first, const int* order, const float* pair_weight, int pairs, int E, int top, int K,
                   int N, int act, float limit, int tensor_cores, int dtype, cudaStream_t stream);
 int bt_moe_expert_tcgen05_supports(int pairs, int E, int K, int N);
+int bt_moe_many_rows_supports(int pairs, int E, int width, int inner, int gated);
 int bt_moe_gather(const void* x, long long x_row_stride, const int* order, int top, void* out, int pairs, int K, cudaStream_t stream);
 int bt_moe_expert_tcgen05(int mode, const void* a, const void* w, void* out, const int* offsets, const int* order,
                           const float* pair_weight, int* status, int pairs, int E, int K, int N, int act, float limit,

@@ -20,6 +20,7 @@
 // The products exist as 32-bit multiply-adds (float32, and every shape), on tensor cores (bfloat16, mma.sync m16n8k16
 // with 32-bit accumulators, K a multiple of 8) and, for steps with few rows an expert, as a kernel that streams the weights
 // into registers (bfloat16).  A row's result never depends on its neighbours in the tile.
+#include "api.h"
 #include "common.cuh"
 
 namespace bt {
@@ -625,6 +626,53 @@ extern "C" int bt_moe_route(const void* x, long long x_row_stride, const void* r
 
 extern "C" int bt_moe_tile_rows() { return bt::MS_BM; }
 
+// ---- which kernel takes the experts' products of bfloat16 rows --------------------------------------------------------
+// Steps of at most 16 rows an expert on average take the kernel that streams the weights into registers (`few`): ahead of the
+// version before it at every size that was measured.  Above, the fastest by an estimate decides, of `few`, the kernel that stages
+// both operands (`mma`) and the tcgen05 product behind a gather (moe_tcgen05.cu: both products, up to 256 experts), in us:
+//   half of `once` + K (k + min(blocks, 4 a multiprocessor) block_k + the blocks beyond more_k) + blocks likewise + E K N weight
+// with the row tiles that rows spread over the experts by chance make.  Fitted to 804 sizes of 2 to 512 experts from 64 x 32 to
+// 2,048 x 768 at 17 to 500 rows, weights beyond L2; nine of ten estimates are within 18 %, and of 100 sizes the choice is within
+// 2 % of the faster of the rules before (mma; few up to 48 rows, tcgen05 above) in 94, behind by more than a tenth in 2.  Both products,
+// few / mma / tcgen05: 16 experts of 512 x 1,024 at 17 rows 27 / 45 / 26, at 48 48 / 60 / 26; 64 experts of 256 x 512 at 48 73 / 38 /
+// 29; 512 of 64 x 128 at 32 93 / 24 / not taken; 4 of 128 x 256 at 48 10 / 11 / 17, at 100 not taken / 11 / 18.
+namespace bt {
+struct MoeTime {
+  float once, k, block, block_k, more, more_k, weight;
+};
+constexpr MoeTime MOE_FEW = {7.34f, 4.73e-4f, 8.88e-3f, 7.77e-6f, 1.38e-2f, 5.55e-6f, 1.56e-7f};
+constexpr MoeTime MOE_MMA = {6.88f, 8.72e-3f, 6.02e-3f, 3.75e-5f, 2.43e-3f, 2.00e-5f, 1.01e-7f};
+constexpr MoeTime MOE_TC = {14.8f, 2.86e-3f, 1.34e-2f, 2.52e-5f, 1.77e-2f, 1.80e-5f, 0.f};
+constexpr int MOE_FEW_ROWS = 16;
+}  // namespace bt
+
+// `tile`: rows of a tile; `spread`: up to that many rows an expert on average they lie in one tile as a rule
+static double moe_us(const bt::MoeTime& t, double pairs, double E, double K, double N, bool pair, double tile, double spread, int cols) {
+  const double tiles = E + (pairs > spread * E ? (pairs - spread * E) / tile : 0.0), blocks = tiles * ((int)(N + cols - 1) / cols);
+  const double full = 4.0 * bt::sm_count(), first = blocks < full ? blocks : full, more = blocks - first;
+  return 0.5 * t.once + K * (t.k + first * t.block_k + more * t.more_k) + first * t.block + more * t.more +
+         E * K * N * (pair ? 2 : 1) * t.weight;
+}
+static double moe_few_us(int pairs, int E, int K, int N, bool pair) { return moe_us(bt::MOE_FEW, pairs, E, K, N, pair, 24, 20, pair ? 16 : 32); }
+static double moe_mma_us(int pairs, int E, int K, int N, bool pair) { return moe_us(bt::MOE_MMA, pairs, E, K, N, pair, 24, 20, 64); }
+static double moe_tc_us(int pairs, int E, int K, int N, bool pair) { return moe_us(bt::MOE_TC, pairs, E, K, N, pair, 128, 64, pair ? 64 : 128); }
+static bool moe_takes_few(int pairs, int E, int K, int N, bool pair) {
+  return pairs <= (long long)bt::MOE_FEW_ROWS * E || moe_few_us(pairs, E, K, N, pair) <= moe_mma_us(pairs, E, K, N, pair);
+}
+
+// Whether the tcgen05 products (moe_tcgen05.cu) are the ones to take for a step's pairs: width -> inner -> width, `gated` with
+// pairs of `inner` columns in the first.
+extern "C" int bt_moe_many_rows_supports(int pairs, int E, int width, int inner, int gated) {
+  if (!bt_moe_expert_tcgen05_supports(pairs, E, width, inner) || !bt_moe_expert_tcgen05_supports(pairs, E, inner, width) ||
+      pairs <= (long long)bt::MOE_FEW_ROWS * E || bt::sm_count() <= 0)
+    return 0;
+  auto other = [&](int K, int N, bool pair) {
+    return moe_takes_few(pairs, E, K, N, pair) ? moe_few_us(pairs, E, K, N, pair) : moe_mma_us(pairs, E, K, N, pair);
+  };
+  return moe_tc_us(pairs, E, width, inner, gated != 0) + moe_tc_us(pairs, E, inner, width, false) <
+         other(width, inner, gated != 0) + other(inner, width, false);
+}
+
 extern "C" int bt_moe_sort(const int* ids, int total, int E, int* offsets, int* tile_first, int* order, int* place,
                            cudaStream_t stream) {
   using namespace bt;
@@ -655,11 +703,7 @@ extern "C" int bt_moe_expert(int first, const void* a, long long a_row_stride, c
   const dim3 grid((N + MS_BN - 1) / MS_BN, tiles);
   const bool pieces = dtype == kBF16 && K % 8 == 0 && a_row_stride % 8 == 0 && (unsigned long long)a % 16 == 0 &&
                       (unsigned long long)w % 16 == 0;
-  // few rows an expert (a decode step, a short prompt): up to 48 on average the kernel that streams its weights into
-  // registers is ahead of the one that stages both operands.  Measured for 16 experts of 512 x 1,024, the two products (us):
-  // 32 rows an expert 22 + 16 against 26 + 14, 50 rows 29 + 20 against 35 + 17, 75 rows 37 + 27 against 34 + 25; for 384 x
-  // 768 at 32 rows 15 + 13 against 18 + 13, 50 rows 22 + 15 against 21 + 13.
-  if (pieces && tensor_cores && pairs <= 48ll * E) {
+  if (pieces && tensor_cores && moe_takes_few(pairs, E, K, N, first == kMoeInPair)) {
     const int cols = first == kMoeInPair ? MF_W / 2 : MF_W;
     const dim3 few((N + cols - 1) / cols, tiles);
     if (first == kMoeInPair)

@@ -1054,10 +1054,12 @@ def moe_expert(first: bool, a, w, out, offsets, tile_first, order, pair_weight, 
                                    c_int(1 if tensor_cores else 0), c_int(_code(a.dtype)), _stream()))
 
 
-def moe_many_rows_supports(pairs, n_experts, k, n) -> bool:
-    """Whether `moe_expert_tcgen05` takes the product and is the one to take: bfloat16 steps with more rows an expert than
-    the kernel that streams the weights into registers is for (bt_moe_expert: 48 on average)."""
-    return pairs > 48 * n_experts and _supports("bt_moe_expert_tcgen05_supports", pairs, n_experts, k, n)
+def moe_many_rows_supports(x, w_in, w_out, *, pairs, gated=True) -> bool:
+    """Whether `moe_gather` and `moe_expert_tcgen05` take a step's products and are the ones to take (csrc/moe.cu has the rule):
+    bfloat16 rows `x` and weights w_in [experts, (2) inner, width], w_out [experts, width, inner]."""
+    experts, width, inner = w_out.shape
+    return (x.dtype == w_in.dtype == w_out.dtype == torch.bfloat16
+            and _supports("bt_moe_many_rows_supports", pairs, experts, width, inner, gated))
 
 
 def moe_gather(x, order, out, *, pairs, top):

@@ -155,8 +155,7 @@ class RoutedFeedForward(FeedForward):
         kernels.moe_sort(ids, offsets, tile_first, order, place, pairs=pairs, n_experts=routes)
         hidden = ctx.ws.take((pairs, self.inner), ctx.dtype)
         part = ctx.ws.take((pairs, self.width), torch.float32)
-        if (ctx.dtype == torch.bfloat16 and kernels.moe_many_rows_supports(pairs, self.n_experts, self.width, self.inner)
-                and kernels.moe_many_rows_supports(pairs, self.n_experts, self.inner, self.width)):
+        if kernels.moe_many_rows_supports(x, self.w_in, self.w_out, pairs=pairs, gated=self.gated):
             rows = ctx.ws.take((pairs, self.width), ctx.dtype)
             kernels.moe_gather(x, order, rows, pairs=pairs, top=top)
             kernels.moe_expert_tcgen05(True, rows, self.w_in, hidden, offsets, order, None, pairs=pairs,
