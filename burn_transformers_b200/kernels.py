@@ -1056,9 +1056,10 @@ def moe_expert(first: bool, a, w, out, offsets, tile_first, order, pair_weight, 
 
 def moe_many_rows_supports(x, w_in, w_out, *, pairs, gated=True) -> bool:
     """Whether `moe_gather` and `moe_expert_tcgen05` take a step's products and are the ones to take (csrc/moe.cu has the rule):
-    bfloat16 rows `x` and weights w_in [experts, (2) inner, width], w_out [experts, width, inner]."""
+    bfloat16 rows `x` and weights w_in [experts, (2) inner, width], w_out [experts, width, inner] on 16-byte boundaries."""
     experts, width, inner = w_out.shape
-    return (x.dtype == w_in.dtype == w_out.dtype == torch.bfloat16
+    return (x.dtype == w_in.dtype == w_out.dtype == torch.bfloat16 and x.stride(0) % 8 == 0
+            and all(t.data_ptr() % 16 == 0 for t in (x, w_in, w_out))
             and _supports("bt_moe_many_rows_supports", pairs, experts, width, inner, gated))
 
 

@@ -1,9 +1,12 @@
 """The routed experts' products below the tcgen05 products' sizes: more of K than a turn of the loop takes, rows that fill one row
-tile and two, each side of the kernels' rule."""
+tile and two, each side of the kernels' rule; and rows and weights that the tcgen05 products do not take."""
+import types
+
 import pytest
 import torch
 
 from burn_transformers_b200 import kernels
+from burn_transformers_b200.parts.routed import RoutedFeedForward
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -39,3 +42,26 @@ def test_products_of_few_rows(counts, width, inner, gated):
     want = torch.cat([hidden[of == e].double() @ w_out[e].double().t() for e in range(experts)]) * weights[order.long()].double()[:, None]
     # (exact products; the accumulator is cut to 24 bits once for 16 of them, the warps' eight sums are rounded)
     assert rel(part, want) < (inner / 16 + 10) * 2.0 ** -23
+
+
+def test_what_the_tcgen05_products_do_not_take_goes_on():
+    """Weights off a 16-byte boundary: as before there were tcgen05 products, another kernel takes them."""
+    width, inner, experts, tokens, top = 256, 128, 16, 2048, 2
+    gen = torch.Generator(device=DEV).manual_seed(4)
+    flat = lambda n, off: (torch.randn(n + off, generator=gen, device=DEV) * 0.06).bfloat16()[off:]  # noqa: E731
+    x = torch.randn(tokens, width, generator=gen, device=DEV).bfloat16()
+    numbers = flat(experts * 2 * inner * width, 0), flat(experts * width * inner, 0)
+    router = torch.randn(experts, width, generator=gen, device=DEV).bfloat16()
+    results = []
+    for shift in (0, 1):
+        part = RoutedFeedForward(width, experts, top, inner, activation="swish")
+        w_in, w_out = (torch.empty(w.numel() + shift, dtype=w.dtype, device=DEV)[shift:].copy_(w) for w in numbers)
+        part.bind({"router.weight": router, "in.weight": w_in.view(-1, width), "out.weight": w_out.view(-1, inner)})
+        assert kernels.moe_many_rows_supports(x, part.w_in, part.w_out, pairs=tokens * top) == (shift == 0)
+        ws = types.SimpleNamespace(take=lambda shape, dtype: torch.empty(shape, dtype=dtype, device=DEV), mark=lambda: 0, release=lambda m: None)
+        ctx = types.SimpleNamespace(n_tokens=tokens, dtype=torch.bfloat16, ws=ws)
+        out = torch.zeros(tokens, width, device=DEV)
+        part.forward(ctx, x, out)
+        results.append(out)
+    # (the experts' inner numbers are rounded to 8 bits, in a few places the other way)
+    assert rel(results[1], results[0].double()) < 2.0 ** -8
