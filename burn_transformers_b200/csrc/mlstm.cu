@@ -443,8 +443,7 @@ __global__ void __launch_bounds__(256) mlstm_chunk_kernel(const T* __restrict__ 
       for (int i = 0; i < 4; ++i) {
         const float4 kv = i0 + i < dim ? *reinterpret_cast<const float4*>(k_t + (i0 + i) * MCP + sx) : make_float4(0.f, 0.f, 0.f, 0.f);
         kw[i][0] = kv.x * wv.x; kw[i][1] = kv.y * wv.y; kw[i][2] = kv.z * wv.z; kw[i][3] = kv.w * wv.w;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) nacc[i] += kw[i][u];
+        nacc[i] = fmaf(kv.w, wv.w, fmaf(kv.z, wv.z, fmaf(kv.y, wv.y, fmaf(kv.x, wv.x, nacc[i]))));      // (each product and sum rounded once)
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
