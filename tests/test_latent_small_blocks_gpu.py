@@ -55,7 +55,7 @@ def test_one_token_a_sequence_in_small_blocks(rank, rot, heads, seqs, runs, wind
 
 
 def test_runs_of_keys_never_leave_the_two_numbers_around_two_blocks():
-    part = LatentAttention(64, 16, 16, 8, 16, 512, 0.1, 1e-5, types.SimpleNamespace(dims=8))
+    part = LatentAttention(64, 16, 16, 8, 16, 512, 0.1, 1e-5, types.SimpleNamespace(rotates=True, dims=8))
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     for seqs in (1, 8, 50, 64, 100, sms, sms + 12, 2 * sms - 1, 2 * sms, 600):
         for bound in (33, 200, 1000):
