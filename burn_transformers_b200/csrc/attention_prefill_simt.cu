@@ -12,7 +12,7 @@
 // Q is 4 where blocks of 32 queries are three a multiprocessor, 2 where blocks of 16 are four for every three
 // multiprocessors, else 1 (decode steps of head sizes that the decode kernels do not take, short or few prompts).  A query's sums
 // are formed in the same order whatever Q is.  Measured with 12 heads, in us: with a warp a query and a lane a key, the version
-// before; with 32 queries in every block; and so.  Prompts of 64 channels, 32-bit: of 37, 268 and 499 tokens 217 / 79 / 68, one of
+// before; with 32 queries in every block; and so.  Prompts of 64 channels, 32-bit: of 37, 268 and 499 tokens 217 / 79 / 76, one of
 // 129 28 / 22 / 12; 2 x 1,024 tokens of 96 channels, bfloat16, 1,097 / 494 / 303; one token for each of 64 sequences behind 900:
 // 50 channels, 32-bit, 267 / 1,187 / 179, 96 channels, bfloat16, 330 / 2,184 / 202.
 //

@@ -656,8 +656,12 @@ static double moe_us(const bt::MoeTime& t, double pairs, double E, double K, dou
 static double moe_few_us(int pairs, int E, int K, int N, bool pair) { return moe_us(bt::MOE_FEW, pairs, E, K, N, pair, 24, 20, pair ? 16 : 32); }
 static double moe_mma_us(int pairs, int E, int K, int N, bool pair) { return moe_us(bt::MOE_MMA, pairs, E, K, N, pair, 24, 20, 64); }
 static double moe_tc_us(int pairs, int E, int K, int N, bool pair) { return moe_us(bt::MOE_TC, pairs, E, K, N, pair, 128, 64, pair ? 64 : 128); }
-static bool moe_takes_few(int pairs, int E, int K, int N, bool pair) {
-  return pairs <= (long long)bt::MOE_FEW_ROWS * E || moe_few_us(pairs, E, K, N, pair) <= moe_mma_us(pairs, E, K, N, pair);
+// `few` or `mma`, one for both products (one of each took longer than either: 16 experts of 128 x 256 at 40 rows 16.2 us, with
+// few 11.4, with mma 12.3), as for experts with a gate, so that the second product's call decides as the first one's
+static bool moe_takes_few(int pairs, int E, int width, int inner) {
+  return pairs <= (long long)bt::MOE_FEW_ROWS * E ||
+         moe_few_us(pairs, E, width, inner, true) + moe_few_us(pairs, E, inner, width, false) <=
+             moe_mma_us(pairs, E, width, inner, true) + moe_mma_us(pairs, E, inner, width, false);
 }
 
 // Whether the tcgen05 products (moe_tcgen05.cu) are the ones to take for a step's pairs: width -> inner -> width, `gated` with
@@ -666,11 +670,9 @@ extern "C" int bt_moe_many_rows_supports(int pairs, int E, int width, int inner,
   if (!bt_moe_expert_tcgen05_supports(pairs, E, width, inner) || !bt_moe_expert_tcgen05_supports(pairs, E, inner, width) ||
       pairs <= (long long)bt::MOE_FEW_ROWS * E || bt::sm_count() <= 0)
     return 0;
-  auto other = [&](int K, int N, bool pair) {
-    return moe_takes_few(pairs, E, K, N, pair) ? moe_few_us(pairs, E, K, N, pair) : moe_mma_us(pairs, E, K, N, pair);
-  };
+  const auto other = moe_takes_few(pairs, E, width, inner) ? moe_few_us : moe_mma_us;
   return moe_tc_us(pairs, E, width, inner, gated != 0) + moe_tc_us(pairs, E, inner, width, false) <
-         other(width, inner, gated != 0) + other(inner, width, false);
+         other(pairs, E, width, inner, gated != 0) + other(pairs, E, inner, width, false);
 }
 
 extern "C" int bt_moe_sort(const int* ids, int total, int E, int* offsets, int* tile_first, int* order, int* place,
@@ -703,7 +705,7 @@ extern "C" int bt_moe_expert(int first, const void* a, long long a_row_stride, c
   const dim3 grid((N + MS_BN - 1) / MS_BN, tiles);
   const bool pieces = dtype == kBF16 && K % 8 == 0 && a_row_stride % 8 == 0 && (unsigned long long)a % 16 == 0 &&
                       (unsigned long long)w % 16 == 0;
-  if (pieces && tensor_cores && moe_takes_few(pairs, E, K, N, first == kMoeInPair)) {
+  if (pieces && tensor_cores && moe_takes_few(pairs, E, first ? K : N, first ? N : K)) {
     const int cols = first == kMoeInPair ? MF_W / 2 : MF_W;
     const dim3 few((N + cols - 1) / cols, tiles);
     if (first == kMoeInPair)
