@@ -524,9 +524,10 @@ sigmoid_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, cons
 // The accumulated O is rescaled only when a row's maximum has grown by more than 2^8 over the reference its weights are
 // formed with (weights up to 2^8 lose nothing in bfloat16, whose rounding is relative, nor in the 32-bit sums); then the warps
 // wait for the products in flight, and read, multiply and write back their rows.
-// What bounds it is the special-function unit: 128 x 128 exponentials a tile are 1,024 cycles of a multiprocessor, and a
-// thread's other work between two tiles (load, maximum, pack, store) is hidden by a second block on the multiprocessor where
-// shared memory has room for it (heads of up to 64 channels; with values of 128, P takes the place of the scores it was made
+// What bounds it is a softmax warp's chain of dependent steps; no unit is full (16 x 1,024 tokens, 25 heads of 64: the
+// special-function pipe is active 47 % of the time, the tensor pipe 23).  128 x 128 exponentials a tile are 1,024 cycles of a
+// multiprocessor, and a thread's other work between two tiles (load, maximum, pack, store) runs beside those of a second block on
+// the multiprocessor where shared memory has room for it (heads of up to 64 channels; with values of 128, P takes the place of the scores it was made
 // of and the next scores wait for the product).  The version with eight softmax warps, P through shared memory and O taken
 // out of TMEM each tile had room for one block a multiprocessor.  16 sequences of 1,024 tokens, 25 heads of 64: 238 us
 // before, 125 now (0.75 us a tile and multiprocessor, 2.4 us a block); 8 x 512, 16 heads: 30.6 to 17.1 us; 2 x 1,024, 12
