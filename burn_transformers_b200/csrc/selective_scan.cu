@@ -41,6 +41,25 @@ __device__ __forceinline__ float ss_decay(float d, float a_scaled) {
   }
 }
 
+__device__ __forceinline__ unsigned long long ss_pack(float lo, float hi) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ void ss_unpack(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long ss_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long ss_mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 // dt[t, c], a block: 256 channels x SS_TT tokens; W_dt's rows of these channels lie transposed in shared memory
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -86,6 +105,109 @@ selective_scan_dt_kernel(const T* __restrict__ low, long long low_row_stride, co
       for (int t = 0; t < SS_TT; ++t)
         if (t < nt) dt[(t0 + t) * channels + c] = ss_softplus(acc[t]);
     }
+  }
+}
+
+// The same for bfloat16 rows and a rank of at most 64, on tensor cores: W_dt's 32-bit numbers go in as three bfloat16 parts, which
+// hold all of their bits, the smallest parts first, so that the products are exact and a result's sum is cut only in its last few
+// additions.  A warp keeps 32 channels' weights in registers as the operand wants them and walks over tiles of 16 tokens, with
+// neither shared memory nor barriers; the softplus, about 45 instructions a number, is what is left.  The kernel above is bound by
+// instructions, a third of them for its weights' way through shared memory.  In us, above and here: 2,439 tokens of 1,536 channels
+// and rank 48 27.5 and 17.8, 2,048 of 1,024 and rank 16 12.5 and 9.6, 100 of 1,536 and rank 48 6.4 and 3.9.
+template <int KS>
+__global__ void __launch_bounds__(128, KS <= 2 ? 5 : KS == 3 ? 4 : 3)
+selective_scan_dt_mma_kernel(const __nv_bfloat16* __restrict__ low, long long low_row_stride, const float* __restrict__ w_dt,
+                             const float* __restrict__ b_dt, float* __restrict__ dt, int n_tokens, int channels, int rank,
+                             int groups, int walkers) {
+  pdl_trigger();
+  const int warp = (int)(blockIdx.x * 4 + (threadIdx.x >> 5)), lane = threadIdx.x & 31, g = lane >> 2, t2 = (lane & 3) * 2;
+  const int group = warp % groups, walker = warp / groups;
+  if (walker >= walkers) return;
+  const int c0 = group * 32;
+  unsigned w[3][KS][4][2];
+#pragma unroll
+  for (int k = 0; k < KS; ++k)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = c0 + 8 * j + g, r = 16 * k + 8 * h + t2;
+        float2 v = c < channels && r < rank ? *reinterpret_cast<const float2*>(w_dt + (long long)c * rank + r) : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const __nv_bfloat162 part = __floats2bfloat162_rn(v.x, v.y);
+          const float2 back = __bfloat1622float2(part);
+          w[q][k][j][h] = *reinterpret_cast<const unsigned*>(&part);
+          v.x -= back.x;
+          v.y -= back.y;
+        }
+      }
+  float2 bias[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int c = c0 + 8 * j + t2;
+    bias[j] = make_float2(c < channels ? b_dt[c] : 0.f, c + 1 < channels ? b_dt[c + 1] : 0.f);
+  }
+  const bool pairs = channels % 2 == 0 && (unsigned long long)dt % 8 == 0;
+  pdl_wait();
+  for (int t0 = walker * 16; t0 < n_tokens; t0 += walkers * 16) {
+    unsigned a[KS][4];
+#pragma unroll
+    for (int k = 0; k < KS; ++k)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int t = t0 + g + 8 * (i & 1), r = 16 * k + 8 * (i >> 1) + t2;
+        a[k][i] = t < n_tokens && r < rank ? *reinterpret_cast<const unsigned*>(low + t * low_row_stride + r) : 0u;
+      }
+    float acc[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[j][i] = 0.f;
+#pragma unroll
+    for (int q = 2; q >= 0; --q)
+#pragma unroll
+      for (int k = 0; k < KS; ++k)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+              : "+f"(acc[j][0]), "+f"(acc[j][1]), "+f"(acc[j][2]), "+f"(acc[j][3])
+              : "r"(a[k][0]), "r"(a[k][1]), "r"(a[k][2]), "r"(a[k][3]), "r"(w[q][k][j][0]), "r"(w[q][k][j][1]));
+    bool whole = true;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        acc[j][i] += i & 1 ? bias[j].y : bias[j].x;
+        whole = whole && isfinite(acc[j][i]);
+      }
+    if (!whole) {      // an infinity times the parts of a weight is no number: such sums are formed again by multiply-adds
+#pragma unroll 1
+      for (int n = 0; n < 16; ++n) {
+        const int t = t0 + g + 8 * (n >> 1 & 1), c = c0 + 8 * (n >> 2) + t2 + (n & 1);
+        if (t >= n_tokens || c >= channels) continue;
+        float z = b_dt[c];
+        for (int r = 0; r < rank; ++r) z = fmaf(w_dt[(long long)c * rank + r], to_float(low[t * low_row_stride + r]), z);
+#pragma unroll
+        for (int m = 0; m < 16; ++m)
+          if (m == n && !isfinite(acc[m >> 2][m & 3])) acc[m >> 2][m & 3] = z;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int t = t0 + g + 8 * h, c = c0 + 8 * j + t2;
+        const float y0 = ss_softplus(acc[j][2 * h]), y1 = ss_softplus(acc[j][2 * h + 1]);
+        float* at = dt + (long long)t * channels + c;
+        if (t >= n_tokens) continue;
+        if (pairs) {
+          if (c < channels) *reinterpret_cast<float2*>(at) = make_float2(y0, y1);
+        } else {
+          if (c < channels) at[0] = y0;
+          if (c + 1 < channels) at[1] = y1;
+        }
+      }
   }
 }
 
@@ -235,6 +357,221 @@ selective_scan_kernel(const T* __restrict__ x, long long x_row_stride, const T* 
   }
 }
 
+// The pieces of long runs for up to 16 state indices: a channel belongs to one thread, or two neighbours above 8 indices, with 8
+// indices each, whose numbers go two an instruction; a token's B and C are read once a warp, and four tokens are worked on at once
+// without a branch between them.  What bounds it: the special-function unit's exponentials, one an index and token, take 14 us a
+// launch at 2,439 tokens of 1,536 channels x 16 indices, the instructions about 11 (the first launch) and 20; the rest is the
+// latency of a warp's chain.  Both launches there, in us, with selective_scan_kernel and so: 90 and 70; 2 x 1,024 tokens of 1,024
+// channels 63 and 51; one run of 300 32 and 31; 8 indices 114 and 51; 32-bit rows 121 and 98.  (A thread for all 16 indices: 84,
+// too few warps to hide an exponential behind.  72 registers a thread, so that 2,439 tokens are one wave of blocks: 68, but 2 x 70
+// tokens 37 instead of 24.)
+// A piece's tokens are asked for SP_AHEAD at a time, one group ahead.  The walk over the earlier pieces goes through the cells as
+// they lie, n_state + 1 numbers a channel in a row over the block's threads, and meets the channels' layout in shared memory.
+constexpr int SP_THREADS = 64, SP_STAGE = 64, SP_AHEAD = 4;
+
+template <typename T, int LANES, bool ENDS>
+__global__ void __launch_bounds__(SP_THREADS, ENDS ? 12 : 10)
+selective_scan_piece_kernel(const T* __restrict__ x, long long x_row_stride, const T* __restrict__ z, long long z_row_stride,
+                            const float* __restrict__ dt, const T* __restrict__ low, long long low_row_stride, int b_off,
+                            int c_off, const float* __restrict__ a_log, const float* __restrict__ d_skip,
+                            float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ seq_start,
+                            T* __restrict__ out, long long out_row_stride, int channels, int n_state, float out_scale,
+                            int piece, float* __restrict__ ends) {
+  constexpr float kLog2e = sizeof(T) == 2 ? 1.4426950408889634f : 1.f;      // (see ss_decay)
+  constexpr int NS = 8, PAD = NS * LANES;                                   // indices a thread, and a channel, has room for
+  constexpr int ROW = ENDS ? PAD : 2 * PAD;                                 // a token's B, and C where it is read
+  constexpr int CPB = SP_THREADS / LANES, CELLS = (CPB * (PAD + 1) + SP_THREADS - 1) / SP_THREADS;
+  __shared__ __align__(16) float bc_s[SP_STAGE * ROW];
+  __shared__ float walk_s[ENDS ? 1 : CPB * (PAD + 1)];
+  pdl_trigger();
+  const int tid = threadIdx.x, seq = blockIdx.y, cl = tid / LANES, n0 = tid % LANES * NS, c0 = blockIdx.x * CPB, c = c0 + cl;
+  const bool owns = c < channels;
+  float a[NS];
+#pragma unroll
+  for (int i = 0; i < NS; ++i) a[i] = owns && n0 + i < n_state ? -expf(a_log[(long long)c * n_state + n0 + i]) * kLog2e : 0.f;
+#pragma unroll
+  for (int i = 0; i < NS; ++i)
+    if (a[i] == -INFINITY) a[i] = -3.4e38f;      // (times a step of zero must be a number, see fetch below)
+  const float skip = !ENDS && owns ? d_skip[c] : 0.f;
+  pdl_wait();
+  const int first = seq_start[seq], n_all = seq_start[seq + 1] - first;
+  const int n_pieces = (n_all + piece - 1) / piece, my_piece = blockIdx.z;
+  if (my_piece >= n_pieces - (ENDS ? 1 : 0)) return;
+  const int t_lo = my_piece * piece, t_hi = min(n_all, t_lo + piece);
+  const int n1 = n_state + 1;
+  const long long es = (long long)channels * n1;
+  float* e_block = ends + ((long long)(first / piece + seq)) * es + (long long)c0 * n1;
+  float* s_block = state + ((long long)slots[seq] * channels + c0) * n_state;
+  float s[NS];
+  if (ENDS) {
+    if (my_piece == 0 && owns) {
+      float* copy = e_block + (long long)(n_pieces - 1) * es + cl * n1;
+#pragma unroll
+      for (int i = 0; i < NS; ++i)
+        if (n0 + i < n_state) copy[n0 + i] = s_block[cl * n_state + n0 + i];
+    }
+#pragma unroll
+    for (int i = 0; i < NS; ++i) s[i] = 0.f;
+  } else if (my_piece == 0) {
+    const float* before = n_pieces > 1 ? e_block + (long long)(n_pieces - 1) * es + cl * n1 : s_block + cl * n_state;
+#pragma unroll
+    for (int i = 0; i < NS; ++i) s[i] = owns && n0 + i < n_state ? before[n0 + i] : 0.f;
+  } else {
+    // number k of this thread is number `tid + 64 k` of the block's cells: channel ch, index n (index n_state: the sum of dt)
+    float w[CELLS], wa[CELLS];
+    int at_d[CELLS];
+    const float* copy = e_block + (long long)(n_pieces - 1) * es;
+    const int step_c = SP_THREADS / n1, step_n = SP_THREADS % n1;
+    int ch = tid / n1, n = tid % n1;
+#pragma unroll
+    for (int k = 0; k < CELLS; ++k) {
+      const bool mine = ch < CPB && c0 + ch < channels && n < n_state;
+      w[k] = mine ? copy[tid + SP_THREADS * k] : 0.f;
+      wa[k] = mine ? -expf(a_log[(long long)(c0 + ch) * n_state + n]) * kLog2e : 0.f;
+      at_d[k] = mine ? ch * n1 + n_state : -1;
+      ch += step_c; n += step_n;
+      if (n >= n1) { n -= n1; ++ch; }
+    }
+#pragma unroll 2
+    for (int j = 0; j < my_piece; ++j) {      // (two pieces' numbers are asked for at once)
+      const float* e = e_block + (long long)j * es;
+      float ev[CELLS], dv[CELLS];
+#pragma unroll
+      for (int k = 0; k < CELLS; ++k) {
+        ev[k] = at_d[k] >= 0 ? e[tid + SP_THREADS * k] : 0.f;
+        dv[k] = at_d[k] >= 0 ? e[at_d[k]] : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < CELLS; ++k) w[k] = fmaf(ss_decay<T>(dv[k], wa[k]), w[k], ev[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < CELLS; ++k)
+      if (at_d[k] >= 0) walk_s[tid + SP_THREADS * k] = w[k];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NS; ++i) s[i] = owns && n0 + i < n_state ? walk_s[cl * n1 + n0 + i] : 0.f;
+  }
+  unsigned long long s2[NS / 2], a2[NS / 2];
+#pragma unroll
+  for (int i = 0; i < NS / 2; ++i) {
+    s2[i] = ss_pack(s[2 * i], s[2 * i + 1]);
+    a2[i] = ss_pack(a[2 * i], a[2 * i + 1]);
+  }
+  const long long cc = owns ? c : 0;      // (a thread past the channels reads the first one's numbers and writes nothing)
+  float dt_sum = 0.f;
+  for (int t0 = t_lo; t0 < t_hi; t0 += SP_STAGE) {
+    const int nt = min(SP_STAGE, t_hi - t0);
+    const long long row0 = first + t0;
+    const float* dt_at = dt + row0 * channels + cc;
+    const T* x_at = x + row0 * x_row_stride + cc;
+    const T* z_at = z + row0 * z_row_stride + cc;
+    T* out_at = out + row0 * out_row_stride + cc;
+    float d[SP_AHEAD];
+    T xv[SP_AHEAD], zv[SP_AHEAD];
+    // the next SP_AHEAD tokens' numbers; a token past the piece has a step of zero, which leaves the state as it is
+    auto fetch = [&](int left, float (&dd)[SP_AHEAD], T (&xx)[SP_AHEAD], T (&zz)[SP_AHEAD]) {
+      if (left >= SP_AHEAD) {
+#pragma unroll
+        for (int u = 0; u < SP_AHEAD; ++u) {
+          dd[u] = dt_at[u * channels];
+          xx[u] = x_at[u * x_row_stride];
+          if (!ENDS) zz[u] = z_at[u * z_row_stride];
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < SP_AHEAD; ++u) {
+          const bool in = u < left;
+          dd[u] = in ? dt_at[u * channels] : 0.f;
+          xx[u] = in ? x_at[u * x_row_stride] : from_float<T>(0.f);
+          if (!ENDS) zz[u] = in ? z_at[u * z_row_stride] : from_float<T>(0.f);
+        }
+      }
+      dt_at += (long long)SP_AHEAD * channels;
+      x_at += SP_AHEAD * x_row_stride;
+      if (!ENDS) z_at += SP_AHEAD * z_row_stride;
+    };
+    fetch(nt, d, xv, zv);
+    __syncthreads();
+#pragma unroll 8
+    for (int i = tid; i < SP_STAGE * ROW; i += SP_THREADS) {      // (zeros past the piece: a number there times zero is no number)
+      const int t = i / ROW, m = i % ROW, n = m % PAD;
+      bc_s[i] = t < nt && n < n_state ? to_float(low[(row0 + t) * low_row_stride + (m < PAD ? b_off : c_off) + n]) : 0.f;
+    }
+    __syncthreads();
+    for (int t = 0; t < nt; t += SP_AHEAD) {
+      float dn[SP_AHEAD];
+      T xn[SP_AHEAD], zn[SP_AHEAD];
+      fetch(nt - t - SP_AHEAD, dn, xn, zn);
+      float y[SP_AHEAD];
+#pragma unroll
+      for (int u = 0; u < SP_AHEAD; ++u) {
+        const float dx = d[u] * to_float(xv[u]);
+        const unsigned long long d2 = ss_pack(d[u], d[u]), dx2 = ss_pack(dx, dx);
+        const ulonglong2* b2 = reinterpret_cast<const ulonglong2*>(bc_s + (t + u) * ROW + n0);
+        unsigned long long y2[2] = {0ull, 0ull};
+#pragma unroll
+        for (int i4 = 0; i4 < NS / 4; ++i4) {
+          const ulonglong2 b = b2[i4];
+          ulonglong2 cv;
+          if (!ENDS) cv = b2[PAD / 4 + i4];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int i = 2 * i4 + h;
+            float e0, e1;
+            ss_unpack(ss_mul2(d2, a2[i]), e0, e1);
+            if constexpr (sizeof(T) == 2) {
+              asm("ex2.approx.ftz.f32 %0, %0;\n" : "+f"(e0));
+              asm("ex2.approx.ftz.f32 %0, %0;\n" : "+f"(e1));
+            } else {
+              e0 = expf(e0);
+              e1 = expf(e1);
+            }
+            s2[i] = ss_fma2(ss_pack(e0, e1), s2[i], ss_mul2(dx2, h ? b.y : b.x));
+            if (!ENDS) y2[h] = ss_fma2(s2[i], h ? cv.y : cv.x, y2[h]);
+          }
+        }
+        if (ENDS) {
+          dt_sum += d[u];
+        } else {
+          float y0, y1, y3, y4;
+          ss_unpack(y2[0], y0, y1);
+          ss_unpack(y2[1], y3, y4);
+          y[u] = (y0 + y1) + (y3 + y4);
+          if (LANES > 1) y[u] += __shfl_xor_sync(0xffffffffu, y[u], 1);
+        }
+      }
+      if (!ENDS) {
+#pragma unroll
+        for (int v = 0; v < SP_AHEAD / LANES; ++v) {      // (a channel's lanes take the tokens' gates in turn)
+          const int u = v * LANES + (LANES > 1 ? tid % LANES : 0);
+          const float yu = LANES == 1 ? y[v] : (tid % LANES ? y[v * LANES + LANES - 1] : y[v * LANES]);
+          const float xf = to_float(LANES == 1 ? xv[v] : (tid % LANES ? xv[v * LANES + LANES - 1] : xv[v * LANES]));
+          const float zf = to_float(LANES == 1 ? zv[v] : (tid % LANES ? zv[v * LANES + LANES - 1] : zv[v * LANES]));
+          const float gate = sizeof(T) == 2 ? __fdividef(zf, 1.f + __expf(-zf)) : zf / (1.f + expf(-zf));
+          if (owns && t + u < nt) out_at[u * out_row_stride] = from_float<T>((yu + skip * xf) * gate * out_scale);
+        }
+        out_at += SP_AHEAD * out_row_stride;
+      }
+#pragma unroll
+      for (int u = 0; u < SP_AHEAD; ++u) {
+        d[u] = dn[u];
+        xv[u] = xn[u];
+        if (!ENDS) zv[u] = zn[u];
+      }
+    }
+  }
+  if (!owns || (!ENDS && my_piece != n_pieces - 1)) return;
+  float* dst = ENDS ? e_block + (long long)my_piece * es + cl * n1 + n0 : s_block + cl * n_state + n0;
+#pragma unroll
+  for (int i = 0; i < NS / 2; ++i) {
+    float lo, hi;
+    ss_unpack(s2[i], lo, hi);
+    if (n0 + 2 * i < n_state) dst[2 * i] = lo;
+    if (n0 + 2 * i + 1 < n_state) dst[2 * i + 1] = hi;
+  }
+  if (ENDS && n0 == 0) dst[n_state] = dt_sum;
+}
+
 template <typename T>
 static int launch_selective_scan(const T* x, long long xs, const T* z, long long zs, const float* dt, const T* low,
                                  long long ls, int b_off, int c_off, const float* a_log, const float* d_skip, float* state,
@@ -249,6 +586,17 @@ static int launch_selective_scan(const T* x, long long xs, const T* z, long long
   else if (n_state <= 256) { ns = 16; lanes = 16; }
   else { ns = 16; lanes = 32; }
   BT_CHECK(n_state <= 512, "selective_scan: %d state indices a channel; the kernel takes up to 512", n_state);
+  if (piece > 0 && n_state <= 16) {      // (steps without pieces are few tokens a sequence: more lanes a channel answer sooner)
+#define BT_SP(LANES, ENDS)                                                                                                   \
+  BT_PDL_OK("selective_scan", launch_pdl(selective_scan_piece_kernel<T, LANES, ENDS>,                                        \
+                                         dim3((channels + SP_THREADS / LANES - 1) / (SP_THREADS / LANES), n_seqs, max_pieces), \
+                                         dim3(SP_THREADS), 0, stream, 1, x, xs, z, zs, dt, low, ls, b_off, c_off, a_log,     \
+                                         d_skip, state, slots, seq_start, out, os, channels, n_state, out_scale, piece, ends))
+    if (n_state <= 8) { BT_SP(1, true); BT_SP(1, false); }
+    else { BT_SP(2, true); BT_SP(2, false); }
+#undef BT_SP
+    return 0;
+  }
   const int cpb = SS_THREADS / lanes;
   const dim3 grid((channels + cpb - 1) / cpb, n_seqs, piece > 0 ? max_pieces : 1);
   const int stage = n_state <= 64 ? 2 * SS_TT : SS_TT;      // tokens staged in shared memory at a time
@@ -270,7 +618,10 @@ static int launch_selective_scan(const T* x, long long xs, const T* z, long long
                                            slots, seq_start, out, os, channels, n_state, out_scale, piece, ends,       \
                                            stage));                                                                   \
   } while (0)
-  if (ns == 4) BT_SS(4, 4);
+  if (ns == 4)      // (its pieces went the other way)
+    BT_PDL_OK("selective_scan", launch_pdl(selective_scan_kernel<T, 4, 4, false>, grid, dim3(SS_THREADS), smem, stream, 1, x, xs, z,
+                                           zs, dt, low, ls, b_off, c_off, a_log, d_skip, state, slots, seq_start, out, os,
+                                           channels, n_state, out_scale, piece, ends, stage));
   else if (ns == 8) BT_SS(8, 4);
   else if (lanes == 4) BT_SS(16, 4);
   else if (lanes == 8) BT_SS(16, 8);
@@ -289,6 +640,25 @@ extern "C" int bt_selective_scan_dt(const void* low, long long low_row_stride, c
   BT_CHECK(channels > 0 && rank > 0 && rank <= 160 && n_tokens >= 0,
            "selective_scan_dt: bad sizes channels=%d rank=%d (at most 160)", channels, rank);
   if (n_tokens == 0) return 0;
+  if (dtype == kBF16 && rank % 2 == 0 && rank <= 64 && n_tokens <= 0x7ffffff0ll && low_row_stride % 2 == 0 &&
+      (unsigned long long)low % 4 == 0 && (unsigned long long)w_dt % 8 == 0) {
+    // (one wave of blocks: 12 warps a multiprocessor and more are resident, with as many tiles of tokens each as that leaves)
+    const int sms = sm_count();
+    BT_CHECK(sms > 0, "selective_scan_dt: cannot read the number of multiprocessors of the current device");
+    const int groups = (channels + 31) / 32, tiles = (int)((n_tokens + 15) / 16);
+    const int most = 12 * sms / groups > 0 ? 12 * sms / groups : 1, walkers = tiles < most ? tiles : (tiles + (tiles + most - 1) / most - 1) / ((tiles + most - 1) / most);
+    const dim3 grid((unsigned)(((long long)groups * walkers + 3) / 4));
+#define BT_SSM(KS)                                                                                                    \
+  BT_PDL_OK("selective_scan_dt", launch_pdl(selective_scan_dt_mma_kernel<KS>, grid, dim3(128), 0, stream, 1,          \
+                                            (const __nv_bfloat16*)low, low_row_stride, w_dt, b_dt, dt, (int)n_tokens, \
+                                            channels, rank, groups, walkers))
+    if (rank <= 16) BT_SSM(1);
+    else if (rank <= 32) BT_SSM(2);
+    else if (rank <= 48) BT_SSM(3);
+    else BT_SSM(4);
+#undef BT_SSM
+    return 0;
+  }
   const size_t smem = sizeof(float) * ((size_t)rank * SS_WS + (size_t)SS_TT * rank);
   const long long tiles = (n_tokens + SS_TT - 1) / SS_TT;
   const long long col_blocks = (channels + 255) / 256, want_rows = (4 * 148 + col_blocks - 1) / col_blocks;
