@@ -1,0 +1,149 @@
+// The products inside a chunk of 64 tokens of a recurrence (lightning.cu, mlstm.cu), on tensor cores with no operand's bits given up:
+// a 32-bit number goes in as the sum of three bfloat16 numbers (the residues are exact), a number that bfloat16 holds as itself,
+// and the products whose parts' orders add up to two at most are formed; what is left out is below 2^-24 of a product.
+//
+// Tensor cores cut their sums where a multiply-add rounds them.  So the products of the first parts begin from zero at every step of
+// 16 along the sum and are added in 32-bit registers; those of the smaller parts, 2^-8 and less of the result, share accumulators.
+//
+// A block is four warps with 16 rows of the result each.  The second operands lie in shared memory, their parts one behind the
+// other, in rows of (columns + 8) numbers: eight rows' 16-byte pieces then meet all banks, however they are read.
+#pragma once
+#include "common.cuh"
+
+namespace bt {
+
+constexpr int CM_CHUNK = 64, CM_THREADS = 128, CM_COLS = 64;
+constexpr int CM_ROW = CM_COLS + 8;      // numbers of a row of value channels in shared memory
+
+__device__ __forceinline__ void cm_mma(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void cm_ldmatrix(unsigned (&r)[4], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ void cm_ldmatrix_t(unsigned (&r)[4], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+}
+
+// two numbers' parts, each as a pair of bfloat16
+template <int PARTS>
+__device__ __forceinline__ void cm_split(float x, float y, unsigned (&part)[PARTS]) {
+#pragma unroll
+  for (int q = 0; q < PARTS; ++q) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    part[q] = *reinterpret_cast<const unsigned*>(&h);
+    if (q + 1 < PARTS) {
+      x -= __uint_as_float(part[q] << 16);
+      y -= __uint_as_float(part[q] & 0xffff0000u);
+    }
+  }
+}
+
+__device__ __forceinline__ void cm_load8(const float* p, float (&x)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+}
+__device__ __forceinline__ void cm_load8(const __nv_bfloat16* p, float (&x)[8]) { unpack16(*reinterpret_cast<const uint4*>(p), x); }
+__device__ __forceinline__ float2 cm_load2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ float2 cm_load2(const __nv_bfloat16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
+
+// Rows of `cols` numbers (whole pieces of 8) into shared memory, part behind part (`part_size` numbers apart), rows `stride` apart:
+// load(row, column, x) gives eight numbers.
+template <int PARTS, typename Load>
+__device__ __forceinline__ void cm_fill(__nv_bfloat16* dst, int rows, int cols, int stride, int part_size, Load load) {
+  const int pieces = cols / 8;
+#pragma unroll 2
+  for (int i = threadIdx.x; i < rows * pieces; i += CM_THREADS) {
+    const int r = i / pieces, c = (i - r * pieces) * 8;
+    float x[8];
+    load(r, c, x);
+    unsigned part[4][PARTS];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) cm_split<PARTS>(x[2 * u], x[2 * u + 1], part[u]);
+#pragma unroll
+    for (int q = 0; q < PARTS; ++q)
+      *reinterpret_cast<uint4*>(dst + q * part_size + r * stride + c) = make_uint4(part[0][q], part[1][q], part[2][q], part[3][q]);
+  }
+}
+
+// big += a0 b0, small += the other products of the parts, for two neighbouring tiles of eight columns (b: their operands, part by
+// part: the first tile's two registers, then the second's)
+template <int AP, int BP>
+__device__ __forceinline__ void cm_products(float (&big0)[4], float (&small0)[4], float (&big1)[4], float (&small1)[4],
+                                            const unsigned (&a)[AP][4], const unsigned (&b)[BP][4]) {
+#pragma unroll
+  for (int q = AP + BP - 2; q >= 0; --q)
+#pragma unroll
+    for (int pa = 0; pa < AP; ++pa) {
+      const int pb = q - pa;
+      if (q > 2 || pb < 0 || pb >= BP) continue;
+      if (q > 0) {
+        cm_mma(small0, a[pa], b[pb][0], b[pb][1]);
+        cm_mma(small1, a[pa], b[pb][2], b[pb][3]);
+      } else {
+        float x[4] = {}, y[4] = {};
+        cm_mma(x, a[0], b[0][0], b[0][1]);
+        cm_mma(y, a[0], b[0][2], b[0][3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          big0[i] += x[i];
+          big1[i] += y[i];
+        }
+      }
+    }
+}
+
+// One step of 16 along the sum over a second operand whose rows run along the sum (S_in or V: [sum][column]): rows row0.., the tiles
+// of columns [0, 8 tiles).
+template <int AP, int BP, int TILES>
+__device__ __forceinline__ void cm_step_rows(float (&big)[TILES][4], float (&small)[TILES][4], const unsigned (&a)[AP][4],
+                                             const __nv_bfloat16* src, int row0, int part_size) {
+  const int lane = threadIdx.x & 31;
+  const __nv_bfloat16* at = src + (row0 + (lane & 15)) * CM_ROW + (lane >> 4) * 8;
+#pragma unroll
+  for (int j = 0; j < TILES; j += 2) {
+    unsigned b[BP][4];
+#pragma unroll
+    for (int q = 0; q < BP; ++q) cm_ldmatrix_t(b[q], at + q * part_size + 8 * j);
+    cm_products<AP, BP>(big[j], small[j], big[j + 1], small[j + 1], a, b);
+  }
+}
+
+// The chunk's contribution to the state, rows d of `dim` (16 a warp and round), columns [0, 64):  sum_s K'[s][d] V[s][c], K' and V in
+// shared memory ([token][channel]; KP and VP parts).  store(d, c, x, y) gets the numbers of columns c and c + 1; ones(d, sum), the sum of
+// K' alone, where SUMS is set.
+template <int KP, int VP, bool SUMS, typename Store, typename Ones>
+__device__ __forceinline__ void cm_state(const __nv_bfloat16* k, int k_stride, int k_part, const __nv_bfloat16* v, int v_part, int dim,
+                                         Store store, Ones ones) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t2 = (lane & 3) * 2;
+  for (int d0 = warp * 16; d0 < dim; d0 += 64) {
+    float big[8][4] = {}, small[8][4] = {}, sums[4] = {};
+#pragma unroll
+    for (int s = 0; s < CM_CHUNK; s += 16) {
+      unsigned a[KP][4];
+      // (matrices: channels d0.. of tokens s.., channels d0 + 8.., then tokens s + 8..)
+      const __nv_bfloat16* at = k + (s + (lane & 7) + (lane >> 4) * 8) * k_stride + d0 + (lane >> 3 & 1) * 8;
+#pragma unroll
+      for (int q = 0; q < KP; ++q) cm_ldmatrix_t(a[q], at + q * k_part);
+      cm_step_rows<KP, VP, 8>(big, small, a, v, s, v_part);
+      if (SUMS)
+#pragma unroll
+        for (int q = KP - 1; q >= 0; --q) cm_mma(sums, a[q], 0x3f803f80u, 0x3f803f80u);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      store(d0 + g, 8 * j + t2, big[j][0] + small[j][0], big[j][1] + small[j][1]);
+      store(d0 + g + 8, 8 * j + t2, big[j][2] + small[j][2], big[j][3] + small[j][3]);
+    }
+    if (SUMS && (lane & 3) == 0) {
+      ones(d0 + g, sums[0]);
+      ones(d0 + g + 8, sums[2]);
+    }
+  }
+}
+
+}  // namespace bt

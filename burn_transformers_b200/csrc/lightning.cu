@@ -9,6 +9,7 @@
 // the state in registers for all tokens of the step, and writes it back once.  Inside a block a value channel belongs
 // to SPLIT adjacent lanes, each with DPT of the head's `dim` key channels; their partial outputs meet by shuffles.
 // The state lives in `state[slot][head][dim][vdim]`; a sequence that starts finds zeros there.
+#include "chunk_mma.cuh"
 #include "common.cuh"
 
 namespace bt {
@@ -362,6 +363,42 @@ lightning_prefix_kernel(float* scratch, float* __restrict__ state, const int* __
   *st = s;
 }
 
+// The same, four neighbouring elements a thread and eight chunks asked for at a time, where a state is whole pieces of 16 bytes on
+// such boundaries: two rounds of loads for 1,024 tokens instead of four.
+__global__ void __launch_bounds__(128)
+lightning_prefix_vec_kernel(float* scratch, float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ seq_start,
+                            const float* __restrict__ decay, int max_chunks, int n_heads, int dim, int vdim) {
+  pdl_trigger();
+  pdl_wait();
+  const int seq = blockIdx.z, head = blockIdx.y;
+  const int e = (blockIdx.x * 128 + threadIdx.x) * 4;
+  if (e >= dim * vdim) return;
+  const int n_new = seq_start[seq + 1] - seq_start[seq];
+  const int n_chunks = (n_new + LC - 1) / LC;
+  const float lam = decay[head];
+  const float full = powf(lam, (float)LC);
+  const float tail = powf(lam, (float)(n_new - (n_chunks - 1) * LC));
+  float* st = state + (((long long)slots[seq] * n_heads + head) * dim) * vdim + e;
+  const long long stride = (long long)n_heads * dim * vdim;
+  float* cell = scratch + (((long long)seq * max_chunks) * n_heads + head) * (long long)dim * vdim + e;
+  float4 s = *reinterpret_cast<float4*>(st);
+  for (int c = 0; c < n_chunks; c += 8) {
+    float4 kv[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      kv[u] = c + u < n_chunks ? __ldcg(reinterpret_cast<const float4*>(cell + (c + u) * stride)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (c + u < n_chunks) {
+        *reinterpret_cast<float4*>(cell + (c + u) * stride) = s;
+        const float f = c + u == n_chunks - 1 ? tail : full;
+        s = make_float4(fmaf(f, s.x, kv[u].x), fmaf(f, s.y, kv[u].y), fmaf(f, s.z, kv[u].z), fmaf(f, s.w, kv[u].w));
+      }
+    }
+  }
+  *reinterpret_cast<float4*>(st) = s;
+}
+
 // out[t] += decay^(t+1) S_in^T q_t for the tokens of a chunk; grid and blocks as lightning_chunk_kernel.
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -446,6 +483,221 @@ lightning_carry_kernel(const T* __restrict__ proj, long long row_stride, int q_o
   }
 }
 
+// The chunks on tensor cores (chunk_mma.cuh), for rows on 16-byte boundaries with channels in whole operand tiles: first every
+// chunk's contribution to the state (lightning_state_kernel), then lightning_prefix_kernel, then all of o at once
+// (lightning_out_kernel), which is written once.  PARTS: 1 where q, k and v are bfloat16 numbers as they are, else 3.
+// The kernels above are bound by shared memory (an operand read for every other multiply-add) and write o, read it and write it
+// again; these by the forming of the features and the parts, and by the products.  All three kernels, above and here, in us: 2 x 1,024
+// tokens of 16 heads of 64 x 64 with act 0 65 and 49, 6 x 1,000 of 12 heads 112 and 88, with act 1 101 and 58, 32-bit rows 2 x 1,024
+// 69 and 39.  Errors against 64 bits 1.2e-7 and 7e-8 (act 0), 1.8e-7 and 9e-8 (act 1).
+// x * sigmoid(x) for these kernels: the library's division is half of its instructions; here a reciprocal and one Newton step (the
+// argument is bounded so that the reciprocal is a normal number)
+__device__ __forceinline__ float cm_feature(float x, int act) {
+  if (act != 0) return x;
+  const float y = 1.f + expf(fminf(-x, 87.f));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(y));
+  return x * fmaf(r, fmaf(-y, r, 1.f), r);
+}
+
+template <typename T, int PARTS>
+__global__ void __launch_bounds__(CM_THREADS, 4)
+lightning_state_kernel(const T* __restrict__ proj, long long row_stride, int k_off, int v_off, const int* __restrict__ seq_start,
+                       const float* __restrict__ decay, float* __restrict__ scratch, int max_chunks, int n_heads, int dim, int vdim,
+                       int col_blocks, int act) {
+  extern __shared__ __align__(16) unsigned char cm_smem[];
+  __nv_bfloat16* k_s = reinterpret_cast<__nv_bfloat16*>(cm_smem);      // [3][64][dim + 8]: decay^(len - 1 - s) k_s
+  const int k_stride = dim + 8, k_part = CM_CHUNK * k_stride, v_part = CM_CHUNK * CM_ROW;
+  __nv_bfloat16* v_s = k_s + 3 * k_part;                               // [PARTS][64][72]
+  __shared__ float pw[CM_CHUNK];
+  pdl_trigger();
+  pdl_wait();
+  const int chunk = blockIdx.x, seq = blockIdx.z;
+  const int head = blockIdx.y / col_blocks, col0 = (blockIdx.y - head * col_blocks) * CM_COLS;
+  const int first = seq_start[seq], n_new = seq_start[seq + 1] - first;
+  if (chunk * CM_CHUNK >= n_new) return;
+  const int len = min(CM_CHUNK, n_new - chunk * CM_CHUNK);
+  const T* rows = proj + (first + (long long)chunk * CM_CHUNK) * row_stride;
+  if (threadIdx.x < CM_CHUNK) pw[threadIdx.x] = powf(decay[head], (float)threadIdx.x);
+  __syncthreads();
+  cm_fill<3>(k_s, CM_CHUNK, dim, k_stride, k_part, [&](int t, int c, float (&x)[8]) {
+    if (t < len) cm_load8(rows + t * row_stride + k_off + head * dim + c, x);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = t < len ? cm_feature(x[u], act) * pw[len - 1 - t] : 0.f;
+  });
+  cm_fill<PARTS>(v_s, CM_CHUNK, CM_COLS, CM_ROW, v_part, [&](int t, int c, float (&x)[8]) {
+    const bool in = t < len && col0 + c < vdim;
+    if (in) cm_load8(rows + t * row_stride + v_off + head * vdim + col0 + c, x);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = in ? cm_feature(x[u], act) : 0.f;
+  });
+  __syncthreads();
+  float* dst = scratch + ((((long long)seq * max_chunks + chunk) * n_heads + head) * dim) * vdim + col0;
+  cm_state<3, PARTS, false>(k_s, k_stride, k_part, v_s, v_part, dim,
+                            [&](int d, int c, float x, float y) {
+                              if (col0 + c < vdim) *reinterpret_cast<float2*>(dst + (long long)d * vdim + c) = make_float2(x, y);
+                            },
+                            [](int, float) {});
+}
+
+template <typename T, int PARTS>
+__global__ void __launch_bounds__(CM_THREADS, 4)
+lightning_out_kernel(const T* __restrict__ proj, long long row_stride, int q_off, int k_off, int v_off, const int* __restrict__ seq_start,
+                     const float* __restrict__ decay, float* __restrict__ out, long long out_row_stride,
+                     const float* __restrict__ scratch, int max_chunks, int n_heads, int dim, int vdim, int col_blocks, int act) {
+  extern __shared__ __align__(16) unsigned char cm_smem[];
+  const int k_stride = dim + 8, k_part = CM_CHUNK * k_stride, s_part = max(dim, CM_CHUNK) * CM_ROW;
+  __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(cm_smem);      // [PARTS][64][dim + 8]
+  __nv_bfloat16* s_s = q_s + PARTS * k_part;                           // [3][dim][72] the state; then [PARTS][64][dim + 8] k; then [PARTS][64][72] v
+  __shared__ float pw[CM_CHUNK + 1];
+  pdl_trigger();
+  pdl_wait();
+  const int chunk = blockIdx.x, seq = blockIdx.z;
+  const int head = blockIdx.y / col_blocks, col0 = (blockIdx.y - head * col_blocks) * CM_COLS;
+  const int first = seq_start[seq], n_new = seq_start[seq + 1] - first;
+  if (chunk * CM_CHUNK >= n_new) return;
+  const int len = min(CM_CHUNK, n_new - chunk * CM_CHUNK);
+  const long long row0 = first + (long long)chunk * CM_CHUNK;
+  const T* rows = proj + row0 * row_stride;
+  if (threadIdx.x <= CM_CHUNK) pw[threadIdx.x] = powf(decay[head], (float)threadIdx.x);
+  const float* src = scratch + ((((long long)seq * max_chunks + chunk) * n_heads + head) * dim) * vdim + col0;
+  cm_fill<3>(s_s, dim, CM_COLS, CM_ROW, s_part, [&](int d, int c, float (&x)[8]) {
+    if (col0 + c < vdim) cm_load8(src + (long long)d * vdim + c, x);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = col0 + c < vdim ? x[u] : 0.f;
+  });
+  auto fill = [&](__nv_bfloat16* dst, int off) {      // q or k
+    cm_fill<PARTS>(dst, CM_CHUNK, dim, k_stride, k_part, [&](int t, int c, float (&x)[8]) {
+      if (t < len) cm_load8(rows + t * row_stride + off + head * dim + c, x);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = t < len ? cm_feature(x[u], act) : 0.f;
+    });
+  };
+  fill(q_s, q_off);
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t2 = (lane & 3) * 2;
+  const int ta = warp * 16 + g, tb = ta + 8;      // this thread's rows
+  auto query = [&](int d, unsigned (&a)[PARTS][4]) {      // the operand of 16 channels from d on
+#pragma unroll
+    for (int q = 0; q < PARTS; ++q) cm_ldmatrix(a[q], q_s + q * k_part + (warp * 16 + (lane & 15)) * k_stride + d + (lane >> 4) * 8);
+  };
+  float o[8][4], o_small[8][4];
+  {
+    // decay^(t + 1) S_in^T q_t
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) o[j][i] = o_small[j][i] = 0.f;
+    for (int d = 0; d < dim; d += 16) {
+      unsigned a[PARTS][4];
+      query(d, a);
+      cm_step_rows<PARTS, 3, 8>(o, o_small, a, s_s, d, s_part);
+    }
+    const float pa = pw[ta + 1], pb = pw[tb + 1];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        o[j][i] = (o[j][i] + o_small[j][i]) * (i < 2 ? pa : pb);
+      }
+  }
+  __syncthreads();      // the state has been read
+  fill(s_s, k_off);
+  __syncthreads();
+  float sc[8][4];
+  {
+    // the scores of this warp's tokens on those up to its last one
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      float small[2][4] = {};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sc[j][i] = sc[j + 1][i] = 0.f;
+      if (j > 2 * warp) continue;
+      for (int d = 0; d < dim; d += 16) {
+        unsigned a[PARTS][4], b[PARTS][4];
+        query(d, a);
+        // (matrices: tokens 8 j.. of channels d.., of channels d + 8.., then tokens 8 j + 8..)
+        const __nv_bfloat16* at = s_s + (8 * j + (lane & 7) + (lane >> 4) * 8) * k_stride + d + (lane >> 3 & 1) * 8;
+#pragma unroll
+        for (int q = 0; q < PARTS; ++q) cm_ldmatrix(b[q], at + q * k_part);
+        cm_products<PARTS, PARTS>(sc[j], small[0], sc[j + 1], small[1], a, b);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        sc[j][i] += small[0][i];
+        sc[j + 1][i] += small[1][i];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int t = i < 2 ? ta : tb, at = 8 * j + t2 + (i & 1);
+        sc[j][i] = at <= t ? sc[j][i] * pw[t - at] : 0.f;
+      }
+  }
+  __syncthreads();      // k has been read
+  cm_fill<PARTS>(s_s, CM_CHUNK, CM_COLS, CM_ROW, s_part, [&](int t, int c, float (&x)[8]) {
+    const bool in = t < len && col0 + c < vdim;
+    if (in) cm_load8(rows + t * row_stride + v_off + head * vdim + col0 + c, x);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = in ? cm_feature(x[u], act) : 0.f;
+  });
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o_small[j][i] = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {      // 16 tokens s at a time
+    if (j > warp) break;
+    unsigned a[3][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      unsigned part[3];
+      cm_split<3>(sc[2 * j + (i >> 1)][2 * (i & 1)], sc[2 * j + (i >> 1)][2 * (i & 1) + 1], part);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) a[q][i] = part[q];
+    }
+    cm_step_rows<3, PARTS, 8>(o, o_small, a, s_s, 16 * j, s_part);
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int c = 8 * j + t2;
+    if (col0 + c >= vdim) break;
+    float* at = out + row0 * out_row_stride + (long long)head * vdim + col0 + c;
+    if (ta < len) *reinterpret_cast<float2*>(at + ta * out_row_stride) = make_float2(o[j][0] + o_small[j][0], o[j][1] + o_small[j][1]);
+    if (tb < len) *reinterpret_cast<float2*>(at + tb * out_row_stride) = make_float2(o[j][2] + o_small[j][2], o[j][3] + o_small[j][3]);
+  }
+}
+
+template <typename T, int PARTS>
+static int launch_lightning_mma(const T* proj, long long row_stride, int q_off, int k_off, int v_off, float* state, const int* slots,
+                                const int* seq_start, const float* decay, float* out, long long out_row_stride, float* scratch,
+                                int max_chunks, int n_seqs, int n_heads, int dim, int vdim, int act, cudaStream_t stream) {
+  const int col_blocks = (vdim + CM_COLS - 1) / CM_COLS;
+  const dim3 grid(max_chunks, n_heads * col_blocks, n_seqs), block(CM_THREADS);
+  const size_t rows_k = (size_t)CM_CHUNK * (dim + 8), rows_v = (size_t)CM_CHUNK * CM_ROW;
+  const size_t smem_s = 2 * (3 * rows_k + PARTS * rows_v), rows_s = 3 * (size_t)(dim > CM_CHUNK ? dim : CM_CHUNK) * CM_ROW;
+  const size_t smem_o = 2 * (PARTS * rows_k + (rows_s > PARTS * rows_k ? rows_s : PARTS * rows_k));
+  static SharedMemoryAllowance allowed_s, allowed_o;
+  BT_CHECK(allow_shared_memory(allowed_s, lightning_state_kernel<T, PARTS>, smem_s) &&
+               allow_shared_memory(allowed_o, lightning_out_kernel<T, PARTS>, smem_o),
+           "lightning_scan: cannot reserve %zu bytes of shared memory", smem_s > smem_o ? smem_s : smem_o);
+  BT_PDL_OK("lightning_state", launch_pdl(lightning_state_kernel<T, PARTS>, grid, block, smem_s, stream, 1, proj, row_stride, k_off, v_off,
+                                          seq_start, decay, scratch, max_chunks, n_heads, dim, vdim, col_blocks, act));
+  if ((unsigned long long)state % 16 == 0)
+    BT_PDL_OK("lightning_prefix", launch_pdl(lightning_prefix_vec_kernel, dim3((dim * vdim + 511) / 512, n_heads, n_seqs), dim3(128), 0,
+                                             stream, 1, scratch, state, slots, seq_start, decay, max_chunks, n_heads, dim, vdim));
+  else
+    BT_PDL_OK("lightning_prefix", launch_pdl(lightning_prefix_kernel, dim3((dim * vdim + 255) / 256, n_heads, n_seqs), dim3(256), 0,
+                                             stream, 1, scratch, state, slots, seq_start, decay, max_chunks, n_heads, dim, vdim));
+  BT_PDL_OK("lightning_out", launch_pdl(lightning_out_kernel<T, PARTS>, grid, block, smem_o, stream, 1, proj, row_stride, q_off, k_off,
+                                        v_off, seq_start, decay, out, out_row_stride, (const float*)scratch, max_chunks, n_heads, dim,
+                                        vdim, col_blocks, act));
+  return 0;
+}
+
 template <typename T>
 static int launch_lightning_chunked(const T* proj, long long row_stride, int q_off, int k_off, int v_off, float* state,
                                     const int* slots, const int* seq_start, const float* decay, float* out,
@@ -461,6 +713,16 @@ static int launch_lightning_chunked(const T* proj, long long row_stride, int q_o
   constexpr int V = 16 / (int)sizeof(T);
   const int vec = dim % V == 0 && vdim % V == 0 && q_off % V == 0 && k_off % V == 0 && v_off % V == 0 && row_stride % V == 0 &&
                   out_row_stride % 4 == 0 && ((unsigned long long)proj | (unsigned long long)out | (unsigned long long)scratch) % 16 == 0;
+  // (below a block a multiprocessor, x * sigmoid(x) by a block's 128 threads takes longer than what the products save: three heads of
+  // 128 x 96 over 700 tokens, 66 blocks, 50 us against 40; 48 blocks 29 against 25; 272 blocks 46 against 50)
+  if (vec && dim % 16 == 0 && dim <= 128 && (act != 0 || (long long)max_chunks * n_heads * col_blocks * n_seqs >= sm_count()) && q_off % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0 && vdim % 8 == 0) {
+    if constexpr (sizeof(T) == 2)
+      if (act == 1)
+        return launch_lightning_mma<T, 1>(proj, row_stride, q_off, k_off, v_off, state, slots, seq_start, decay, out, out_row_stride,
+                                          scratch, max_chunks, n_seqs, n_heads, dim, vdim, act, stream);
+    return launch_lightning_mma<T, 3>(proj, row_stride, q_off, k_off, v_off, state, slots, seq_start, decay, out, out_row_stride,
+                                      scratch, max_chunks, n_seqs, n_heads, dim, vdim, act, stream);
+  }
   auto chunk_kernel = lightning_chunk_kernel<T>;
   auto carry_kernel = lightning_carry_kernel<T>;
   if (smem_a > 48 * 1024)
