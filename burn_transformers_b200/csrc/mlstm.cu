@@ -13,6 +13,7 @@
 // block keeps its own copy (the block of the first channel group writes them back).  A value channel belongs to SPLIT
 // adjacent lanes, each with DPT of the head's key channels; partial sums meet by shuffles.
 // State: s[slot][head][dim][vdim], n[slot][head][dim], m[slot][head]; a sequence that starts finds zeros there.
+#include "chunk_mma.cuh"
 #include "common.cuh"
 
 namespace bt {
@@ -507,6 +508,43 @@ __global__ void __launch_bounds__(256) mlstm_prefix_kernel(MlstmChunked c) {
   *st = s;
 }
 
+// The same, four neighbouring elements a thread and eight chunks asked for at a time, where rows of S and n are whole pieces of 16
+// bytes on such boundaries (12 to 6 us beside other work at 2 x 1,024 tokens).
+__global__ void __launch_bounds__(128) mlstm_prefix_vec_kernel(MlstmChunked c) {
+  const MlstmArgs& p = c.a;
+  pdl_trigger();
+  pdl_wait();
+  const int seq = blockIdx.z, head = blockIdx.y, H = p.n_heads, dim = p.dim, vdim = p.vdim;
+  const int e = (blockIdx.x * 128 + threadIdx.x) * 4;
+  if (e >= dim * (vdim + 1)) return;
+  const int n_new = p.seq_start[seq + 1] - p.seq_start[seq];
+  const int n_chunks = (n_new + MC - 1) / MC;
+  const long long slot_head = (long long)p.slots[seq] * H + head;
+  const bool is_s = e < dim * vdim;
+  float* st = is_s ? p.s + slot_head * dim * vdim + e : p.n + slot_head * dim + (e - dim * vdim);
+  const long long base = ((long long)seq * c.max_chunks) * H + head;
+  float* cell = is_s ? c.ds + base * dim * vdim + e : c.dn + base * dim + (e - dim * vdim);
+  const long long stride = (long long)H * (is_s ? dim * vdim : dim);
+  float4 s = *reinterpret_cast<float4*>(st);
+  for (int k = 0; k < n_chunks; k += 8) {
+    float4 kv[8];
+    float f[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      kv[u] = k + u < n_chunks ? __ldcg(reinterpret_cast<const float4*>(cell + (k + u) * stride)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      f[u] = k + u < n_chunks ? c.carry[base + (long long)(k + u) * H] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (k + u < n_chunks) {
+        *reinterpret_cast<float4*>(cell + (k + u) * stride) = s;
+        s = make_float4(fmaf(f[u], s.x, kv[u].x), fmaf(f[u], s.y, kv[u].y), fmaf(f[u], s.z, kv[u].z), fmaf(f[u], s.w, kv[u].w));
+      }
+    }
+  }
+  *reinterpret_cast<float4*>(st) = s;
+}
+
 // out[t] = (out[t] + f_t S_in^T q_t) / (max(|den_t + f_t n_in . q_t|, exp(-m_t)) + 1e-6), f_t = exp(c_t + m_in - m_t);
 // grid and blocks as mlstm_chunk_kernel.
 template <typename T>
@@ -606,6 +644,224 @@ __global__ void __launch_bounds__(256) mlstm_carry_kernel(const T* __restrict__ 
   }
 }
 
+// The chunks on tensor cores (chunk_mma.cuh), for rows on 16-byte boundaries with channels in whole operand tiles: first every
+// chunk's contribution to S and n, then mlstm_prefix_kernel, then all of o at once, which is written once.  bfloat16 q, k and v go
+// in as they are; the weights, the state and n in three parts.  The whole chain (gates, the
+// three kernels) at 2 x 1,024 tokens of 16 heads of 64 x 64 takes 81 us with the kernels above and 49 so, 32-bit rows 86 and 62,
+// 6 x 1,000 of 12 heads 122 and 76, one run of 400 44 and 32; errors against 64 bits are those of the kernels above.
+template <typename T>
+__global__ void __launch_bounds__(CM_THREADS, 4) mlstm_state_kernel(const T* __restrict__ proj, MlstmChunked c) {
+  constexpr int PARTS = sizeof(T) == 2 ? 1 : 3;
+  const MlstmArgs& p = c.a;
+  const int dim = p.dim, vdim = p.vdim, H = p.n_heads;
+  extern __shared__ __align__(16) unsigned char cm_smem[];
+  __nv_bfloat16* k_s = reinterpret_cast<__nv_bfloat16*>(cm_smem);      // [3][64][dim + 8]: exp(c_L - c_s + a_s - m_L) k_s
+  const int k_stride = dim + 8, k_part = CM_CHUNK * k_stride, v_part = CM_CHUNK * CM_ROW;
+  __nv_bfloat16* v_s = k_s + 3 * k_part;                               // [PARTS][64][72]
+  __shared__ float w_end[CM_CHUNK];
+  pdl_trigger();
+  pdl_wait();
+  const int chunk = blockIdx.x, seq = blockIdx.z;
+  const int head = blockIdx.y / c.col_blocks, col_block = blockIdx.y - head * c.col_blocks, col0 = col_block * CM_COLS;
+  const int first = p.seq_start[seq], n_new = p.seq_start[seq + 1] - first;
+  if (chunk * MC >= n_new) return;
+  const int len = min(MC, n_new - chunk * MC);
+  const long long row0 = first + (long long)chunk * MC;
+  const T* rows = proj + row0 * p.row_stride;
+  if (threadIdx.x < MC) {
+    const long long g = (row0 + threadIdx.x) * H + head, gl = (row0 + len - 1) * H + head;
+    w_end[threadIdx.x] = threadIdx.x < len ? expf(c.gc[gl] - c.gm[gl] + c.ga[g] - c.gc[g]) : 0.f;
+  }
+  __syncthreads();
+  cm_fill<3>(k_s, MC, dim, k_stride, k_part, [&](int t, int ch, float (&x)[8]) {
+    if (t < len) cm_load8(rows + t * p.row_stride + p.k_off + head * dim + ch, x);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = t < len ? x[u] * w_end[t] : 0.f;
+  });
+  cm_fill<PARTS>(v_s, MC, CM_COLS, CM_ROW, v_part, [&](int t, int ch, float (&x)[8]) {
+    const bool in = t < len && col0 + ch < vdim;
+    if (in) cm_load8(rows + t * p.row_stride + p.v_off + head * vdim + col0 + ch, x);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = in ? x[u] : 0.f;
+  });
+  __syncthreads();
+  const long long cell = ((long long)seq * c.max_chunks + chunk) * H + head;
+  float* dst = c.ds + cell * dim * vdim + col0;
+  cm_state<3, PARTS, true>(k_s, k_stride, k_part, v_s, v_part, dim,
+                           [&](int d, int ch, float x, float y) {
+                             if (col0 + ch < vdim) *reinterpret_cast<float2*>(dst + (long long)d * vdim + ch) = make_float2(x, y);
+                           },
+                           [&](int d, float sum) {
+                             if (col_block == 0) c.dn[cell * dim + d] = sum;
+                           });
+}
+
+template <typename T>
+__global__ void __launch_bounds__(CM_THREADS, 4) mlstm_out_kernel(const T* __restrict__ proj, MlstmChunked c) {
+  constexpr int PARTS = sizeof(T) == 2 ? 1 : 3;
+  const MlstmArgs& p = c.a;
+  const int dim = p.dim, vdim = p.vdim, H = p.n_heads;
+  extern __shared__ __align__(16) unsigned char cm_smem[];
+  const int k_stride = dim + 8, k_part = CM_CHUNK * k_stride, s_part = max(dim, CM_CHUNK) * CM_ROW;
+  __nv_bfloat16* k_s = reinterpret_cast<__nv_bfloat16*>(cm_smem);      // [PARTS][64][dim + 8]
+  __nv_bfloat16* q_s = k_s + PARTS * k_part;                           // [PARTS][64][dim + 8]
+  __nv_bfloat16* s_s = q_s + PARTS * k_part;                           // [3][dim][72] the state and, in column 64, n; then [PARTS][64][72] v
+  __shared__ float g_a[MC], g_c[MC], f_s[MC], floor_s[MC];             // a_s - c_s, c_t - m_t, exp(c_t + m_in - m_t), exp(-m_t)
+  pdl_trigger();
+  pdl_wait();
+  const int chunk = blockIdx.x, seq = blockIdx.z;
+  const int head = blockIdx.y / c.col_blocks, col0 = (blockIdx.y - head * c.col_blocks) * CM_COLS;
+  const int first = p.seq_start[seq], n_new = p.seq_start[seq + 1] - first;
+  if (chunk * MC >= n_new) return;
+  const int len = min(MC, n_new - chunk * MC);
+  const long long row0 = first + (long long)chunk * MC;
+  const T* rows = proj + row0 * p.row_stride;
+  const long long cell = ((long long)seq * c.max_chunks + chunk) * H + head;
+  if (threadIdx.x < MC) {
+    float ga = 0.f, gc = 0.f, gm = 0.f;
+    if (threadIdx.x < len) {
+      const long long g = (row0 + threadIdx.x) * H + head;
+      ga = c.ga[g]; gc = c.gc[g]; gm = c.gm[g];
+    }
+    g_a[threadIdx.x] = ga - gc;
+    g_c[threadIdx.x] = gc - gm;
+    f_s[threadIdx.x] = threadIdx.x < len ? expf(gc + c.m_start[cell] - gm) : 0.f;
+    floor_s[threadIdx.x] = expf(-gm);
+  }
+  const float* src = c.ds + cell * dim * vdim + col0;
+  cm_fill<3>(s_s, dim, CM_ROW, CM_ROW, s_part, [&](int d, int ch, float (&x)[8]) {
+    const bool state = ch < CM_COLS && col0 + ch < vdim;
+    if (state) cm_load8(src + (long long)d * vdim + ch, x);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = state ? x[u] : 0.f;
+    if (ch == CM_COLS) x[0] = c.dn[cell * dim + d];
+  });
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    cm_fill<PARTS>(i ? q_s : k_s, MC, dim, k_stride, k_part, [&](int t, int ch, float (&x)[8]) {
+      if (t < len) cm_load8(rows + t * p.row_stride + (i ? p.q_off : p.k_off) + head * dim + ch, x);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = t < len ? x[u] : 0.f;
+    });
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t2 = (lane & 3) * 2;
+  const int ta = warp * 16 + g, tb = ta + 8;      // this thread's rows
+  auto query = [&](int d, unsigned (&a)[PARTS][4]) {      // the operand of 16 channels from d on
+#pragma unroll
+    for (int q = 0; q < PARTS; ++q) cm_ldmatrix(a[q], q_s + q * k_part + (warp * 16 + (lane & 15)) * k_stride + d + (lane >> 4) * 8);
+  };
+  float o[8][4], o_small[8][4], div_a, div_b;
+  {
+    // f_t S_in^T q_t and f_t n_in . q_t
+    float nq[4] = {}, nq_small[4] = {};
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) o[j][i] = o_small[j][i] = 0.f;
+    for (int d = 0; d < dim; d += 16) {
+      unsigned a[PARTS][4];
+      query(d, a);
+      cm_step_rows<PARTS, 3, 8>(o, o_small, a, s_s, d, s_part);
+#pragma unroll
+      for (int pb = 2; pb >= 0; --pb) {
+        unsigned b0, b1;
+        asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(b0), "=r"(b1)
+                     : "r"((unsigned)__cvta_generic_to_shared(s_s + pb * s_part + (d + (lane & 15)) * CM_ROW + CM_COLS)) : "memory");
+#pragma unroll
+        for (int pa = 0; pa < PARTS; ++pa)
+          if (pa + pb <= 2) cm_mma(pa + pb == 0 ? nq : nq_small, a[pa], b0, b1);
+      }
+    }
+    const float fa = f_s[ta] * p.q_scale, fb = f_s[tb] * p.q_scale;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        o[j][i] = (o[j][i] + o_small[j][i]) * (i < 2 ? fa : fb);
+      }
+    div_a = __shfl_sync(0xffffffffu, nq[0] + nq_small[0], lane & ~3) * fa;
+    div_b = __shfl_sync(0xffffffffu, nq[2] + nq_small[2], lane & ~3) * fb;
+  }
+  float sc[8][4];
+  {
+    // the weighted scores of this warp's tokens on those up to its last one, and their sums
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      float small[2][4] = {};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sc[j][i] = sc[j + 1][i] = 0.f;
+      if (j > 2 * warp) continue;
+      for (int d = 0; d < dim; d += 16) {
+        unsigned a[PARTS][4], b[PARTS][4];
+        query(d, a);
+        // (matrices: tokens 8 j.. of channels d.., of channels d + 8.., then tokens 8 j + 8..)
+        const __nv_bfloat16* at = k_s + (8 * j + (lane & 7) + (lane >> 4) * 8) * k_stride + d + (lane >> 3 & 1) * 8;
+#pragma unroll
+        for (int q = 0; q < PARTS; ++q) cm_ldmatrix(b[q], at + q * k_part);
+        cm_products<PARTS, PARTS>(sc[j], small[0], sc[j + 1], small[1], a, b);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        sc[j][i] += small[0][i];
+        sc[j + 1][i] += small[1][i];
+      }
+    }
+    float den_a = 0.f, den_b = 0.f;
+    const float ca = g_c[ta], cb = g_c[tb];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int t = i < 2 ? ta : tb, at = 8 * j + t2 + (i & 1);
+        sc[j][i] = at <= t && t < len ? sc[j][i] * p.q_scale * expf((i < 2 ? ca : cb) + g_a[at]) : 0.f;
+        if (i < 2) den_a += sc[j][i];
+        else den_b += sc[j][i];
+      }
+#pragma unroll
+    for (int x = 1; x < 4; x <<= 1) {
+      den_a += __shfl_xor_sync(0xffffffffu, den_a, x);
+      den_b += __shfl_xor_sync(0xffffffffu, den_b, x);
+    }
+    div_a = fmaxf(fabsf(den_a + div_a), floor_s[ta]) + 1e-6f;
+    div_b = fmaxf(fabsf(den_b + div_b), floor_s[tb]) + 1e-6f;
+  }
+  __syncthreads();      // the state has been read
+  cm_fill<PARTS>(s_s, MC, CM_COLS, CM_ROW, s_part, [&](int t, int ch, float (&x)[8]) {
+    const bool in = t < len && col0 + ch < vdim;
+    if (in) cm_load8(rows + t * p.row_stride + p.v_off + head * vdim + col0 + ch, x);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = in ? x[u] : 0.f;
+  });
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o_small[j][i] = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {      // 16 tokens s at a time
+    if (j > warp) break;
+    unsigned a[3][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      unsigned part[3];
+      cm_split<3>(sc[2 * j + (i >> 1)][2 * (i & 1)], sc[2 * j + (i >> 1)][2 * (i & 1) + 1], part);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) a[q][i] = part[q];
+    }
+    cm_step_rows<3, PARTS, 8>(o, o_small, a, s_s, 16 * j, s_part);
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int ch = 8 * j + t2;
+    if (col0 + ch >= vdim) break;
+    float* at = p.out + row0 * p.out_row_stride + (long long)head * vdim + col0 + ch;
+    if (ta < len)
+      *reinterpret_cast<float2*>(at + ta * p.out_row_stride) = make_float2((o[j][0] + o_small[j][0]) / div_a, (o[j][1] + o_small[j][1]) / div_a);
+    if (tb < len)
+      *reinterpret_cast<float2*>(at + tb * p.out_row_stride) = make_float2((o[j][2] + o_small[j][2]) / div_b, (o[j][3] + o_small[j][3]) / div_b);
+  }
+}
+
 static long long mlstm_scratch_floats(long long n_rows, int n_seqs, int max_new, int n_heads, int dim, int vdim) {
   const long long chunks = (max_new + MC - 1) / MC;
   const long long cells = (long long)n_seqs * chunks * n_heads;
@@ -634,6 +890,26 @@ static int launch_mlstm_chunked(const T* proj, MlstmArgs p, float* scratch, long
   constexpr int V = 16 / (int)sizeof(T);
   c.vec = p.dim % V == 0 && p.vdim % V == 0 && p.q_off % V == 0 && p.k_off % V == 0 && p.v_off % V == 0 && p.row_stride % V == 0 &&
           p.out_row_stride % 4 == 0 && ((unsigned long long)proj | (unsigned long long)p.out | (unsigned long long)c.ds) % 16 == 0;
+  // (with few blocks the chain of a block counts, and 256 threads make it shorter: 60 blocks 30 us against 27; 64 blocks 36 against 46)
+  if (c.vec && p.dim % 16 == 0 && p.dim <= 128 && (long long)c.max_chunks * p.n_heads * c.col_blocks * n_seqs * 7 >= sm_count() * 3 && p.vdim % 8 == 0 && p.q_off % 8 == 0 && p.k_off % 8 == 0 && p.v_off % 8 == 0) {
+    constexpr int PARTS = sizeof(T) == 2 ? 1 : 3;
+    const dim3 cells(c.max_chunks, p.n_heads * c.col_blocks, n_seqs);
+    const size_t rows_k = (size_t)MC * (p.dim + 8), rows_s = (size_t)(p.dim > MC ? p.dim : MC) * CM_ROW;
+    const size_t smem_s = 2 * (3 * rows_k + PARTS * (size_t)MC * CM_ROW), smem_o = 2 * (2 * PARTS * rows_k + 3 * rows_s);
+    static SharedMemoryAllowance allowed_s, allowed_o;
+    BT_CHECK(allow_shared_memory(allowed_s, mlstm_state_kernel<T>, smem_s) && allow_shared_memory(allowed_o, mlstm_out_kernel<T>, smem_o),
+             "mlstm_scan: cannot reserve %zu bytes of shared memory", smem_s > smem_o ? smem_s : smem_o);
+    BT_PDL_OK("mlstm_gates", launch_pdl(mlstm_gates_kernel<T>, dim3(p.n_heads, n_seqs), dim3(256), 0, stream, 1, proj, c));
+    BT_PDL_OK("mlstm_state", launch_pdl(mlstm_state_kernel<T>, cells, dim3(CM_THREADS), smem_s, stream, 1, proj, c));
+    if (((unsigned long long)p.s | (unsigned long long)p.n | (unsigned long long)c.dn) % 16 == 0)
+      BT_PDL_OK("mlstm_prefix", launch_pdl(mlstm_prefix_vec_kernel, dim3((p.dim * (p.vdim + 1) + 511) / 512, p.n_heads, n_seqs), dim3(128),
+                                           0, stream, 1, c));
+    else
+      BT_PDL_OK("mlstm_prefix", launch_pdl(mlstm_prefix_kernel, dim3((p.dim * (p.vdim + 1) + 255) / 256, p.n_heads, n_seqs), dim3(256),
+                                           0, stream, 1, c));
+    BT_PDL_OK("mlstm_out", launch_pdl(mlstm_out_kernel<T>, cells, dim3(CM_THREADS), smem_o, stream, 1, proj, c));
+    return 0;
+  }
   const dim3 grid(c.max_chunks, p.n_heads * c.col_blocks, n_seqs), block(256);
   const size_t smem_a = ((size_t)2 * p.dim * MCP + (size_t)MC * 64 + (size_t)MC * MCP + 3 * MC) * sizeof(float);
   const size_t smem_c = ((size_t)p.dim * MCP + (size_t)p.dim * 64 + p.dim + 2 * MC) * sizeof(float);
