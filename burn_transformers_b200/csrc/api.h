@@ -78,6 +78,10 @@ int bt_head_rows_tcgen05(const void* a, long long a_row, const void* w, void* ou
                          int M, int heads, int N, int K, cudaStream_t stream);
 int bt_linear_tcgen05(const void* a, const void* w, const float* bias, const float* residual, void* out, int* status,
                       int M, int N, int K, int act, int out_is_f32, cudaStream_t stream);
+// out[M, inner] = rule(gate) * up, gate and up the halves of a[M, K] @ w[2 inner, K]^T, all bfloat16.
+int bt_gated_tcgen05_supports(int M, int inner, int K);
+int bt_gated_tcgen05(const void* a, const void* w, void* out, int* status, int M, int inner, int K, int act, float limit,
+                     cudaStream_t stream);
 // out[M, N] = act(x[M, K] @ w[N, K]^T + bias) (+ residual) for at most 128 bfloat16 rows over large weights, on the
 // tcgen05 tensor cores with the weights on their M side; split: blocks per cluster along K (0: chosen from the shape).
 int bt_linear_few_tcgen05_supports(int M, int N, int K);

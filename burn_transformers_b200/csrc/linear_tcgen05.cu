@@ -44,14 +44,45 @@ struct TcParams {
   int head_cols;
   long long out_row, head_stride;
   int band;                 // tiles of rows that go over all columns before the next rows are begun (at least 1)
+  // a gated product (bfloat16 results of N / 2 columns): W's first N / 2 rows are the gate's, the others up's
+  float limit;
 };
 
+
+// A warp's 32 rows of 32 numbers as bfloat16: a thread's 64-byte row goes into the patch (rows 80 bytes apart: no bank conflicts),
+// then lane 4 r + c writes 16 bytes of rows r, r + 8, r + 16, r + 24: four lanes cover a row's 64 bytes, an instruction 8 lines
+// instead of 32.  dst: the first column of row 0; rows from row0 on, up to `rows`, are written.
+__device__ __forceinline__ void tc_store32(unsigned char* patch, int stride, const float (&v)[32], int lane, __nv_bfloat16* dst,
+                                           long long row_stride, int row0, int rows) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint4 x;
+    x.x = tc_pack(v[8 * j], v[8 * j + 1]);
+    x.y = tc_pack(v[8 * j + 2], v[8 * j + 3]);
+    x.z = tc_pack(v[8 * j + 4], v[8 * j + 5]);
+    x.w = tc_pack(v[8 * j + 6], v[8 * j + 7]);
+    *reinterpret_cast<uint4*>(patch + lane * stride + 16 * j) = x;
+  }
+  __syncwarp();
+  const int cq = lane & 3, rq = lane >> 2;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int r = rq + 8 * k;
+    const uint4 x = *reinterpret_cast<const uint4*>(patch + r * stride + 16 * cq);
+    if (row0 + r < rows) *reinterpret_cast<uint4*>(dst + (long long)(row0 + r) * row_stride + 8 * cq) = x;
+  }
+  __syncwarp();      // the patch is free again
+}
 
 // Persistent: a block walks over output tiles (tile, tile + grid, ...).  The accumulator is double-buffered in
 // tensor memory (2 x BN columns), so the epilogue of one tile runs while the products of the next are issued.
 // Shared memory: STAGES x (A tile 128 x 64, W tile BN x 64), each tile 1024-byte aligned, then a 32 x 20 float
 // patch per epilogue warp through which accumulator rows are turned into coalesced global rows.
-template <int BN, int STAGES, bool PAIR>
+// GATED: half of a tile's BN rows of W are the gate's and half up's, of the same BN / 2 columns of the result (each block of a
+// pair loads one of the halves), so that the epilogue has both numbers of a result and writes rule(gate) * up: the rows of 2 N
+// numbers between the product and an activation kernel, written and read again, are gone.  2,048 rows of 5,632 x 1,024
+// and the activation in a recorded layer: 20 and 12 us as two kernels, 24 as one.
+template <int BN, int STAGES, bool PAIR, bool GATED>
 __global__ void __launch_bounds__(TC_THREADS)
 linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, TcParams p) {
   extern __shared__ unsigned char tc_smem_raw[];
@@ -72,6 +103,11 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const int tiles_m = (p.M + BM - 1) / BM, tiles_n = (p.N + BN - 1) / BN;
   const int n_tiles = tiles_m * tiles_n;
   const int k_blocks = (p.K + TC_BK - 1) / TC_BK;
+  // the first row of W that this block loads for the tn-th tile of columns, of half `h` where it loads two
+  auto w_row = [&](int tn, int h) {
+    if constexpr (GATED) return tn * (BN / 2) + (PAIR ? rank : h) * (p.N / 2);
+    else return tn * BN + rank * W_ROWS;
+  };
   // Where a tile lies: bands of `band` tiles of rows, a band's rows first, then its columns (the band's A comes from L2 then)
   auto place = [&](int tile, int& tm, int& tn) {
     const int b = tile / (p.band * tiles_n), first = b * p.band, in_band = tile - first * tiles_n;
@@ -122,13 +158,18 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         if constexpr (PAIR) tc_tma_load_pair(dst, weights ? &map_w : &map_a, kb * TC_BK, row, tc_first_block(&full[s]));
         else tc_tma_load(dst, weights ? &map_w : &map_a, kb * TC_BK, row, &full[s]);
       };
+      auto load_w = [&](int s, int kb, int tn) {
+        load(s, true, kb, w_row(tn, 0));
+        if constexpr (GATED && !PAIR)
+          tc_tma_load(tiles + (size_t)s * (A_BYTES + W_BYTES) + A_BYTES + W_BYTES / 2, &map_w, kb * TC_BK, w_row(tn, 1), &full[s]);
+      };
       {
         int tm = 0, tn = 0;
         place(tile0, tm, tn);
-        const int m0 = tm * BM + rank * TC_BM, n0 = tn * BN + rank * W_ROWS;
+        const int m0 = tm * BM + rank * TC_BM;
         for (int kb = 0; kb < pre; ++kb) {
           expect(kb);
-          load(kb, true, kb, n0);
+          load_w(kb, kb, tn);
         }
         pdl_wait();
         for (int kb = 0; kb < pre; ++kb) load(kb, false, kb, m0);
@@ -139,7 +180,7 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       for (int tile = tile0; tile < n_tiles; tile += tile_step, kb = 0) {
         int tm, tn;
         place(tile, tm, tn);
-        const int m0 = tm * BM + rank * TC_BM, n0 = tn * BN + rank * W_ROWS;
+        const int m0 = tm * BM + rank * TC_BM;
         for (; kb < k_blocks; ++kb) {
           if (!tc_bar_wait(&empty[s], parity)) {
             failed = 1;
@@ -148,7 +189,7 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           }
           expect(s);
           load(s, false, kb, m0);
-          load(s, true, kb, n0);
+          load_w(s, kb, tn);
           if (++s == STAGES) {
             s = 0;
             parity ^= 1u;
@@ -230,11 +271,29 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       const int row = m0 + quarter * 32 + lane;
       const bool row_ok = row < p.M;
       // (the first warp of a quarter takes the larger part when the 32-column chunks are an odd number)
-      constexpr int SPLIT = (BN / 32 + 1) / 2 * 32;
+      constexpr int COLS = GATED ? BN / 2 : BN;      // of the result
+      constexpr int SPLIT = (COLS / 32 + 1) / 2 * 32;
 #pragma unroll 1
-      for (int c0 = half ? SPLIT : 0; c0 < (half ? BN : SPLIT); c0 += 32) {
+      for (int c0 = half ? SPLIT : 0; c0 < (half ? COLS : SPLIT); c0 += 32) {
         float v[32];
         tc_ld32(tmem_acc + ((unsigned)(quarter * 32) << 16) + (unsigned)(buf * ACC + c0), v);
+        if constexpr (GATED) {
+          float up[32];
+          tc_ld32(tmem_acc + ((unsigned)(quarter * 32) << 16) + (unsigned)(buf * ACC + COLS + c0), up);
+          const int cols = p.N / 2, col0 = tn * COLS + c0;
+          if (col0 >= cols) continue;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = tc_gated(v[i], up[i], p.act, p.limit);
+          __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out);
+          if (cols % 8 == 0 && col0 + 32 <= cols) {
+            tc_store32(reinterpret_cast<unsigned char*>(patch), TC_PATCH_STRIDE * 4, v, lane, out + col0, cols, m0 + quarter * 32, p.M);
+          } else if (row_ok) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (col0 + i < cols) out[(long long)row * cols + col0 + i] = __float2bfloat16_rn(v[i]);
+          }
+          continue;
+        }
         const int col0 = n0 + c0;
         if (col0 >= p.N) continue;                 // (uniform in the warp; the load above is collective)
         const long long o0 = (long long)row * p.N + col0;
@@ -300,31 +359,11 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
               *reinterpret_cast<float4*>(dst + 4 * j) = x;
             }
           } else {
-            // bfloat16: the thread's 64-byte row goes into the patch (rows 80 bytes apart: no bank conflicts), then
-            // lane 4 r + c writes 16 bytes of rows r, r + 8, r + 16, r + 24: four lanes cover a row's 64 bytes,
-            // an instruction 8 lines instead of 32
-            unsigned char* patch8 = reinterpret_cast<unsigned char*>(patch);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint4 x;
-              x.x = tc_pack(v[8 * j], v[8 * j + 1]);
-              x.y = tc_pack(v[8 * j + 2], v[8 * j + 3]);
-              x.z = tc_pack(v[8 * j + 4], v[8 * j + 5]);
-              x.w = tc_pack(v[8 * j + 6], v[8 * j + 7]);
-              *reinterpret_cast<uint4*>(patch8 + lane * (TC_PATCH_STRIDE * 4) + 16 * j) = x;
-            }
-            __syncwarp();
-            const int cq = lane & 3, rq = lane >> 2;
             // (a chunk of 32 columns lies in one head)
             const int head = p.head_cols > 0 ? col0 / p.head_cols : 0;
-            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out) + head * p.head_stride + (col0 - head * p.head_cols) + 8 * cq;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const int r = rq + 8 * k, grow = m0 + quarter * 32 + r;
-              const uint4 x = *reinterpret_cast<const uint4*>(patch8 + r * (TC_PATCH_STRIDE * 4) + 16 * cq);
-              if (grow < p.M) *reinterpret_cast<uint4*>(dst + (long long)grow * p.out_row) = x;
-            }
-            __syncwarp();      // the patch is free again
+            tc_store32(reinterpret_cast<unsigned char*>(patch), TC_PATCH_STRIDE * 4, v, lane,
+                       reinterpret_cast<__nv_bfloat16*>(p.out) + head * p.head_stride + (col0 - head * p.head_cols), p.out_row,
+                       m0 + quarter * 32, p.M);
           }
         } else if (row_ok) {
           // a ragged edge, or rows that are no multiple of 16 bytes: one element at a time
@@ -376,11 +415,11 @@ constexpr TcTile TC_TILES[] = {{256, false, 8900, 296}, {192, false, 7600, 265},
                                {64, false, 5200, 233}, {256, true, 9400, 294}, {224, true, 8900, 260}, {192, true, 8400, 217},
                                {160, true, 7900, 196}, {128, true, 7400, 170}, {96, true, 6900, 167}, {64, true, 6400, 163}};
 
-template <int BN, int STAGES, bool PAIR>
+template <int BN, int STAGES, bool PAIR, bool GATED = false>
 static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mw, const TcParams& p, cudaStream_t stream) {
   constexpr size_t smem = (size_t)STAGES * (TC_BM * TC_BK * 2 + (PAIR ? BN / 2 : BN) * TC_BK * 2) + 1024 + (size_t)TC_EPI_WARPS * 32 * TC_PATCH_STRIDE * 4;
   static_assert(smem <= 227 * 1024, "a multiprocessor's shared memory");
-  auto kern = linear_tcgen05_kernel<BN, STAGES, PAIR>;
+  auto kern = linear_tcgen05_kernel<BN, STAGES, PAIR, GATED>;
   static SharedMemoryAllowance allowed;
   BT_CHECK(allow_shared_memory(allowed, kern, smem), "linear_tcgen05: cannot reserve %zu bytes of shared memory", smem);
   constexpr int GROUP = PAIR ? 2 : 1;
@@ -398,7 +437,7 @@ extern "C" int bt_linear_tcgen05_supports(int M, int N, int K) {
   return M >= 1 && N >= 8 && K >= 8 && K % 8 == 0;   // rows of A and W are 16-byte multiples
 }
 
-static int run_linear_tcgen05(const void* a, long long a_row, const void* w, bt::TcParams p, cudaStream_t stream) {
+static int run_linear_tcgen05(const void* a, long long a_row, const void* w, bt::TcParams p, bool gated, cudaStream_t stream) {
   using namespace bt;
   const int M = p.M, N = p.N, K = p.K;
   // The tile: wide ones reuse every loaded row of A for more columns, narrow ones cover the GPU with fewer idle
@@ -411,6 +450,7 @@ static int run_linear_tcgen05(const void* a, long long a_row, const void* w, bt:
   long long best = -1;
   const int k_blocks = (K + TC_BK - 1) / TC_BK;
   for (const TcTile& t : TC_TILES) {
+    if (gated && t.bn % 64 != 0) continue;      // (half of the tile's columns are whole chunks of the epilogue)
     const long long rows = t.pair ? 2 * TC_BM : TC_BM, groups = t.pair ? sms / 2 : sms;
     const long long tiles = ((M + rows - 1) / rows) * ((N + t.bn - 1) / t.bn), rounds = (tiles + groups - 1) / groups;
     // (more than three rounds: the whole GPU takes in no more than about 85 GB/s a multiprocessor)
@@ -431,7 +471,19 @@ static int run_linear_tcgen05(const void* a, long long a_row, const void* w, bt:
   p.band = (int)(band < 1 ? 1 : (band < tiles_m ? band : tiles_m));
   CUtensorMap ma, mw;
   if (int rc = tensor_map_2d_bf16(&ma, a, (unsigned long long)M, (unsigned long long)K, (unsigned long long)a_row, TC_BM)) return rc;
-  if (int rc = tensor_map_2d_bf16(&mw, w, (unsigned long long)N, (unsigned long long)K, (unsigned long long)K, (unsigned)(pair ? bn / 2 : bn))) return rc;
+  if (int rc = tensor_map_2d_bf16(&mw, w, (unsigned long long)N, (unsigned long long)K, (unsigned long long)K, (unsigned)(pair || gated ? bn / 2 : bn))) return rc;
+  if (gated && pair) {
+    if (bn == 64) return launch_tc<64, 8, true, true>(ma, mw, p, stream);
+    if (bn == 128) return launch_tc<128, 8, true, true>(ma, mw, p, stream);
+    if (bn == 192) return launch_tc<192, 7, true, true>(ma, mw, p, stream);
+    return launch_tc<256, 6, true, true>(ma, mw, p, stream);
+  }
+  if (gated) {
+    if (bn == 64) return launch_tc<64, 8, false, true>(ma, mw, p, stream);
+    if (bn == 128) return launch_tc<128, 6, false, true>(ma, mw, p, stream);
+    if (bn == 192) return launch_tc<192, 5, false, true>(ma, mw, p, stream);
+    return launch_tc<256, 4, false, true>(ma, mw, p, stream);
+  }
   if (pair) {
     if (bn == 64) return launch_tc<64, 8, true>(ma, mw, p, stream);
     if (bn == 96) return launch_tc<96, 8, true>(ma, mw, p, stream);
@@ -455,7 +507,7 @@ extern "C" int bt_linear_tcgen05(const void* a, const void* w, const float* bias
   BT_CHECK(bt_linear_tcgen05_supports(M, N, K), "linear_tcgen05: sizes M=%d N=%d K=%d are not supported", M, N, K);
   BT_CHECK(act >= 0 && act <= 2, "linear_tcgen05: unknown activation %d", act);
   BT_CHECK(!(residual && !out_is_f32), "linear_tcgen05: a residual needs a 32-bit output");
-  return run_linear_tcgen05(a, K, w, TcParams{bias, residual, out, status, M, N, K, act, out_is_f32, 0, N, 0}, stream);
+  return run_linear_tcgen05(a, K, w, TcParams{bias, residual, out, status, M, N, K, act, out_is_f32, 0, N, 0}, false, stream);
 }
 
 // Per-head rows of one product: out[h][t][:] = a[t] @ w[h]^T for heads of N numbers (a multiple of 32), all bfloat16.
@@ -469,5 +521,19 @@ extern "C" int bt_head_rows_tcgen05(const void* a, long long a_row, const void* 
   BT_CHECK(heads > 0 && bt_head_rows_tcgen05_supports(M, N, K, a_row, out_row, head_stride) &&
                ((unsigned long long)a | (unsigned long long)w | (unsigned long long)out) % 16 == 0,
            "head_rows_tcgen05: sizes or strides that are not supported (M=%d heads=%d N=%d K=%d)", M, heads, N, K);
-  return run_linear_tcgen05(a, a_row, w, TcParams{nullptr, nullptr, out, status, M, heads * N, K, 0, 0, N, out_row, head_stride}, stream);
+  return run_linear_tcgen05(a, a_row, w, TcParams{nullptr, nullptr, out, status, M, heads * N, K, 0, 0, N, out_row, head_stride}, false, stream);
+}
+
+// out[M, inner] = rule(gate) * up (gated_pair of common.cuh), gate and up the halves of a[M, K] @ w[2 inner, K]^T, all bfloat16;
+// both halves and the rule in 32 bits, the result rounded once.  act: an Activation; limit: kActSwishClamp's.
+extern "C" int bt_gated_tcgen05_supports(int M, int inner, int K) {
+  return M >= 1 && inner >= 8 && inner <= 0x3fffffff && K >= 8 && K % 8 == 0;
+}
+extern "C" int bt_gated_tcgen05(const void* a, const void* w, void* out, int* status, int M, int inner, int K, int act, float limit,
+                                cudaStream_t stream) {
+  using namespace bt;
+  BT_CHECK(bt_gated_tcgen05_supports(M, inner, K) && ((unsigned long long)a | (unsigned long long)w | (unsigned long long)out) % 16 == 0,
+           "gated_tcgen05: sizes or addresses that are not supported (M=%d inner=%d K=%d)", M, inner, K);
+  BT_CHECK(act >= kActGeluTanh && act <= kActSwish, "gated_tcgen05: unknown rule %d", act);
+  return run_linear_tcgen05(a, K, w, TcParams{nullptr, nullptr, out, status, M, 2 * inner, K, act, 0, 0, inner, 0, 0, limit}, true, stream);
 }

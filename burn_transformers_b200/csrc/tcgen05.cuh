@@ -141,6 +141,20 @@ __device__ __forceinline__ float tc_activation(float x, int act, bool exact) {
   if (act == kActGeluErf) return gelu_erf(x);
   return x;
 }
+// gated_pair (common.cuh) for results that are rounded to bfloat16: the same rules with the special-function unit's exponential and
+// reciprocal (a few units of 2^-23; the tanh form as x sigmoid(2 z)).
+__device__ __forceinline__ float tc_gated(float g, float u, int act, float limit) {
+  if (act == kActGeluErf) return gelu_erf(g) * u;
+  float e = g;
+  if (act == kActSwishClamp) {
+    g = fminf(g, limit);
+    u = fminf(fmaxf(u, -limit), limit) + 1.f;
+    e = 1.702f * g;
+  } else if (act == kActGeluTanh) {
+    e = 2.f * 0.7978845608028654f * (g + 0.044715f * g * g * g);
+  }
+  return __fdividef(g, 1.f + __expf(-e)) * u;
+}
 __device__ __forceinline__ void tc_bar_arrive(unsigned long long* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc_smem(bar)) : "memory");
 }

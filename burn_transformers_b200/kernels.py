@@ -355,6 +355,26 @@ def linear_tcgen05(a, w, bias, out, *, m, activation=None, residual=None):
                                        _stream()))
 
 
+def gated_tcgen05_supports(m, inner, k) -> bool:
+    return _supports("bt_gated_tcgen05_supports", m, inner, k)
+
+
+def gated_tcgen05(a, w, out, *, m, activation, limit: float = 0.0):
+    """out[:m] = rule(gate) * up (see gated_activation), gate and up the halves of a[:m] @ w^T on the tcgen05 tensor cores, both in
+    32 bits until the result is rounded; a [M, K], w [2 * inner, K] (the gate's rows, then up's) and out [M, inner] bfloat16."""
+    inner, k = out.shape[1], w.shape[1]
+    _need(a, "a", torch.bfloat16, (None, k))
+    _need(w, "w", torch.bfloat16, (2 * inner, k))
+    _need(out, "out", torch.bfloat16, (None, inner))
+    if a.shape[0] < m or out.shape[0] < m:
+        raise ShapeError(f"gated_tcgen05: {m} rows asked of a[{a.shape[0]}] and out[{out.shape[0]}]")
+    if activation not in PAIR_RULES:
+        raise ShapeError(f"gated_tcgen05: unknown activation {activation!r}")
+    _linear_work(m, 2 * inner, k, a, w, out)
+    _check(library().bt_gated_tcgen05(_ptr(a), _ptr(w), _ptr(out), _ptr(kernel_status(a.device)), c_int(m), c_int(inner), c_int(k),
+                                      c_int(PAIR_RULES[activation]), c_float(limit), _stream()))
+
+
 def linear_few_tcgen05_supports(m, n, k) -> bool:
     return _supports("bt_linear_few_tcgen05_supports", m, n, k)
 

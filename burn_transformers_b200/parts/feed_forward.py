@@ -1,10 +1,12 @@
 """Feed-forward parts."""
 from __future__ import annotations
 
+import torch
+
 from ..weights.spec import MATRIX, VECTOR, TensorSpec
 from .. import kernels
 from .base import FeedForward
-from .linear import linear
+from .linear import LazyNorm, linear
 
 ACTIVATIONS = ("gelu_new", "gelu")
 # rules for the (gate, up) pair of a gated feed-forward: an activation or x sigmoid(x) on the gate, or the clamped rule
@@ -47,7 +49,8 @@ class DenseFeedForward(FeedForward):
 class GatedFeedForward(FeedForward):
     """down(act(gate(x)) * up(x)), added to the residual stream; no biases.  The gate and up matrices are one product:
     `gate_up.weight` is [2 * inner, width] (stored [out, in]: the gate's rows, then up's), `down.weight` [width, inner].
-    The activation (`swish`: x sigmoid(x)) and the product of the two halves are formed in 32-bit and rounded once.  With the rule
+    The activation (`swish`: x sigmoid(x)) and the product of the two halves are formed in 32-bit and rounded once (in steps of more
+    than 64 bfloat16 rows by the product itself).  With the rule
     `swish_clamp` the hidden row is g' sigmoid(1.702 g') (u' + 1), g' = min(gate x, limit), u' = up x clamped to
     [-limit, limit]."""
 
@@ -67,16 +70,26 @@ class GatedFeedForward(FeedForward):
         return {"gate_up.weight": TensorSpec((2 * self.inner, self.width), MATRIX, ("normal", self.init_std)),
                 "down.weight": TensorSpec((self.width, self.inner), MATRIX, ("normal", self.down_init_std))}
 
+    def _one_product(self, ctx, n) -> bool:
+        """Whether the pair is formed in the product's epilogue: where `linear` would take the same tcgen05 product for many rows
+        (csrc/linear_tcgen05.cu; up to 128 rows over a long K another one is ahead by more than the activation takes)."""
+        return (ctx.dtype == torch.bfloat16 and n > 64 and not (n <= 128 and self.width >= 4096)
+                and kernels.gated_tcgen05_supports(n, self.inner, self.width))
+
     def forward(self, ctx, x, residual, store=False):
         if getattr(ctx, "program", None) is not None:
             from ..engine.program import ProgramUnsupported
             raise ProgramUnsupported("a gated feed-forward has no phase in the fused step")
         n = ctx.n_tokens
         mark = ctx.ws.mark()
-        both = ctx.ws.take((n, 2 * self.inner), ctx.dtype)
-        linear(ctx, x, self.t_gate_up_weight, None, both, m=n, w_is_nk=True)
         hidden = ctx.ws.take((n, self.inner), ctx.dtype)
-        kernels.gated_activation(both, hidden, n_rows=n, activation=self.activation, limit=self.limit)
+        if self._one_product(ctx, n):
+            kernels.gated_tcgen05(x.materialize(ctx) if isinstance(x, LazyNorm) else x, self.t_gate_up_weight, hidden, m=n,
+                                  activation=self.activation, limit=self.limit)
+        else:
+            both = ctx.ws.take((n, 2 * self.inner), ctx.dtype)
+            linear(ctx, x, self.t_gate_up_weight, None, both, m=n, w_is_nk=True)
+            kernels.gated_activation(both, hidden, n_rows=n, activation=self.activation, limit=self.limit)
         linear(ctx, hidden, self.t_down_weight, None, residual, m=n, residual=None if store else residual, w_is_nk=True)
         ctx.ws.release(mark)
 
