@@ -1,6 +1,6 @@
 // out[M,N] = act(A[M,K] @ W + bias) (+ residual), accumulated in 32-bit with plain fused
 // multiply-adds (no tensor cores, no reduced-precision matrix mode).  This is the matrix
-// product of the true 32-bit path and the fallback for shapes the tensor-core kernels refuse.
+// product of the true 32-bit path (weights with a long K: linear_split_tcgen05.cu) and the fallback for shapes the tensor-core kernels refuse.
 // W is either [K,N] with N contiguous (a Conv1D weight as stored) or [N,K] with K contiguous
 // (an embedding table used as a tied readout).  Every output element is a sum over k in an order
 // that its sizes alone decide, so a row's result does not depend on which other rows are in the call.

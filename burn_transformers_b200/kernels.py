@@ -221,8 +221,9 @@ def layernorm(x, gamma, beta, out, eps: float, rows=None, n_rows=None):
                                   c_float(eps), c_int(_code(out.dtype)), _stream()))
 
 
-def linear_simt(a, w, bias, out, *, m=None, w_is_nk=False, activation=None, residual=None):
-    """out = act(a @ w + bias) (+ residual) with 32-bit fused multiply-adds.
+def linear_simt(a, w, bias, out, *, m=None, w_is_nk=False, activation=None, residual=None, split=0):
+    """out = act(a @ w + bias) (+ residual) with 32-bit products and sums: fused multiply-adds, or, for 32-bit weights with a long K,
+    tensor cores on exact parts of the operands (`split`: how many blocks share a tile there; 0: by the sizes).
 
     a: [M, K]; w: [K, N] (or [N, K] when w_is_nk); bias: [N] float32 or None; residual: [M, N]
     float32 (may be `out` itself); out: [M, N] float32 or a's dtype.
@@ -242,6 +243,13 @@ def linear_simt(a, w, bias, out, *, m=None, w_is_nk=False, activation=None, resi
     if activation not in ACTIVATIONS:
         raise ShapeError(f"linear: unknown activation {activation!r}")
     _linear_work(m, n, k, a, w, out)
+    if (a.dtype == torch.float32 and _supports("bt_linear_split_takes", n, k, 1 if w_is_nk else 0)
+            and (a.data_ptr() | w.data_ptr()) % 16 == 0):
+        # tcgen05 with the operands in three bfloat16 parts, which hold all of their bits (csrc/linear_split_tcgen05.cu)
+        _check(library().bt_linear_split(_ptr(a), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out), _ptr(kernel_status(a.device)),
+                                         c_int(m), c_int(n), c_int(k), c_int(1 if w_is_nk else 0),
+                                         c_int(ACTIVATIONS[activation]), c_int(split), _stream()))
+        return
     _check(library().bt_linear_simt(_ptr(a), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out), c_int(m), c_int(n), c_int(k),
                                     c_int(1 if w_is_nk else 0), c_int(ACTIVATIONS[activation]), c_int(_code(a.dtype)),
                                     c_int(_code(out.dtype)), _stream()))

@@ -22,8 +22,8 @@ class LazyNorm:
 def linear(ctx, a, w, bias, out, *, m, w_is_nk=False, activation=None, residual=None):
     """out[:m] = act(a[:m] @ w + bias) (+ residual[:m]);  w is [K, N], or [N, K] when `w_is_nk`.
 
-    32-bit operands always take the plain fused-multiply-add kernel: the 32-bit path has no reduced-precision
-    matrix mode.  bfloat16 products of at most 16 rows take a weight-streaming kernel, which can also normalise
+    32-bit operands always take kernels.linear_simt, by weight either fused multiply-adds or tensor cores on exact parts of
+    the operands: the 32-bit path has no reduced-precision matrix mode.  bfloat16 products of at most 16 rows take a weight-streaming kernel, which can also normalise
     its rows on the way in; 17 to 64 rows ([N, K] weights) take the kernel that is fed by tensor-map copies (large
     weights with a short K the tcgen05 product for many rows); up to 128 rows over a large weight (any K at up to 16
     rows, a long K above) take the tcgen05 product with the weights on the M side; with more rows they run on the
