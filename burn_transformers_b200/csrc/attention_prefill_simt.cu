@@ -1,6 +1,7 @@
 // Causal attention for steps that bring several tokens per sequence, with plain 32-bit
 // arithmetic: scores, online softmax, and the value mix are all fused multiply-adds in 32-bit,
-// so this kernel serves the true 32-bit path (and any head size the tensor-core kernel refuses).
+// so this kernel serves the true 32-bit path (but for what attention_prefill_parts.cuh takes: more than a few queries of heads of 16,
+// 32, 48 or 64 channels on 16-byte boundaries) and any head size the tensor-core kernel refuses.
 // The S x S score plane is never stored.
 //
 // A block is 8 Q queries of one (sequence, head) and walks their keys in tiles of 64; a thread holds Q queries x 4 keys of the
@@ -33,19 +34,12 @@ constexpr int PF_MAXG = 4;     // groups of 64 channels: head_dim <= 256
 __host__ __device__ __forceinline__ int pf_stride(int head_dim) { return (head_dim + 3) / 4 * 4 + 4; }
 
 // G: groups of 64 channels that hold a head.  VEC: rows whose heads start on 16-byte boundaries.  Q: queries a thread holds.
+// the block's part of sequence `seq` and head `head`: queries q0 to q0 + 8 Q
 template <typename T, int G, bool VEC, int Q>
-__global__ void __launch_bounds__(PF_THREADS)
-attention_prefill_simt_kernel(const T* __restrict__ q, long long q_row_stride, KvView kv, T* __restrict__ out,
-                              const int* __restrict__ seq_start, const int* __restrict__ past_len, int n_heads,
-                              int n_kv_heads, int head_dim, float scale, int causal, int window) {
+__device__ __forceinline__ void pf_block(float* smem, const T* __restrict__ q, long long q_row_stride, const KvView& kv, T* __restrict__ out,
+                                         int seq, int head, int q0, int t0, int n_new, int past, int n_heads, int n_kv_heads, int head_dim,
+                                         float scale, int causal, int window) {
   constexpr int BQ = 8 * Q;      // queries per block
-  extern __shared__ __align__(16) float smem[];
-  const int seq = blockIdx.y, head = blockIdx.z;
-  const int t0 = seq_start[seq], n_new = seq_start[seq + 1] - t0;
-  // longest tiles first: they see the most keys
-  const int q0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * BQ;
-  if (q0 >= n_new) return;
-  const int past = past_len[seq];
   const int kv_len = past + n_new;
   const int kv_head = head / (n_heads / n_kv_heads);
   const int nq = min(BQ, n_new - q0);
@@ -275,6 +269,20 @@ attention_prefill_simt_kernel(const T* __restrict__ q, long long q_row_stride, K
 }
 
 template <typename T, int G, bool VEC, int Q>
+__global__ void __launch_bounds__(PF_THREADS)
+attention_prefill_simt_kernel(const T* __restrict__ q, long long q_row_stride, KvView kv, T* __restrict__ out,
+                              const int* __restrict__ seq_start, const int* __restrict__ past_len, int n_heads,
+                              int n_kv_heads, int head_dim, float scale, int causal, int window) {
+  extern __shared__ __align__(16) float smem[];
+  const int seq = blockIdx.y, t0 = seq_start[seq], n_new = seq_start[seq + 1] - t0;
+  // longest tiles first: they see the most keys
+  const int q0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 8 * Q;
+  if (q0 >= n_new) return;
+  pf_block<T, G, VEC, Q>(smem, q, q_row_stride, kv, out, seq, blockIdx.z, q0, t0, n_new, past_len[seq], n_heads, n_kv_heads, head_dim, scale,
+                         causal, window);
+}
+
+template <typename T, int G, bool VEC, int Q>
 static int launch_pf(const void* q, long long q_row_stride, const KvView& view, void* out, const int* seq_start, const int* past_len,
                      int n_seqs, int max_new, int n_heads, int n_kv_heads, int head_dim, float scale, int causal, int window,
                      cudaStream_t stream) {
@@ -307,6 +315,8 @@ static int launch_pf_queries(int queries, int head_dim, Args... args) {
 
 }  // namespace bt
 
+#include "attention_prefill_parts.cuh"
+
 // kv_table == nullptr selects the packed view: keys and values are read from the step's own
 // projections (k, v point at the first key/value channel of row 0, rows kv_row_stride apart).
 extern "C" int bt_attention_prefill_simt(const void* q, long long q_row_stride, const void* k, const void* v,
@@ -324,6 +334,9 @@ extern "C" int bt_attention_prefill_simt(const void* q, long long q_row_stride, 
   if (n_seqs == 0 || max_new == 0) return 0;
   KvView view{k, v, kv_table, table_stride, table_len > 0 ? table_len : 1, page_size > 0 ? page_size : 1,
               kv_row_stride, seq_start};
+  if (dtype == kF32 && attention_prefill_parts_takes(q, q_row_stride, view, out, head_dim, max_new))
+    return launch_attention_prefill_parts((const float*)q, q_row_stride, view, (float*)out, seq_start, past_len, n_seqs, max_new, n_heads,
+                                          n_kv_heads, head_dim, scale, causal, window, stream);
   // 16-byte copies need every head of every row on a 16-byte boundary
   const int piece = dtype == kF32 ? 4 : 8;
   const bool vec = head_dim % piece == 0 && ((unsigned long long)k | (unsigned long long)v) % 16 == 0 &&

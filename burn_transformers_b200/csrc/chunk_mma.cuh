@@ -20,6 +20,19 @@ __device__ __forceinline__ void cm_mma(float (&d)[4], const unsigned (&a)[4], un
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// the same from zero
+__device__ __forceinline__ void cm_mma_zero(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// (two sums an instruction)
+__device__ __forceinline__ void cm_add(float (&d)[4], const float (&x)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; i += 2)
+    asm("{\n.reg .b64 a, b;\nmov.b64 a, {%0, %1};\nmov.b64 b, {%2, %3};\nadd.rn.f32x2 a, a, b;\nmov.b64 {%0, %1}, a;\n}\n"
+        : "+f"(d[i]), "+f"(d[i + 1]) : "f"(x[i]), "f"(x[i + 1]));
+}
 __device__ __forceinline__ void cm_ldmatrix(unsigned (&r)[4], const __nv_bfloat16* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
@@ -37,8 +50,9 @@ __device__ __forceinline__ void cm_split(float x, float y, unsigned (&part)[PART
     const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
     part[q] = *reinterpret_cast<const unsigned*>(&h);
     if (q + 1 < PARTS) {
-      x -= __uint_as_float(part[q] << 16);
-      y -= __uint_as_float(part[q] & 0xffff0000u);
+      // (both differences at once; they are exact)
+      asm("{\n.reg .b64 a, b, c;\nmov.b64 a, {%0, %1};\nmov.b64 b, {%2, %3};\nmov.b64 c, {%4, %4};\nfma.rn.f32x2 a, b, c, a;\n"
+          "mov.b64 {%0, %1}, a;\n}\n" : "+f"(x), "+f"(y) : "r"(part[q] << 16), "r"(part[q] & 0xffff0000u), "r"(0xbf800000u));
     }
   }
 }
@@ -85,14 +99,11 @@ __device__ __forceinline__ void cm_products(float (&big0)[4], float (&small0)[4]
         cm_mma(small0, a[pa], b[pb][0], b[pb][1]);
         cm_mma(small1, a[pa], b[pb][2], b[pb][3]);
       } else {
-        float x[4] = {}, y[4] = {};
-        cm_mma(x, a[0], b[0][0], b[0][1]);
-        cm_mma(y, a[0], b[0][2], b[0][3]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          big0[i] += x[i];
-          big1[i] += y[i];
-        }
+        float x[4], y[4];
+        cm_mma_zero(x, a[0], b[0][0], b[0][1]);
+        cm_mma_zero(y, a[0], b[0][2], b[0][3]);
+        cm_add(big0, x);
+        cm_add(big1, y);
       }
     }
 }
