@@ -39,15 +39,29 @@ layernorm_kernel(const float* __restrict__ x, const int* __restrict__ rows, cons
 
 // The same for many rows that are not long: a warp holds one row in registers (J vectors of four per lane), so the
 // row is read once and nothing is handed over between warps.  width is a multiple of 4, at most 128 J.
-template <typename TOut, int J>
+// EARLY: gamma and beta, which no step writes, are asked for before the wait for the predecessor and held in registers: a step of few
+// rows is a chain of latencies, and from memory they are the longest of this kernel's two.  The last rows come first: the
+// kernel before wrote them last, so that of many rows more are still in L2 (16,384 x 1,600 after the residual stream was written: 34 to 30 us).
+template <typename TOut, int J, bool EARLY>
 __global__ void __launch_bounds__(256)
 layernorm_rows_kernel(const float* __restrict__ x, const int* __restrict__ rows, const float* __restrict__ gamma,
                       const float* __restrict__ beta, TOut* __restrict__ out, int n_rows, int width, float eps) {
   pdl_trigger();
-  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r = blockIdx.x * (blockDim.x >> 5) + warp;
-  if (r >= n_rows) return;
+  const int r = n_rows - 1 - (int)(blockIdx.x * (blockDim.x >> 5) + warp);
+  auto weights = [&](int j, float4& g, float4& b) {
+    const int c = (j * 32 + lane) * 4;
+    g = b = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c >= width) return;
+    g = *reinterpret_cast<const float4*>(gamma + c);
+    if (beta) b = *reinterpret_cast<const float4*>(beta + c);
+  };
+  float4 gs[EARLY ? J : 1], bs[EARLY ? J : 1];
+  if constexpr (EARLY)
+#pragma unroll
+    for (int j = 0; j < J; ++j) weights(j, gs[j], bs[j]);
+  pdl_wait();
+  if (r < 0) return;
   const float* src = x + (long long)(rows ? rows[r] : r) * width;
   float4 v[J];
 #pragma unroll
@@ -72,9 +86,13 @@ layernorm_rows_kernel(const float* __restrict__ x, const int* __restrict__ rows,
   for (int j = 0; j < J; ++j) {
     const int c = (j * 32 + lane) * 4;
     if (c < width) {
-      const float4 g = *reinterpret_cast<const float4*>(gamma + c);
-      float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (beta) b = *reinterpret_cast<const float4*>(beta + c);
+      float4 g, b;
+      if constexpr (EARLY) {
+        g = gs[j];
+        b = bs[j];
+      } else {
+        weights(j, g, b);
+      }
       const float o0 = (v[j].x - mean) * rstd * g.x + b.x, o1 = (v[j].y - mean) * rstd * g.y + b.y;
       const float o2 = (v[j].z - mean) * rstd * g.z + b.z, o3 = (v[j].w - mean) * rstd * g.w + b.w;
       if constexpr (sizeof(TOut) == 4) {
@@ -102,9 +120,14 @@ static int launch_layernorm(const float* x, const int* rows, const float* gamma,
     // rows in flight than blocks of eight, and registers only for the vectors that a row has do the same: 16,384 rows of 1,600
     // took 37.5 us with eight warps and 16 vectors, 31.0 so; of 1,024 22.5, 21.6 so)
     const dim3 grid((n_rows + 1) / 2), block(64);
-#define BT_LN_ROWS(J)                                                                                                    \
-  BT_PDL_OK("layernorm", launch_pdl(layernorm_rows_kernel<TOut, J>, grid, block, 0, stream, 1, x, rows, gamma, beta, out, \
-                                    n_rows, width, eps))
+    // (gamma and beta ahead of the wait: rows and weights cold, before / after, us: 64 x 1,600 4.2 / 2.1, 2,048 x 768 4.3 / 3.2, 4,096 x 1,600
+    // 13.6 / 11.9, 8,192 x 1,600 16.8 / 21.3, 16,384 x 1,024 18.4 / 19.4: beyond 4,096 rows the registers cost more than the wait did)
+    const bool early = n_rows <= 4096;
+#define BT_LN_ROWS(J)                                                                                                              \
+  BT_PDL_OK("layernorm", early ? launch_pdl(layernorm_rows_kernel<TOut, J, true>, grid, block, 0, stream, 1, x, rows, gamma, beta, \
+                                            out, n_rows, width, eps)                                                              \
+                               : launch_pdl(layernorm_rows_kernel<TOut, J, false>, grid, block, 0, stream, 1, x, rows, gamma, beta, \
+                                            out, n_rows, width, eps))
     if (width <= 1024) BT_LN_ROWS(8);
     else if (width <= 1280) BT_LN_ROWS(10);
     else if (width <= 1664) BT_LN_ROWS(13);
