@@ -48,8 +48,8 @@ int bt_sigmoid_attention_tcgen05(const void* q, long long q_rows, long long q_ro
 int bt_attention_prefill_tcgen05(const void* q, long long q_rows, long long q_row_stride, const void* k, const void* v,
                                  long long pool_pages, const int* kv_table, int table_stride, int table_len, int page_size,
                                  void* out, int* status, const int* seq_start, const int* past_len, int n_seqs, int max_new,
-                                 int n_heads, int n_kv_heads, int head_dim, float scale, int causal, int window,
-                                 cudaStream_t stream);
+                                 int n_heads, int n_kv_heads, int head_dim, float scale, int causal, int window, void* file_k,
+                                 void* file_v, long long file_pages, const int* file_table, int file_stride, cudaStream_t stream);
 
 long long bt_attention_decode_scratch_floats(int n_seqs, int n_heads, int head_dim, int n_splits);
 // out[M, N] = act(a[M, K] @ w[N, K]^T + bias) (+ residual) for at most 64 bfloat16 rows (made for 17..64).

@@ -73,6 +73,15 @@ struct TaParams {
   int maps, k_map_cols;        // paged: a pool row holds `maps` keys `k_map_cols` columns apart; head h reads key h % maps
 };
 
+// Where a softmax block files the step's own keys and values (see the kernel): the pools, a sequence's pages, and the rows they come from.
+struct TaFile {
+  __nv_bfloat16 *k_pool, *v_pool;              // [pages][n_kv_heads][64][HD]
+  const int* table;
+  int table_stride;
+  const __nv_bfloat16 *k_rows, *v_rows;        // the first key / value channel of the projections' row 0
+  long long row_stride;
+};
+
 __device__ __forceinline__ unsigned ta_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void ta_bar_init(unsigned long long* bar, int count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(ta_smem(bar)), "r"(count));
@@ -99,6 +108,11 @@ __device__ __forceinline__ void ta_tma(void* dst, const CUtensorMap* map, int co
           ta_smem(dst)),
       "l"(map), "r"(col), "r"(row), "r"(ta_smem(bar))
       : "memory");
+}
+__device__ __forceinline__ void ta_tma_store(const CUtensorMap* map, int col, int row, const void* src) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];\n" ::"l"(map), "r"(col), "r"(row),
+               "r"(ta_smem(src))
+               : "memory");
 }
 // Shared-memory operand descriptor for tiles of 128-byte rows with the 128-byte swizzle.  K-major operands (Q, K, P):
 // groups of 8 rows lie 1024 bytes apart (stride offset); the leading offset is not used.  The MN-major operand (V:
@@ -602,10 +616,16 @@ struct TsShape {
   static constexpr int COLS = TWO ? 256 : 512;
 };
 
-template <int HD, int HV>
+// FILE: sequences that start at position 0, causal, keys and values in the projections' rows.  A block's last tile of keys then holds its
+// own 128 tokens; the block of a key head's first query head also writes that tile to the pages, whole pages from shared memory by
+// the TMA, the rows of a page that the sequence does not fill by the producer's warp.  The copy that ran beside this kernel before read
+// the projections once more and held its multiprocessors first (16 x 1,024 tokens of 25 heads of 64: attention and copy 184 to 158 us; 2 x 1,024 of
+// 12: 20.1 to 18.2).
+template <int HD, int HV, bool FILE>
 __global__ void __launch_bounds__(TS_THREADS, TsShape<HD, HV>::TWO ? 2 : 1)
 attention_prefill_softmax_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
-                                 const __grid_constant__ CUtensorMap v_map, TaParams p) {
+                                 const __grid_constant__ CUtensorMap v_map, TaParams p, const __grid_constant__ CUtensorMap k_pages,
+                                 const __grid_constant__ CUtensorMap v_pages, TaFile file) {
   using Shape = TsShape<HD, HV>;
   constexpr int CB = HD / 64, CBV = HV / 64;
   constexpr int TILE_BYTES = Shape::TILE_BYTES, TILE_V = Shape::TILE_V;
@@ -733,6 +753,38 @@ attention_prefill_softmax_kernel(const __grid_constant__ CUtensorMap q_map, cons
           break;
         }
         load(it + TA_STAGES, true);
+      }
+      if (FILE && head % (p.n_heads / p.n_kv_heads) == 0) {
+        const int s = (n_tiles - 1) % TA_STAGES;
+        const unsigned parity = (unsigned)((n_tiles - 1) / TA_STAGES) & 1u;
+        for (int values = 0; values < 2; ++values) {
+          if (*failed || !ta_bar_wait(values ? &v_full[s] : &k_full[s], parity)) {
+            *failed = 1;
+            break;
+          }
+          const unsigned char* src = values ? Vs + s * TILE_V : Ks + s * TILE_BYTES;
+          for (int h = 0; h < 2; ++h) {
+            if (n_new - q0 < 64 * (h + 1)) continue;
+            const int page = file.table[(long long)seq * file.table_stride + q0 / 64 + h];
+            for (int cb = 0; cb < (values ? CBV : CB); ++cb)
+              ta_tma_store(values ? &v_pages : &k_pages, cb * 64, (page * p.n_kv_heads + kv_head) * 64,
+                           src + cb * 2 * TA_BOX_BYTES + h * TA_BOX_BYTES);
+          }
+        }
+        asm volatile("cp.async.bulk.commit_group;\ncp.async.bulk.wait_group 0;\n" ::: "memory");
+      }
+    }
+    __syncwarp();
+    if (FILE && head % (p.n_heads / p.n_kv_heads) == 0 && nq % 64 != 0) {
+      const int first = q0 + nq / 64 * 64;
+      const int page = file.table[(long long)seq * file.table_stride + first / 64];
+      const long long dst = ((long long)page * p.n_kv_heads + kv_head) * 64;
+      for (int i = lane; i < nq % 64 * (HD / 8); i += 32) {
+        const int r = i / (HD / 8), c = i % (HD / 8) * 8;
+        const long long from = (t0 + first + r) * file.row_stride + kv_head * HD + c, to = (dst + r) * HD + c;
+        const uint4 k = *reinterpret_cast<const uint4*>(file.k_rows + from), v = *reinterpret_cast<const uint4*>(file.v_rows + from);
+        *reinterpret_cast<uint4*>(file.k_pool + to) = k;
+        *reinterpret_cast<uint4*>(file.v_pool + to) = v;
       }
     }
   } else if (warp == TS_SOFTMAX_WARPS + 1) {
@@ -957,17 +1009,17 @@ attention_prefill_softmax_kernel(const __grid_constant__ CUtensorMap q_map, cons
   if (threadIdx.x == 0 && *failed && p.status) atomicExch(p.status, 6);
 }
 
-template <int HD, int HV>
+template <int HD, int HV, bool FILE = false>
 static int launch_ts(const CUtensorMap& qm, const CUtensorMap& km, const CUtensorMap& vm, const TaParams& p, int n_seqs, int max_new,
-                     cudaStream_t stream) {
+                     cudaStream_t stream, const CUtensorMap& kp = {}, const CUtensorMap& vp = {}, const TaFile& file = {}) {
   constexpr size_t smem = TsShape<HD, HV>::SMEM;
-  auto kern = attention_prefill_softmax_kernel<HD, HV>;
+  auto kern = attention_prefill_softmax_kernel<HD, HV, FILE>;
   static SharedMemoryAllowance allowed;
   BT_CHECK(allow_shared_memory(allowed, kern, smem), "attention_prefill_tcgen05: cannot reserve %zu bytes of shared memory", smem);
   const int q_tiles = (max_new + TA_BQ - 1) / TA_BQ;
   BT_CHECK(q_tiles <= 65535, "attention_prefill_tcgen05: %d new tokens in one sequence are too many for one launch", max_new);
   dim3 grid(n_seqs * p.n_heads, q_tiles);
-  BT_PDL_OK("attention_prefill_tcgen05", launch_pdl(kern, grid, dim3(TS_THREADS), smem, stream, 1, qm, km, vm, p));
+  BT_PDL_OK("attention_prefill_tcgen05", launch_pdl(kern, grid, dim3(TS_THREADS), smem, stream, 1, qm, km, vm, p, kp, vp, file));
   return 0;
 }
 
@@ -1000,7 +1052,8 @@ static int run_attention_prefill_tcgen05(const void* q, long long q_rows, long l
                                          int page_size, void* out, int* status, const int* seq_start, const int* past_len,
                                          int n_seqs, int max_new, int n_heads, int n_kv_heads, int head_dim, float scale,
                                          int causal, int window, int sigmoid, const float* bias, int keep_first,
-                                         long long pool_row_stride, int v_dim, cudaStream_t stream) {
+                                         long long pool_row_stride, int v_dim, void* file_k, void* file_v, long long file_pages,
+                                         const int* file_table, int file_stride, cudaStream_t stream) {
   using namespace bt;
   BT_CHECK(bt_attention_prefill_tcgen05_supports(head_dim, page_size > 0 ? page_size : 64),
            "attention_prefill_tcgen05: head_dim %d (page size %d) is not supported", head_dim, page_size);
@@ -1044,18 +1097,33 @@ static int run_attention_prefill_tcgen05(const void* q, long long q_rows, long l
     if (v_dim == 64) return launch_ta<128, 64>(qm, km, vm, p, n_seqs, max_new, stream);
     return launch_ta<128, 128>(qm, km, vm, p, n_seqs, max_new, stream);
   }
+  if (file_table != nullptr) {
+    BT_CHECK(kv_table == nullptr && causal && file_pages >= 1 && file_pages * n_kv_heads * 64 < (1ll << 31),
+             "attention_prefill_tcgen05: only a causal step's own keys and values can be filed");
+    CUtensorMap kp, vp;
+    const unsigned long long rows = (unsigned long long)file_pages * n_kv_heads * 64;
+    if (int rc = tensor_map_2d_bf16(&kp, file_k, rows, head_dim, head_dim, 64)) return rc;
+    if (int rc = tensor_map_2d_bf16(&vp, file_v, rows, head_dim, head_dim, 64)) return rc;
+    const TaFile file{(__nv_bfloat16*)file_k, (__nv_bfloat16*)file_v, file_table, file_stride, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, q_row_stride};
+    if (head_dim == 64) return launch_ts<64, 64, true>(qm, km, vm, p, n_seqs, max_new, stream, kp, vp, file);
+    return launch_ts<128, 128, true>(qm, km, vm, p, n_seqs, max_new, stream, kp, vp, file);
+  }
   if (head_dim == 64) return launch_ts<64, 64>(qm, km, vm, p, n_seqs, max_new, stream);
   return launch_ts<128, 128>(qm, km, vm, p, n_seqs, max_new, stream);
 }
 
+// file_table (may be null): the step's sequences start at position 0 and their keys and values are also written to the pools file_k and
+// file_v, [file_pages][n_kv_heads][64][head_dim], at the pages of file_table's rows, which hold every new token's page.
 extern "C" int bt_attention_prefill_tcgen05(const void* q, long long q_rows, long long q_row_stride, const void* k, const void* v,
                                             long long pool_pages, const int* kv_table, int table_stride, int table_len,
                                             int page_size, void* out, int* status, const int* seq_start, const int* past_len,
                                             int n_seqs, int max_new, int n_heads, int n_kv_heads, int head_dim, float scale,
-                                            int causal, int window, cudaStream_t stream) {
+                                            int causal, int window, void* file_k, void* file_v, long long file_pages,
+                                            const int* file_table, int file_stride, cudaStream_t stream) {
   return run_attention_prefill_tcgen05(q, q_rows, q_row_stride, k, v, pool_pages, kv_table, table_stride, table_len, page_size,
                                        out, status, seq_start, past_len, n_seqs, max_new, n_heads, n_kv_heads, head_dim, scale,
-                                       causal, window, 0, nullptr, 0, 0, head_dim, stream);
+                                       causal, window, 0, nullptr, 0, 0, head_dim, file_k, file_v, file_pages, file_table, file_stride,
+                                       stream);
 }
 
 // The same for attention whose weights are sigmoid(score * scale + bias[head]), not normalised over the keys; always
@@ -1072,7 +1140,7 @@ extern "C" int bt_sigmoid_attention_tcgen05(const void* q, long long q_rows, lon
   BT_CHECK(window >= 0 && keep_first >= 0, "sigmoid_attention_tcgen05: bad window %d or kept positions %d", window, keep_first);
   return run_attention_prefill_tcgen05(q, q_rows, q_row_stride, k, v, pool_pages, kv_table, table_stride, table_len, page_size,
                                        out, status, seq_start, past_len, n_seqs, max_new, n_heads, n_kv_heads, head_dim, scale,
-                                       1, window, 1, bias, keep_first, pool_row_stride, v_dim, stream);
+                                       1, window, 1, bias, keep_first, pool_row_stride, v_dim, nullptr, nullptr, 0, nullptr, 0, stream);
 }
 
 // Causal multi-head attention of sequences that start at position 0 with a sink and an output gate (each optional): query

@@ -516,7 +516,7 @@ def attention_prefill(q_proj, out, seq_start, past_len, n_seqs, max_new, n_heads
 
 def _attention_prefill_tcgen05(q_proj, out, seq_start, past_len, n_seqs, max_new, n_heads, n_kv_heads, head_dim, scale,
                                *, causal=True, window=0, k_pool=None, v_pool=None, table=None, table_len=0,
-                               k_offset=None, v_offset=None):
+                               k_offset=None, v_offset=None, file=None):
     _need(q_proj, "q_proj", torch.bfloat16)
     _need(out, "out", torch.bfloat16, (None, n_heads * head_dim))
     stride = q_proj.shape[1]
@@ -529,11 +529,29 @@ def _attention_prefill_tcgen05(q_proj, out, seq_start, past_len, n_seqs, max_new
         _need(v_pool, "v_pool", torch.bfloat16)
         _need(table, "table", torch.int32)
         k_ptr, v_ptr, t_ptr, t_stride, pages = _ptr(k_pool), _ptr(v_pool), _ptr(table), table.shape[1], k_pool.shape[0]
+    file_k, file_v, file_table = file or (None, None, None)
+    if file is not None:
+        if table is not None or not causal:
+            raise ShapeError("attention_prefill: only a causal step's own keys and values can be filed")
+        _need(file_k, "file_k", torch.bfloat16, (None, n_kv_heads, PAGE_SIZE, head_dim))
+        _need(file_v, "file_v", torch.bfloat16, tuple(file_k.shape))
+        _need(file_table, "file_table", torch.int32)
+        if file_table.shape[1] * PAGE_SIZE < max_new:
+            raise ShapeError(f"attention_prefill: {max_new} new tokens do not fit the {file_table.shape[1]} pages of a row")
     _check(library().bt_attention_prefill_tcgen05(
         _ptr(q_proj), c_longlong(q_proj.shape[0]), c_longlong(stride), k_ptr, v_ptr, c_longlong(pages), t_ptr,
         c_int(t_stride), c_int(table_len), c_int(PAGE_SIZE), _ptr(out), _ptr(kernel_status(q_proj.device)),
         _ptr(seq_start), _ptr(past_len), c_int(n_seqs), c_int(max_new), c_int(n_heads), c_int(n_kv_heads),
-        c_int(head_dim), c_float(scale), c_int(1 if causal else 0), c_int(window), _stream()))
+        c_int(head_dim), c_float(scale), c_int(1 if causal else 0), c_int(window), _ptr(file_k), _ptr(file_v),
+        c_longlong(file_k.shape[0] if file else 0), _ptr(file_table), c_int(file_table.shape[1] if file else 0), _stream()))
+
+
+def attention_prefill_files(q_proj, k_pool, head_dim, causal) -> bool:
+    """Whether attention_prefill takes `file` = (keys' pool, values' pool, table): the attention of sequences that start at position
+    0 then also writes their keys and values to their pages, so that no kv_append is needed.  The table's rows must hold a
+    page for every 64 of a sequence's tokens, none of them twice."""
+    return (q_proj.dtype == torch.bfloat16 and causal and k_pool.numel() // head_dim < 1 << 31
+            and _supports("bt_attention_prefill_tcgen05_supports", head_dim, PAGE_SIZE))
 
 
 def attention_decode_supports(head_dim: int, row_stride: int, dtype) -> bool:

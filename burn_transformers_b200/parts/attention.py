@@ -102,7 +102,10 @@ class CausalSelfAttention(Mixer):
         k_pool, v_pool, group, g = ctx.cache.layer_pools(entry)
         table = ctx.tables[g]
         window = self.window or 0
-        if owns_cache and not ctx.is_decode:
+        # fresh sequences attend over the step's own projections; where the kernel can, it files their keys and values as it goes
+        files = (owns_cache and ctx.fresh and not ctx.is_decode and not group.is_ring
+                 and kernels.attention_prefill_files(proj, k_pool, self.head_dim, self.causal))
+        if owns_cache and not ctx.is_decode and not files:
             side = getattr(ctx, "side", None) if ctx.fresh else None
             if side is not None:
                 # fresh sequences attend over the step's own projections: nothing in this step reads the pages, so
@@ -143,7 +146,8 @@ class CausalSelfAttention(Mixer):
             kernels.attention_prefill(proj, mixed, ctx.seq_start, ctx.past_len, ctx.n_seqs, ctx.max_new,
                                            self.n_heads, self.n_kv_heads, self.head_dim, self.scale,
                                            causal=self.causal, window=window,
-                                           k_offset=self.q_width, v_offset=self.q_width + self.kv_width)
+                                           k_offset=self.q_width, v_offset=self.q_width + self.kv_width,
+                                           **({"file": (k_pool, v_pool, table)} if files else {}))
         else:
             if group.is_ring and ctx.max_new > group.table_len * PAGE_SIZE - self.window + 1:
                 # (the engine refuses such a step before the cache changes; this guards direct users of the part)
