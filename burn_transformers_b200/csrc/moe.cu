@@ -23,6 +23,8 @@
 #include "api.h"
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace bt {
 
 __device__ __forceinline__ void warp_argmax(float& v, int& i) {
@@ -66,79 +68,29 @@ __device__ __forceinline__ void unpack_piece(const uint4& v, float (&o)[8]) {
   }
 }
 
-// NP > 0: the token's row is whole 16-byte pieces, at most NP a lane; the lane keeps them in registers and asks for the
-// pieces of four experts' rows at once, so that a token costs a few trips to memory, not one per expert and piece.
-template <typename T, int NP>
-__global__ void __launch_bounds__(ROUTE_WARPS * 32)
-moe_route_kernel(const T* __restrict__ x, long long x_row_stride, const T* __restrict__ router, int n_tokens, int K, int E,
-                 int top, int n_groups, int keep, float scale, int rule, const float* __restrict__ logit_bias,
-                 const float* __restrict__ choice_bias, int normalise, int* __restrict__ ids, float* __restrict__ weights) {
-  extern __shared__ float sm[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* score = sm + (size_t)warp * 3 * E;   // [E] sigmoid scores
+struct RouteArgs {
+  int n_tokens, K, E, top, n_groups, keep;
+  float scale;
+  int rule, normalise;
+  const float *logit_bias, *choice_bias;
+  int* ids;
+  float* weights;
+  int sets;      // of TB tokens a block takes, each with as many warps (1, 2 or 4)
+};
+
+// What a warp makes of its token's scores z (+ logit_bias): the score itself, and, once all are there, the choice.
+__device__ __forceinline__ float route_score(const RouteArgs& p, int e, float z) {
+  if (p.logit_bias != nullptr) z += p.logit_bias[e];
+  return p.rule != kRouteSigmoid ? z : 1.f / (1.f + expf(-z));
+}
+__device__ __forceinline__ void route_choose(const RouteArgs& p, int t, float* score, int lane) {
+  const int E = p.E, top = p.top, n_groups = p.n_groups, keep = p.keep, rule = p.rule, normalise = p.normalise;
+  const float scale = p.scale;
+  const float* choice_bias = p.choice_bias;
+  int* ids = p.ids;
+  float* weights = p.weights;
   float* cand = score + E;                    // [E] scores still to choose from (-inf: not allowed, or taken)
   float* group = cand + E;                    // [n_groups] group scores
-  pdl_trigger();
-  pdl_wait();
-  const int t = blockIdx.x * ROUTE_WARPS + warp;
-  if (t >= n_tokens) return;
-  const T* row = x + (long long)t * x_row_stride;
-  constexpr int V = 16 / (int)sizeof(T), EB = 4;
-  if (NP > 0) {
-    float xv[NP > 0 ? NP : 1][V];
-#pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      const int k = (lane + 32 * i) * V;
-      uint4 raw = make_uint4(0, 0, 0, 0);
-      if (k < K) raw = *reinterpret_cast<const uint4*>(row + k);
-      unpack_piece(raw, xv[i]);
-    }
-    for (int e0 = 0; e0 < E; e0 += EB) {
-      uint4 raw[EB][NP > 0 ? NP : 1];
-#pragma unroll
-      for (int j = 0; j < EB; ++j)
-#pragma unroll
-        for (int i = 0; i < NP; ++i) {
-          const int k = (lane + 32 * i) * V;
-          raw[j][i] = (e0 + j < E && k < K) ? *reinterpret_cast<const uint4*>(router + (long long)(e0 + j) * K + k)
-                                            : make_uint4(0, 0, 0, 0);
-        }
-#pragma unroll
-      for (int j = 0; j < EB; ++j) {
-        float acc = 0.f;
-#pragma unroll
-        for (int i = 0; i < NP; ++i) {
-          float wv[V];
-          unpack_piece(raw[j][i], wv);
-#pragma unroll
-          for (int u = 0; u < V; ++u) acc = fmaf(xv[i][u], wv[u], acc);
-        }
-        acc = warp_sum(acc);
-        if (lane == 0 && e0 + j < E) {
-          if (logit_bias != nullptr) acc += logit_bias[e0 + j];
-          score[e0 + j] = rule != kRouteSigmoid ? acc : 1.f / (1.f + expf(-acc));
-        }
-      }
-    }
-  } else {
-    for (int e0 = 0; e0 < E; e0 += EB) {
-      float acc[EB] = {0.f, 0.f, 0.f, 0.f};
-      for (int k = lane; k < K; k += 32) {
-        const float xs = to_float(row[k]);
-#pragma unroll
-        for (int j = 0; j < EB; ++j)
-          if (e0 + j < E) acc[j] = fmaf(xs, to_float(router[(long long)(e0 + j) * K + k]), acc[j]);
-      }
-#pragma unroll
-      for (int j = 0; j < EB; ++j) {
-        float z = warp_sum(acc[j]);
-        if (lane == 0 && e0 + j < E) {
-          if (logit_bias != nullptr) z += logit_bias[e0 + j];
-          score[e0 + j] = rule != kRouteSigmoid ? z : 1.f / (1.f + expf(-z));
-        }
-      }
-    }
-  }
   __syncwarp();
   if (rule == kRouteSoftmax) {
     float top_z = -INFINITY;
@@ -208,8 +160,121 @@ moe_route_kernel(const T* __restrict__ x, long long x_row_stride, const T* __res
   }
 }
 
+// Rows of any length: a warp a token, element by element.
+template <typename T>
+__global__ void __launch_bounds__(ROUTE_WARPS * 32)
+moe_route_plain_kernel(const T* __restrict__ x, long long x_row_stride, const T* __restrict__ router, RouteArgs p) {
+  extern __shared__ float sm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, K = p.K, E = p.E;
+  float* score = sm + (size_t)warp * 3 * E;   // [E] scores, and two more [E] for the choice
+  pdl_trigger();
+  pdl_wait();
+  const int t = blockIdx.x * ROUTE_WARPS + warp;
+  if (t >= p.n_tokens) return;
+  const T* row = x + (long long)t * x_row_stride;
+  constexpr int EB = 4;
+  for (int e0 = 0; e0 < E; e0 += EB) {
+    float acc[EB] = {0.f, 0.f, 0.f, 0.f};
+    for (int k = lane; k < K; k += 32) {
+      const float xs = to_float(row[k]);
+#pragma unroll
+      for (int j = 0; j < EB; ++j)
+        if (e0 + j < E) acc[j] = fmaf(xs, to_float(router[(long long)(e0 + j) * K + k]), acc[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < EB; ++j) {
+      const float z = warp_sum(acc[j]);
+      if (lane == 0 && e0 + j < E) score[e0 + j] = route_score(p, e0 + j, z);
+    }
+  }
+  route_choose(p, t, score, lane);
+}
+
+// Rows of whole 16-byte pieces, at most NP a lane: a block takes TB tokens (their rows in registers, or in shared memory where they are
+// several), and its eight warps take the experts in turn, EB at once: the router's rows are read once for TB tokens, and a token's experts do not wait for one another.
+// With a warp a token and all experts one after the other, 2,048 tokens read the router 2,048 times from L2 and 64 tokens were a
+// chain of E / 4 reads.  Before / now, us, 64 experts of 1,024: 64 tokens 26.7 / 6.3, 804 31.8 / 11.6, 2,048 61 / 22; 8 of 512: 4.7 / 2.6 and
+// 7.9 / 6.6 (2,048); 256 of 1,024: 93 / 12.5 and 219 / 57.  A score's sum has the order it had: a lane's pieces one after
+// the other, then lanes 16, 8, 4, 2 and 1 apart; here lanes that are done with a number's half take another number's.
+constexpr int ROUTE_BLOCK = 256;
+template <typename T, int NP, int TB>
+__global__ void __launch_bounds__(ROUTE_BLOCK, 2)
+moe_route_kernel(const T* __restrict__ x, long long x_row_stride, const T* __restrict__ router, RouteArgs p) {
+  extern __shared__ float sm[];
+  constexpr int V = 16 / (int)sizeof(T), EB = 4, SUMS = TB * EB;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, K = p.K, E = p.E;
+  const int mates = ROUTE_BLOCK / 32 / p.sets, set = warp / mates, step = mates * EB;      // warps for the same tokens
+  const int t0 = (blockIdx.x * p.sets + set) * TB;
+  float* score = sm + set * TB * 3 * ((E + 3) & ~3);
+  uint4 raw[EB][NP];
+  auto fetch = [&](int e0) {
+#pragma unroll
+    for (int j = 0; j < EB; ++j)
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        const int k = (lane + 32 * i) * V;
+        raw[j][i] = (e0 + j < E && k < K) ? *reinterpret_cast<const uint4*>(router + (long long)(e0 + j) * K + k) : make_uint4(0, 0, 0, 0);
+      }
+  };
+  pdl_trigger();
+  fetch(warp % mates * EB);      // (no kernel of a step writes the router)
+  pdl_wait();
+  auto piece = [&](int t, int i) {      // piece lane + 32 i of token t0 + t
+    const int k = (lane + 32 * i) * V;
+    return (t0 + t < p.n_tokens && k < K) ? *reinterpret_cast<const uint4*>(x + (t0 + t) * x_row_stride + k) : make_uint4(0, 0, 0, 0);
+  };
+  uint4 xr[TB == 1 ? NP : 1];
+  uint4* x_s = reinterpret_cast<uint4*>(sm + p.sets * TB * 3 * ((E + 3) & ~3)) + set * TB * NP * 32;      // [TB][32 NP]
+  if constexpr (TB == 1) {
+#pragma unroll
+    for (int i = 0; i < NP; ++i) xr[i] = piece(0, i);
+  } else {
+    for (int i = warp % mates; i < TB * NP; i += mates) x_s[i * 32 + lane] = piece(i / NP, i % NP);
+    __syncthreads();
+  }
+  for (int e0 = warp % mates * EB; e0 < E; e0 += step) {
+    float acc[SUMS];
+#pragma unroll
+    for (int i = 0; i < SUMS; ++i) acc[i] = 0.f;
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      float wv[EB][V];
+#pragma unroll
+      for (int j = 0; j < EB; ++j) unpack_piece(raw[j][i], wv[j]);
+#pragma unroll
+      for (int t = 0; t < TB; ++t) {
+        float xv[V];
+        if constexpr (TB == 1) unpack_piece(xr[i], xv);
+        else unpack_piece(x_s[(t * NP + i) * 32 + lane], xv);
+#pragma unroll
+        for (int j = 0; j < EB; ++j)
+#pragma unroll
+          for (int u = 0; u < V; ++u) acc[t * EB + j] = fmaf(xv[u], wv[j][u], acc[t * EB + j]);
+      }
+    }
+    fetch(e0 + step);
+#pragma unroll
+    for (int o = 16, n = SUMS / 2; o > 0; o >>= 1, n >>= 1) {
+      const bool high = (lane & o) != 0;
+      if (n == 0) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        const float give = high ? acc[i] : acc[i + n], keep = high ? acc[i + n] : acc[i];
+        acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+    }
+    const int sum = lane / (32 / SUMS), t = sum / EB, e = e0 + sum % EB;
+    if (lane % (32 / SUMS) == 0 && e < E) score[t * 3 * ((E + 3) & ~3) + e] = route_score(p, e, acc[0]);
+  }
+  __syncthreads();
+  for (int t = warp % mates; t < TB; t += mates)
+    if (t0 + t < p.n_tokens) route_choose(p, t0 + t, score + t * 3 * ((E + 3) & ~3), lane);
+}
+
 // One block.  offsets[e]: first sorted row of expert e (offsets[E] = all rows); tile_first[e]: first row tile of expert e
 // (tile_first[E] = all tiles); order[r]: the pair (token * top + choice) that lies in sorted row r; place[pair]: its row.
+// HELD: pairs a thread keeps, whose ids are read together and once.
+template <int HELD>
 __global__ void __launch_bounds__(1024)
 moe_sort_kernel(const int* __restrict__ ids, int total, int E, int tile_rows, int* __restrict__ offsets,
                 int* __restrict__ tile_first, int* __restrict__ order, int* __restrict__ place) {
@@ -218,37 +283,64 @@ moe_sort_kernel(const int* __restrict__ ids, int total, int E, int tile_rows, in
   int* cursor = ism + E;    // [E]
   pdl_trigger();
   pdl_wait();
+  int mine[HELD], rank[HELD];
+#pragma unroll
+  for (int u = 0; u < HELD; ++u) {
+    const int i = threadIdx.x + u * blockDim.x;
+    mine[u] = i < total ? ids[i] : -1;
+  }
   for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < total; i += blockDim.x) atomicAdd(&count[ids[i]], 1);
+  // a pair's place among its expert's is what the count was; which pair gets which of an expert's rows does not matter: a row's result
+  // does not depend on its place
+#pragma unroll
+  for (int u = 0; u < HELD; ++u)
+    if (mine[u] >= 0) rank[u] = atomicAdd(&count[mine[u]], 1);
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (total > HELD * (int)blockDim.x) {
+    for (int i = threadIdx.x + HELD * blockDim.x; i < total; i += blockDim.x) atomicAdd(&count[ids[i]], 1);
+    __syncthreads();
+  }
+  if (threadIdx.x < 32) {
+    // a warp adds up the experts before each, 32 at a time
     int rows = 0, tiles = 0;
-    for (int e = 0; e < E; ++e) {
-      offsets[e] = rows;
-      tile_first[e] = tiles;
-      cursor[e] = rows;
-      rows += count[e];
-      tiles += (count[e] + tile_rows - 1) / tile_rows;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + threadIdx.x, n = e < E ? count[e] : 0, n_tiles = (n + tile_rows - 1) / tile_rows;
+      int upto = n, tiles_upto = n_tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, upto, o), b = __shfl_up_sync(0xffffffffu, tiles_upto, o);
+        if (threadIdx.x >= o) {
+          upto += a;
+          tiles_upto += b;
+        }
+      }
+      if (e < E) {
+        offsets[e] = cursor[e] = rows + upto - n;
+        tile_first[e] = tiles + tiles_upto - n_tiles;
+      }
+      rows += __shfl_sync(0xffffffffu, upto, 31);
+      tiles += __shfl_sync(0xffffffffu, tiles_upto, 31);
     }
-    offsets[E] = rows;
-    tile_first[E] = tiles;
+    if (threadIdx.x == 0) {
+      offsets[E] = rows;
+      tile_first[E] = tiles;
+    }
   }
   __syncthreads();
-  // lanes of a warp that hold the same expert take consecutive rows from one atomic; which pair gets which of an
-  // expert's rows does not matter: a row's result does not depend on its place
-  for (int base = 0; base < total; base += blockDim.x) {
-    const int i = base + threadIdx.x;
-    if (i < total) {
-      const int e = ids[i];
-      const unsigned same = __match_any_sync(__activemask(), e);
-      const int rank = __popc(same & ((1u << (threadIdx.x & 31)) - 1));
-      int first = 0;
-      if (rank == 0) first = atomicAdd(&cursor[e], __popc(same));
-      first = __shfl_sync(same, first, __ffs(same) - 1);
-      order[first + rank] = i;
-      place[i] = first + rank;
-    }
+#pragma unroll
+  for (int u = 0; u < HELD; ++u) {
+    if (mine[u] < 0) continue;
+    const int i = threadIdx.x + u * blockDim.x, row = cursor[mine[u]] + rank[u];
+    order[row] = i;
+    place[i] = row;
+  }
+  if (total <= HELD * (int)blockDim.x) return;
+  // the rest lies from an expert's last rows backwards (the held ones have its first)
+  for (int i = threadIdx.x + HELD * blockDim.x; i < total; i += blockDim.x) {
+    const int e = ids[i], row = cursor[e] + atomicSub(&count[e], 1) - 1;
+    order[row] = i;
+    place[i] = row;
   }
 }
 
@@ -596,8 +688,6 @@ extern "C" int bt_moe_route(const void* x, long long x_row_stride, const void* r
   BT_CHECK(rule >= kRouteSigmoid && rule <= kRouteChosen && (rule != kRouteChosen || (n_groups == 1 && normalise)),
            "moe_route: rule %d; a softmax over the chosen goes with one group of experts and weights that sum to one", rule);
   if (n_tokens == 0) return 0;
-  const dim3 grid((n_tokens + ROUTE_WARPS - 1) / ROUTE_WARPS), block(ROUTE_WARPS * 32);
-  const size_t smem = (size_t)ROUTE_WARPS * 3 * E * sizeof(float);
   // pieces of 16 bytes a lane holds of a token's row: 1, 2 or 4 (rows of up to 128 pieces); 0: element by element
   auto pieces_of = [&](int elem) {
     const int v = 16 / elem;
@@ -605,23 +695,38 @@ extern "C" int bt_moe_route(const void* x, long long x_row_stride, const void* r
     const int per_lane = (K / v + 31) / 32;
     return per_lane <= 1 ? 1 : per_lane <= 2 ? 2 : per_lane <= 4 ? 4 : 0;
   };
-#define BT_ROUTE(T, NP)                                                                                              \
-  BT_PDL_OK("moe_route", launch_pdl(moe_route_kernel<T, NP>, grid, block, smem, stream, 1, (const T*)x, x_row_stride, \
-                                    (const T*)router, n_tokens, K, E, top, n_groups, keep, scale, rule, logit_bias, \
-                                    choice_bias, normalise, ids, weights))
-  if (dtype == kF32) {
-    const int np = pieces_of(4);
-    if (np == 1) BT_ROUTE(float, 1); else if (np == 2) BT_ROUTE(float, 2); else if (np == 4) BT_ROUTE(float, 4);
-    else BT_ROUTE(float, 0);
-  } else if (dtype == kBF16) {
-    const int np = pieces_of(2);
-    if (np == 1) BT_ROUTE(__nv_bfloat16, 1); else if (np == 2) BT_ROUTE(__nv_bfloat16, 2);
-    else if (np == 4) BT_ROUTE(__nv_bfloat16, 4); else BT_ROUTE(__nv_bfloat16, 0);
-  } else {
-    return fail("moe_route: unknown dtype %d", dtype);
-  }
+  const int sms = sm_count();
+  BT_CHECK(sms > 0, "moe_route: cannot read the number of multiprocessors of the current device");
+  // A token a block while that leaves at most two blocks a multiprocessor, else four; several times as many where the experts are too few
+  // for eight warps and the blocks still reach every multiprocessor.  One / four tokens a block, us, 64 experts of 1,024: 200 tokens 7.6 / 8.4, 400 12.9 / 10.2, 2,048 48 / 21.
+  const size_t row = 3 * (size_t)((E + 3) & ~3) * sizeof(float);
+  const int tokens = n_tokens <= 2 * sms || 4 * row + 4 * 4 * 512 > 48 * 1024 ? 1 : 4;
+  int sets = tokens == 1 || E > 16 ? 1 : E > 8 ? 2 : 4;
+  while (sets > 1 && n_tokens < 4 * sets * sms) sets /= 2;
+  const RouteArgs p{n_tokens, K, E, top, n_groups, keep, scale, rule, normalise, logit_bias, choice_bias, ids, weights, sets};
+  auto launch = [&](auto kernel, int at_once, int threads, size_t held, const auto* x_, const auto* router_) -> int {
+    BT_PDL_OK("moe_route", launch_pdl(kernel, dim3((n_tokens + at_once - 1) / at_once), dim3(threads), at_once * (row + held), stream, 1,
+                                      x_, x_row_stride, router_, p));
+    return 0;
+  };
+  auto by_type = [&](auto* x_, auto* router_) -> int {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(x_)>>;
+    const int np = pieces_of(sizeof(T));
+    if (np == 0) return launch(moe_route_plain_kernel<T>, ROUTE_WARPS, ROUTE_WARPS * 32, 0, x_, router_);
+#define BT_ROUTE(NP, TB) return launch(moe_route_kernel<T, NP, TB>, TB * sets, ROUTE_BLOCK, TB == 1 ? 0 : (size_t)NP * 512, x_, router_)
+    if (tokens == 1) {
+      if (np == 1) BT_ROUTE(1, 1);
+      if (np == 2) BT_ROUTE(2, 1);
+      BT_ROUTE(4, 1);
+    }
+    if (np == 1) BT_ROUTE(1, 4);
+    if (np == 2) BT_ROUTE(2, 4);
+    BT_ROUTE(4, 4);
 #undef BT_ROUTE
-  return 0;
+  };
+  if (dtype == kF32) return by_type((const float*)x, (const float*)router);
+  if (dtype == kBF16) return by_type((const __nv_bfloat16*)x, (const __nv_bfloat16*)router);
+  return fail("moe_route: unknown dtype %d", dtype);
 }
 
 extern "C" int bt_moe_tile_rows() { return bt::MS_BM; }
@@ -680,8 +785,15 @@ extern "C" int bt_moe_sort(const int* ids, int total, int E, int* offsets, int* 
   using namespace bt;
   static_assert(MS_BM == MM_BM, "both product kernels read the same row tiles");
   BT_CHECK(total >= 0 && E > 0 && E <= 4096, "moe_sort: bad sizes pairs=%d experts=%d", total, E);
-  BT_PDL_OK("moe_sort", launch_pdl(moe_sort_kernel, dim3(1), dim3(1024), (size_t)2 * E * sizeof(int), stream, 1, ids,
-                                   total, E, MS_BM, offsets, tile_first, order, place));
+  auto launch = [&](auto kernel) -> int {
+    BT_PDL_OK("moe_sort", launch_pdl(kernel, dim3(1), dim3(1024), (size_t)2 * E * sizeof(int), stream, 1, ids, total, E, MS_BM, offsets,
+                                     tile_first, order, place));
+    return 0;
+  };
+  // (One pass of atomics and ids in registers instead of two passes over them, a warp instead of a thread for the experts' offsets, us: 512
+  // pairs of 64 experts 5.0 to 1.7, 16,384 39 to 11, 65,536 145 to 44.  Sixteen pairs a thread for the few: 2.9.)
+  if (total > 1024) return launch(moe_sort_kernel<16>);
+  return launch(moe_sort_kernel<1>);
   return 0;
 }
 
