@@ -14,6 +14,7 @@
 // g * sigmoid(g), and writes the row that the output projection reads.
 //
 // Long runs go by chunks, further below.
+#include "chunk_mma.cuh"
 #include "common.cuh"
 
 namespace bt {
@@ -530,12 +531,413 @@ gla_carry_kernel(const float* __restrict__ aged_q, const int* __restrict__ seq_s
   }
 }
 
+// The chunks on tensor cores (chunk_mma.cuh), for heads of whole operand tiles up to 64 channels: first every chunk's contribution to the
+// state (gla_state_kernel), then gla_prefix_vec_kernel, then all of o at once (gla_out_kernel), written once; no aged q in memory.
+// The weights are products of factors of at most one as above, with sub-blocks of 16 tokens between the chunk and the groups of four:
+// q_t e^{b_t - B} k_s e^{B - b_s}, B at the end of s's sub-block, is a product of matrices for every later sub-block; inside a
+// sub-block the groups' weights are multiply-adds.  The kernels above are bound by shared memory; these by forming factors and parts.
+// Before / now, us, all three kernels: 2 x 1,024 tokens of 16 heads of 64 x 64 70 / 40, 6 x 1,000 of 12 heads 135 / 77, one prompt of 129 tokens
+// 39 / 31; 32-bit rows 2 x 1,024 68 / 45; errors against 64 bits 1.6e-7 / 1.4e-7.  Heads of 128 channels leave two blocks a multiprocessor
+// and took 121 where the kernels above take 104, 32-bit heads of 16 15.4 against 13.7.
+
+// A chunk's contribution to the state: sum_s (k_s e^{b_end - b_s}) v_s^T.  A thread takes two key channels of 16 tokens and adds the log
+// decays up from the end.
+template <typename T, int PARTS>
+__global__ void __launch_bounds__(CM_THREADS, 4)
+gla_state_kernel(const T* __restrict__ proj, long long row_stride, int k_off, int v_off, const float* __restrict__ dt, float log_scale,
+                 const int* __restrict__ seq_start, float* __restrict__ states, float* __restrict__ ends, int max_chunks, int n_heads,
+                 int dim, int vdim, int col_blocks) {
+  extern __shared__ __align__(16) unsigned char cm_smem[];
+  const int k_stride = dim + 8, k_part = CM_CHUNK * k_stride, v_part = CM_CHUNK * CM_ROW;
+  __nv_bfloat16* k_s = reinterpret_cast<__nv_bfloat16*>(cm_smem);      // [3][64][dim + 8]
+  __nv_bfloat16* v_s = k_s + 3 * k_part;                               // [PARTS][64][72]
+  float2* sums = reinterpret_cast<float2*>(v_s + PARTS * v_part);      // [4][dim / 2] of 16 tokens each
+  pdl_trigger();
+  pdl_wait();
+  const int chunk = blockIdx.x, seq = blockIdx.z;
+  const int head = blockIdx.y / col_blocks, col_block = blockIdx.y - head * col_blocks, col0 = col_block * CM_COLS;
+  const int first = seq_start[seq], n_new = seq_start[seq + 1] - first;
+  if (chunk * CM_CHUNK >= n_new) return;
+  const int len = min(CM_CHUNK, n_new - chunk * CM_CHUNK), pairs = dim / 2;
+  const long long row0 = first + (long long)chunk * CM_CHUNK;
+  const T* rows = proj + row0 * row_stride;
+  const float* dt_rows = dt + (row0 * n_heads + head) * dim;
+  const long long dt_stride = (long long)n_heads * dim;
+  // (at most 64 channels: a pair of channels and a quarter of the tokens a thread.  A token past the last one: the last one's
+  // numbers, so that all reads are asked for together)
+  const int quarter = threadIdx.x / pairs, d = (threadIdx.x - quarter * pairs) * 2;
+  float2 x[16], k[16];
+  if (quarter < 4) {
+    float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const long long t = min(quarter * 16 + i, len - 1);
+      x[i] = *reinterpret_cast<const float2*>(dt_rows + t * dt_stride + d);
+      k[i] = cm_load2(rows + t * row_stride + k_off + head * dim + d);
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      if (quarter * 16 + i >= len) x[i] = k[i] = make_float2(0.f, 0.f);
+      sum.x += x[i].x;
+      sum.y += x[i].y;
+    }
+    sums[threadIdx.x] = sum;
+  }
+  cm_fill<PARTS>(v_s, CM_CHUNK, CM_COLS, CM_ROW, v_part, [&](int t, int c, float (&y)[8]) {
+    const bool in = t < len && col0 + c < vdim;
+    if (in) cm_load8(rows + t * row_stride + v_off + head * vdim + col0 + c, y);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) y[u] = in ? y[u] : 0.f;
+  });
+  __syncthreads();
+  if (quarter < 4) {
+    float2 after = make_float2(0.f, 0.f);      // of the tokens behind the one in hand
+    for (int h = quarter + 1; h < 4; ++h) {
+      const float2 y = sums[h * pairs + d / 2];
+      after.x += y.x;
+      after.y += y.y;
+    }
+    if (quarter == 0 && col_block == 0) {
+      const float2 y = sums[d / 2];
+      *reinterpret_cast<float2*>(ends + (((long long)seq * max_chunks + chunk) * n_heads + head) * dim + d) =
+          make_float2(gla_exp<T>(log_scale * (y.x + after.x)), gla_exp<T>(log_scale * (y.y + after.y)));
+    }
+#pragma unroll
+    for (int i = 15; i >= 0; --i) {
+      unsigned part[3];
+      cm_split<3>(k[i].x * gla_exp<T>(log_scale * after.x), k[i].y * gla_exp<T>(log_scale * after.y), part);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) *reinterpret_cast<unsigned*>(k_s + q * k_part + (quarter * 16 + i) * k_stride + d) = part[q];
+      after.x += x[i].x;
+      after.y += x[i].y;
+    }
+  }
+  __syncthreads();
+  float* dst = states + ((((long long)seq * max_chunks + chunk) * n_heads + head) * dim) * vdim + col0;
+  cm_state<3, PARTS, false>(k_s, k_stride, k_part, v_s, v_part, dim,
+                            [&](int c, int at, float a, float b) {
+                              if (col0 + at < vdim) *reinterpret_cast<float2*>(dst + (long long)c * vdim + at) = make_float2(a, b);
+                            },
+                            [](int, float) {});
+}
+
+// gla_prefix_kernel with four value channels a thread and eight chunks asked for at a time.
+__global__ void __launch_bounds__(128)
+gla_prefix_vec_kernel(float* states, const float* __restrict__ ends, float* __restrict__ state, const int* __restrict__ slots,
+                      const int* __restrict__ seq_start, int max_chunks, int n_heads, int dim, int vdim) {
+  pdl_trigger();
+  pdl_wait();
+  const int seq = blockIdx.z, head = blockIdx.y, e = (blockIdx.x * 128 + threadIdx.x) * 4;
+  if (e >= dim * vdim) return;
+  const int n_chunks = (seq_start[seq + 1] - seq_start[seq] + GC - 1) / GC;
+  float4* st = reinterpret_cast<float4*>(state + (((long long)slots[seq] * n_heads + head) * dim) * vdim + e);
+  const long long stride = (long long)n_heads * dim * vdim / 4, end_stride = (long long)n_heads * dim;
+  float4* cell = reinterpret_cast<float4*>(states + (((long long)seq * max_chunks) * n_heads + head) * (long long)dim * vdim + e);
+  const float* end = ends + ((long long)seq * max_chunks * n_heads + head) * dim + e / vdim;
+  float4 s = *st;
+  for (int c = 0; c < n_chunks; c += 8) {
+    float4 kv[8];
+    float decay[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      kv[u] = c + u < n_chunks ? __ldcg(cell + (c + u) * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+      decay[u] = c + u < n_chunks ? end[(c + u) * end_stride] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (c + u >= n_chunks) break;
+      cell[(c + u) * stride] = s;
+      s = make_float4(fmaf(decay[u], s.x, kv[u].x), fmaf(decay[u], s.y, kv[u].y), fmaf(decay[u], s.z, kv[u].z), fmaf(decay[u], s.w, kv[u].w));
+    }
+  }
+  *st = s;
+}
+
+// N sums over lanes at once: lanes `from` apart and then nearer ones, down to `to` apart, hand each other half of their numbers; once a
+// lane is left with one, x[0], the rest of the distances add it up.
+template <int N>
+__device__ __forceinline__ void gla_lane_sums(float (&x)[N], int from, int to) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = from, n = N / 2; o >= to; o >>= 1, n >>= 1) {
+    const bool high = (lane & o) != 0;
+    if (n == 0) x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float give = high ? x[i] : x[i + n], keep = high ? x[i + n] : x[i];
+      x[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+}
+
+constexpr int GD = 20;      // row length of a sub-block's weights ([token s][token t])
+template <typename T, int PARTS>
+__global__ void __launch_bounds__(CM_THREADS, 4)
+gla_out_kernel(const T* __restrict__ proj, long long row_stride, int q_off, int k_off, int v_off, float q_scale, const float* __restrict__ dt,
+               float log_scale, const int* __restrict__ seq_start, float* __restrict__ out, long long out_row_stride,
+               const float* __restrict__ states, int max_chunks, int n_heads, int dim, int vdim, int col_blocks, int held) {
+  extern __shared__ __align__(16) unsigned char cm_smem[];
+  float* q_t = reinterpret_cast<float*>(cm_smem);                      // [dim][GCP]   q_t e^{b_t - B_g(t)}
+  float* k_t = q_t + dim * GCP;                                        // [dim][GCP]   k_s e^{B_(g(s)+1) - b_s}; in its place then
+  const int k_stride = dim + 8, k_part = CM_CHUNK * k_stride, s_part = CM_CHUNK * CM_ROW;
+  __nv_bfloat16* parts = reinterpret_cast<__nv_bfloat16*>(k_t);        // [3][64][dim + 8] k; [3][dim][72] the state; [PARTS][64][72] v
+  float* bs = reinterpret_cast<float*>(cm_smem + held);                // [GG + 1][bsp]  B_0 .. B_16
+  const int bsp = dim | 1;
+  float* a_t = bs + (((GG + 1) * bsp + 3) & ~3);                       // [4][16][GD]  a sub-block's weights on itself
+  pdl_trigger();
+  pdl_wait();
+  const int chunk = blockIdx.x, seq = blockIdx.z;
+  const int head = blockIdx.y / col_blocks, col0 = (blockIdx.y - head * col_blocks) * CM_COLS;
+  const int first = seq_start[seq], n_new = seq_start[seq + 1] - first;
+  if (chunk * CM_CHUNK >= n_new) return;
+  const int len = min(CM_CHUNK, n_new - chunk * CM_CHUNK);
+  const long long row0 = first + (long long)chunk * CM_CHUNK;
+  const T* rows = proj + row0 * row_stride;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // two groups of a warp at a time, a lane two channels: the groups' q, k and decays, and the weights inside a group
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    float w[2][16] = {};
+    const int d = 2 * lane;
+    if (d < dim) {
+      float2 q[2][4], k[2][4], la[2][4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          // (a token past the last one: the last one's numbers, so that all reads are asked for together)
+          const long long t = min(4 * (4 * warp + 2 * pass + h) + i, len - 1);
+          const T* src = rows + t * row_stride + head * dim + d;
+          q[h][i] = cm_load2(src + q_off);
+          k[h][i] = cm_load2(src + k_off);
+          la[h][i] = *reinterpret_cast<const float2*>(dt + ((row0 + t) * n_heads + head) * dim + d);
+        }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int g = 4 * warp + 2 * pass + h;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (4 * g + i >= len) q[h][i] = k[h][i] = la[h][i] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          float qh[4], kh[4], a[4], log_a[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            qh[i] = (u ? q[h][i].y : q[h][i].x) * q_scale;
+            kh[i] = u ? k[h][i].y : k[h][i].x;
+            log_a[i] = (u ? la[h][i].y : la[h][i].x) * log_scale;
+            a[i] = gla_exp<T>(log_a[i]);
+          }
+          bs[(g + 1) * bsp + d + u] = (log_a[0] + log_a[1]) + (log_a[2] + log_a[3]);
+          const float a12 = a[1] * a[2], a23 = a[2] * a[3], a123 = a12 * a[3];
+          // (numbers 4 s + t of a cell of 4 x 4)
+          w[h][0] = fmaf(qh[0], kh[0], w[h][0]);
+          w[h][5] = fmaf(qh[1], kh[1], w[h][5]);
+          w[h][10] = fmaf(qh[2], kh[2], w[h][10]);
+          w[h][15] = fmaf(qh[3], kh[3], w[h][15]);
+          w[h][1] = fmaf(qh[1], kh[0] * a[1], w[h][1]);
+          w[h][6] = fmaf(qh[2], kh[1] * a[2], w[h][6]);
+          w[h][11] = fmaf(qh[3], kh[2] * a[3], w[h][11]);
+          w[h][2] = fmaf(qh[2], kh[0] * a12, w[h][2]);
+          w[h][7] = fmaf(qh[3], kh[1] * a23, w[h][7]);
+          w[h][3] = fmaf(qh[3], kh[0] * a123, w[h][3]);
+          const float p1 = a[0] * a[1], p2 = p1 * a[2], p3 = p2 * a[3];
+          *reinterpret_cast<float4*>(q_t + (d + u) * GCP + 4 * g) = make_float4(qh[0] * a[0], qh[1] * p1, qh[2] * p2, qh[3] * p3);
+          *reinterpret_cast<float4*>(k_t + (d + u) * GCP + 4 * g) = make_float4(kh[0] * a123, kh[1] * a23, kh[2] * a[3], kh[3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      gla_lane_sums(w[h], 16, 1);      // (a lane pair's number: lane / 2)
+      const int g = 2 * pass + h, number = lane >> 1;
+      if ((lane & 1) == 0) a_t[(warp * 16 + 4 * g + number / 4) * GD + 4 * g + number % 4] = w[h][0];
+    }
+  }
+  __syncthreads();
+  if (tid < dim) {
+    float sum = 0.f;
+    bs[tid] = 0.f;
+#pragma unroll
+    for (int g = 1; g <= GG; ++g) {
+      sum += bs[g * bsp + tid];
+      bs[g * bsp + tid] = sum;
+    }
+  }
+  __syncthreads();
+  {
+    // weights between the groups of a sub-block: 24 pairs (later group gt, earlier group gs), four lanes each with a quarter of the channels
+    const int pair = min(tid >> 2, 23), block = pair / 6, r = pair - block * 6;
+    const int later = r < 1 ? 1 : r < 3 ? 2 : 3, earlier = r - later * (later - 1) / 2, gt = 4 * block + later, gs = 4 * block + earlier;
+    float acc[16] = {};
+    const float* bt_ = bs + gt * bsp;
+    const float* bq = bs + (gs + 1) * bsp;
+#pragma unroll 4
+    for (int d = tid & 3; d < dim; d += 4) {
+      const float f = gla_exp<T>(bt_[d] - bq[d]);
+      const float4 qv = *reinterpret_cast<const float4*>(q_t + d * GCP + gt * 4);
+      const float4 kv = *reinterpret_cast<const float4*>(k_t + d * GCP + gs * 4);
+      const float qa[4] = {qv.x, qv.y, qv.z, qv.w}, ka[4] = {kv.x * f, kv.y * f, kv.z * f, kv.w * f};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[4 * j + i] = fmaf(qa[i], ka[j], acc[4 * j + i]);
+    }
+    gla_lane_sums(acc, 2, 1);      // (a lane's four numbers: those of token s = 4 gs + its place among the four)
+    if (tid < 96)
+      *reinterpret_cast<float4*>(a_t + (block * 16 + 4 * earlier + (tid & 3)) * GD + 4 * later) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  }
+  {
+    // k_s e^{B - b_s} with B at the end of s's sub-block, in parts (a thread's numbers wait in registers until k_t has been read)
+    const int t = tid & 63, c0 = (tid >> 6) * 32, g = t >> 2, end = (t >> 4) * 4 + 4;
+    const bool there = t < 48 && c0 < dim;      // (the last sub-block's weights on itself are all there is of it)
+    float x[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const int d = c0 + i;
+      x[i] = there && d < dim ? k_t[d * GCP + t] * gla_exp<T>(bs[end * bsp + d] - bs[(g + 1) * bsp + d]) : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 32; i += 8) {
+      if (!there || c0 + i >= dim) break;
+      unsigned part[4][3];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) cm_split<3>(x[i + 2 * u], x[i + 2 * u + 1], part[u]);
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
+        *reinterpret_cast<uint4*>(parts + p * k_part + t * k_stride + c0 + i) = make_uint4(part[0][p], part[1][p], part[2][p], part[3][p]);
+    }
+  }
+  __syncthreads();
+  const int g = lane >> 2, t2 = (lane & 3) * 2, ta = warp * 16 + g, tb = ta + 8;      // this thread's rows
+  // the operand of 16 channels from d on of q_t e^{b_t - B_ref}
+  auto query = [&](int d, int ref, unsigned (&a)[3][4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = i & 1 ? tb : ta, c = d + t2 + 8 * (i >> 1);
+      const float* b = bs + (t >> 2) * bsp + c;
+      const float* r = bs + ref * bsp + c;
+      unsigned part[3];
+      cm_split<3>(q_t[c * GCP + t] * gla_exp<T>(b[0] - r[0]), q_t[(c + 1) * GCP + t] * gla_exp<T>(b[1] - r[1]), part);
+#pragma unroll
+      for (int p = 0; p < 3; ++p) a[p][i] = part[p];
+    }
+  };
+  float sc[8][4];      // the weights of this warp's tokens on those up to its last one
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float small[2][4] = {};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sc[2 * j][i] = sc[2 * j + 1][i] = 0.f;
+    if (j < warp) {
+      for (int d = 0; d < dim; d += 16) {
+        unsigned a[3][4], b[3][4];
+        query(d, 4 * j + 4, a);
+        // (matrices: tokens 16 j.. of channels d.., of channels d + 8.., then tokens 16 j + 8..)
+        const __nv_bfloat16* at = parts + (16 * j + (lane & 7) + (lane >> 4) * 8) * k_stride + d + (lane >> 3 & 1) * 8;
+#pragma unroll
+        for (int p = 0; p < 3; ++p) cm_ldmatrix(b[p], at + p * k_part);
+        cm_products<3, 3>(sc[2 * j], small[0], sc[2 * j + 1], small[1], a, b);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        sc[2 * j][i] += small[0][i];
+        sc[2 * j + 1][i] += small[1][i];
+      }
+    } else if (j == warp) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int t = g + 8 * (i >> 1), at = 8 * h + t2 + (i & 1);
+          sc[2 * j + h][i] = at <= t ? a_t[(warp * 16 + at) * GD + t] : 0.f;
+        }
+    }
+  }
+  __syncthreads();      // k has been read
+  const float* src = states + ((((long long)seq * max_chunks + chunk) * n_heads + head) * dim) * vdim + col0;
+  cm_fill<3>(parts, dim, CM_COLS, CM_ROW, s_part, [&](int d, int c, float (&x)[8]) {
+    if (col0 + c < vdim) cm_load8(src + (long long)d * vdim + c, x);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = col0 + c < vdim ? x[u] : 0.f;
+  });
+  __syncthreads();
+  float o[8][4], o_small[8][4];
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[j][i] = o_small[j][i] = 0.f;
+  for (int d = 0; d < dim; d += 16) {
+    unsigned a[3][4];
+    query(d, 0, a);
+    cm_step_rows<3, 3, 8>(o, o_small, a, parts, d, s_part);
+  }
+  __syncthreads();      // the state has been read
+  cm_fill<PARTS>(parts, CM_CHUNK, CM_COLS, CM_ROW, s_part, [&](int t, int c, float (&x)[8]) {
+    const bool in = t < len && col0 + c < vdim;
+    if (in) cm_load8(rows + t * row_stride + v_off + head * vdim + col0 + c, x);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = in ? x[u] : 0.f;
+  });
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {      // 16 tokens s at a time
+    if (j > warp) break;
+    unsigned a[3][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      unsigned part[3];
+      cm_split<3>(sc[2 * j + (i >> 1)][2 * (i & 1)], sc[2 * j + (i >> 1)][2 * (i & 1) + 1], part);
+#pragma unroll
+      for (int p = 0; p < 3; ++p) a[p][i] = part[p];
+    }
+    cm_step_rows<3, PARTS, 8>(o, o_small, a, parts, 16 * j, s_part);
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int c = 8 * j + t2;
+    if (col0 + c >= vdim) break;
+    float* at = out + row0 * out_row_stride + (long long)head * vdim + col0 + c;
+    if (ta < len) *reinterpret_cast<float2*>(at + ta * out_row_stride) = make_float2(o[j][0] + o_small[j][0], o[j][1] + o_small[j][1]);
+    if (tb < len) *reinterpret_cast<float2*>(at + tb * out_row_stride) = make_float2(o[j][2] + o_small[j][2], o[j][3] + o_small[j][3]);
+  }
+}
+
 // Scratch of the chunked form: [states | ends | aged_q].
 static inline long long gla_state_floats(int n_seqs, int max_new, int n_heads, int dim, int vdim) {
   return (long long)n_seqs * ((max_new + GC - 1) / GC) * n_heads * dim * vdim;
 }
 static inline long long gla_end_floats(int n_seqs, int max_new, int n_heads, int dim) {
   return (long long)n_seqs * ((max_new + GC - 1) / GC) * n_heads * dim;
+}
+
+template <typename T, int PARTS>
+static int launch_gla_mma(const T* proj, long long row_stride, int q_off, int k_off, int v_off, float q_scale, const float* dt,
+                          float log_scale, float* state, const int* slots, const int* seq_start, float* out, long long out_row_stride,
+                          float* states, float* ends, int max_chunks, int n_seqs, int n_heads, int dim, int vdim, int col_blocks,
+                          cudaStream_t stream) {
+  const dim3 grid(max_chunks, n_heads * col_blocks, n_seqs), block(CM_THREADS);
+  const size_t rows_k = 2 * 3 * (size_t)CM_CHUNK * (dim + 8), rows_v = 2 * (size_t)PARTS * CM_CHUNK * CM_ROW;
+  const size_t smem_s = rows_k + rows_v + (size_t)2 * dim * sizeof(float2);
+  // (k_t, the parts of k, of the state and of v lie in one place in turn; the state's are the longest)
+  const size_t held = (size_t)dim * GCP * sizeof(float) + 2 * 3 * (size_t)CM_CHUNK * CM_ROW;
+  const size_t smem_o = held + ((((size_t)(GG + 1) * (dim | 1) + 3) & ~(size_t)3) + 4 * 16 * GD) * sizeof(float);
+  static SharedMemoryAllowance allowed_s, allowed_o;
+  BT_CHECK(allow_shared_memory(allowed_s, gla_state_kernel<T, PARTS>, smem_s) && allow_shared_memory(allowed_o, gla_out_kernel<T, PARTS>, smem_o),
+           "gla: cannot reserve %zu bytes of shared memory", smem_s > smem_o ? smem_s : smem_o);
+  BT_PDL_OK("gla_state", launch_pdl(gla_state_kernel<T, PARTS>, grid, block, smem_s, stream, 1, proj, row_stride, k_off, v_off, dt,
+                                    log_scale, seq_start, states, ends, max_chunks, n_heads, dim, vdim, col_blocks));
+  if ((unsigned long long)state % 16 == 0)
+    BT_PDL_OK("gla_prefix", launch_pdl(gla_prefix_vec_kernel, dim3((dim * vdim + 511) / 512, n_heads, n_seqs), dim3(128), 0, stream, 1, states,
+                                       (const float*)ends, state, slots, seq_start, max_chunks, n_heads, dim, vdim));
+  else
+    BT_PDL_OK("gla_prefix", launch_pdl(gla_prefix_kernel, dim3((dim * vdim + 255) / 256, n_heads, n_seqs), dim3(256), 0, stream, 1, states,
+                                       (const float*)ends, state, slots, seq_start, max_chunks, n_heads, dim, vdim));
+  BT_PDL_OK("gla_out", launch_pdl(gla_out_kernel<T, PARTS>, grid, block, smem_o, stream, 1, proj, row_stride, q_off, k_off, v_off, q_scale,
+                                  dt, log_scale, seq_start, out, out_row_stride, (const float*)states, max_chunks, n_heads, dim, vdim,
+                                  col_blocks, (int)held));
+  return 0;
 }
 
 template <typename T>
@@ -562,6 +964,11 @@ static int launch_gla_chunked(const T* proj, long long row_stride, int q_off, in
   constexpr int V = 16 / (int)sizeof(T);
   const int vec = dim % 4 == 0 && vdim % V == 0 && v_off % V == 0 && row_stride % V == 0 && out_row_stride % 4 == 0 &&
                   ((unsigned long long)proj | (unsigned long long)out | (unsigned long long)states | (unsigned long long)aged_q) % 16 == 0;
+  if (vec && dim % 16 == 0 && dim >= (sizeof(T) == 4 ? 32 : 16) && dim <= 64 && vdim % 8 == 0 && v_off % 8 == 0 && q_off % 2 == 0 && k_off % 2 == 0 && row_stride % 8 == 0 &&
+      (unsigned long long)dt % 8 == 0 && (unsigned long long)ends % 8 == 0)
+    return launch_gla_mma<T, sizeof(T) == 2 ? 1 : 3>(proj, row_stride, q_off, k_off, v_off, q_scale, dt, log_scale, state, slots, seq_start,
+                                                     out, out_row_stride, states, ends, max_chunks, n_seqs, n_heads, dim, vdim, col_blocks,
+                                                     stream);
   BT_PDL_OK("gla_chunk", launch_pdl(chunk_kernel, grid, block, smem_a, stream, 1, proj, row_stride, q_off, k_off, v_off, q_scale,
                                     dt, log_scale, seq_start, out, out_row_stride, states, ends, aged_q, max_chunks, n_heads,
                                     dim, vdim, col_blocks, vec));
