@@ -490,14 +490,15 @@ lightning_carry_kernel(const T* __restrict__ proj, long long row_stride, int q_o
 // again; these by the forming of the features and the parts, and by the products.  All three kernels, above and here, in us: 2 x 1,024
 // tokens of 16 heads of 64 x 64 with act 0 65 and 49, 6 x 1,000 of 12 heads 112 and 88, with act 1 101 and 58, 32-bit rows 2 x 1,024
 // 69 and 39.  Errors against 64 bits 1.2e-7 and 7e-8 (act 0), 1.8e-7 and 9e-8 (act 1).
-// x * sigmoid(x) for these kernels: the library's division is half of its instructions; here a reciprocal and one Newton step (the
-// argument is bounded so that the reciprocal is a normal number)
+// x * sigmoid(x) for these kernels: the library's division is half of its instructions; here a reciprocal and one Newton step, of a number
+// between one and two: e^-|x| neither overflows nor makes the reciprocal a number that is not normal.
 __device__ __forceinline__ float cm_feature(float x, int act) {
   if (act != 0) return x;
-  const float y = 1.f + expf(fminf(-x, 87.f));
+  const float e = expf(-fabsf(x)), y = 1.f + e;
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(y));
-  return x * fmaf(r, fmaf(-y, r, 1.f), r);
+  r = fmaf(r, fmaf(-y, r, 1.f), r);
+  return x * (x < 0.f ? e * r : r);
 }
 
 template <typename T, int PARTS>
