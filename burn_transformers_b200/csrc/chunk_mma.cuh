@@ -1,9 +1,15 @@
 // The products inside a chunk of 64 tokens of a recurrence (lightning.cu, mlstm.cu), on tensor cores with no operand's bits given up:
 // a 32-bit number goes in as the sum of three bfloat16 numbers (the residues are exact), a number that bfloat16 holds as itself,
-// and the products whose parts' orders add up to two at most are formed; what is left out is below 2^-24 of a product.
+// and the products whose parts' orders add up to two at most are formed; what is left out is below 2^-24 of a product (of a number below
+// 2^-110 the parts end at 2^-133, bfloat16's last).
 //
 // Tensor cores cut their sums where a multiply-add rounds them.  So the products of the first parts begin from zero at every step of
 // 16 along the sum and are added in 32-bit registers; those of the smaller parts, 2^-8 and less of the result, share accumulators.
+//
+// A number that is infinite, or that bfloat16 rounds to infinity, has no parts: its residue is none.  And a weight of zero that stands for a
+// later token meets that token's values all the same.  Either way the sum that it meets is no finite number, whatever else is in it; the
+// kernels look for such results when they have written them and form them again by multiply-adds (cm_state says whether there are
+// any, cm_bad_rows where; cm_plain_row forms a row).
 //
 // A block is four warps with 16 rows of the result each.  The second operands lie in shared memory, their parts one behind the
 // other, in rows of (columns + 8) numbers: eight rows' 16-byte pieces then meet all banks, however they are read.
@@ -126,11 +132,12 @@ __device__ __forceinline__ void cm_step_rows(float (&big)[TILES][4], float (&sma
 
 // The chunk's contribution to the state, rows d of `dim` (16 a warp and round), columns [0, 64):  sum_s K'[s][d] V[s][c], K' and V in
 // shared memory ([token][channel]; KP and VP parts).  store(d, c, x, y) gets the numbers of columns c and c + 1; ones(d, sum), the sum of
-// K' alone, where SUMS is set.
+// K' alone, where SUMS is set.  Whether one of this thread's numbers is not finite.
 template <int KP, int VP, bool SUMS, typename Store, typename Ones>
-__device__ __forceinline__ void cm_state(const __nv_bfloat16* k, int k_stride, int k_part, const __nv_bfloat16* v, int v_part, int dim,
+__device__ __forceinline__ bool cm_state(const __nv_bfloat16* k, int k_stride, int k_part, const __nv_bfloat16* v, int v_part, int dim,
                                          Store store, Ones ones) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t2 = (lane & 3) * 2;
+  float zeros = 0.f;      // (zero times every number)
   for (int d0 = warp * 16; d0 < dim; d0 += 64) {
     float big[8][4] = {}, small[8][4] = {}, sums[4] = {};
 #pragma unroll
@@ -147,14 +154,62 @@ __device__ __forceinline__ void cm_state(const __nv_bfloat16* k, int k_stride, i
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      store(d0 + g, 8 * j + t2, big[j][0] + small[j][0], big[j][1] + small[j][1]);
-      store(d0 + g + 8, 8 * j + t2, big[j][2] + small[j][2], big[j][3] + small[j][3]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        big[j][i] += small[j][i];
+        zeros = fmaf(big[j][i], 0.f, zeros);
+      }
+      store(d0 + g, 8 * j + t2, big[j][0], big[j][1]);
+      store(d0 + g + 8, 8 * j + t2, big[j][2], big[j][3]);
     }
     if (SUMS && (lane & 3) == 0) {
       ones(d0 + g, sums[0]);
       ones(d0 + g + 8, sums[2]);
     }
   }
+  return zeros != 0.f;      // (no number, where one is not finite)
+}
+
+// Of a warp's 16 rows those with a number that is not finite, a bit each; a, b: whether this thread has one in its rows lane / 4 and lane / 4 + 8.
+__device__ __forceinline__ unsigned cm_bad_rows(bool a, bool b) {
+  unsigned rows = 0;
+  const unsigned all_a = __ballot_sync(0xffffffffu, a), all_b = __ballot_sync(0xffffffffu, b);
+#pragma unroll
+  for (int g = 0; g < 8; ++g) {
+    rows |= (unsigned)((all_a >> (4 * g) & 15u) != 0) << g;
+    rows |= (unsigned)((all_b >> (4 * g) & 15u) != 0) << (g + 8);
+  }
+  return rows;
+}
+
+// The chunk's token t by multiply-adds, a warp together, columns lane and lane + 32 of a block's: x = carry * sum_d q(d) in(d, c) and then, token
+// by token, weigh(s, q . k_s) v(s, c).  The sum of the weights is returned.
+template <typename Q, typename K, typename V, typename In, typename Weigh>
+__device__ __forceinline__ float cm_plain_row(int t, int dim, int cols, float carry, Q q, K k, V v, In in, Weigh weigh, float (&x)[2]) {
+  const int lane = threadIdx.x & 31;
+  float sum = 0.f;
+  x[0] = x[1] = 0.f;
+#pragma unroll 1
+  for (int d = 0; d < dim; ++d) {
+    const float y = q(d);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (lane + 32 * i < cols) x[i] = fmaf(y, in(d, lane + 32 * i), x[i]);
+  }
+  x[0] *= carry;
+  x[1] *= carry;
+#pragma unroll 1
+  for (int s = 0; s <= t; ++s) {
+    float w = 0.f;
+#pragma unroll 1
+    for (int d = lane; d < dim; d += 32) w = fmaf(q(d), k(s, d), w);
+    w = weigh(s, warp_sum(w));
+    sum += w;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (lane + 32 * i < cols) x[i] = fmaf(w, v(s, lane + 32 * i), x[i]);
+  }
+  return sum;
 }
 
 }  // namespace bt

@@ -534,11 +534,26 @@ lightning_state_kernel(const T* __restrict__ proj, long long row_stride, int k_o
   });
   __syncthreads();
   float* dst = scratch + ((((long long)seq * max_chunks + chunk) * n_heads + head) * dim) * vdim + col0;
-  cm_state<3, PARTS, false>(k_s, k_stride, k_part, v_s, v_part, dim,
-                            [&](int d, int c, float x, float y) {
-                              if (col0 + c < vdim) *reinterpret_cast<float2*>(dst + (long long)d * vdim + c) = make_float2(x, y);
-                            },
-                            [](int, float) {});
+  const bool bad = cm_state<3, PARTS, false>(k_s, k_stride, k_part, v_s, v_part, dim,
+                                             [&](int d, int c, float x, float y) {
+                                               if (col0 + c < vdim) *reinterpret_cast<float2*>(dst + (long long)d * vdim + c) = make_float2(x, y);
+                                             },
+                                             [](int, float) {});
+  if (!__syncthreads_or(bad)) return;
+  const int cols = min(CM_COLS, vdim - col0);
+  for (int i = threadIdx.x; i < dim * cols; i += CM_THREADS) {
+    const int d = i / cols, c = i - d * cols;
+    float* at = dst + (long long)d * vdim + c;
+    if (isfinite(*at)) continue;
+    float x = 0.f;
+#pragma unroll 1
+    for (int s = 0; s < len; ++s) {
+      const T* row = rows + s * row_stride;
+      x = fmaf(feature(to_float(row[k_off + head * dim + d]), act) * pw[len - 1 - s],
+               feature(to_float(row[v_off + head * vdim + col0 + c]), act), x);
+    }
+    *at = x;
+  }
 }
 
 template <typename T, int PARTS>
@@ -662,13 +677,37 @@ lightning_out_kernel(const T* __restrict__ proj, long long row_stride, int q_off
     }
     cm_step_rows<3, PARTS, 8>(o, o_small, a, s_s, 16 * j, s_part);
   }
+  float zeros[2] = {0.f, 0.f};      // (zero times every number of a row)
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int c = 8 * j + t2;
     if (col0 + c >= vdim) break;
     float* at = out + row0 * out_row_stride + (long long)head * vdim + col0 + c;
-    if (ta < len) *reinterpret_cast<float2*>(at + ta * out_row_stride) = make_float2(o[j][0] + o_small[j][0], o[j][1] + o_small[j][1]);
-    if (tb < len) *reinterpret_cast<float2*>(at + tb * out_row_stride) = make_float2(o[j][2] + o_small[j][2], o[j][3] + o_small[j][3]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      o[j][i] += o_small[j][i];
+      zeros[i >> 1] = fmaf(o[j][i], 0.f, zeros[i >> 1]);
+    }
+    if (ta < len) *reinterpret_cast<float2*>(at + ta * out_row_stride) = make_float2(o[j][0], o[j][1]);
+    if (tb < len) *reinterpret_cast<float2*>(at + tb * out_row_stride) = make_float2(o[j][2], o[j][3]);
+  }
+  unsigned redo = cm_bad_rows(ta < len && zeros[0] != 0.f, tb < len && zeros[1] != 0.f);
+  if (redo == 0) return;
+  __syncwarp();
+  const int cols = min(CM_COLS, vdim - col0);
+  for (; redo; redo &= redo - 1) {
+    const int t = warp * 16 + __ffs(redo) - 1;
+    auto number = [&](int token, int at) { return feature(to_float(rows[token * row_stride + at]), act); };
+    float x[2];
+    cm_plain_row(t, dim, cols, pw[t + 1], [&](int d) { return number(t, q_off + head * dim + d); },
+                 [&](int s, int d) { return number(s, k_off + head * dim + d); },
+                 [&](int s, int c) { return number(s, v_off + head * vdim + col0 + c); },
+                 [&](int d, int c) { return src[(long long)d * vdim + c]; }, [&](int s, float w) { return w * pw[t - s]; }, x);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float* at = out + (row0 + t) * out_row_stride + (long long)head * vdim + col0 + lane + 32 * i;
+      if (lane + 32 * i < cols && !isfinite(*at)) *at = x[i];
+    }
   }
 }
 

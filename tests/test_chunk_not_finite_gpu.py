@@ -1,4 +1,6 @@
-"""The recurrences' chunks on tensor cores at the ends of the numbers' range: x sigmoid(x) far below zero."""
+"""The recurrences' chunks on tensor cores at the ends of the numbers' range.  Values that have no parts: infinities, and 32-bit numbers that
+bfloat16 rounds to one, against the chunks' formulas in 64 bits, token by token in the order of time: what is a number there is one here, what
+is an infinity has its sign, and no token's result depends on a later token.  And x sigmoid(x) far below zero."""
 import pytest
 import torch
 
@@ -6,6 +8,85 @@ from burn_transformers_b200 import kernels
 
 pytestmark = pytest.mark.gpu
 DEV, F64 = "cuda", torch.float64
+CHUNK, LENGTHS, HEADS = 64, [70, 300], 16
+
+
+def step(lengths):
+    starts = [sum(lengths[:i]) for i in range(len(lengths) + 1)]
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    return starts, ints(starts), ints(list(range(len(lengths), 0, -1)))
+
+
+def outer(k, v):
+    return k[:, :, None] * v[:, None, :]
+
+
+def dot(q, m):      # sum over the key channels, without a library product (whose padding would meet the infinities)
+    return (q[:, :, None] * m).sum(1)
+
+
+def same(got, want, size):
+    """Equal kinds everywhere; where `want` is a number, within what sums of some hundred 32-bit terms of total `size` may lose."""
+    got, inf = got.to(F64).reshape(want.shape), torch.isinf(want)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(got[inf], want[inf])
+    ok = torch.isfinite(want) & torch.isfinite(size)
+    assert float(((got - want).abs()[ok] / size[ok].clamp_min(1e-300)).max()) < 256 * 2.0 ** -23
+
+
+def spoil(rows, lo, v, kind, dim, vdim):
+    """Puts the numbers in question into the values (at offset v) of the sequence whose rows begin at lo."""
+    if kind == "infinite":
+        rows[lo + 21, v + 2 * vdim + 5] = float("inf")
+        rows[lo + 100, v + 3 * vdim] = float("-inf")
+        rows[lo + 5, v + 4 * vdim + vdim - 1] = float("nan")
+    else:
+        rows[lo + 30, v + 2 * vdim + 5] = 3.4e38
+        rows[lo + 77, v + 3 * vdim] = -3.4e38
+
+
+KINDS = [(torch.bfloat16, "infinite"), (torch.float32, "infinite"), (torch.float32, "largest")]
+
+
+@pytest.mark.parametrize("dim, vdim", [(16, 24), (64, 64), (128, 72)])
+@pytest.mark.parametrize("dtype, kind", KINDS)
+@pytest.mark.parametrize("activation", ["swish", None])
+def test_decayed_chunks(dim, vdim, dtype, kind, activation):
+    torch.manual_seed(dim)
+    starts, seq_start, slots = step(LENGTHS)
+    n, wide = starts[-1], HEADS * (2 * dim + vdim)
+    rows = torch.randn(n, wide, device=DEV) * (1e-3 if kind == "largest" else 1.0)
+    spoil(rows, starts[1], 2 * HEADS * dim, kind, dim, vdim)
+    if activation and kind == "infinite":
+        rows.nan_to_num_(nan=float("nan"), posinf=float("inf"), neginf=float("inf"))      # (x sigmoid(x) of minus infinity is no number)
+    proj, decay = rows.to(dtype), torch.rand(HEADS, device=DEV) * 0.2 + 0.8
+    state = torch.randn(3, HEADS, dim, vdim, device=DEV)
+    first, out = state.clone(), torch.empty(n, HEADS * vdim, device=DEV)
+    scratch = torch.empty(kernels.lightning_chunked_scratch_floats(2, max(LENGTHS), HEADS, dim, vdim), device=DEV)
+    kernels.lightning_scan(proj, 0, HEADS * dim, 2 * HEADS * dim, state, slots, seq_start, decay, out, n_seqs=2, n_heads=HEADS, dim=dim,
+                           vdim=vdim, max_new=max(LENGTHS), scratch=scratch, activation=activation)
+    x, lam = proj.to(F64), decay.to(F64)[:, None]
+    x = x * torch.sigmoid(x) if activation else x
+    for i in range(2):
+        S = first[2 - i].to(F64)
+        T = S.abs()      # the same with every number's size
+        want, size = [], []
+        for lo in range(starts[i], starts[i + 1], CHUNK):
+            hi = min(lo + CHUNK, starts[i + 1])
+            q, k, v = (x[lo:hi, a:a + HEADS * d].view(hi - lo, HEADS, d) for a, d in ((0, dim), (HEADS * dim, dim), (2 * HEADS * dim, vdim)))
+            for t in range(hi - lo):
+                o, u = lam ** (t + 1) * dot(q[t], S), lam ** (t + 1) * dot(q[t].abs(), T)
+                for s in range(t + 1):
+                    o = o + lam ** (t - s) * (q[t] * k[s]).sum(-1, keepdim=True) * v[s]
+                    u = u + lam ** (t - s) * (q[t] * k[s]).abs().sum(-1, keepdim=True) * v[s].abs()
+                want.append(o)
+                size.append(u)
+            fall = lam[:, :, None] ** (hi - lo)
+            S, T = fall * S, fall * T
+            for s in range(hi - lo):
+                f = lam[:, :, None] ** (hi - lo - 1 - s)
+                S, T = S + f * outer(k[s], v[s]), T + f * outer(k[s], v[s]).abs()
+        same(out[starts[i]:starts[i + 1]], torch.stack(want), torch.stack(size))
+        same(state[2 - i], S, T)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
