@@ -1,4 +1,4 @@
-// The products inside a chunk of 64 tokens of a recurrence (lightning.cu, mlstm.cu), on tensor cores with no operand's bits given up:
+// The products inside a chunk of 64 tokens of a recurrence (lightning.cu, mlstm.cu, gla.cu), on tensor cores with no operand's bits given up:
 // a 32-bit number goes in as the sum of three bfloat16 numbers (the residues are exact), a number that bfloat16 holds as itself,
 // and the products whose parts' orders add up to two at most are formed; what is left out is below 2^-24 of a product (of a number below
 // 2^-110 the parts end at 2^-133, bfloat16's last).
@@ -131,15 +131,15 @@ __device__ __forceinline__ void cm_step_rows(float (&big)[TILES][4], float (&sma
 }
 
 // The chunk's contribution to the state, rows d of `dim` (16 a warp and round), columns [0, 64):  sum_s K'[s][d] V[s][c], K' and V in
-// shared memory ([token][channel]; KP and VP parts).  store(d, c, x, y) gets the numbers of columns c and c + 1; ones(d, sum), the sum of
-// K' alone, where SUMS is set.  Whether one of this thread's numbers is not finite.
-template <int KP, int VP, bool SUMS, typename Store, typename Ones>
+// shared memory ([token][channel]; KP and VP parts).  store(d, c, x, y) gets the numbers of columns c and c + 1.  Whether one of this
+// thread's numbers is not finite.
+template <int KP, int VP, typename Store>
 __device__ __forceinline__ bool cm_state(const __nv_bfloat16* k, int k_stride, int k_part, const __nv_bfloat16* v, int v_part, int dim,
-                                         Store store, Ones ones) {
+                                         Store store) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t2 = (lane & 3) * 2;
   float zeros = 0.f;      // (zero times every number)
   for (int d0 = warp * 16; d0 < dim; d0 += 64) {
-    float big[8][4] = {}, small[8][4] = {}, sums[4] = {};
+    float big[8][4] = {}, small[8][4] = {};
 #pragma unroll
     for (int s = 0; s < CM_CHUNK; s += 16) {
       unsigned a[KP][4];
@@ -148,9 +148,6 @@ __device__ __forceinline__ bool cm_state(const __nv_bfloat16* k, int k_stride, i
 #pragma unroll
       for (int q = 0; q < KP; ++q) cm_ldmatrix_t(a[q], at + q * k_part);
       cm_step_rows<KP, VP, 8>(big, small, a, v, s, v_part);
-      if (SUMS)
-#pragma unroll
-        for (int q = KP - 1; q >= 0; --q) cm_mma(sums, a[q], 0x3f803f80u, 0x3f803f80u);
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -161,10 +158,6 @@ __device__ __forceinline__ bool cm_state(const __nv_bfloat16* k, int k_stride, i
       }
       store(d0 + g, 8 * j + t2, big[j][0], big[j][1]);
       store(d0 + g + 8, 8 * j + t2, big[j][2], big[j][3]);
-    }
-    if (SUMS && (lane & 3) == 0) {
-      ones(d0 + g, sums[0]);
-      ones(d0 + g + 8, sums[2]);
     }
   }
   return zeros != 0.f;      // (no number, where one is not finite)

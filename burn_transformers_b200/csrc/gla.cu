@@ -614,11 +614,9 @@ gla_state_kernel(const T* __restrict__ proj, long long row_stride, int k_off, in
   }
   __syncthreads();
   float* dst = states + ((((long long)seq * max_chunks + chunk) * n_heads + head) * dim) * vdim + col0;
-  cm_state<3, PARTS, false>(k_s, k_stride, k_part, v_s, v_part, dim,
-                            [&](int c, int at, float a, float b) {
-                              if (col0 + at < vdim) *reinterpret_cast<float2*>(dst + (long long)c * vdim + at) = make_float2(a, b);
-                            },
-                            [](int, float) {});
+  cm_state<3, PARTS>(k_s, k_stride, k_part, v_s, v_part, dim, [&](int c, int at, float a, float b) {
+    if (col0 + at < vdim) *reinterpret_cast<float2*>(dst + (long long)c * vdim + at) = make_float2(a, b);
+  });
 }
 
 // gla_prefix_kernel with four value channels a thread and eight chunks asked for at a time.

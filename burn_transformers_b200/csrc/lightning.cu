@@ -534,11 +534,9 @@ lightning_state_kernel(const T* __restrict__ proj, long long row_stride, int k_o
   });
   __syncthreads();
   float* dst = scratch + ((((long long)seq * max_chunks + chunk) * n_heads + head) * dim) * vdim + col0;
-  const bool bad = cm_state<3, PARTS, false>(k_s, k_stride, k_part, v_s, v_part, dim,
-                                             [&](int d, int c, float x, float y) {
-                                               if (col0 + c < vdim) *reinterpret_cast<float2*>(dst + (long long)d * vdim + c) = make_float2(x, y);
-                                             },
-                                             [](int, float) {});
+  const bool bad = cm_state<3, PARTS>(k_s, k_stride, k_part, v_s, v_part, dim, [&](int d, int c, float x, float y) {
+    if (col0 + c < vdim) *reinterpret_cast<float2*>(dst + (long long)d * vdim + c) = make_float2(x, y);
+  });
   if (!__syncthreads_or(bad)) return;
   const int cols = min(CM_COLS, vdim - col0);
   for (int i = threadIdx.x; i < dim * cols; i += CM_THREADS) {

@@ -673,11 +673,30 @@ __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_state_kernel(const T* __r
     w_end[threadIdx.x] = threadIdx.x < len ? expf(c.gc[gl] - c.gm[gl] + c.ga[g] - c.gc[g]) : 0.f;
   }
   __syncthreads();
-  cm_fill<3>(k_s, MC, dim, k_stride, k_part, [&](int t, int ch, float (&x)[8]) {
-    if (t < len) cm_load8(rows + t * p.row_stride + p.k_off + head * dim + ch, x);
+  // Keys times their weights, in parts; and n in multiply-adds, each product and sum rounded once: a thread's tokens of eight channels here,
+  // the threads of a channel in order further below.  (As a product of the parts with ones, n was cut twelve times a chunk: 1.3e-7 of it
+  // on average, where the multiply-adds' errors of 8e-8 have no sign.)
+  const int pieces = dim / 8, at_once = CM_THREADS / pieces, k_first = threadIdx.x / pieces, k_ch = (threadIdx.x - k_first * pieces) * 8;
+  float n[8] = {};
+  if (k_first < at_once) {
+#pragma unroll 2
+    for (int t = k_first; t < MC; t += at_once) {
+      float x[8] = {};
+      if (t < len) cm_load8(rows + t * p.row_stride + p.k_off + head * dim + k_ch, x);
+      const float w = w_end[t];
+      unsigned part[4][3];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) x[u] = t < len ? x[u] * w_end[t] : 0.f;
-  });
+      for (int u = 0; u < 8; ++u) {
+        n[u] = fmaf(x[u], w, n[u]);
+        x[u] *= w;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) cm_split<3>(x[2 * u], x[2 * u + 1], part[u]);
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        *reinterpret_cast<uint4*>(k_s + q * k_part + t * k_stride + k_ch) = make_uint4(part[0][q], part[1][q], part[2][q], part[3][q]);
+    }
+  }
   cm_fill<PARTS>(v_s, MC, CM_COLS, CM_ROW, v_part, [&](int t, int ch, float (&x)[8]) {
     const bool in = t < len && col0 + ch < vdim;
     if (in) cm_load8(rows + t * p.row_stride + p.v_off + head * vdim + col0 + ch, x);
@@ -687,13 +706,21 @@ __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_state_kernel(const T* __r
   __syncthreads();
   const long long cell = ((long long)seq * c.max_chunks + chunk) * H + head;
   float* dst = c.ds + cell * dim * vdim + col0;
-  cm_state<3, PARTS, true>(k_s, k_stride, k_part, v_s, v_part, dim,
-                           [&](int d, int ch, float x, float y) {
-                             if (col0 + ch < vdim) *reinterpret_cast<float2*>(dst + (long long)d * vdim + ch) = make_float2(x, y);
-                           },
-                           [&](int d, float sum) {
-                             if (col_block == 0) c.dn[cell * dim + d] = sum;
-                           });
+  cm_state<3, PARTS>(k_s, k_stride, k_part, v_s, v_part, dim, [&](int d, int ch, float x, float y) {
+    if (col0 + ch < vdim) *reinterpret_cast<float2*>(dst + (long long)d * vdim + ch) = make_float2(x, y);
+  });
+  if (col_block != 0) return;
+  __syncthreads();      // the keys have been read
+  float* n_s = reinterpret_cast<float*>(cm_smem);      // [at_once][dim]
+  if (k_first < at_once)
+#pragma unroll
+    for (int u = 0; u < 8; u += 4) *reinterpret_cast<float4*>(n_s + k_first * dim + k_ch + u) = make_float4(n[u], n[u + 1], n[u + 2], n[u + 3]);
+  __syncthreads();
+  for (int d = threadIdx.x; d < dim; d += CM_THREADS) {
+    float sum = n_s[d];
+    for (int i = 1; i < at_once; ++i) sum += n_s[i * dim + d];
+    c.dn[cell * dim + d] = sum;
+  }
 }
 
 template <typename T>
