@@ -795,8 +795,15 @@ __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_out_kernel(const T* __res
         asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(b0), "=r"(b1)
                      : "r"((unsigned)__cvta_generic_to_shared(s_s + pb * s_part + (d + (lane & 15)) * CM_ROW + CM_COLS)) : "memory");
 #pragma unroll
-        for (int pa = 0; pa < PARTS; ++pa)
-          if (pa + pb <= 2) cm_mma(pa + pb == 0 ? nq : nq_small, a[pa], b0, b1);
+        for (int pa = 0; pa < PARTS; ++pa) {
+          if (pa + pb == 0) {
+            float x[4];
+            cm_mma_zero(x, a[0], b0, b1);
+            cm_add(nq, x);
+          } else if (pa + pb <= 2) {
+            cm_mma(nq_small, a[pa], b0, b1);
+          }
+        }
       }
     }
     const float fa = f_s[ta] * p.q_scale, fb = f_s[tb] * p.q_scale;
