@@ -132,12 +132,12 @@ __device__ __forceinline__ void cm_step_rows(float (&big)[TILES][4], float (&sma
 
 // The chunk's contribution to the state, rows d of `dim` (16 a warp and round), columns [0, 64):  sum_s K'[s][d] V[s][c], K' and V in
 // shared memory ([token][channel]; KP and VP parts).  store(d, c, x, y) gets the numbers of columns c and c + 1.  Whether one of this
-// thread's numbers is not finite.
+// thread's numbers may not be finite.
 template <int KP, int VP, typename Store>
 __device__ __forceinline__ bool cm_state(const __nv_bfloat16* k, int k_stride, int k_part, const __nv_bfloat16* v, int v_part, int dim,
                                          Store store) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t2 = (lane & 3) * 2;
-  float zeros = 0.f;      // (zero times every number)
+  float zeros = 0.f;      // (zero times all numbers' sum, which is no finite number if one of them is none)
   for (int d0 = warp * 16; d0 < dim; d0 += 64) {
     float big[8][4] = {}, small[8][4] = {};
 #pragma unroll
@@ -152,15 +152,13 @@ __device__ __forceinline__ bool cm_state(const __nv_bfloat16* k, int k_stride, i
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        big[j][i] += small[j][i];
-        zeros = fmaf(big[j][i], 0.f, zeros);
-      }
+      for (int i = 0; i < 4; ++i) big[j][i] += small[j][i];
+      zeros = fmaf((big[j][0] + big[j][1]) + (big[j][2] + big[j][3]), 0.f, zeros);
       store(d0 + g, 8 * j + t2, big[j][0], big[j][1]);
       store(d0 + g + 8, 8 * j + t2, big[j][2], big[j][3]);
     }
   }
-  return zeros != 0.f;      // (no number, where one is not finite)
+  return zeros != 0.f;
 }
 
 // Of a warp's 16 rows those with a number that is not finite, a bit each; a, b: whether this thread has one in its rows lane / 4 and lane / 4 + 8.

@@ -675,17 +675,16 @@ lightning_out_kernel(const T* __restrict__ proj, long long row_stride, int q_off
     }
     cm_step_rows<3, PARTS, 8>(o, o_small, a, s_s, 16 * j, s_part);
   }
-  float zeros[2] = {0.f, 0.f};      // (zero times every number of a row)
+  float zeros[2] = {0.f, 0.f};      // (zero times a row's numbers)
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int c = 8 * j + t2;
     if (col0 + c >= vdim) break;
     float* at = out + row0 * out_row_stride + (long long)head * vdim + col0 + c;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      o[j][i] += o_small[j][i];
-      zeros[i >> 1] = fmaf(o[j][i], 0.f, zeros[i >> 1]);
-    }
+    for (int i = 0; i < 4; ++i) o[j][i] += o_small[j][i];
+    zeros[0] = fmaf(o[j][0] + o[j][1], 0.f, zeros[0]);
+    zeros[1] = fmaf(o[j][2] + o[j][3], 0.f, zeros[1]);
     if (ta < len) *reinterpret_cast<float2*>(at + ta * out_row_stride) = make_float2(o[j][0], o[j][1]);
     if (tb < len) *reinterpret_cast<float2*>(at + tb * out_row_stride) = make_float2(o[j][2], o[j][3]);
   }

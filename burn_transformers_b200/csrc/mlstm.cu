@@ -706,11 +706,25 @@ __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_state_kernel(const T* __r
   __syncthreads();
   const long long cell = ((long long)seq * c.max_chunks + chunk) * H + head;
   float* dst = c.ds + cell * dim * vdim + col0;
-  cm_state<3, PARTS>(k_s, k_stride, k_part, v_s, v_part, dim, [&](int d, int ch, float x, float y) {
+  const bool bad = cm_state<3, PARTS>(k_s, k_stride, k_part, v_s, v_part, dim, [&](int d, int ch, float x, float y) {
     if (col0 + ch < vdim) *reinterpret_cast<float2*>(dst + (long long)d * vdim + ch) = make_float2(x, y);
   });
+  if (__syncthreads_or(bad)) {      // (and the keys have been read)
+    const int cols = min(CM_COLS, vdim - col0);
+    for (int i = threadIdx.x; i < dim * cols; i += CM_THREADS) {
+      const int d = i / cols, ch = i - d * cols;
+      float* at = dst + (long long)d * vdim + ch;
+      if (isfinite(*at)) continue;
+      float x = 0.f;
+#pragma unroll 1
+      for (int t = 0; t < len; ++t) {
+        const T* row = rows + t * p.row_stride;
+        x = fmaf(to_float(row[p.k_off + head * dim + d]) * w_end[t], to_float(row[p.v_off + head * vdim + col0 + ch]), x);
+      }
+      *at = x;
+    }
+  }
   if (col_block != 0) return;
-  __syncthreads();      // the keys have been read
   float* n_s = reinterpret_cast<float*>(cm_smem);      // [at_once][dim]
   if (k_first < at_once)
 #pragma unroll
@@ -721,6 +735,28 @@ __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_state_kernel(const T* __r
     for (int i = 1; i < at_once; ++i) sum += n_s[i * dim + d];
     c.dn[cell * dim + d] = sum;
   }
+}
+
+// A token's whole row by multiply-adds (the divisor is every channel's), a warp together: qk and v are the chunk's rows from the head's
+// channels on, v's the block's; f: the incoming state's factor.  (A call of its own: inside, it costs the kernel registers.)
+template <typename T>
+__device__ __noinline__ void mlstm_plain_row(const T* qk, const T* v, long long stride, int q_off, int k_off, float q_scale, const float* state,
+                                             int vdim, const float* n, float f, float floor, float g_c, const float* g_a, int t, int dim,
+                                             int cols, float* out) {
+  const int lane = threadIdx.x & 31;
+  auto query = [&](int d) { return to_float(qk[t * stride + q_off + d]) * q_scale; };
+  float x[2], nq = 0.f;
+#pragma unroll 1
+  for (int d = lane; d < dim; d += 32) nq = fmaf(query(d), n[d], nq);
+  nq = warp_sum(nq) * f;
+  const float den = cm_plain_row(t, dim, cols, f, query, [&](int s, int d) { return to_float(qk[s * stride + k_off + d]); },
+                                 [&](int s, int c) { return to_float(v[s * stride + c]); },
+                                 [&](int d, int c) { return state[(long long)d * vdim + c]; },
+                                 [&](int s, float w) { return w * expf(g_c + g_a[s]); }, x);
+  const float by = fmaxf(fabsf(den + nq), floor) + 1e-6f;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (lane + 32 * i < cols) out[lane + 32 * i] = x[i] / by;
 }
 
 template <typename T>
@@ -778,6 +814,7 @@ __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_out_kernel(const T* __res
     for (int q = 0; q < PARTS; ++q) cm_ldmatrix(a[q], q_s + q * k_part + (warp * 16 + (lane & 15)) * k_stride + d + (lane >> 4) * 8);
   };
   float o[8][4], o_small[8][4], div_a, div_b;
+  float zeros[2];      // (zero times a row's numbers and its divisor's sum)
   {
     // f_t S_in^T q_t and f_t n_in . q_t
     float nq[4] = {}, nq_small[4] = {};
@@ -856,8 +893,12 @@ __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_out_kernel(const T* __res
       den_a += __shfl_xor_sync(0xffffffffu, den_a, x);
       den_b += __shfl_xor_sync(0xffffffffu, den_b, x);
     }
-    div_a = fmaxf(fabsf(den_a + div_a), floor_s[ta]) + 1e-6f;
-    div_b = fmaxf(fabsf(den_b + div_b), floor_s[tb]) + 1e-6f;
+    div_a += den_a;
+    div_b += den_b;
+    zeros[0] = div_a * 0.f;
+    zeros[1] = div_b * 0.f;
+    div_a = fmaxf(fabsf(div_a), floor_s[ta]) + 1e-6f;
+    div_b = fmaxf(fabsf(div_b), floor_s[tb]) + 1e-6f;
   }
   __syncthreads();      // the state has been read
   cm_fill<PARTS>(s_s, MC, CM_COLS, CM_ROW, s_part, [&](int t, int ch, float (&x)[8]) {
@@ -889,10 +930,21 @@ __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_out_kernel(const T* __res
     const int ch = 8 * j + t2;
     if (col0 + ch >= vdim) break;
     float* at = p.out + row0 * p.out_row_stride + (long long)head * vdim + col0 + ch;
-    if (ta < len)
-      *reinterpret_cast<float2*>(at + ta * p.out_row_stride) = make_float2((o[j][0] + o_small[j][0]) / div_a, (o[j][1] + o_small[j][1]) / div_a);
-    if (tb < len)
-      *reinterpret_cast<float2*>(at + tb * p.out_row_stride) = make_float2((o[j][2] + o_small[j][2]) / div_b, (o[j][3] + o_small[j][3]) / div_b);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[j][i] += o_small[j][i];
+    zeros[0] = fmaf(o[j][0] + o[j][1], 0.f, zeros[0]);
+    zeros[1] = fmaf(o[j][2] + o[j][3], 0.f, zeros[1]);
+    if (ta < len) *reinterpret_cast<float2*>(at + ta * p.out_row_stride) = make_float2(o[j][0] / div_a, o[j][1] / div_a);
+    if (tb < len) *reinterpret_cast<float2*>(at + tb * p.out_row_stride) = make_float2(o[j][2] / div_b, o[j][3] / div_b);
+  }
+  unsigned redo = cm_bad_rows(ta < len && zeros[0] != 0.f, tb < len && zeros[1] != 0.f);
+  if (redo == 0) return;
+  __syncwarp();
+  for (; redo; redo &= redo - 1) {
+    const int t = warp * 16 + __ffs(redo) - 1;
+    mlstm_plain_row<T>(rows + head * dim, rows + p.v_off + head * vdim + col0, p.row_stride, p.q_off, p.k_off, p.q_scale, src, vdim,
+                       c.dn + cell * dim, f_s[t], floor_s[t], g_c[t], g_a, t, dim, min(CM_COLS, vdim - col0),
+                       p.out + (row0 + t) * p.out_row_stride + (long long)head * vdim + col0);
   }
 }
 

@@ -89,6 +89,63 @@ def test_decayed_chunks(dim, vdim, dtype, kind, activation):
         same(state[2 - i], S, T)
 
 
+@pytest.mark.parametrize("dim, vdim", [(16, 24), (64, 64), (128, 72)])
+@pytest.mark.parametrize("dtype, kind", KINDS + [(torch.bfloat16, "key"), (torch.float32, "key")])
+def test_memory_chunks(dim, vdim, dtype, kind):
+    torch.manual_seed(dim)
+    starts, seq_start, slots = step(LENGTHS)
+    n, wide = starts[-1], HEADS * (2 * dim + vdim)
+    rows = torch.randn(n, wide + 2 * HEADS, device=DEV)
+    if kind == "largest":
+        rows[:, :wide] *= 1e-3
+    if kind == "key":
+        rows[starts[1] + 37, HEADS * dim + 6 * dim + 3] = float("inf")
+    else:
+        spoil(rows, starts[1], 2 * HEADS * dim, kind, dim, vdim)
+    proj = rows.to(dtype)
+    bias_i, bias_f = torch.randn(HEADS, device=DEV) - 1.0, torch.rand(HEADS, device=DEV) * 2.0 + 2.0
+    s, nn, m = (torch.randn(3, HEADS, *d, device=DEV) for d in ((dim, vdim), (dim,), ()))
+    before, out = tuple(t.clone() for t in (s, nn, m)), torch.empty(n, HEADS * vdim, device=DEV)
+    scratch = torch.empty(kernels.mlstm_chunked_scratch_floats(n, 2, max(LENGTHS), HEADS, dim, vdim), device=DEV)
+    kernels.mlstm_scan(proj, (0, HEADS * dim, 2 * HEADS * dim, wide, wide + HEADS), bias_i, bias_f, 15.0, dim ** -0.5, s, nn, m, slots,
+                       seq_start, out, n_seqs=2, n_heads=HEADS, dim=dim, vdim=vdim, max_new=max(LENGTHS), scratch=scratch)
+    x = proj.to(F64)
+    a = 15.0 * torch.tanh((x[:, wide:wide + HEADS] + bias_i.to(F64)) / 15.0)
+    b = torch.nn.functional.logsigmoid(15.0 * torch.tanh((x[:, wide + HEADS:] + bias_f.to(F64)) / 15.0))
+    for i in range(2):
+        S, N, top = (t[2 - i].to(F64) for t in before)
+        T, M = S.abs(), N.abs()
+        want, size = [], []
+        for lo in range(starts[i], starts[i + 1], CHUNK):
+            hi = min(lo + CHUNK, starts[i + 1])
+            q, k, v = (x[lo:hi, c:c + HEADS * d].view(hi - lo, HEADS, d) for c, d in ((0, dim), (HEADS * dim, dim), (2 * HEADS * dim, vdim)))
+            ca, ab, m_in, tops = torch.cumsum(b[lo:hi], 0), a[lo:hi], top, []
+            for t in range(hi - lo):
+                top = torch.maximum(b[lo + t] + top, ab[t])
+                tops.append(top)
+                f, qt = torch.exp(ca[t] + m_in - top)[:, None], q[t] * dim ** -0.5
+                num, den = f * dot(qt, S), f * (qt * N).sum(-1, keepdim=True)
+                num_s, den_s = f * dot(qt.abs(), T), f * (qt.abs() * M).sum(-1, keepdim=True)
+                for r in range(t + 1):
+                    w = torch.exp(ca[t] - ca[r] + ab[r] - top)[:, None]
+                    num, den = num + w * (qt * k[r]).sum(-1, keepdim=True) * v[r], den + w * (qt * k[r]).sum(-1, keepdim=True)
+                    grown = w * (qt * k[r]).abs().sum(-1, keepdim=True)
+                    num_s, den_s = num_s + grown * v[r].abs(), den_s + grown
+                by = torch.fmax(den.abs(), torch.exp(-top)[:, None]) + 1e-6
+                want.append(num / by)
+                size.append(num_s / by + (num / by).abs() * den_s / by)
+            keep = torch.exp(ca[-1] + m_in - top)
+            S, T, N, M = keep[:, None, None] * S, keep[:, None, None] * T, keep[:, None] * N, keep[:, None] * M
+            for r in range(hi - lo):
+                w = torch.exp(ca[-1] - ca[r] + ab[r] - top)[:, None]
+                S, T = S + outer(w * k[r], v[r]), T + outer(w * k[r], v[r]).abs()
+                N, M = N + w * k[r], M + (w * k[r]).abs()
+        # (a weight is e to a 32-bit sum of up to 64 log gates: an error of some units in its exponent of up to about 100)
+        same(out[starts[i]:starts[i + 1]], torch.stack(want), 8.0 * torch.stack(size))
+        same(s[2 - i], S, 8.0 * T)
+        same(nn[2 - i], N, 8.0 * M)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_feature_far_below_zero(dtype):
     heads, dim, n = 16, 16, 640
