@@ -614,9 +614,24 @@ gla_state_kernel(const T* __restrict__ proj, long long row_stride, int k_off, in
   }
   __syncthreads();
   float* dst = states + ((((long long)seq * max_chunks + chunk) * n_heads + head) * dim) * vdim + col0;
-  cm_state<3, PARTS>(k_s, k_stride, k_part, v_s, v_part, dim, [&](int c, int at, float a, float b) {
+  const bool bad = cm_state<3, PARTS>(k_s, k_stride, k_part, v_s, v_part, dim, [&](int c, int at, float a, float b) {
     if (col0 + at < vdim) *reinterpret_cast<float2*>(dst + (long long)c * vdim + at) = make_float2(a, b);
   });
+  if (!__syncthreads_or(bad)) return;
+  const int cols = min(CM_COLS, vdim - col0);
+  for (int i = threadIdx.x; i < dim * cols; i += CM_THREADS) {
+    const int c = i / cols, at = i - c * cols;
+    float* to = dst + (long long)c * vdim + at;
+    if (isfinite(*to)) continue;
+    float y = 0.f, after = 0.f;
+#pragma unroll 1
+    for (int t = len - 1; t >= 0; --t) {
+      const T* row = rows + t * row_stride;
+      y = fmaf(to_float(row[k_off + head * dim + c]) * gla_exp<T>(log_scale * after), to_float(row[v_off + head * vdim + col0 + at]), y);
+      after += dt_rows[t * dt_stride + c];
+    }
+    *to = y;
+  }
 }
 
 // gla_prefix_kernel with four value channels a thread and eight chunks asked for at a time.
@@ -666,6 +681,44 @@ __device__ __forceinline__ void gla_lane_sums(float (&x)[N], int from, int to) {
       x[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
     }
   }
+}
+
+// The results of token t of a chunk that are no finite numbers, by multiply-adds, a warp together, a lane two of the (at most 64) key channels:
+// token by token back from t, then the incoming state.  qk, v and dt are the chunk's rows from the head's channels on, v's the block's.
+template <typename T>
+__device__ __noinline__ void gla_plain_row(const T* qk, const T* v, long long stride, int q_off, int k_off, float q_scale, const float* dt,
+                                           long long dt_stride, float log_scale, const float* state, int vdim, int t, int dim, int cols,
+                                           float* out) {
+  const int lane = threadIdx.x & 31;
+  float x[2] = {0.f, 0.f}, q[2], sum[2] = {0.f, 0.f};      // q, and what lies of dt between the token in hand and t
+#pragma unroll
+  for (int i = 0; i < 2; ++i) q[i] = lane + 32 * i < dim ? to_float(qk[t * stride + q_off + lane + 32 * i]) * q_scale : 0.f;
+#pragma unroll 1
+  for (int s = t; s >= 0; --s) {
+    float w = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if (lane + 32 * i >= dim) continue;
+      w = fmaf(q[i] * gla_exp<T>(log_scale * sum[i]), to_float(qk[s * stride + k_off + lane + 32 * i]), w);
+      sum[i] += dt[s * dt_stride + lane + 32 * i];
+    }
+    w = warp_sum(w);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (lane + 32 * i < cols) x[i] = fmaf(w, to_float(v[s * stride + lane + 32 * i]), x[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) q[i] *= gla_exp<T>(log_scale * sum[i]);
+#pragma unroll 1
+  for (int d = 0; d < dim; ++d) {
+    const float y = __shfl_sync(0xffffffffu, d < 32 ? q[0] : q[1], d & 31);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (lane + 32 * i < cols) x[i] = fmaf(y, state[(long long)d * vdim + lane + 32 * i], x[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (lane + 32 * i < cols && !isfinite(out[lane + 32 * i])) out[lane + 32 * i] = x[i];
 }
 
 constexpr int GD = 20;      // row length of a sub-block's weights ([token s][token t])
@@ -892,13 +945,27 @@ gla_out_kernel(const T* __restrict__ proj, long long row_stride, int q_off, int 
     }
     cm_step_rows<3, PARTS, 8>(o, o_small, a, parts, 16 * j, s_part);
   }
+  float zeros[2] = {0.f, 0.f};      // (zero times a row's numbers)
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int c = 8 * j + t2;
     if (col0 + c >= vdim) break;
     float* at = out + row0 * out_row_stride + (long long)head * vdim + col0 + c;
-    if (ta < len) *reinterpret_cast<float2*>(at + ta * out_row_stride) = make_float2(o[j][0] + o_small[j][0], o[j][1] + o_small[j][1]);
-    if (tb < len) *reinterpret_cast<float2*>(at + tb * out_row_stride) = make_float2(o[j][2] + o_small[j][2], o[j][3] + o_small[j][3]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[j][i] += o_small[j][i];
+    zeros[0] = fmaf(o[j][0] + o[j][1], 0.f, zeros[0]);
+    zeros[1] = fmaf(o[j][2] + o[j][3], 0.f, zeros[1]);
+    if (ta < len) *reinterpret_cast<float2*>(at + ta * out_row_stride) = make_float2(o[j][0], o[j][1]);
+    if (tb < len) *reinterpret_cast<float2*>(at + tb * out_row_stride) = make_float2(o[j][2], o[j][3]);
+  }
+  unsigned redo = cm_bad_rows(ta < len && zeros[0] != 0.f, tb < len && zeros[1] != 0.f);
+  if (redo == 0) return;
+  __syncwarp();
+  for (; redo; redo &= redo - 1) {
+    const int t = warp * 16 + __ffs(redo) - 1;
+    gla_plain_row<T>(rows + head * dim, rows + v_off + head * vdim + col0, row_stride, q_off, k_off, q_scale, dt + (row0 * n_heads + head) * dim,
+                     (long long)n_heads * dim, log_scale, src, vdim, t, dim, min(CM_COLS, vdim - col0),
+                     out + (row0 + t) * out_row_stride + (long long)head * vdim + col0);
   }
 }
 

@@ -146,6 +146,45 @@ def test_memory_chunks(dim, vdim, dtype, kind):
         same(nn[2 - i], N, 8.0 * M)
 
 
+@pytest.mark.parametrize("dim, vdim", [(32, 24), (64, 64), (48, 72)])
+@pytest.mark.parametrize("dtype, kind", KINDS)
+def test_gated_chunks(dim, vdim, dtype, kind):
+    torch.manual_seed(dim)
+    starts, seq_start, slots = step(LENGTHS)
+    n, wide = starts[-1], HEADS * (2 * dim + vdim)
+    rows = torch.randn(n, wide, device=DEV) * (1e-3 if kind == "largest" else 1.0)
+    spoil(rows, starts[1], 2 * HEADS * dim, kind, dim, vdim)
+    proj, dt = rows.to(dtype), torch.rand(n, HEADS * dim, device=DEV)
+    state = torch.randn(3, HEADS, dim, vdim, device=DEV)
+    first, out = state.clone(), torch.empty(n, HEADS * vdim, device=DEV)
+    scratch = torch.empty(kernels.gla_chunked_scratch_floats(n, 2, max(LENGTHS), HEADS, dim, vdim), device=DEV)
+    kernels.gla_scan(proj, 0, HEADS * dim, 2 * HEADS * dim, dim ** -0.5, dt, -0.25, state, slots, seq_start, out, n_seqs=2, n_heads=HEADS,
+                     dim=dim, vdim=vdim, max_new=max(LENGTHS), scratch=scratch)
+    x, log_a = proj.to(F64), -0.25 * dt.to(F64).view(n, HEADS, dim)
+    for i in range(2):
+        S = first[2 - i].to(F64)
+        T = S.abs()
+        want, size = [], []
+        for lo in range(starts[i], starts[i + 1], CHUNK):
+            hi = min(lo + CHUNK, starts[i + 1])
+            q, k, v = (x[lo:hi, a:a + HEADS * d].view(hi - lo, HEADS, d) for a, d in ((0, dim), (HEADS * dim, dim), (2 * HEADS * dim, vdim)))
+            b = torch.cumsum(log_a[lo:hi], 0)
+            for t in range(hi - lo):
+                qt = q[t] * dim ** -0.5
+                o, u = dot(qt * torch.exp(b[t]), S), dot(qt.abs() * torch.exp(b[t]), T)
+                for s in range(t + 1):
+                    w = qt * k[s] * torch.exp(b[t] - b[s])
+                    o, u = o + w.sum(-1, keepdim=True) * v[s], u + w.abs().sum(-1, keepdim=True) * v[s].abs()
+                want.append(o)
+                size.append(u)
+            S, T = torch.exp(b[-1])[:, :, None] * S, torch.exp(b[-1])[:, :, None] * T
+            for s in range(hi - lo):
+                f = torch.exp(b[-1] - b[s])
+                S, T = S + outer(f * k[s], v[s]), T + outer(f * k[s], v[s]).abs()
+        same(out[starts[i]:starts[i + 1]], torch.stack(want), 4.0 * torch.stack(size))      # (a decay of up to 64 times 1/4 in its exponent)
+        same(state[2 - i], S, 4.0 * T)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_feature_far_below_zero(dtype):
     heads, dim, n = 16, 16, 640
