@@ -396,6 +396,17 @@ latent_decode_finish_mma_kernel(const float* __restrict__ part, const __nv_bfloa
     float acc = 0.f;
 #pragma unroll
     for (int q = 0; q < LF_WARPS; ++q) acc += red[(q * LF_TOKENS + r) * vdim + j];
+    if (JOIN && !isfinite(acc)) {      // (an infinity, or a number that bfloat16 rounds to one, has no parts: by multiply-adds)
+      const float* src = part + ((long long)token * n_heads + h) * n_splits * (rank + 2);
+      acc = 0.f;
+#pragma unroll 1
+      for (int k = 0; k < rank; ++k) {
+        float x = 0.f;
+#pragma unroll 1
+        for (int s = 0; s < n_splits; ++s) x = fmaf(src[(long long)s * (rank + 2) + k], share[r][s], x);
+        acc = fmaf(x, to_float(w_s[k * ld + j]), acc);
+      }
+    }
     if (gate) acc *= 1.f / (1.f + expf(-to_float(gate[(long long)token * gate_row_stride + (gate_per_head ? h : (long long)h * vdim + j)])));
     out[(long long)token * out_row_stride + (long long)h * vdim + j] = from_float<__nv_bfloat16>(acc);
   }

@@ -88,3 +88,23 @@ def test_after(rank, vdim, n, splits, per_head):
         kernels.latent_decode_finish(uv, out, n_tokens=n, n_splits=splits, scratch=part, gate=gate)
     want = np.einsum("thr,hrv->thv", merged, host(uv)) * plain.sigmoid(host(gate).reshape(n, heads, -1))
     assert rel(host(out[:n]).reshape(n, heads, vdim), want) < 2.5e-3 and bool((out[n:] == 0).all())
+
+
+def test_after_of_what_is_not_finite():
+    """A latent channel that is infinite, or that bfloat16 would round to infinity: the results are those of multiply-adds."""
+    rng = np.random.default_rng(3)
+    n, heads, rank, vdim, splits = 9, 3, 64, 32, 4
+    uv = dev(rng.uniform(0.5, 1.5, (heads, rank, vdim)) / rank)
+    part, _ = partial_results(rng, n, heads, splits, rank)
+    cells = part.view(n, heads, splits, rank + 2)
+    cells[2, 1, 0, 7], cells[8, 0, 2, 63], cells[4, 2, 3, 20] = float("inf"), float("-inf"), float("nan")
+    cells[5, 1, 0, 9], cells[5, 1, :, rank], cells[5, 1, 0, rank + 1] = 3.4e38, -30.0, 1.0
+    cells[5, 1, 0, rank] = 0.0
+    out = torch.empty((n, heads * vdim), dtype=torch.bfloat16, device=DEV)
+    kernels.latent_decode_finish(uv, out, n_tokens=n, n_splits=splits, scratch=part)
+    out = out.view(n, heads, vdim)
+    assert bool((out[2, 1] == float("inf")).all()) and bool((out[8, 0] == float("-inf")).all()) and bool(torch.isnan(out[4, 2]).all())
+    want = 3.4e38 * uv[1, 9].double()
+    assert float(((out[5, 1].double() - want) / want).abs().max()) < 2.0 ** -8
+    out[2, 1], out[8, 0], out[4, 2], out[5, 1] = 0.0, 0.0, 0.0, 0.0
+    assert bool(torch.isfinite(out).all())
