@@ -369,7 +369,8 @@ selective_scan_kernel(const T* __restrict__ x, long long x_row_stride, const T* 
 // they lie, n_state + 1 numbers a channel in a row over the block's threads, and meets the channels' layout in shared memory.
 constexpr int SP_THREADS = 64, SP_STAGE = 64, SP_AHEAD = 4;
 
-template <typename T, int LANES, bool ENDS>
+// FULL: every thread's 8 indices are a channel's; else those past n_state stay zero (a zero times an infinite step would not).
+template <typename T, int LANES, bool ENDS, bool FULL>
 __global__ void __launch_bounds__(SP_THREADS, ENDS ? 12 : 10)
 selective_scan_piece_kernel(const T* __restrict__ x, long long x_row_stride, const T* __restrict__ z, long long z_row_stride,
                             const float* __restrict__ dt, const T* __restrict__ low, long long low_row_stride, int b_off,
@@ -527,6 +528,11 @@ selective_scan_piece_kernel(const T* __restrict__ x, long long x_row_stride, con
               e1 = expf(e1);
             }
             s2[i] = ss_fma2(ss_pack(e0, e1), s2[i], ss_mul2(dx2, h ? b.y : b.x));
+            if (!FULL) {
+              float lo, hi;
+              ss_unpack(s2[i], lo, hi);
+              s2[i] = ss_pack(n0 + 2 * i < n_state ? lo : 0.f, n0 + 2 * i + 1 < n_state ? hi : 0.f);
+            }
             if (!ENDS) y2[h] = ss_fma2(s2[i], h ? cv.y : cv.x, y2[h]);
           }
         }
@@ -587,13 +593,15 @@ static int launch_selective_scan(const T* x, long long xs, const T* z, long long
   else { ns = 16; lanes = 32; }
   BT_CHECK(n_state <= 512, "selective_scan: %d state indices a channel; the kernel takes up to 512", n_state);
   if (piece > 0 && n_state <= 16) {      // (steps without pieces are few tokens a sequence: more lanes a channel answer sooner)
-#define BT_SP(LANES, ENDS)                                                                                                   \
-  BT_PDL_OK("selective_scan", launch_pdl(selective_scan_piece_kernel<T, LANES, ENDS>,                                        \
+#define BT_SP(LANES, ENDS, FULL)                                                                                             \
+  BT_PDL_OK("selective_scan", launch_pdl(selective_scan_piece_kernel<T, LANES, ENDS, FULL>,                                  \
                                          dim3((channels + SP_THREADS / LANES - 1) / (SP_THREADS / LANES), n_seqs, max_pieces), \
                                          dim3(SP_THREADS), 0, stream, 1, x, xs, z, zs, dt, low, ls, b_off, c_off, a_log,     \
                                          d_skip, state, slots, seq_start, out, os, channels, n_state, out_scale, piece, ends))
-    if (n_state <= 8) { BT_SP(1, true); BT_SP(1, false); }
-    else { BT_SP(2, true); BT_SP(2, false); }
+    if (n_state == 8) { BT_SP(1, true, true); BT_SP(1, false, true); }
+    else if (n_state < 8) { BT_SP(1, true, false); BT_SP(1, false, false); }
+    else if (n_state == 16) { BT_SP(2, true, true); BT_SP(2, false, true); }
+    else { BT_SP(2, true, false); BT_SP(2, false, false); }
 #undef BT_SP
     return 0;
   }
