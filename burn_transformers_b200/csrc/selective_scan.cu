@@ -553,7 +553,7 @@ selective_scan_piece_kernel(const T* __restrict__ x, long long x_row_stride, con
           const float yu = LANES == 1 ? y[v] : (tid % LANES ? y[v * LANES + LANES - 1] : y[v * LANES]);
           const float xf = to_float(LANES == 1 ? xv[v] : (tid % LANES ? xv[v * LANES + LANES - 1] : xv[v * LANES]));
           const float zf = to_float(LANES == 1 ? zv[v] : (tid % LANES ? zv[v * LANES + LANES - 1] : zv[v * LANES]));
-          const float gate = sizeof(T) == 2 ? __fdividef(zf, 1.f + __expf(-zf)) : zf / (1.f + expf(-zf));
+          const float gate = zf / (1.f + expf(-zf));
           if (owns && t + u < nt) out_at[u * out_row_stride] = from_float<T>((yu + skip * xf) * gate * out_scale);
         }
         out_at += SP_AHEAD * out_row_stride;

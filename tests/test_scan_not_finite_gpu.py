@@ -37,3 +37,14 @@ def test_an_infinite_row(n_state, dtype):
     assert torch.equal(out[~ok], want[~ok]) and float(((out - want).abs()[ok] / want[ok]).max()) < 2.0 ** -8
     ok = torch.isfinite(S)
     assert torch.equal(state[0].to(F64)[~ok], S[~ok]) and float(((state[0].to(F64) - S).abs()[ok] / S[ok]).max()) < 1e-5
+
+
+@pytest.mark.parametrize("n_state", [7, 8, 16])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_gate_far_below_zero(n_state, dtype):
+    inner, total = 70, 200
+    z = torch.tensor([-1.0, -20.0, -60.0, -85.0, -87.5, -88.0, -88.5], device=DEV).to(dtype).repeat(total * inner // 7).view(total, inner)
+    x = torch.full((total, inner), 1e30, device=DEV, dtype=dtype)
+    out, want, _ = scan(dtype, inner, n_state, x, z, torch.zeros(1, inner, n_state, device=DEV))
+    # (the gates themselves are down to 2^-120, with all of their bits)
+    assert float(((out - want).abs() / want.abs()).max()) < (2.0 ** -8 if dtype is torch.bfloat16 else 1e-5)
