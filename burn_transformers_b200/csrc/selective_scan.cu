@@ -18,6 +18,7 @@
 // pieces of sequence s begin at first_row(s) / piece + s.  Nothing orders the second launch's blocks, so none of them may
 // read what another one writes: the first launch copies the stored state into the cell of the sequence's last piece (which
 // leaves no ends), and all pieces start from that copy.
+#include "chunk_mma.cuh"
 #include "common.cuh"
 
 namespace bt {
@@ -109,11 +110,11 @@ selective_scan_dt_kernel(const T* __restrict__ low, long long low_row_stride, co
 }
 
 // The same for bfloat16 rows and a rank of at most 64, on tensor cores: W_dt's 32-bit numbers go in as three bfloat16 parts, which
-// hold all of their bits, the smallest parts first, so that the products are exact and a result's sum is cut only in its last few
-// additions.  A warp keeps 32 channels' weights in registers as the operand wants them and walks over tiles of 16 tokens, with
+// hold all of their bits (chunk_mma.cuh; the first parts' sums begin from zero every 16 of the rank).  Errors against 64 bits, above and
+// here, rank 48: 1.3e-7 and 1.9e-8 with normal numbers, 1.8e-7 and 1.2e-7 beside one large channel (3.2e-7 in one accumulator).  A warp keeps 32 channels' weights in registers as the operand wants them and walks over tiles of 16 tokens, with
 // neither shared memory nor barriers; the softplus, about 45 instructions a number, is what is left.  The kernel above is bound by
 // instructions, a third of them for its weights' way through shared memory.  In us, above and here: 2,439 tokens of 1,536 channels
-// and rank 48 27.5 and 17.8, 2,048 of 1,024 and rank 16 12.5 and 9.6, 100 of 1,536 and rank 48 6.4 and 3.9.
+// and rank 48 27.8 and 18.2, 2,048 of 1,024 and rank 16 12.5 and 9.6, 100 of 1,536 and rank 48 6.9 and 3.9.
 template <int KS>
 __global__ void __launch_bounds__(128, KS <= 2 ? 5 : KS == 3 ? 4 : 3)
 selective_scan_dt_mma_kernel(const __nv_bfloat16* __restrict__ low, long long low_row_stride, const float* __restrict__ w_dt,
@@ -159,26 +160,27 @@ selective_scan_dt_mma_kernel(const __nv_bfloat16* __restrict__ low, long long lo
         const int t = t0 + g + 8 * (i & 1), r = 16 * k + 8 * (i >> 1) + t2;
         a[k][i] = t < n_tokens && r < rank ? *reinterpret_cast<const unsigned*>(low + t * low_row_stride + r) : 0u;
       }
-    float acc[4][4];
+    float acc[4][4] = {}, small[4][4] = {};
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc[j][i] = 0.f;
-#pragma unroll
-    for (int q = 2; q >= 0; --q)
+    for (int q = 2; q > 0; --q)
 #pragma unroll
       for (int k = 0; k < KS; ++k)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-              : "+f"(acc[j][0]), "+f"(acc[j][1]), "+f"(acc[j][2]), "+f"(acc[j][3])
-              : "r"(a[k][0]), "r"(a[k][1]), "r"(a[k][2]), "r"(a[k][3]), "r"(w[q][k][j][0]), "r"(w[q][k][j][1]));
+        for (int j = 0; j < 4; ++j) cm_mma(small[j], a[k], w[q][k][j][0], w[q][k][j][1]);
+#pragma unroll
+    for (int k = 0; k < KS; ++k)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float x[4];
+        cm_mma_zero(x, a[k], w[0][k][j][0], w[0][k][j][1]);
+        cm_add(acc[j], x);
+      }
     bool whole = true;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        acc[j][i] += i & 1 ? bias[j].y : bias[j].x;
+        acc[j][i] = acc[j][i] + small[j][i] + (i & 1 ? bias[j].y : bias[j].x);
         whole = whole && isfinite(acc[j][i]);
       }
     if (!whole) {      // an infinity times the parts of a weight is no number: such sums are formed again by multiply-adds

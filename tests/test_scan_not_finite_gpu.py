@@ -1,4 +1,4 @@
-"""Long runs of the selective scan at the ends of the numbers' range, against the recurrence in 64 bits."""
+"""Long runs of the selective scan, and its step sizes, at the ends of the numbers' range and beside large ones, against 64 bits."""
 import pytest
 import torch
 
@@ -48,3 +48,15 @@ def test_a_gate_far_below_zero(n_state, dtype):
     out, want, _ = scan(dtype, inner, n_state, x, z, torch.zeros(1, inner, n_state, device=DEV))
     # (the gates themselves are down to 2^-120, with all of their bits)
     assert float(((out - want).abs() / want.abs()).max()) < (2.0 ** -8 if dtype is torch.bfloat16 else 1e-5)
+
+
+@pytest.mark.parametrize("rank", [32, 48, 64])
+def test_step_sizes_beside_a_large_channel(rank):
+    torch.manual_seed(rank)
+    low, w = torch.rand(640, rank, device=DEV) + 0.5, torch.rand(512, rank, device=DEV) + 0.5
+    low[:, 0] = 4096.0
+    low, dt = low.bfloat16(), torch.empty(640, 512, device=DEV)
+    kernels.selective_scan_dt(low, w, torch.zeros(512, device=DEV), dt, n_tokens=640)
+    want = low.to(F64) @ w.to(F64).T      # (a softplus of thousands is its argument)
+    # the sum of the large channel's 16 is cut once, by 2^-23 at most, and the up to three others are added with a rounding each
+    assert float(((dt.to(F64) - want) / want).pow(2).mean().sqrt()) < 2.0 ** -22.5
