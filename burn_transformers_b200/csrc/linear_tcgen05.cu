@@ -295,8 +295,10 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           tc_ld32(tmem_acc + ((unsigned)(quarter * 32) << 16) + (unsigned)(buf * ACC + COLS + c0), up);
           const int cols = p.N / 2, col0 = tn * COLS + c0;
           if (col0 >= cols) continue;
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = tc_gated(v[i], up[i], p.act, p.limit);
+          if (p.act == kActSwish) tc_gated_all<kActSwish>(v, up, p.limit);
+          else if (p.act == kActSwishClamp) tc_gated_all<kActSwishClamp>(v, up, p.limit);
+          else if (p.act == kActGeluTanh) tc_gated_all<kActGeluTanh>(v, up, p.limit);
+          else tc_gated_all<kActGeluErf>(v, up, p.limit);
           __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out);
           if (cols % 8 == 0 && col0 + 32 <= cols) {
             tc_store32(reinterpret_cast<unsigned char*>(patch), TC_PATCH_STRIDE * 4, v, lane, out + col0, cols, m0 + quarter * 32, p.M);

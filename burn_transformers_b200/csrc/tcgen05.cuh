@@ -142,18 +142,27 @@ __device__ __forceinline__ float tc_activation(float x, int act, bool exact) {
   return x;
 }
 // gated_pair (common.cuh) for results that are rounded to bfloat16: the same rules with the special-function unit's exponential and
-// reciprocal (a few units of 2^-23; the tanh form as x sigmoid(2 z)).
-__device__ __forceinline__ float tc_gated(float g, float u, int act, float limit) {
-  if (act == kActGeluErf) return gelu_erf(g) * u;
+// reciprocal (a few units of 2^-23, more where the exponential is small; the tanh form as x sigmoid(2 z)).  Where 1 + e^x is too large for
+// the reciprocal both sides of the division are taken down by 2^32.
+template <int ACT>
+__device__ __forceinline__ float tc_gated(float g, float u, float limit) {
+  if (ACT == kActGeluErf) return gelu_erf(g) * u;
   float e = g;
-  if (act == kActSwishClamp) {
+  if (ACT == kActSwishClamp) {
     g = fminf(g, limit);
     u = fminf(fmaxf(u, -limit), limit) + 1.f;
     e = 1.702f * g;
-  } else if (act == kActGeluTanh) {
+  } else if (ACT == kActGeluTanh) {
     e = 2.f * 0.7978845608028654f * (g + 0.044715f * g * g * g);
   }
-  return __fdividef(g, 1.f + __expf(-e)) * u;
+  const float y = 1.f + __expf(-e), down = y > 0x1p125f ? 0x1p-32f : 1.f;
+  return __fdividef(g * down, y * down) * u;
+}
+// v = rule(v) * up
+template <int ACT>
+__device__ __forceinline__ void tc_gated_all(float (&v)[32], const float (&up)[32], float limit) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = tc_gated<ACT>(v[i], up[i], limit);
 }
 __device__ __forceinline__ void tc_bar_arrive(unsigned long long* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc_smem(bar)) : "memory");

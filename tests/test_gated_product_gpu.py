@@ -43,3 +43,16 @@ def test_large_gates_saturate():
         kernels.gated_tcgen05(a, w, out, m=80, activation=rule)
         want = paired((a.double() @ w.double().T)[:, :16], (a.double() @ w.double().T)[:, 16:], rule, 0.0)
         assert bool((out[0::2].double() - want[0::2]).abs().max() <= 2.0 ** -8 * want.abs().max()) and bool((out[1::2].float().abs() < 1e-30).all())
+
+
+def test_gates_far_below_zero():
+    # gates of which a large second factor leaves something: sigmoids down to 2^-128
+    gates = torch.tensor([-20.0, -60.0, -85.0, -86.0, -87.0, -87.5, -88.0, -88.5], device=DEV)
+    a = torch.ones(80, 8, device=DEV).bfloat16()
+    w = torch.cat([gates[:, None] / 8.0 * torch.ones(8, device=DEV), torch.full((8, 8), 1e30, device=DEV)]).bfloat16()
+    both, out = a.double() @ w.double().T, torch.empty(80, 8, device=DEV).bfloat16()
+    kernels.gated_tcgen05(a, w, out, m=80, activation="swish")
+    want = paired(both[:, :8], both[:, 8:], "swish", 0.0)
+    # a rounding to bfloat16, and an exponential whose argument was rounded at 2^7: 2^-17 of it
+    error = float(((out.double() - want) / want).abs().max())
+    assert error < 2.0 ** -8
