@@ -173,32 +173,72 @@ __device__ __forceinline__ unsigned cm_bad_rows(bool a, bool b) {
   return rows;
 }
 
+// Columns lane and lane + 32 of a block whose incoming state holds a NaN: so do their results, which need not be formed again (in(d, c) as
+// below; a state that has become NaN would bring every later token here).
+template <typename In>
+__device__ __forceinline__ void cm_nan_columns(int dim, int cols, In in, bool (&nan)[2]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float sum = 0.f;
+#pragma unroll 8
+    for (int d = 0; d < dim; ++d) {
+      const float y = lane + 32 * h < cols ? in(d, lane + 32 * h) : 0.f;
+      sum = isnan(y) ? y : sum;
+    }
+    nan[h] = isnan(sum) || lane + 32 * h >= cols;
+  }
+}
+
 // The chunk's token t by multiply-adds, a warp together, columns lane and lane + 32 of a block's: x = carry * sum_d q(d) in(d, c) and then, token
-// by token, weigh(s, q . k_s) v(s, c).  The sum of the weights is returned.
+// by token, weigh(s, q . k_s) v(s, c), up to 128 channels d.  The sum of the weights is returned.  (Eight channels' or tokens' numbers are asked
+// for at once: a state that has become infinite brings every later token here.)
 template <typename Q, typename K, typename V, typename In, typename Weigh>
 __device__ __forceinline__ float cm_plain_row(int t, int dim, int cols, float carry, Q q, K k, V v, In in, Weigh weigh, float (&x)[2]) {
   const int lane = threadIdx.x & 31;
-  float sum = 0.f;
-  x[0] = x[1] = 0.f;
-#pragma unroll 1
-  for (int d = 0; d < dim; ++d) {
-    const float y = q(d);
+  float sum = 0.f, own[4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-      if (lane + 32 * i < cols) x[i] = fmaf(y, in(d, lane + 32 * i), x[i]);
-  }
+  for (int i = 0; i < 4; ++i) own[i] = lane + 32 * i < dim ? q(lane + 32 * i) : 0.f;
+  x[0] = x[1] = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll 1
+    for (int d = 32 * i; d < min(dim, 32 * i + 32); d += 8) {      // (dim is whole operand tiles)
+      float y[8][2];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) y[u][h] = lane + 32 * h < cols ? in(d + u, lane + 32 * h) : 0.f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const float z = __shfl_sync(0xffffffffu, own[i], (d + u) & 31);
+        x[0] = fmaf(z, y[u][0], x[0]);
+        x[1] = fmaf(z, y[u][1], x[1]);
+      }
+    }
   x[0] *= carry;
   x[1] *= carry;
 #pragma unroll 1
-  for (int s = 0; s <= t; ++s) {
-    float w = 0.f;
-#pragma unroll 1
-    for (int d = lane; d < dim; d += 32) w = fmaf(q(d), k(s, d), w);
-    w = weigh(s, warp_sum(w));
-    sum += w;
+  for (int s = 0; s <= t; s += 8) {
+    float w[8], y[8][2];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-      if (lane + 32 * i < cols) x[i] = fmaf(w, v(s, lane + 32 * i), x[i]);
+    for (int u = 0; u < 8; ++u) {
+      const int token = min(s + u, t);
+      w[u] = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (lane + 32 * i < dim) w[u] = fmaf(own[i], k(token, lane + 32 * i), w[u]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) y[u][h] = lane + 32 * h < cols ? v(token, lane + 32 * h) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float z = weigh(min(s + u, t), warp_sum(w[u]));
+      if (s + u > t) break;
+      sum += z;
+      x[0] = fmaf(z, y[u][0], x[0]);
+      x[1] = fmaf(z, y[u][1], x[1]);
+    }
   }
   return sum;
 }

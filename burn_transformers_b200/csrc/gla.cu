@@ -540,6 +540,24 @@ gla_carry_kernel(const float* __restrict__ aged_q, const int* __restrict__ seq_s
 // 39 / 31; 32-bit rows 2 x 1,024 68 / 45; errors against 64 bits 1.6e-7 / 1.4e-7.  Heads of 128 channels leave two blocks a multiprocessor
 // and took 121 where the kernels above take 104, 32-bit heads of 16 15.4 against 13.7.
 
+// The numbers of a chunk's contribution to the state that are not finite, by multiply-adds (a call of its own: inside, it costs the kernel registers).
+template <typename T>
+__device__ __noinline__ void gla_plain_state(const T* k, const T* v, long long stride, const float* dt, long long dt_stride, float log_scale, int len,
+                                             int dim, int cols, float* dst, int vdim) {
+  for (int i = threadIdx.x; i < dim * cols; i += CM_THREADS) {
+    const int d = i / cols, c = i - d * cols;
+    float* at = dst + (long long)d * vdim + c;
+    if (isfinite(*at)) continue;
+    float x = 0.f, after = 0.f;
+#pragma unroll 8
+    for (int t = len - 1; t >= 0; --t) {
+      x = fmaf(to_float(k[t * stride + d]) * gla_exp<T>(log_scale * after), to_float(v[t * stride + c]), x);
+      after += dt[t * dt_stride + d];
+    }
+    *at = x;
+  }
+}
+
 // A chunk's contribution to the state: sum_s (k_s e^{b_end - b_s}) v_s^T.  A thread takes two key channels of 16 tokens and adds the log
 // decays up from the end.
 template <typename T, int PARTS>
@@ -617,21 +635,9 @@ gla_state_kernel(const T* __restrict__ proj, long long row_stride, int k_off, in
   const bool bad = cm_state<3, PARTS>(k_s, k_stride, k_part, v_s, v_part, dim, [&](int c, int at, float a, float b) {
     if (col0 + at < vdim) *reinterpret_cast<float2*>(dst + (long long)c * vdim + at) = make_float2(a, b);
   });
-  if (!__syncthreads_or(bad)) return;
-  const int cols = min(CM_COLS, vdim - col0);
-  for (int i = threadIdx.x; i < dim * cols; i += CM_THREADS) {
-    const int c = i / cols, at = i - c * cols;
-    float* to = dst + (long long)c * vdim + at;
-    if (isfinite(*to)) continue;
-    float y = 0.f, after = 0.f;
-#pragma unroll 1
-    for (int t = len - 1; t >= 0; --t) {
-      const T* row = rows + t * row_stride;
-      y = fmaf(to_float(row[k_off + head * dim + c]) * gla_exp<T>(log_scale * after), to_float(row[v_off + head * vdim + col0 + at]), y);
-      after += dt_rows[t * dt_stride + c];
-    }
-    *to = y;
-  }
+  if (__syncthreads_or(bad))
+    gla_plain_state<T>(rows + k_off + head * dim, rows + v_off + head * vdim + col0, row_stride, dt_rows, dt_stride, log_scale, len, dim,
+                       min(CM_COLS, vdim - col0), dst, vdim);
 }
 
 // gla_prefix_kernel with four value channels a thread and eight chunks asked for at a time.
@@ -683,42 +689,71 @@ __device__ __forceinline__ void gla_lane_sums(float (&x)[N], int from, int to) {
   }
 }
 
-// The results of token t of a chunk that are no finite numbers, by multiply-adds, a warp together, a lane two of the (at most 64) key channels:
-// token by token back from t, then the incoming state.  qk, v and dt are the chunk's rows from the head's channels on, v's the block's.
+// The results of a chunk's tokens (bits of `redo`, from token `first_token` on) that are no finite numbers, by multiply-adds, a warp together, a lane
+// two of the (at most 64) key channels: token by token back from a row's own, then the incoming state.  qk, v and dt are the chunk's rows
+// from the head's channels on, v's and out's the block's.
 template <typename T>
-__device__ __noinline__ void gla_plain_row(const T* qk, const T* v, long long stride, int q_off, int k_off, float q_scale, const float* dt,
-                                           long long dt_stride, float log_scale, const float* state, int vdim, int t, int dim, int cols,
-                                           float* out) {
+__device__ __noinline__ void gla_plain_rows(unsigned redo, const T* qk, const T* v, long long stride, int q_off, int k_off, float q_scale,
+                                            const float* dt, long long dt_stride, float log_scale, const float* state, int vdim,
+                                            int first_token, int dim, int cols, float* out, long long out_stride) {
   const int lane = threadIdx.x & 31;
-  float x[2] = {0.f, 0.f}, q[2], sum[2] = {0.f, 0.f};      // q, and what lies of dt between the token in hand and t
+  bool nan[2];
+  cm_nan_columns(dim, cols, [&](int d, int c) { return state[(long long)d * vdim + c]; }, nan);
+  for (; redo; redo &= redo - 1) {
+    const int t = first_token + __ffs(redo) - 1;
+    float* at = out + t * out_stride + lane;
+    const bool need[2] = {!nan[0] && !isfinite(at[0]), !nan[1] && !isfinite(at[32])};
+    if (!__any_sync(0xffffffffu, need[0] || need[1])) continue;
+    float x[2] = {0.f, 0.f}, q[2], sum[2] = {0.f, 0.f};      // q, and what lies of dt between the token in hand and t
 #pragma unroll
-  for (int i = 0; i < 2; ++i) q[i] = lane + 32 * i < dim ? to_float(qk[t * stride + q_off + lane + 32 * i]) * q_scale : 0.f;
+    for (int i = 0; i < 2; ++i) q[i] = lane + 32 * i < dim ? to_float(qk[t * stride + q_off + lane + 32 * i]) * q_scale : 0.f;
 #pragma unroll 1
-  for (int s = t; s >= 0; --s) {
-    float w = 0.f;
+    for (int s = t; s >= 0; s -= 8) {      // (eight tokens', and eight channels', numbers are asked for at once)
+      float k[8][2], a[8][2], y[8][2];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int token = max(s - u, 0), c = lane + 32 * i;
+          k[u][i] = c < dim ? to_float(qk[token * stride + k_off + c]) : 0.f;
+          a[u][i] = c < dim ? dt[token * dt_stride + c] : 0.f;
+          y[u][i] = c < cols ? to_float(v[token * stride + c]) : 0.f;
+        }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        float w = 0.f;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          if (lane + 32 * i < dim) w = fmaf(q[i] * gla_exp<T>(log_scale * sum[i]), k[u][i], w);
+          sum[i] += s - u >= 0 ? a[u][i] : 0.f;
+        }
+        w = warp_sum(w);
+        if (s - u < 0) break;
+        x[0] = fmaf(w, y[u][0], x[0]);
+        x[1] = fmaf(w, y[u][1], x[1]);
+      }
+    }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      if (lane + 32 * i >= dim) continue;
-      w = fmaf(q[i] * gla_exp<T>(log_scale * sum[i]), to_float(qk[s * stride + k_off + lane + 32 * i]), w);
-      sum[i] += dt[s * dt_stride + lane + 32 * i];
-    }
-    w = warp_sum(w);
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-      if (lane + 32 * i < cols) x[i] = fmaf(w, to_float(v[s * stride + lane + 32 * i]), x[i]);
-  }
-#pragma unroll
-  for (int i = 0; i < 2; ++i) q[i] *= gla_exp<T>(log_scale * sum[i]);
+      q[i] *= gla_exp<T>(log_scale * sum[i]);
 #pragma unroll 1
-  for (int d = 0; d < dim; ++d) {
-    const float y = __shfl_sync(0xffffffffu, d < 32 ? q[0] : q[1], d & 31);
+      for (int d = 32 * i; d < min(dim, 32 * i + 32); d += 8) {
+        float y[8][2];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-      if (lane + 32 * i < cols) x[i] = fmaf(y, state[(long long)d * vdim + lane + 32 * i], x[i]);
+        for (int u = 0; u < 8; ++u)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) y[u][h] = lane + 32 * h < cols ? state[(long long)(d + u) * vdim + lane + 32 * h] : 0.f;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const float z = __shfl_sync(0xffffffffu, q[i], (d + u) & 31);
+          x[0] = fmaf(z, y[u][0], x[0]);
+          x[1] = fmaf(z, y[u][1], x[1]);
+        }
+      }
+    }
+    if (need[0]) at[0] = x[0];
+    if (need[1]) at[32] = x[1];
   }
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-    if (lane + 32 * i < cols && !isfinite(out[lane + 32 * i])) out[lane + 32 * i] = x[i];
 }
 
 constexpr int GD = 20;      // row length of a sub-block's weights ([token s][token t])
@@ -958,15 +993,12 @@ gla_out_kernel(const T* __restrict__ proj, long long row_stride, int q_off, int 
     if (ta < len) *reinterpret_cast<float2*>(at + ta * out_row_stride) = make_float2(o[j][0], o[j][1]);
     if (tb < len) *reinterpret_cast<float2*>(at + tb * out_row_stride) = make_float2(o[j][2], o[j][3]);
   }
-  unsigned redo = cm_bad_rows(ta < len && zeros[0] != 0.f, tb < len && zeros[1] != 0.f);
+  const unsigned redo = cm_bad_rows(ta < len && zeros[0] != 0.f, tb < len && zeros[1] != 0.f);
   if (redo == 0) return;
   __syncwarp();
-  for (; redo; redo &= redo - 1) {
-    const int t = warp * 16 + __ffs(redo) - 1;
-    gla_plain_row<T>(rows + head * dim, rows + v_off + head * vdim + col0, row_stride, q_off, k_off, q_scale, dt + (row0 * n_heads + head) * dim,
-                     (long long)n_heads * dim, log_scale, src, vdim, t, dim, min(CM_COLS, vdim - col0),
-                     out + (row0 + t) * out_row_stride + (long long)head * vdim + col0);
-  }
+  gla_plain_rows<T>(redo, rows + head * dim, rows + v_off + head * vdim + col0, row_stride, q_off, k_off, q_scale, dt + (row0 * n_heads + head) * dim,
+                    (long long)n_heads * dim, log_scale, src, vdim, warp * 16, dim, min(CM_COLS, vdim - col0),
+                    out + row0 * out_row_stride + (long long)head * vdim + col0, out_row_stride);
 }
 
 // Scratch of the chunked form: [states | ends | aged_q].

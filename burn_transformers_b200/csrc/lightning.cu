@@ -501,6 +501,22 @@ __device__ __forceinline__ float cm_feature(float x, int act) {
   return x * (x < 0.f ? e * r : r);
 }
 
+// The numbers of a chunk's contribution to the state that are not finite, by multiply-adds (a call of its own: inside, it costs the kernel registers).
+template <typename T>
+__device__ __noinline__ void lightning_plain_state(const T* k, const T* v, long long stride, int act, const float* pw, int len, int dim, int cols,
+                                                   float* dst, int vdim) {
+  for (int i = threadIdx.x; i < dim * cols; i += CM_THREADS) {
+    const int d = i / cols, c = i - d * cols;
+    float* at = dst + (long long)d * vdim + c;
+    if (isfinite(*at)) continue;
+    float x = 0.f;
+#pragma unroll 8
+    for (int s = 0; s < len; ++s)
+      x = fmaf(cm_feature(to_float(k[s * stride + d]), act) * pw[len - 1 - s], cm_feature(to_float(v[s * stride + c]), act), x);
+    *at = x;
+  }
+}
+
 template <typename T, int PARTS>
 __global__ void __launch_bounds__(CM_THREADS, 4)
 lightning_state_kernel(const T* __restrict__ proj, long long row_stride, int k_off, int v_off, const int* __restrict__ seq_start,
@@ -537,20 +553,31 @@ lightning_state_kernel(const T* __restrict__ proj, long long row_stride, int k_o
   const bool bad = cm_state<3, PARTS>(k_s, k_stride, k_part, v_s, v_part, dim, [&](int d, int c, float x, float y) {
     if (col0 + c < vdim) *reinterpret_cast<float2*>(dst + (long long)d * vdim + c) = make_float2(x, y);
   });
-  if (!__syncthreads_or(bad)) return;
-  const int cols = min(CM_COLS, vdim - col0);
-  for (int i = threadIdx.x; i < dim * cols; i += CM_THREADS) {
-    const int d = i / cols, c = i - d * cols;
-    float* at = dst + (long long)d * vdim + c;
-    if (isfinite(*at)) continue;
-    float x = 0.f;
-#pragma unroll 1
-    for (int s = 0; s < len; ++s) {
-      const T* row = rows + s * row_stride;
-      x = fmaf(feature(to_float(row[k_off + head * dim + d]), act) * pw[len - 1 - s],
-               feature(to_float(row[v_off + head * vdim + col0 + c]), act), x);
-    }
-    *at = x;
+  if (__syncthreads_or(bad))
+    lightning_plain_state<T>(rows + k_off + head * dim, rows + v_off + head * vdim + col0, row_stride, act, pw, len, dim, min(CM_COLS, vdim - col0), dst, vdim);
+}
+
+// The results of a chunk's tokens (bits of `redo`, from token `first` on) that are no finite numbers, by multiply-adds, a warp together: qk and v
+// are the chunk's rows from the head's channels on, v's and out's the block's; pw: the decay's powers.
+template <typename T>
+__device__ __noinline__ void lightning_plain_rows(unsigned redo, const T* qk, const T* v, long long stride, int q_off, int k_off, int act,
+                                                  const float* state, int vdim, const float* pw, int first, int dim, int cols, float* out,
+                                                  long long out_stride) {
+  const int lane = threadIdx.x & 31;
+  auto in = [&](int d, int c) { return state[(long long)d * vdim + c]; };
+  bool nan[2];
+  cm_nan_columns(dim, cols, in, nan);
+  for (; redo; redo &= redo - 1) {
+    const int t = first + __ffs(redo) - 1;
+    float* at = out + t * out_stride + lane;
+    const bool need[2] = {!nan[0] && !isfinite(at[0]), !nan[1] && !isfinite(at[32])};
+    if (!__any_sync(0xffffffffu, need[0] || need[1])) continue;
+    float x[2];
+    cm_plain_row(t, dim, cols, pw[t + 1], [&](int d) { return cm_feature(to_float(qk[t * stride + q_off + d]), act); },
+                 [&](int s, int d) { return cm_feature(to_float(qk[s * stride + k_off + d]), act); },
+                 [&](int s, int c) { return cm_feature(to_float(v[s * stride + c]), act); }, in, [&](int s, float w) { return w * pw[t - s]; }, x);
+    if (need[0]) at[0] = x[0];
+    if (need[1]) at[32] = x[1];
   }
 }
 
@@ -692,20 +719,8 @@ lightning_out_kernel(const T* __restrict__ proj, long long row_stride, int q_off
   if (redo == 0) return;
   __syncwarp();
   const int cols = min(CM_COLS, vdim - col0);
-  for (; redo; redo &= redo - 1) {
-    const int t = warp * 16 + __ffs(redo) - 1;
-    auto number = [&](int token, int at) { return feature(to_float(rows[token * row_stride + at]), act); };
-    float x[2];
-    cm_plain_row(t, dim, cols, pw[t + 1], [&](int d) { return number(t, q_off + head * dim + d); },
-                 [&](int s, int d) { return number(s, k_off + head * dim + d); },
-                 [&](int s, int c) { return number(s, v_off + head * vdim + col0 + c); },
-                 [&](int d, int c) { return src[(long long)d * vdim + c]; }, [&](int s, float w) { return w * pw[t - s]; }, x);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      float* at = out + (row0 + t) * out_row_stride + (long long)head * vdim + col0 + lane + 32 * i;
-      if (lane + 32 * i < cols && !isfinite(*at)) *at = x[i];
-    }
-  }
+  lightning_plain_rows<T>(redo, rows + head * dim, rows + v_off + head * vdim + col0, row_stride, q_off, k_off, act, src, vdim, pw, warp * 16,
+                          dim, min(CM_COLS, vdim - col0), out + row0 * out_row_stride + (long long)head * vdim + col0, out_row_stride);
 }
 
 template <typename T, int PARTS>

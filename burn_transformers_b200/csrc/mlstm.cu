@@ -644,6 +644,21 @@ __global__ void __launch_bounds__(256) mlstm_carry_kernel(const T* __restrict__ 
   }
 }
 
+// The numbers of a chunk's contribution to S that are not finite, by multiply-adds (a call of its own: inside, it costs the kernel registers).
+template <typename T>
+__device__ __noinline__ void mlstm_plain_state(const T* k, const T* v, long long stride, const float* w_end, int len, int dim, int cols, float* dst,
+                                               int vdim) {
+  for (int i = threadIdx.x; i < dim * cols; i += CM_THREADS) {
+    const int d = i / cols, c = i - d * cols;
+    float* at = dst + (long long)d * vdim + c;
+    if (isfinite(*at)) continue;
+    float x = 0.f;
+#pragma unroll 8
+    for (int t = 0; t < len; ++t) x = fmaf(to_float(k[t * stride + d]) * w_end[t], to_float(v[t * stride + c]), x);
+    *at = x;
+  }
+}
+
 // The chunks on tensor cores (chunk_mma.cuh), for rows on 16-byte boundaries with channels in whole operand tiles: first every
 // chunk's contribution to S and n, then mlstm_prefix_kernel, then all of o at once, which is written once.  bfloat16 q, k and v go
 // in as they are; the weights, the state and n in three parts.  The whole chain (gates, the
@@ -709,21 +724,8 @@ __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_state_kernel(const T* __r
   const bool bad = cm_state<3, PARTS>(k_s, k_stride, k_part, v_s, v_part, dim, [&](int d, int ch, float x, float y) {
     if (col0 + ch < vdim) *reinterpret_cast<float2*>(dst + (long long)d * vdim + ch) = make_float2(x, y);
   });
-  if (__syncthreads_or(bad)) {      // (and the keys have been read)
-    const int cols = min(CM_COLS, vdim - col0);
-    for (int i = threadIdx.x; i < dim * cols; i += CM_THREADS) {
-      const int d = i / cols, ch = i - d * cols;
-      float* at = dst + (long long)d * vdim + ch;
-      if (isfinite(*at)) continue;
-      float x = 0.f;
-#pragma unroll 1
-      for (int t = 0; t < len; ++t) {
-        const T* row = rows + t * p.row_stride;
-        x = fmaf(to_float(row[p.k_off + head * dim + d]) * w_end[t], to_float(row[p.v_off + head * vdim + col0 + ch]), x);
-      }
-      *at = x;
-    }
-  }
+  if (__syncthreads_or(bad))      // (and the keys have been read)
+    mlstm_plain_state<T>(rows + p.k_off + head * dim, rows + p.v_off + head * vdim + col0, p.row_stride, w_end, len, dim, min(CM_COLS, vdim - col0), dst, vdim);
   if (col_block != 0) return;
   float* n_s = reinterpret_cast<float*>(cm_smem);      // [at_once][dim]
   if (k_first < at_once)
@@ -737,26 +739,35 @@ __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_state_kernel(const T* __r
   }
 }
 
-// A token's whole row by multiply-adds (the divisor is every channel's), a warp together: qk and v are the chunk's rows from the head's
-// channels on, v's the block's; f: the incoming state's factor.  (A call of its own: inside, it costs the kernel registers.)
+// A chunk's tokens (bits of `redo`, from token `first` on; of `den` those whose divisor is in doubt) by multiply-adds, a warp together, whole rows
+// (the divisor is every channel's): qk and v are the chunk's rows from the head's channels on, v's and out's the block's; n the incoming
+// normaliser.  (A call of its own: inside, it costs the kernel registers.)
 template <typename T>
-__device__ __noinline__ void mlstm_plain_row(const T* qk, const T* v, long long stride, int q_off, int k_off, float q_scale, const float* state,
-                                             int vdim, const float* n, float f, float floor, float g_c, const float* g_a, int t, int dim,
-                                             int cols, float* out) {
+__device__ __noinline__ void mlstm_plain_rows(unsigned redo, unsigned den, const T* qk, const T* v, long long stride, int q_off, int k_off,
+                                              float q_scale, const float* state, int vdim, const float* n, const float* f_s,
+                                              const float* floor_s, const float* g_c, const float* g_a, int first, int dim, int cols, float* out,
+                                              long long out_stride) {
   const int lane = threadIdx.x & 31;
-  auto query = [&](int d) { return to_float(qk[t * stride + q_off + d]) * q_scale; };
-  float x[2], nq = 0.f;
+  auto in = [&](int d, int c) { return state[(long long)d * vdim + c]; };
+  bool nan[2];
+  cm_nan_columns(dim, cols, in, nan);
+  for (; redo; redo &= redo - 1) {
+    const int t = first + __ffs(redo) - 1;
+    float* at = out + t * out_stride + lane;
+    const bool doubt = (den & redo & (0u - redo)) != 0;
+    if (!__any_sync(0xffffffffu, (!nan[0] && (doubt || !isfinite(at[0]))) || (!nan[1] && (doubt || !isfinite(at[32]))))) continue;
+    auto query = [&](int d) { return to_float(qk[t * stride + q_off + d]) * q_scale; };
+    float x[2], nq = 0.f;
 #pragma unroll 1
-  for (int d = lane; d < dim; d += 32) nq = fmaf(query(d), n[d], nq);
-  nq = warp_sum(nq) * f;
-  const float den = cm_plain_row(t, dim, cols, f, query, [&](int s, int d) { return to_float(qk[s * stride + k_off + d]); },
-                                 [&](int s, int c) { return to_float(v[s * stride + c]); },
-                                 [&](int d, int c) { return state[(long long)d * vdim + c]; },
-                                 [&](int s, float w) { return w * expf(g_c + g_a[s]); }, x);
-  const float by = fmaxf(fabsf(den + nq), floor) + 1e-6f;
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-    if (lane + 32 * i < cols) out[lane + 32 * i] = x[i] / by;
+    for (int d = lane; d < dim; d += 32) nq = fmaf(query(d), n[d], nq);
+    nq = warp_sum(nq) * f_s[t];
+    const float sum = cm_plain_row(t, dim, cols, f_s[t], query, [&](int s, int d) { return to_float(qk[s * stride + k_off + d]); },
+                                   [&](int s, int c) { return to_float(v[s * stride + c]); }, in,
+                                   [&](int s, float w) { return w * expf(g_c[t] + g_a[s]); }, x);
+    const float by = fmaxf(fabsf(sum + nq), floor_s[t]) + 1e-6f;
+    if (!nan[0]) at[0] = x[0] / by;
+    if (!nan[1]) at[32] = x[1] / by;
+  }
 }
 
 template <typename T>
@@ -814,7 +825,8 @@ __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_out_kernel(const T* __res
     for (int q = 0; q < PARTS; ++q) cm_ldmatrix(a[q], q_s + q * k_part + (warp * 16 + (lane & 15)) * k_stride + d + (lane >> 4) * 8);
   };
   float o[8][4], o_small[8][4], div_a, div_b;
-  float zeros[2];      // (zero times a row's numbers and its divisor's sum)
+  bool doubt_a, doubt_b;      // of the divisors
+  float zeros[2];             // (zero times a row's numbers, where the divisor is not in doubt)
   {
     // f_t S_in^T q_t and f_t n_in . q_t
     float nq[4] = {}, nq_small[4] = {};
@@ -895,8 +907,10 @@ __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_out_kernel(const T* __res
     }
     div_a += den_a;
     div_b += den_b;
-    zeros[0] = div_a * 0.f;
-    zeros[1] = div_b * 0.f;
+    doubt_a = !isfinite(div_a);
+    doubt_b = !isfinite(div_b);
+    zeros[0] = doubt_a ? 1.f : 0.f;
+    zeros[1] = doubt_b ? 1.f : 0.f;
     div_a = fmaxf(fabsf(div_a), floor_s[ta]) + 1e-6f;
     div_b = fmaxf(fabsf(div_b), floor_s[tb]) + 1e-6f;
   }
@@ -937,15 +951,12 @@ __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_out_kernel(const T* __res
     if (ta < len) *reinterpret_cast<float2*>(at + ta * p.out_row_stride) = make_float2(o[j][0] / div_a, o[j][1] / div_a);
     if (tb < len) *reinterpret_cast<float2*>(at + tb * p.out_row_stride) = make_float2(o[j][2] / div_b, o[j][3] / div_b);
   }
-  unsigned redo = cm_bad_rows(ta < len && zeros[0] != 0.f, tb < len && zeros[1] != 0.f);
+  const unsigned redo = cm_bad_rows(ta < len && zeros[0] != 0.f, tb < len && zeros[1] != 0.f);
   if (redo == 0) return;
   __syncwarp();
-  for (; redo; redo &= redo - 1) {
-    const int t = warp * 16 + __ffs(redo) - 1;
-    mlstm_plain_row<T>(rows + head * dim, rows + p.v_off + head * vdim + col0, p.row_stride, p.q_off, p.k_off, p.q_scale, src, vdim,
-                       c.dn + cell * dim, f_s[t], floor_s[t], g_c[t], g_a, t, dim, min(CM_COLS, vdim - col0),
-                       p.out + (row0 + t) * p.out_row_stride + (long long)head * vdim + col0);
-  }
+  mlstm_plain_rows<T>(redo, cm_bad_rows(doubt_a, doubt_b), rows + head * dim, rows + p.v_off + head * vdim + col0, p.row_stride, p.q_off, p.k_off,
+                      p.q_scale, src, vdim, c.dn + cell * dim, f_s, floor_s, g_c, g_a, warp * 16, dim, min(CM_COLS, vdim - col0),
+                      p.out + row0 * p.out_row_stride + (long long)head * vdim + col0, p.out_row_stride);
 }
 
 static long long mlstm_scratch_floats(long long n_rows, int n_seqs, int max_new, int n_heads, int dim, int vdim) {
