@@ -765,9 +765,10 @@ static int launch_lightning_chunked(const T* proj, long long row_stride, int q_o
   constexpr int V = 16 / (int)sizeof(T);
   const int vec = dim % V == 0 && vdim % V == 0 && q_off % V == 0 && k_off % V == 0 && v_off % V == 0 && row_stride % V == 0 &&
                   out_row_stride % 4 == 0 && ((unsigned long long)proj | (unsigned long long)out | (unsigned long long)scratch) % 16 == 0;
-  // (below a block a multiprocessor, x * sigmoid(x) by a block's 128 threads takes longer than what the products save: three heads of
-  // 128 x 96 over 700 tokens, 66 blocks, 50 us against 40; 48 blocks 29 against 25; 272 blocks 46 against 50)
-  if (vec && dim % 16 == 0 && dim <= 128 && (act != 0 || (long long)max_chunks * n_heads * col_blocks * n_seqs >= sm_count()) && q_off % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0 && vdim % 8 == 0) {
+  // By the layer's sizes and addresses alone: a sequence's bits must not depend on what else is in the call.  Multiply-adds / parts, us,
+  // bfloat16: heads of 64 x 64 with x sigmoid(x) 36 blocks 27 / 32, 192 40 / 39, 512 68 / 47, without it 23 / 21, 35 / 24, 60 / 30; heads
+  // of 128 x 128 with it 16 blocks 40 / 49, 256 64 / 55, 1,024 205 / 207.  So few blocks with x sigmoid(x) pay for many.
+  if (vec && dim % 16 == 0 && dim <= 128 && vdim % 8 == 0 && q_off % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0) {
     if constexpr (sizeof(T) == 2)
       if (act == 1)
         return launch_lightning_mma<T, 1>(proj, row_stride, q_off, k_off, v_off, state, slots, seq_start, decay, out, out_row_stride,
