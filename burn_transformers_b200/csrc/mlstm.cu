@@ -987,8 +987,10 @@ static int launch_mlstm_chunked(const T* proj, MlstmArgs p, float* scratch, long
   constexpr int V = 16 / (int)sizeof(T);
   c.vec = p.dim % V == 0 && p.vdim % V == 0 && p.q_off % V == 0 && p.k_off % V == 0 && p.v_off % V == 0 && p.row_stride % V == 0 &&
           p.out_row_stride % 4 == 0 && ((unsigned long long)proj | (unsigned long long)p.out | (unsigned long long)c.ds) % 16 == 0;
-  // (with few blocks the chain of a block counts, and 256 threads make it shorter: 60 blocks 30 us against 27; 64 blocks 36 against 46)
-  if (c.vec && p.dim % 16 == 0 && p.dim <= 128 && (long long)c.max_chunks * p.n_heads * c.col_blocks * n_seqs * 7 >= sm_count() * 3 && p.vdim % 8 == 0 && p.q_off % 8 == 0 && p.k_off % 8 == 0 && p.v_off % 8 == 0) {
+  // By the layer's sizes and addresses alone: a sequence's bits must not depend on what else is in the call.  Multiply-adds / parts, us:
+  // bfloat16 heads of 64 x 64 36 blocks 24.5 / 26.6, 84 29.1 / 31.2, 132 45 / 36, 512 80 / 46; 128 x 128 16 blocks 33 / 29, 1,024 193 / 137.
+  // 32-bit rows 64 x 64 36 blocks 25.7 / 24.7, 1,152 143 / 123; 128 x 64 256 blocks 74 / 67, 1,152 252 / 278.
+  if (c.vec && p.dim % 16 == 0 && p.dim <= 128 && p.vdim % 8 == 0 && p.q_off % 8 == 0 && p.k_off % 8 == 0 && p.v_off % 8 == 0) {
     constexpr int PARTS = sizeof(T) == 2 ? 1 : 3;
     const dim3 cells(c.max_chunks, p.n_heads * c.col_blocks, n_seqs);
     const size_t rows_k = (size_t)MC * (p.dim + 8), rows_s = (size_t)(p.dim > MC ? p.dim : MC) * CM_ROW;
