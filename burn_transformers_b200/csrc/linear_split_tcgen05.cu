@@ -497,6 +497,27 @@ extern "C" int bt_linear_split_takes(int N, int K, int w_is_nk) {
   return K % 4 == 0 && (w_is_nk || N % 4 == 0) && N >= 256 && N <= 2048 && K >= 768 && K >= N;
 }
 
+// How many blocks share a tile (1, 2, 4 or 8) on a device of `sms` multiprocessors, by what the tiles take: a k-block 1.35 us, start and end
+// 2.5, the exchange 1.5.  Of 4 blocks 32 clusters are resident together on 148 multiprocessors, of 8 blocks 14; a device with too few for
+// any by that measure does without.  (Any answer gives the same bits.)
+extern "C" int bt_linear_split_blocks(int M, int N, int K, int sms) {
+  using namespace bt;
+  const long long tiles = (long long)((M + LS_BM - 1) / LS_BM) * ((N + LS_BN - 1) / LS_BN), k_blocks = (K + TC_BK - 1) / TC_BK;
+  long long best = -1;
+  int split = 1;
+  for (const int s : {1, 2, 4, 8}) {
+    const long long places = s <= 2 ? sms / s : s == 4 ? sms / 4 - 5 : sms / 8 - 4;
+    if (places < 1) continue;
+    const long long rounds = (tiles + places - 1) / places;
+    const long long cost = 2500 + (s > 1 ? 1500 : 0) + rounds * ((k_blocks + s - 1) / s * 1350 + (s > 1 && rounds > 1 ? 3000 : 0));
+    if (best < 0 || cost < best) {
+      best = cost;
+      split = s;
+    }
+  }
+  return split;
+}
+
 // All operands 32-bit, A and W on 16-byte boundaries with rows of such pieces (K, and N of a [K,N] weight, multiples of 4).
 // split: 0 by the sizes; 1, 2, 4 or 8 blocks a tile.
 extern "C" int bt_linear_split(const float* a, const float* w, const float* bias, const float* residual, float* out, int* status, int M,
@@ -510,18 +531,9 @@ extern "C" int bt_linear_split(const float* a, const float* w, const float* bias
   const int rows16 = N % 4 == 0 && ((unsigned long long)out | (unsigned long long)residual | (unsigned long long)bias) % 16 == 0;
   const SplitParams p{a, w, bias, residual, out, status, M, N, K, act, rows16};
   if (split == 0) {
-    const long long tiles = (long long)((M + LS_BM - 1) / LS_BM) * ((N + LS_BN - 1) / LS_BN), k_blocks = (K + TC_BK - 1) / TC_BK;
     const int sms = sm_count();
-    long long best = -1;
-    // (a k-block 1.35 us, start and end 2.5, the exchange 1.5; of 4 blocks 32 clusters are resident together, of 8 blocks 14)
-    for (const int s : {1, 2, 4, 8}) {
-      const long long places = s <= 2 ? sms / s : s == 4 ? sms / 4 - 5 : sms / 8 - 4, rounds = (tiles + places - 1) / places;
-      const long long cost = 2500 + (s > 1 ? 1500 : 0) + rounds * ((k_blocks + s - 1) / s * 1350 + (s > 1 && rounds > 1 ? 3000 : 0));
-      if (best < 0 || cost < best) {
-        best = cost;
-        split = s;
-      }
-    }
+    BT_CHECK(sms > 0, "linear_split: cannot read the number of multiprocessors of the current device");
+    split = bt_linear_split_blocks(M, N, K, sms);
   }
   if (split == 8) return w_is_nk ? launch_split<true, 8>(p, stream) : launch_split<false, 8>(p, stream);
   if (split == 2) return w_is_nk ? launch_split<true, 2>(p, stream) : launch_split<false, 2>(p, stream);
