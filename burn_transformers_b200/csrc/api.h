@@ -22,8 +22,8 @@ int bt_layernorm(const float* x, const int* rows, const float* gamma, const floa
 int bt_linear_simt(const void* A, const void* W, const float* bias, const float* residual, void* out, int M, int N,
                    int K, int w_is_nk, int act, int in_dtype, int out_dtype, cudaStream_t stream);
 
-// The same for 32-bit operands on tcgen05 in exact bfloat16 parts, where bt_linear_split_takes says so.
-int bt_linear_split_takes(int N, int K, int w_is_nk);
+// The same for 32-bit operands on tcgen05 in exact bfloat16 parts, where bt_linear_split_supports says so.
+int bt_linear_split_supports(int N, int K, int w_is_nk);
 int bt_linear_split_blocks(int M, int N, int K, int sms);
 int bt_linear_split(const float* a, const float* w, const float* bias, const float* residual, float* out, int* status, int M, int N, int K,
                     int w_is_nk, int act, int split, cudaStream_t stream);

@@ -493,7 +493,7 @@ static int launch_split(const SplitParams& p, cudaStream_t stream) {
 // rows: 768 x 768 8.3 / 12.0 / 33.8 and 7.3 / 10.2 / 25.5; 768 x 3072 28 / 41 / 126 and 12 / 22 / 68; 1024 x 4096 36 / 48 / 180 and 23 / 28 /
 // 105; 1600 x 6400 56 / 118 / 448 and 33 / 76 / 269; 256 x 768 8.3 / 8.7 / 14.5 and 6.4 / 7.5 / 10.6.  Not 512 x 512 (6.1 / 6.5 / 16 and
 // 6.5 / 8.4 / 13), nor wide ones: 2304 x 768 8.2 / 21 / 80 and 13 / 16 / 48, and behind by more where the weights come from memory.
-extern "C" int bt_linear_split_takes(int N, int K, int w_is_nk) {
+extern "C" int bt_linear_split_supports(int N, int K, int w_is_nk) {
   return K % 4 == 0 && (w_is_nk || N % 4 == 0) && N >= 256 && N <= 2048 && K >= 768 && K >= N;
 }
 

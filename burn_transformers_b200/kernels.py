@@ -243,7 +243,7 @@ def linear_simt(a, w, bias, out, *, m=None, w_is_nk=False, activation=None, resi
     if activation not in ACTIVATIONS:
         raise ShapeError(f"linear: unknown activation {activation!r}")
     _linear_work(m, n, k, a, w, out)
-    if (a.dtype == torch.float32 and _supports("bt_linear_split_takes", n, k, 1 if w_is_nk else 0)
+    if (a.dtype == torch.float32 and _supports("bt_linear_split_supports", n, k, 1 if w_is_nk else 0)
             and (a.data_ptr() | w.data_ptr()) % 16 == 0):
         # tcgen05 with the operands in three bfloat16 parts, which hold all of their bits (csrc/linear_split_tcgen05.cu)
         _check(library().bt_linear_split(_ptr(a), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out), _ptr(kernel_status(a.device)),

@@ -61,3 +61,11 @@ def test_what_is_not_finite(split):
     assert float((out[70] - want[70]).abs().max()) < 1e-38
     rest = [r for r in range(200) if r not in (3, 50, 60, 61, 70)]
     assert rel(out[rest], a[rest].double() @ w.double()) < 2e-7
+
+
+def test_a_profile_shows_the_product_alone():
+    a, w, out = torch.randn(5, 1076, device=DEV), torch.randn(1076, 1052, device=DEV), torch.empty(5, 1052, device=DEV)
+    with kernels.KernelProfile() as profile:      # (a size that no other test has asked for: the first question is asked here)
+        kernels.linear_simt(a, w, None, out)
+    (row,) = profile.summary()
+    assert row["kernel"] == "linear_split" and row["flops"] == 2.0 * 5 * 1052 * 1076
