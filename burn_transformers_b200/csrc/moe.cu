@@ -794,7 +794,6 @@ extern "C" int bt_moe_sort(const int* ids, int total, int E, int* offsets, int* 
   // pairs of 64 experts 5.0 to 1.7, 16,384 39 to 11, 65,536 145 to 44.  Sixteen pairs a thread for the few: 2.9.)
   if (total > 1024) return launch(moe_sort_kernel<16>);
   return launch(moe_sort_kernel<1>);
-  return 0;
 }
 
 // first: 1 = the experts' first product (a: the tokens' rows [tokens, K]; w: [E][2N][K]; out: [pairs, N] of the
