@@ -21,6 +21,7 @@ def paired(g, u, rule, limit):
 @pytest.mark.parametrize("m", [1, 65, 127, 128, 129, 256, 257, 1030, 5000])
 @pytest.mark.parametrize("inner, k", [(8, 8), (30, 64), (32, 72), (100, 200), (160, 1024), (2816, 136)])
 def test_gated_product(m, inner, k):
+    torch.manual_seed(m + inner)
     a = torch.randn(m, k, device=DEV).bfloat16()
     w = (torch.randn(2 * inner, k, device=DEV) * 2.0 * k ** -0.5).bfloat16()
     both = a.double() @ w.double().T
@@ -28,8 +29,9 @@ def test_gated_product(m, inner, k):
         out = torch.full((m + 2, inner), 3.0, device=DEV).bfloat16()
         kernels.gated_tcgen05(a, w, out, m=m, activation=rule, limit=limit)
         want = paired(both[:, :inner], both[:, inner:], rule, limit)
-        # one rounding to bfloat16 of each result: 2^-9 of its size at most, 2^-10 as a mean; the sums' errors are far below
-        assert float((out[:m].double() - want).norm() / want.norm()) < 2.0 ** -8.5
+        # one rounding to bfloat16 of each result: half a unit of 2^-7, so 2^-8 of its size at most, and less than 2^-9 in the norm of many;
+        # the sums' errors are far below
+        assert float((out[:m].double() - want).norm() / want.norm()) < (2.0 ** -8.5 if m * inner > 1000 else 2.0 ** -8)
         assert float(((out[:m].double() - want).abs() - 2.0 ** -8 * want.abs()).max()) < 1e-4
         assert bool((out[m:] == 3.0).all())
     kernels.check_status(a.device)

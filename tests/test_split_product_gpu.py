@@ -30,7 +30,14 @@ def test_product_in_parts(m, n, k, nk):
         assert rel(out[:m], product) < 2e-7 and bool((out[m:] == 7.0).all())
         seen.append(out)
     assert all(torch.equal(seen[0], other) for other in seen[1:])
-    kernels.linear_simt(a, w_arg, bias, res, w_is_nk=nk, activation="gelu_new", residual=res.clone())
+    want, seen_res = torch.nn.functional.gelu(product + bias.double(), approximate="tanh") + res.double(), []
+    for split in (0, 1, 2, 4, 8):
+        out = torch.full((m + 2, n), 7.0, device=DEV)
+        out[:m] = res
+        kernels.linear_simt(a, w_arg, bias, out, m=m, w_is_nk=nk, activation="gelu_new", residual=out, split=split)      # in place
+        assert rel(out[:m], want) < 5e-7 and bool((out[m:] == 7.0).all())
+        seen_res.append(out)
+    assert all(torch.equal(seen_res[0], other) for other in seen_res[1:])
     alone = torch.empty(1, n, device=DEV)
     kernels.linear_simt(a[m - 1:].contiguous(), w_arg, None, alone, w_is_nk=nk)
     assert torch.equal(alone[0], seen[0][m - 1])
