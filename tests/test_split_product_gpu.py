@@ -76,3 +76,12 @@ def test_a_profile_shows_the_product_alone():
         kernels.linear_simt(a, w, None, out)
     (row,) = profile.summary()
     assert row["kernel"] == "linear_split" and row["flops"] == 2.0 * 5 * 1052 * 1076
+
+
+@pytest.mark.parametrize("split", [0, 1, 8])
+def test_rows_of_no_whole_pieces(split):
+    torch.manual_seed(3)
+    a, w = torch.randn(130, 772, device=DEV), torch.randn(257, 772, device=DEV) * 772 ** -0.5      # ([N,K]: N is free)
+    bias, out = torch.randn(257, device=DEV), torch.full((132, 257), 7.0, device=DEV)
+    kernels.linear_simt(a, w, bias, out, m=130, w_is_nk=True, split=split)
+    assert rel(out[:130], a.double() @ w.double().T + bias.double()) < 2e-7 and bool((out[130:] == 7.0).all())
