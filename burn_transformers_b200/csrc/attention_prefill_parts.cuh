@@ -58,7 +58,7 @@ __device__ __noinline__ void ap_plain(const float* __restrict__ q, KvView kv, fl
                                       int n_kv_heads, float scale, int first, int last, int part) {
   const int lane = threadIdx.x & 31;
   float m = -INFINITY, l = 0.f, acc[2] = {0.f, 0.f};
-  for (int j = first; j <= last; ++j) {
+  for (int j = first; j <= last && !isnan(l); ++j) {      // (once the sum of the weights is NaN the rest changes nothing)
     const long long at = (long long)(t0 + j) * kv.row_stride + kv_head * HD;
     const float* k = kv.table ? kv_row<float>(kv.k, kv, seq, kv_head, n_kv_heads, HD, j) : reinterpret_cast<const float*>(kv.k) + at;
     const float* v = kv.table ? kv_row<float>(kv.v, kv, seq, kv_head, n_kv_heads, HD, j) : reinterpret_cast<const float*>(kv.v) + at;
