@@ -400,7 +400,7 @@ latent_decode_finish_mma_kernel(const float* __restrict__ part, const __nv_bfloa
       const float* src = part + ((long long)token * n_heads + h) * n_splits * (rank + 2);
       acc = 0.f;
 #pragma unroll 1
-      for (int k = 0; k < rank; ++k) {
+      for (int k = 0; k < rank && !isnan(acc); ++k) {
         float x = 0.f;
 #pragma unroll 1
         for (int s = 0; s < n_splits; ++s) x = fmaf(src[(long long)s * (rank + 2) + k], share[r][s], x);
