@@ -6,8 +6,8 @@
 // A block is 16, 32 or 64 queries of one (sequence, head) and walks their keys in tiles of 64; two or four warps share 16 queries: each
 // forms the scores of a part of a tile's keys, reads all of them back, forms the same softmax and mixes a part of the channels.  The
 // parts of the queries, of a tile's keys and of its values lie in shared memory; the next tile waits in registers as 32-bit numbers.  The
-// multiply-add kernel is bound by its reads of shared memory, this one by its instructions and the chains of a tile (half of all issue
-// slots and 42 % of the tensor pipe at 64 queries).  A sequence with eight new tokens or fewer is formed by multiply-adds here too: of a
+// multiply-add kernel is bound by its reads of shared memory, this one by its instructions and the chains of a tile (45 % of all issue
+// slots and 41 % of the tensor pipe at 64 queries).  A sequence with eight new tokens or fewer is formed by multiply-adds here too: of a
 // tile's 16 rows most would be empty, and splitting the keys and values costs what it does for 16 (64 sequences with one token
 // behind 900: 153 us in parts, 123 by multiply-adds).  Multiply-adds / parts, us, 12 heads of 64: prompts of 37, 268 and 499 tokens 76 / 36,
 // one of 129 11.4 / 10.0, one of 1,024 116 / 69, 24 tokens behind 300 for each of 32 sequences 67 / 51; 16 heads, 4 x 1,000 428 / 214; three of

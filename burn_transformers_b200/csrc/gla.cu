@@ -536,8 +536,8 @@ gla_carry_kernel(const float* __restrict__ aged_q, const int* __restrict__ seq_s
 // The weights are products of factors of at most one as above, with sub-blocks of 16 tokens between the chunk and the groups of four:
 // q_t e^{b_t - B} k_s e^{B - b_s}, B at the end of s's sub-block, is a product of matrices for every later sub-block; inside a
 // sub-block the groups' weights are multiply-adds.  The kernels above are bound by shared memory; these by forming factors and parts.
-// Before / now, us, all three kernels: 2 x 1,024 tokens of 16 heads of 64 x 64 70 / 40, 6 x 1,000 of 12 heads 135 / 77, one prompt of 129 tokens
-// 39 / 31; 32-bit rows 2 x 1,024 68 / 45; errors against 64 bits 1.6e-7 / 1.4e-7.  Heads of 128 channels leave two blocks a multiprocessor
+// The kernels above / here, us, all three: 2 x 1,024 tokens of 16 heads of 64 x 64 73 / 44, one prompt of 700 of 12 heads 49 / 31; 32-bit rows
+// 72 / 49 and 48 / 31; errors against 64 bits 1.6e-7 / 1.4e-7.  Heads of 128 channels leave two blocks a multiprocessor
 // and took 121 where the kernels above take 104, 32-bit heads of 16 15.4 against 13.7.
 
 // The numbers of a chunk's contribution to the state that are not finite, by multiply-adds (a call of its own: inside, it costs the kernel registers).
@@ -1001,7 +1001,8 @@ gla_out_kernel(const T* __restrict__ proj, long long row_stride, int q_off, int 
                     out + row0 * out_row_stride + (long long)head * vdim + col0, out_row_stride);
 }
 
-// Scratch of the chunked form: [states | ends | aged_q].
+// Scratch of the chunked form: [states | ends | aged_q].  (The kernels in parts leave aged_q as it is; which kernels take a call is known
+// with its addresses only.)
 static inline long long gla_state_floats(int n_seqs, int max_new, int n_heads, int dim, int vdim) {
   return (long long)n_seqs * ((max_new + GC - 1) / GC) * n_heads * dim * vdim;
 }
@@ -1061,8 +1062,8 @@ static int launch_gla_chunked(const T* proj, long long row_stride, int q_off, in
   constexpr int V = 16 / (int)sizeof(T);
   const int vec = dim % 4 == 0 && vdim % V == 0 && v_off % V == 0 && row_stride % V == 0 && out_row_stride % 4 == 0 &&
                   ((unsigned long long)proj | (unsigned long long)out | (unsigned long long)states | (unsigned long long)aged_q) % 16 == 0;
-  if (vec && dim % 16 == 0 && dim >= (sizeof(T) == 4 ? 32 : 16) && dim <= 64 && vdim % 8 == 0 && v_off % 8 == 0 && q_off % 2 == 0 && k_off % 2 == 0 && row_stride % 8 == 0 &&
-      (unsigned long long)dt % 8 == 0 && (unsigned long long)ends % 8 == 0)
+  if (vec && dim % 16 == 0 && dim >= (sizeof(T) == 4 ? 32 : 16) && dim <= 64 && vdim % 8 == 0 && v_off % 8 == 0 && q_off % 2 == 0 &&
+      k_off % 2 == 0 && row_stride % 8 == 0 && (unsigned long long)dt % 8 == 0 && (unsigned long long)ends % 8 == 0)
     return launch_gla_mma<T, sizeof(T) == 2 ? 1 : 3>(proj, row_stride, q_off, k_off, v_off, q_scale, dt, log_scale, state, slots, seq_start,
                                                      out, out_row_stride, states, ends, max_chunks, n_seqs, n_heads, dim, vdim, col_blocks,
                                                      stream);

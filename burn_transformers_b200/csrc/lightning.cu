@@ -488,8 +488,8 @@ lightning_carry_kernel(const T* __restrict__ proj, long long row_stride, int q_o
 // (lightning_out_kernel), which is written once.  PARTS: 1 where q, k and v are bfloat16 numbers as they are, else 3.
 // The kernels above are bound by shared memory (an operand read for every other multiply-add) and write o, read it and write it
 // again; these by the forming of the features and the parts, and by the products.  All three kernels, above and here, in us: 2 x 1,024
-// tokens of 16 heads of 64 x 64 with act 0 65 and 49, 6 x 1,000 of 12 heads 112 and 88, with act 1 101 and 58, 32-bit rows 2 x 1,024
-// 69 and 39.  Errors against 64 bits 1.2e-7 and 7e-8 (act 0), 1.8e-7 and 9e-8 (act 1).
+// tokens of 16 heads of 64 x 64 with act 0 68 and 47, 6 x 1,000 of 12 heads 115 and 92, with act 1 60 and 30, 105 and 60; 32-bit rows 2 x 1,024
+// 71 and 46, with act 1 66 and 37.  Errors against 64 bits 1.2e-7 and 7e-8 (act 0), 1.8e-7 and 9e-8 (act 1).
 // x * sigmoid(x) for these kernels: the library's division is half of its instructions; here a reciprocal and one Newton step, of a number
 // between one and two: e^-|x| neither overflows nor makes the reciprocal a number that is not normal.
 __device__ __forceinline__ float cm_feature(float x, int act) {

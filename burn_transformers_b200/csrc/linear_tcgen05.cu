@@ -81,7 +81,7 @@ __device__ __forceinline__ void tc_store32(unsigned char* patch, int stride, con
 // GATED: half of a tile's BN rows of W are the gate's and half up's, of the same BN / 2 columns of the result (each block of a
 // pair loads one of the halves), so that the epilogue has both numbers of a result and writes rule(gate) * up: the rows of 2 N
 // numbers between the product and an activation kernel, written and read again, are gone.  2,048 rows of 5,632 x 1,024
-// and the activation in a recorded layer: 20 and 12 us as two kernels, 24 as one.
+// and the activation in a recorded layer: 20 and 12 us as two kernels, 25 as one.
 template <int BN, int STAGES, bool PAIR, bool GATED>
 __global__ void __launch_bounds__(TC_THREADS)
 linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, TcParams p) {

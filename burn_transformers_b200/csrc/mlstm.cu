@@ -662,8 +662,8 @@ __device__ __noinline__ void mlstm_plain_state(const T* k, const T* v, long long
 // The chunks on tensor cores (chunk_mma.cuh), for rows on 16-byte boundaries with channels in whole operand tiles: first every
 // chunk's contribution to S and n, then mlstm_prefix_kernel, then all of o at once, which is written once.  bfloat16 q, k and v go
 // in as they are; the weights, the state and n in three parts.  The whole chain (gates, the
-// three kernels) at 2 x 1,024 tokens of 16 heads of 64 x 64 takes 81 us with the kernels above and 49 so, 32-bit rows 86 and 62,
-// 6 x 1,000 of 12 heads 122 and 76, one run of 400 44 and 32; errors against 64 bits are those of the kernels above.
+// three kernels) at 2 x 1,024 tokens of 16 heads of 64 x 64 takes 80 us with the kernels above and 46 so, 32-bit rows 85 and 62,
+// 6 x 1,000 of 12 heads 123 and 76, one run of 700 45 and 36, of 400 29 and 31.  n is summed by multiply-adds (see there).
 template <typename T>
 __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_state_kernel(const T* __restrict__ proj, MlstmChunked c) {
   constexpr int PARTS = sizeof(T) == 2 ? 1 : 3;
@@ -959,6 +959,7 @@ __global__ void __launch_bounds__(CM_THREADS, 4) mlstm_out_kernel(const T* __res
                       p.out + row0 * p.out_row_stride + (long long)head * vdim + col0, p.out_row_stride);
 }
 
+// (den is asked for and not used by the kernels in parts; which kernels take a call is known with its addresses only.)
 static long long mlstm_scratch_floats(long long n_rows, int n_seqs, int max_new, int n_heads, int dim, int vdim) {
   const long long chunks = (max_new + MC - 1) / MC;
   const long long cells = (long long)n_seqs * chunks * n_heads;

@@ -362,7 +362,7 @@ selective_scan_kernel(const T* __restrict__ x, long long x_row_stride, const T* 
 // The pieces of long runs for up to 16 state indices: a channel belongs to one thread, or two neighbours above 8 indices, with 8
 // indices each, whose numbers go two an instruction; a token's B and C are read once a warp, and four tokens are worked on at once
 // without a branch between them.  What bounds it: the special-function unit's exponentials, one an index and token, take 14 us a
-// launch at 2,439 tokens of 1,536 channels x 16 indices, the instructions about 11 (the first launch) and 20; the rest is the
+// launch at 2,439 tokens of 1,536 channels x 16 indices (its pipe is busy 50 and 32 % of the two launches), the instructions about 11 (the first launch) and 20; the rest is the
 // latency of a warp's chain.  Both launches there, in us, with selective_scan_kernel and so: 90 and 70; 2 x 1,024 tokens of 1,024
 // channels 63 and 51; one run of 300 32 and 31; 8 indices 114 and 51; 32-bit rows 121 and 98.  (A thread for all 16 indices: 84,
 // too few warps to hide an exponential behind.  72 registers a thread, so that 2,439 tokens are one wave of blocks: 68, but 2 x 70
